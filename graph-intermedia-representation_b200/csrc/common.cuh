@@ -231,7 +231,9 @@ void release(gir_dev* g, DevBuf& b);
 void release_scratch(gir_dev* g, size_t min_bytes);
 constexpr size_t kKeepScratchBelow = 64u << 20;
 
-// Pinned host scratch of at least `bytes`.
+// Pinned host scratch of at least `bytes` (kPinnedBytes are there from create on, so pointers to it
+// stay valid across calls that ask for no more).
+constexpr size_t kPinnedBytes = 4096;
 int pinned(gir_dev* g, size_t bytes, void** out);
 
 bool is_device_ptr(const void* p);
@@ -451,30 +453,25 @@ __device__ __forceinline__ void warp_append(bool pred, int32_t value, int32_t* q
     if (pred) q[base + __popc(m & ((1u << lane_id()) - 1))] = value;
 }
 
-// Grid-wide barrier of a cooperative launch: every CTA meets here. `bar` holds the arrival count
-// at bar[0] and the generation at bar[32] (own 128-byte lines), zeroed by the host before the
-// launch. The wait is bounded: after `spins` polls a CTA sets *err and leaves; every CTA also
+// Grid-wide barrier of a cooperative launch: every CTA meets here. `bar` is one counter on its own
+// 128-byte line, zeroed by the host before the launch; arrivals only count up, so a CTA waits until
+// the counter reaches the end of its own round (one atomic and the polls, no reset and no second
+// word). The wait is bounded: after `spins_max` polls a CTA sets *err and leaves; every CTA also
 // leaves once it sees *err set. Returns false once any CTA has flagged an error.
 __device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned long long* err, unsigned spins_max) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        volatile unsigned int* gen = bar + 32;
-        const unsigned int g0 = *gen;
         __threadfence();
-        if (atomicAdd(bar, 1u) == gridDim.x - 1) {
-            atomicExch(bar, 0u);
-            __threadfence();
-            atomicAdd(bar + 32, 1u);
-        } else {
-            unsigned int spins = 0;
-            while (*gen == g0) {
-                if (++spins > spins_max) {
-                    atomicExch(err, 1ull);
-                    break;
-                }
-                if ((spins & 63) == 0 && __ldcg(err) != 0ull) break;
-                __nanosleep(64);
+        const unsigned int mine = atomicAdd(bar, 1u);
+        const unsigned int end = mine - mine % gridDim.x + gridDim.x;
+        volatile unsigned int* now = bar;
+        unsigned int spins = 0;
+        while ((int)(*now - end) < 0) {
+            if (++spins > spins_max) {
+                atomicExch(err, 1ull);
+                break;
             }
+            if ((spins & 63) == 0 && __ldcg(err) != 0ull) break;
         }
         __threadfence();
     }

@@ -52,20 +52,46 @@ __host__ __device__ inline void bfs_features(double V, double E, double nf, doub
     out[7] = 0.f;  // task: BFS direction
 }
 
-// The direction of the next level: the fixed switch (alpha / beta, gir_query.cpp:159-169), or the
-// network when `params` is given and its margin is large enough. x receives the features.
+// The fixed direction switch (alpha / beta, gir_query.cpp:159-169).
+__device__ __forceinline__ int fixed_direction(double V, double nf, double mf, double mu, int bottom_up, double alpha,
+                                               double beta) {
+    if (!bottom_up && mf * alpha > mu) return 1;
+    if (bottom_up && nf * beta < V) return 0;
+    return bottom_up;
+}
+
+// The direction of the next level: the fixed switch, or the network when `params` is given and its
+// margin is large enough. x receives the features.
 __device__ __forceinline__ int decide_direction(const float* params, double V, double E, double nf, double mf,
                                                 double mu, int bottom_up, int lanes, double alpha, double beta,
                                                 float* x) {
-    int fixed = bottom_up;
-    if (!bottom_up && mf * alpha > mu) fixed = 1;
-    else if (bottom_up && nf * beta < V) fixed = 0;
+    const int fixed = fixed_direction(V, nf, mf, mu, bottom_up, alpha, beta);
     bfs_features(V, E, nf, mf, mu, bottom_up != 0, lanes, x);
     if (!params) return fixed;
     float h[HID], o[OUT];
     forward_one(layout(params), x, h, o);
     const int net = o[1] > o[0] ? 1 : 0;
     return fabsf(o[1] - o[0]) >= kDirMargin ? net : fixed;
+}
+
+// The same decision by one warp (all lanes call it and get the result): lane j computes hidden unit
+// j, lanes 0 and 1 the two direction logits, each sum in forward_one's order.
+__device__ __forceinline__ int decide_direction_warp(const float* params, double V, double E, double nf, double mf,
+                                                     double mu, int bottom_up, int lanes, double alpha, double beta) {
+    static_assert(HID == 32, "one hidden unit per lane");
+    const int j = threadIdx.x & 31;
+    const Layout l = layout(params);
+    float x[IN];
+    bfs_features(V, E, nf, mf, mu, bottom_up != 0, lanes, x);
+    float z = l.b1[j];
+    for (int i = 0; i < IN; ++i) z += l.W1[j * IN + i] * x[i];
+    const float h = tanhf(z);
+    const int k = j & 1;
+    float o = l.b2[k];
+    for (int i = 0; i < HID; ++i) o += l.W2[k * HID + i] * __shfl_sync(0xffffffffu, h, i);
+    const float o0 = __shfl_sync(0xffffffffu, o, 0), o1 = __shfl_sync(0xffffffffu, o, 1);
+    if (fabsf(o1 - o0) >= kDirMargin) return o1 > o0 ? 1 : 0;
+    return fixed_direction(V, nf, mf, mu, bottom_up, alpha, beta);
 }
 
 }  // namespace sched_net

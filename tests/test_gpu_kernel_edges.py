@@ -1,0 +1,78 @@
+"""Sizes at which the query and layer kernels change path (edges of tiles, of launches, of the rules
+that pick a variant), each against the oracle. Integer work: bit-exact."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _graph(pkg, V, u, v):
+    key = np.unique(np.asarray(u, np.int64) * V + np.asarray(v, np.int64))
+    return pkg.graphs.from_edges(V, key // V, key % V)
+
+
+def _brooms(pkg, V, hub):
+    """Hubs with rows of `hub` entries (longer than one warp's run of edge positions), hanging on a
+    directed ring through every vertex (as many levels as vertices), and a few random edges."""
+    rng = np.random.default_rng(V + hub)
+    ring = np.arange(V, dtype=np.int64)
+    u, v = [ring, np.zeros(hub, np.int64), np.full(hub, V // 2)], [(ring + 1) % V, 1 + ring[:hub] % (V - 1), ring[-hub:]]
+    u.append(rng.integers(0, V, V // 50))
+    v.append(rng.integers(0, V, V // 50))
+    u, v = np.concatenate(u), np.concatenate(v)
+    return _graph(pkg, V, u[u != v], v[u != v])
+
+
+@pytest.mark.parametrize("V,hub,alpha", [(33, 3, 15), (4095, 700, 15), (4096, 513, 15), (4097, 512, 1e-6), (9000, 8999, 15),
+                                         (9000, 4000, 1e9)])
+def test_bfs_levels_across_launch_rules(pkg, orc, V, hub, alpha):
+    """The device-resident level loop: below and above 4,096 vertices (where directions are chosen),
+    thousands of levels (more decisions than are read with the counters), hub rows longer than a run,
+    both directions forced, 1 to 65 lanes with repeated and out-of-range sources."""
+    g = _brooms(pkg, V, hub)
+    fb, fa = orc.normalize(g.V, g.fw_beg, g.fw_adj)
+    deg = np.diff(fb)
+    d = pkg.DeviceGraph.from_graph(g, weights=False)
+    d.set_param(pkg.native.PARAM_ALPHA, alpha)
+    if alpha > 1e6:
+        d.set_param(pkg.native.PARAM_BETA, 1e9)
+    rng = np.random.default_rng(1)
+    for lanes in (1, 2, 33, 65):
+        src = rng.integers(0, V, lanes).astype(np.int32)
+        src[-1] = src[0]
+        if lanes > 2:
+            src[1] = -1
+            src[2] = V
+        exp = np.stack([orc.bfs(g.V, fb, fa, [int(s)]) for s in src])
+        np.testing.assert_array_equal(d.bfs(src), exp)
+        st = d.query_stats()
+        assert st["reached"] == (exp >= 0).sum() and st["edges"] == ((exp >= 0) * deg).sum()
+        if V >= 4096 and lanes < 65:
+            assert len(d.sched_trace()[1]) >= st["iterations"]
+    sets = [rng.integers(0, V, n).astype(np.int32) for n in (1, 5, 0, 40)]
+    got = d.bfs_sets(sets)
+    for row, s in zip(got, sets):
+        np.testing.assert_array_equal(row, orc.bfs(g.V, fb, fa, [int(x) for x in s]) if len(s) else np.full(V, -1))
+    d.close()
+
+
+def test_bfs_of_a_graph_whose_bottom_up_levels_leave_the_launch(pkg, orc):
+    """More than 2^20 vertices: bottom-up levels, and frontiers of over 2^22 out-edges, run as their own
+    launches between two device-resident stretches."""
+    V = (1 << 20) + 77
+    rng = np.random.default_rng(5)
+    tail = np.arange(V - 300, V - 1)
+    u = np.concatenate([rng.integers(0, V - 300, 6 * V), tail, [0]])
+    v = np.concatenate([rng.integers(0, V - 300, 6 * V), tail + 1, [V - 300]])
+    g = _graph(pkg, V, u[u != v], v[u != v])
+    fb, fa = orc.normalize(g.V, g.fw_beg, g.fw_adj)
+    d = pkg.DeviceGraph.from_graph(g, weights=False)
+    src = np.array([0, V - 300, 17, V - 1], np.int32)
+    exp = np.stack([orc.bfs(g.V, fb, fa, [int(s)]) for s in src])
+    for alpha in (15, 1e-6):
+        d.set_param(pkg.native.PARAM_ALPHA, alpha)
+        np.testing.assert_array_equal(d.bfs(src), exp)
+        st = d.query_stats()
+        assert 0 < st["persistent_levels"] < st["iterations"]
+        assert (st["bottom_up"] > 0) == (alpha > 1)
+    d.close()
