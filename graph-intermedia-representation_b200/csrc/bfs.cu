@@ -17,6 +17,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "frontier.cuh"
 #include "sched_net.cuh"
 
 namespace gir {
@@ -33,18 +34,6 @@ constexpr int kBlock = 256;
 // [4] the device-decided direction of the next level and [5..8] its features (learned schedule)
 enum { C_Q = 0, C_PAIRS = 1, C_MEDGES = 2, C_DIR = 4, C_FEAT = 5, C_N = 9 };
 
-// A frontier queue is two arrays: the vertices and, for each, the number of out-edges of the
-// entries before it. Appends reserve both at once by one atomicAdd of (entries << 33 | edges), so
-// the offsets ascend with the slots and the next level can cut the frontier's out-edges into equal
-// runs without a scan pass (an edge count is below 2^32, an entry count below 2^31).
-constexpr int kQShift = 33;
-constexpr unsigned long long kQEdges = (1ull << kQShift) - 1;
-
-struct Queue {
-    int32_t* v;
-    uint32_t* off;
-};
-
 __device__ __forceinline__ void write_levels(int32_t* level, int64_t V, int32_t v, uint64_t nb, int32_t L) {
     while (nb) {
         const int s = __ffsll((long long)nb) - 1;
@@ -58,62 +47,11 @@ __device__ __forceinline__ void warp_add_u64(unsigned long long* p, unsigned lon
     if (lane_id() == 0 && x) atomicAdd(p, x);
 }
 
-__device__ __forceinline__ uint32_t warp_incl_u32(uint32_t x) {
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane_id() >= o) x += t;
-    }
-    return x;
-}
-
-// Writes a warp's s_n staged vertices to the queue from slot `slot` and edge offset `e0` on.
-__device__ __forceinline__ void queue_write(const int32_t* s_buf, int s_n, const Queue& q, const int32_t* deg,
-                                            unsigned long long slot, uint32_t e0) {
-    for (int b = 0; b < s_n; b += 32) {
-        const int i = b + lane_id();
-        const int32_t v = i < s_n ? s_buf[i] : 0;
-        const uint32_t d = i < s_n ? (uint32_t)deg[v] : 0u;
-        const uint32_t incl = warp_incl_u32(d);
-        if (i < s_n) {
-            q.v[slot + i] = v;
-            q.off[slot + i] = e0 + incl - d;
-        }
-        e0 += __shfl_sync(0xffffffffu, incl, 31);
-    }
-}
-
-// Out-edges of a warp's staged vertices (warp-uniform result).
-__device__ __forceinline__ uint32_t staged_edges(const int32_t* s_buf, int s_n, const int32_t* deg) {
-    uint32_t e = 0;
-    for (int i = lane_id(); i < s_n; i += 32) {
-        e += (uint32_t)deg[s_buf[i]];
-    }
-    return __reduce_add_sync(0xffffffffu, e);
-}
-
-__device__ __forceinline__ void queue_flush(int32_t* s_buf, int& s_n, const Queue& q, const int32_t* deg,
-                                            unsigned long long* cnt) {
-    if (s_n == 0) return;
-    const uint32_t e = staged_edges(s_buf, s_n, deg);
-    unsigned long long at = 0;
-    if (lane_id() == 0) at = atomicAdd(cnt, ((unsigned long long)s_n << kQShift) | e);
-    at = __shfl_sync(0xffffffffu, at, 0);
-    queue_write(s_buf, s_n, q, deg, at >> kQShift, (uint32_t)(at & kQEdges));
-    __syncwarp();
-    s_n = 0;
-}
-
-// Staged append (warp-uniform call): collects in shared memory, one reservation per kStage entries.
-__device__ __forceinline__ void queue_push(bool pred, int32_t v, int32_t* s_buf, int& s_n, const Queue& q,
-                                           const int32_t* deg, unsigned long long* cnt) {
-    const unsigned m = __ballot_sync(0xffffffffu, pred);
-    if (!m) return;
-    const int k = __popc(m);
-    if (s_n + k > kStage) queue_flush(s_buf, s_n, q, deg, cnt);
-    if (pred) s_buf[s_n + __popc(m & ((1u << lane_id()) - 1))] = v;
-    __syncwarp();
-    s_n += k;
-}
+// Row lengths of queue entries.
+struct RowLen {
+    const int32_t* deg;
+    __device__ __forceinline__ int32_t operator()(int32_t v) const { return deg[v]; }
+};
 
 // Sources: lane s of the group starts at every vertex of set s (set_beg is device memory). Counts
 // the sources' (vertex, lane) pairs and out-edges with the queue.
@@ -141,9 +79,9 @@ __global__ void k_init_sources(const int64_t* set_beg, int n_lanes, const int32_
                 medges += (unsigned long long)deg[v];
             }
         }
-        queue_push(on, v, s_stage[threadIdx.x >> 5], n_st, q, deg, &cnt[C_Q]);
+        queue_push(on, v, s_stage[threadIdx.x >> 5], n_st, q, RowLen{deg}, &cnt[C_Q]);
     }
-    queue_flush(s_stage[threadIdx.x >> 5], n_st, q, deg, &cnt[C_Q]);
+    queue_flush(s_stage[threadIdx.x >> 5], n_st, q, RowLen{deg}, &cnt[C_Q]);
     warp_add_u64(&cnt[C_PAIRS], pairs);
     warp_add_u64(&cnt[C_MEDGES], medges);
 }
@@ -165,98 +103,36 @@ struct LevelMasks {
     int64_t V;
 };
 
-// Top-down over the out-edges [c0, c1) of the frontier (edge positions as the queue's offsets count
-// them), by one warp; i0 is the largest entry whose offset is at most c0. One pass does the whole
-// level: the atomicOr on seen[w] hands every newly reached (w, lane) pair to exactly one thread,
-// which writes its level and adds it to the next frontier; the pair's bit is for the next level, so
-// no thread of this level reads what another writes, beyond the pre-check of seen[w] that only saves
-// atomics. A warp holds 32 queue entries in registers (one load each) and finds a position's entry by
-// shuffles; two positions a thread keep two rows of dependent loads in flight.
-__device__ __forceinline__ void td_edges(const Queue& q, int64_t nq, int64_t total, int64_t c0, int64_t c1, int64_t i0,
-                                         const CSRView& fw, const LevelMasks& k, int32_t L, const Queue& out,
-                                         unsigned long long* cnt, LevelAcc& acc) {
-    constexpr int U = 2;
-    const int ln = lane_id();
-    int64_t p = c0;
-    while (p < c1) {
-        const int64_t ij = i0 + ln;
-        uint32_t offj = 0xffffffffu;
-        int64_t begj = 0;
-        unsigned long long mj = 0;
-        if (ij < nq) {
-            const int32_t u = __ldcg(q.v + ij);
-            offj = __ldcg(q.off + ij);
-            begj = fw.beg[u] - offj;
-            mj = __ldcg((const unsigned long long*)k.front + u);
-        }
-        const int64_t wnext = i0 + 32 < nq ? (int64_t)__ldcg(q.off + i0 + 32) : total;
-        const int64_t wend = wnext < c1 ? wnext : c1;
-        for (; p < wend; p += 32 * U) {
-            int32_t w[U];
-            unsigned long long bits[U];
-#pragma unroll
-            for (int j = 0; j < U; ++j) {
-                const int64_t pos = p + j * 32 + ln;
-                int x = 0;  // largest window entry with offset <= pos (rows without edges share an offset)
-#pragma unroll
-                for (int b = 16; b; b >>= 1)
-                    if ((int64_t)__shfl_sync(0xffffffffu, offj, x + b) <= pos) x += b;
-                const int64_t bx = __shfl_sync(0xffffffffu, begj, x);
-                bits[j] = __shfl_sync(0xffffffffu, mj, x);
-                w[j] = -1;
-                if (pos < wend) w[j] = fw.adj[bx + pos];
-            }
-#pragma unroll
-            for (int j = 0; j < U; ++j)
-                bits[j] = w[j] >= 0 ? bits[j] & ~__ldcg((const unsigned long long*)k.seen + w[j]) : 0ull;
-#pragma unroll
-            for (int j = 0; j < U; ++j) {
-                bool fresh = false;
-                if (bits[j]) {
-                    const unsigned long long nb = bits[j] & ~atomicOr((unsigned long long*)k.seen + w[j], bits[j]);
-                    if (nb) {
-                        fresh = atomicOr((unsigned long long*)k.next + w[j], nb) == 0ull;
-                        write_levels(k.level, k.V, w[j], nb, L);
-                        const unsigned c = __popcll(nb);
-                        acc.pairs += c;
-                        acc.medges += (unsigned long long)c * (unsigned long long)fw.deg[w[j]];
-                    }
-                }
-                queue_push(fresh, w[j], acc.s_buf, acc.n, out, fw.deg, cnt);
-            }
-        }
-        p = wend;
-        i0 += 32;
+// A top-down level (walk_rows). One pass does the whole level: the atomicOr on seen[w] hands every
+// newly reached (w, lane) pair to exactly one thread, which writes its level and adds it to the next
+// frontier; the pair's bit is for the next level, so no thread of this level reads what another
+// writes, beyond the pre-check of seen[w] that only saves atomics.
+struct TopDown {
+    CSRView fw;
+    LevelMasks k;
+    int32_t L;
+    unsigned long long pairs, medges;  // this thread's sums
+    __device__ __forceinline__ int32_t deg(int32_t u) const { return fw.deg[u]; }
+    __device__ __forceinline__ void row(int32_t u, int64_t& beg, unsigned long long& lanes) const {
+        beg = fw.beg[u];
+        lanes = __ldcg((const unsigned long long*)k.front + u);
     }
-}
-
-// Largest i in [0, n) with off[i] <= key (off[0] = 0): one warp, 32 probes a round.
-__device__ __forceinline__ int64_t queue_find(const uint32_t* off, int64_t n, int64_t key) {
-    int64_t lo = 0, hi = n - 1;
-    while (hi > lo) {
-        const int64_t step = (hi - lo + 31) / 32;
-        const int64_t i = lo + (int64_t)(lane_id() + 1) * step;
-        const bool c = i <= hi && (int64_t)__ldcg(off + i) <= key;
-        const int t = __popc(__ballot_sync(0xffffffffu, c));
-        if (t > 0) lo += (int64_t)t * step;
-        hi = lo + step - 1 < hi ? lo + step - 1 : hi;
+    __device__ __forceinline__ int32_t adj(int64_t i, unsigned long long) const { return fw.adj[i]; }
+    __device__ __forceinline__ unsigned long long want(int32_t w, unsigned long long lanes) const {
+        return lanes & ~__ldcg((const unsigned long long*)k.seen + w);
     }
-    return lo;
-}
-
-// One top-down level's share of a warp: equal runs of the frontier's out-edges, at most kRun long,
-// so that a short frontier still spreads over every warp.
-constexpr int64_t kRun = 32 * 16;
-__device__ __forceinline__ void td_level(const Queue& q, int64_t nq, int64_t total, int64_t warp, int64_t nwarps,
-                                         const CSRView& fw, const LevelMasks& k, int32_t L, const Queue& out,
-                                         unsigned long long* cnt, LevelAcc& acc) {
-    int64_t run = ((total + nwarps - 1) / nwarps + 31) & ~(int64_t)31;
-    run = run < kRun ? run : kRun;
-    for (int64_t c0 = warp * run; c0 < total; c0 += nwarps * run) {
-        const int64_t c1 = c0 + run < total ? c0 + run : total;
-        td_edges(q, nq, total, c0, c1, queue_find(q.off, nq, c0), fw, k, L, out, cnt, acc);
+    __device__ __forceinline__ bool apply(int32_t w, unsigned long long, unsigned long long bits, int32_t& e) {
+        const unsigned long long nb = bits & ~atomicOr((unsigned long long*)k.seen + w, bits);
+        if (!nb) return false;
+        const bool fresh = atomicOr((unsigned long long*)k.next + w, nb) == 0ull;
+        write_levels(k.level, k.V, w, nb, L);
+        const unsigned c = __popcll(nb);
+        pairs += c;
+        medges += (unsigned long long)c * (unsigned long long)fw.deg[w];
+        e = w;
+        return fresh;
     }
-}
+};
 
 __device__ __forceinline__ uint64_t warp_or_u64(uint64_t x) {
     const unsigned lo = __reduce_or_sync(0xffffffffu, (unsigned)(x & 0xffffffffu));
@@ -308,7 +184,7 @@ __device__ __forceinline__ void bu_threads(const int32_t* ids, int64_t n, int64_
                 }
             }
         }
-        queue_push(on, v, acc.s_buf, acc.n, out, outdeg, cnt);
+        queue_push(on, v, acc.s_buf, acc.n, out, RowLen{outdeg}, cnt);
     }
 }
 
@@ -340,7 +216,7 @@ __device__ __forceinline__ void bu_warps(const int32_t* ids, int64_t n, int64_t 
             acc.pairs += c;
             acc.medges += (unsigned long long)c * (unsigned long long)outdeg[v];
         }
-        queue_push(lane == 0 && nb != 0, v, acc.s_buf, acc.n, out, outdeg, cnt);
+        queue_push(lane == 0 && nb != 0, v, acc.s_buf, acc.n, out, RowLen{outdeg}, cnt);
         // lanes split the level writes of this vertex
         if ((nb >> lane) & 1ull) k.level[(int64_t)lane * k.V + v] = L;
         if ((nb >> 32 >> lane) & 1ull) k.level[(int64_t)(lane + 32) * k.V + v] = L;
@@ -378,7 +254,7 @@ __device__ __forceinline__ void bu_ctas(const int32_t* ids, int64_t n, const CSR
             acc.pairs += c;
             acc.medges += (unsigned long long)c * (unsigned long long)outdeg[v];
         }
-        if (threadIdx.x < 32) queue_push(threadIdx.x == 0 && nb != 0, v, acc.s_buf, acc.n, out, outdeg, cnt);
+        if (threadIdx.x < 32) queue_push(threadIdx.x == 0 && nb != 0, v, acc.s_buf, acc.n, out, RowLen{outdeg}, cnt);
         if (threadIdx.x < 64 && ((nb >> threadIdx.x) & 1ull)) k.level[(int64_t)threadIdx.x * k.V + v] = L;
         __syncthreads();
     }
@@ -443,14 +319,13 @@ __device__ __forceinline__ unsigned long long ldcg_u64(const unsigned long long*
 
 __global__ void __launch_bounds__(kPersistThreads, 1) k_bfs_persistent(PersistArgs a) {
     __shared__ int32_t s_stage[kPersistWarps][kStage];
-    __shared__ unsigned long long s_sum[kPersistWarps][2];
-    __shared__ uint32_t s_n[kPersistWarps], s_e[kPersistWarps];
-    __shared__ unsigned long long s_base, s_acc;
+    __shared__ LevelShared<kPersistWarps> sh;
+    __shared__ unsigned long long s_acc;
     __shared__ int s_dir;
     unsigned long long* err = a.ctl + P_ERR;
     unsigned int* bar = reinterpret_cast<unsigned int*>(a.ctl + kCtlBarrier);
     double* trace = reinterpret_cast<double*>(a.ctl + kCtlTrace);
-    const int lane = lane_id(), wib = threadIdx.x >> 5;
+    const int wib = threadIdx.x >> 5;
     // (warps numbered across the CTAs first, so that a short frontier spreads over the SMs)
     const int64_t warp = (int64_t)wib * gridDim.x + blockIdx.x, nwarps = (int64_t)gridDim.x * kPersistWarps;
     const int64_t tid = blockIdx.x * (int64_t)kPersistThreads + threadIdx.x, nthreads = (int64_t)gridDim.x * kPersistThreads;
@@ -498,46 +373,18 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_bfs_persistent(PersistAr
         acc.s_buf = s_stage[wib];
         const int32_t L = a.L0 + lev + 1;
         if (!dir) {
-            td_level(qa, nq, vedges, warp, nwarps, a.fw, k, L, qb, &sl[S_Q], acc);
+            TopDown op{a.fw, k, L, 0, 0};
+            walk_level(qa, nq, vedges, warp, nwarps, op, qb, &sl[S_Q], acc.s_buf, acc.n);
+            acc.pairs = op.pairs;
+            acc.medges = op.medges;
         } else {
             bu_ctas(a.bins + a.bin_n[0] + a.bin_n[1], a.bin_n[2], a.bw, k, a.all, a.fw.deg, L, qb, &sl[S_Q], acc, &s_acc);
             bu_warps(a.bins + a.bin_n[0], a.bin_n[1], warp, nwarps, a.bw, k, a.all, a.fw.deg, L, qb, &sl[S_Q], acc);
             bu_threads(a.bins, a.bin_n[0], warp * 32, nwarps * 32, a.bw, k, a.all, a.fw.deg, L, qb, &sl[S_Q], acc);
             ++n_bu;
         }
-        // end of the level: the CTA's staged entries and sums go out with one reservation
-        const uint32_t e_w = staged_edges(acc.s_buf, acc.n, a.fw.deg);
-        for (int o = 16; o; o >>= 1) {
-            acc.pairs += __shfl_xor_sync(0xffffffffu, acc.pairs, o);
-            acc.medges += __shfl_xor_sync(0xffffffffu, acc.medges, o);
-        }
-        if (lane == 0) {
-            s_sum[wib][0] = acc.pairs;
-            s_sum[wib][1] = acc.medges;
-            s_n[wib] = (uint32_t)acc.n;
-            s_e[wib] = e_w;
-        }
-        __syncthreads();
-        if (wib == 0) {
-            unsigned long long sp = s_sum[lane][0], sm = s_sum[lane][1];
-            const uint32_t n_in = warp_incl_u32(s_n[lane]), e_in = warp_incl_u32(s_e[lane]);
-            for (int o = 16; o; o >>= 1) {
-                sp += __shfl_xor_sync(0xffffffffu, sp, o);
-                sm += __shfl_xor_sync(0xffffffffu, sm, o);
-            }
-            s_n[lane] = n_in - s_n[lane];
-            s_e[lane] = e_in - s_e[lane];
-            if (lane == 31) {
-                s_base = n_in ? atomicAdd(&sl[S_Q], ((unsigned long long)n_in << kQShift) | e_in) : 0ull;
-                if (sp) atomicAdd(&sl[S_PAIRS], sp);
-                if (sm) atomicAdd(&sl[S_MEDGES], sm);
-            }
-        }
-        __syncthreads();
-        if (acc.n) {
-            const unsigned long long at = s_base;
-            queue_write(acc.s_buf, acc.n, qb, a.fw.deg, (at >> kQShift) + s_n[wib], (uint32_t)(at & kQEdges) + s_e[wib]);
-        }
+        block_publish<kPersistWarps>(sh, acc.s_buf, acc.n, qb, RowLen{a.fw.deg}, &sl[S_Q], acc.pairs, acc.medges,
+                                     &sl[S_PAIRS]);
         if (!grid_barrier(bar, err, kBarrierSpins)) break;
         n_last = nq;
         packed = ldcg_u64(&sl[S_Q]);
@@ -573,7 +420,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_bfs_persistent(PersistAr
 
 __device__ __forceinline__ void level_end(LevelAcc& acc, const Queue& out, const int32_t* outdeg,
                                           unsigned long long* cnt) {
-    queue_flush(acc.s_buf, acc.n, out, outdeg, &cnt[C_Q]);
+    queue_flush(acc.s_buf, acc.n, out, RowLen{outdeg}, &cnt[C_Q]);
     warp_add_u64(&cnt[C_PAIRS], acc.pairs);
     warp_add_u64(&cnt[C_MEDGES], acc.medges);
 }
@@ -584,7 +431,10 @@ __global__ void __launch_bounds__(kBlock) k_td_level(Queue q, int64_t nq, int64_
     LevelAcc acc;
     acc.s_buf = s_stage[threadIdx.x >> 5];
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    td_level(q, nq, total, warp, ((int64_t)gridDim.x * blockDim.x) >> 5, fw, k, L, out, &cnt[C_Q], acc);
+    TopDown op{fw, k, L, 0, 0};
+    walk_level(q, nq, total, warp, ((int64_t)gridDim.x * blockDim.x) >> 5, op, out, &cnt[C_Q], acc.s_buf, acc.n);
+    acc.pairs = op.pairs;
+    acc.medges = op.medges;
     level_end(acc, out, fw.deg, cnt);
 }
 
@@ -644,10 +494,10 @@ int bfs_run(gir_dev* g, const int64_t* set_beg_h, const int32_t* srcs_d, int64_t
     GIR_TRY(ensure_n(g, g->scratch[1], V, &front[0]));
     GIR_TRY(ensure_n(g, g->scratch[2], V, &front[1]));
     GIR_TRY(ensure_n(g, g->scratch[8], V, &front[2]));
-    const int q_slots[3] = {3, 4, 9};
+    const int q_slots[3] = {3, 4, 9}, off_slots[3] = {5, 7, 11};
     for (int i = 0; i < 3; ++i) {
-        GIR_TRY(ensure_n(g, g->scratch[q_slots[i]], 2 * (V + 1), &q[i].v));
-        q[i].off = reinterpret_cast<uint32_t*>(q[i].v + V + 1);
+        GIR_TRY(ensure_n(g, g->scratch[q_slots[i]], V + 1, &q[i].v));
+        GIR_TRY(ensure_n(g, g->scratch[off_slots[i]], V + 1, &q[i].off));
     }
     GIR_TRY(ensure_n(g, g->scratch[6], 65, &sbeg));
     GIR_TRY(ensure_n(g, g->scratch[10], kCtlTrace + kTraceW * kPersistTrace, &ctl));

@@ -6,7 +6,8 @@
 // small SCCs, gir.cpp:541-587; Tarjan-Vishkin over a BFS tree for large ones, gir.cpp:1804-2022).
 // An SCC of one vertex is a singleton block (gir.cpp:584). Here Tarjan-Vishkin runs on every
 // SCC at once:
-//  1. BFS spanning forest of H from every SCC's smallest vertex (level-synchronous);
+//  1. BFS spanning forest of H from every SCC's smallest vertex (level-synchronous), or on a deep H a
+//     forest from union-find, rooted by Euler tours, with 2. and 3. to match (see "Deep graphs");
 //  2. subtree sizes nd (levels bottom-up) and preorder numbers pre (children grouped by parent
 //     by a radix sort, sibling offsets by a scan, levels top-down);
 //  3. low / high: min / max pre over each subtree and its non-tree neighbours;
@@ -19,6 +20,8 @@
 //     articulation point (-1 for the block a tree root belongs to first), bcnt = number of
 //     blocks containing the vertex (AP iff >= 2).
 #include "common.cuh"
+#include "frontier.cuh"
+#include "unionfind.cuh"
 
 namespace gir {
 
@@ -53,10 +56,11 @@ __global__ void k_h_deg(int64_t V, const int32_t* scc, const uint8_t* nontrivial
 }
 
 // Forest roots: every SCC's smallest vertex; only those of non-singleton SCCs start the BFS.
-__global__ void k_roots(int64_t V, const int32_t* scc, const uint8_t* nontrivial, int32_t* parent, int32_t* depth,
-                        int32_t* order, unsigned long long* cnt) {
+__global__ void k_roots(int64_t V, const int32_t* scc, const uint8_t* nontrivial, const int32_t* hdeg, int32_t* parent,
+                        Queue q, unsigned long long* cnt) {
     __shared__ int32_t s_st[kBlock / 32][kStage];
     int n_st = 0;
+    auto deg = [&](int32_t x) { return hdeg[x]; };
     for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < V; base += (int64_t)gridDim.x * blockDim.x) {
         const int64_t v = base + threadIdx.x;
         bool root = false;
@@ -64,58 +68,178 @@ __global__ void k_roots(int64_t V, const int32_t* scc, const uint8_t* nontrivial
             const bool r = scc[v] == (int32_t)v;
             root = r && nontrivial[v];
             parent[v] = r ? (int32_t)v : -1;
-            depth[v] = r ? 0 : -1;
         }
-        stage_append(root, (int32_t)v, s_st[threadIdx.x >> 5], n_st, order, &cnt[C_Q]);
+        queue_push(root, (int32_t)v, s_st[threadIdx.x >> 5], n_st, q, deg, cnt);
     }
-    stage_flush(s_st[threadIdx.x >> 5], n_st, order, &cnt[C_Q]);
+    queue_flush(s_st[threadIdx.x >> 5], n_st, q, deg, cnt);
 }
 
-// One BFS level of the spanning forest: the level's vertices are order[lo, lo + n); new ones are
-// appended to order after it. Edge-balanced: the level's H rows are cut into equal chunks after
-// a scan of their lengths, so hubs of the giant SCC do not serialize a warp.
-__global__ void k_level_deg(const int32_t* q, int64_t n, const int32_t* deg, int64_t* pref) {
-    GRID_STRIDE(i, n) pref[i] = deg[q[i]];
-    if (blockIdx.x == 0 && threadIdx.x == 0) pref[n] = 0;
+// One BFS level of the spanning forest over H (frontier.cuh): the atomicCAS on parent[w] gives w its
+// parent and queues it. The levels end up back to back in the queue array.
+// Bound by the latency of the parents' and SCC labels' random accesses. A level was a degree pass, a
+// scan and a launch whose warps took 512 row entries each: 42 us a level of an 803 x 803 lattice.
+struct ForestLevel {
+    CSRView sym;  // (row lengths: H's)
+    const int32_t* scc;
+    int32_t* parent;
+    __device__ __forceinline__ int32_t deg(int32_t u) const { return sym.deg[u]; }
+    __device__ __forceinline__ void row(int32_t u, int64_t& beg, unsigned long long& who) const {
+        beg = sym.beg[u];
+        who = ((unsigned long long)(uint32_t)scc[u] << 32) | (uint32_t)u;
+    }
+    __device__ __forceinline__ int32_t adj(int64_t i, unsigned long long) const { return sym.adj[i]; }
+    __device__ __forceinline__ unsigned long long want(int32_t w, unsigned long long who) const {
+        return __ldcg(parent + w) == -1 && scc[w] == (int32_t)(who >> 32);
+    }
+    __device__ __forceinline__ bool apply(int32_t w, unsigned long long who, unsigned long long, int32_t& e) {
+        e = w;
+        return atomicCAS(&parent[w], -1, (int32_t)(uint32_t)who) == -1;
+    }
+};
+
+// ---- Deep graphs: a spanning forest without levels ---------------------------------------------
+// Tarjan-Vishkin takes any rooted spanning forest. Where the BFS forest is still growing after
+// deep_levels(V) levels (a road network has thousands), the forest comes from union-find over H
+// instead: every hook of one root under another is a tree edge. Each tree is rooted at its SCC's
+// smallest vertex by its Euler tour: the two arcs of every tree edge, sorted, give each vertex its
+// arcs; the arc after x -> y is the one after y -> x in y's list, cyclically, and the tour starts at
+// the root's first arc. Pointer doubling over the arcs gives each its distance to the tour's end; the
+// arc of a tree edge that comes first points down, the arcs between the two are twice the subtree,
+// and the number of down arcs so far is the preorder. A subtree is then an interval of preorder
+// positions, and low / high over it the minimum / maximum of an interval (doubling windows).
+// 803 x 803 lattice, blocks only: about 1,300 levels of four launches each (94 ms) against some
+// sixty launches in all (about 1.5 ms). The arcs' indices are 32 bits wide: below 2^30 vertices.
+constexpr int64_t kEulerMaxV = 1ll << 30;
+
+// Tree edges: the slot of the hooked root holds (u << 32 | w); ~0 elsewhere.
+__global__ void __launch_bounds__(kBlock) k_tree_link(int64_t V, CSRView h, const int32_t* scc, int32_t* uf,
+                                                      uint64_t* edge, unsigned long long* err) {
+    __shared__ int64_t s_excl[kBlock / 32][33];
+    __shared__ int32_t s_u[kBlock / 32][32];
+    const int wib = threadIdx.x >> 5;
+    warp_sweep_rows(h.beg, h.deg, h.adj, 0, V, s_excl[wib], s_u[wib], [&](int32_t u, int32_t w, int64_t) {
+        if (u > w || scc[u] != scc[w]) return;  // (every pair is in both rows)
+        const int32_t hooked = uf_union(uf, u, w, err);
+        if (hooked >= 0) edge[hooked] = ((uint64_t)(uint32_t)u << 32) | (uint32_t)w;
+    });
 }
 
-constexpr int kForestChunk = 32 * 16;
+__global__ void k_tree_flags(int64_t V, const uint64_t* edge, uint8_t* flag) {
+    GRID_STRIDE(v, V) flag[v] = edge[v] != ~0ull;
+}
 
-__global__ void __launch_bounds__(kBlock) k_forest_balanced(const int32_t* q, int64_t nq, const int64_t* pref, HView h,
-                                                            int32_t* parent, int32_t* depth, int32_t L, int32_t* out,
-                                                            unsigned long long* cnt) {
-    __shared__ int32_t s_st[kBlock / 32][kStage];
-    int n_st = 0;
-    const int64_t total = pref[nq];
-    const int lane = lane_id();
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t c0 = warp * kForestChunk; c0 < total; c0 += nwarps * kForestChunk) {
-        const int64_t c1 = c0 + kForestChunk < total ? c0 + kForestChunk : total;
-        const int64_t key = c0 + lane < total ? c0 + lane : total - 1;
-        int64_t lo = 0, hi = nq - 1;
-        while (lo < hi) {
-            const int64_t m = (lo + hi + 1) >> 1;
-            if (pref[m] <= key) lo = m; else hi = m - 1;
+__global__ void k_tree_arcs(const uint64_t* edge, int64_t n, uint64_t* arcs) {
+    GRID_STRIDE(i, n) {
+        arcs[2 * i] = edge[i];
+        arcs[2 * i + 1] = (edge[i] << 32) | (edge[i] >> 32);
+    }
+}
+
+// Twins and successors of the sorted arcs: twin[i], and jump[i] = (next arc, 1); the arc that would
+// enter its root's first arc again ends the tour: (n, 0) with slot n a fixed point.
+__global__ void k_euler_next(const uint64_t* arcs, int64_t n, const int32_t* scc, int32_t* twin, int2* jump) {
+    GRID_STRIDE(i, n) {
+        const uint64_t a = arcs[i];
+        const int32_t y = (int32_t)(a & 0xffffffffULL);
+        const int64_t t = lower_bound_dev(arcs, (int64_t)0, n, (a << 32) | (a >> 32));
+        twin[i] = (int32_t)t;
+        int64_t nx = t + 1;
+        bool end = false;
+        if (nx == n || (int32_t)(arcs[nx] >> 32) != y) {  // the twin is y's last arc: on to its first
+            nx = lower_bound_dev(arcs, (int64_t)0, n, (uint64_t)(uint32_t)y << 32);
+            end = scc[y] == y;
         }
-        int64_t i = lo;
-        for (int64_t base = c0; base < c1; base += 32) {
-            const int64_t p = base + lane;
-            bool push = false;
-            int32_t w = 0;
-            if (p < c1) {
-                while (pref[i + 1] <= p) ++i;
-                const int32_t u = q[i];
-                w = h.sym.adj[h.sym.beg[u] + (p - pref[i])];
-                if (parent[w] == -1 && h.scc[w] == h.scc[u] && atomicCAS(&parent[w], -1, u) == -1) {
-                    depth[w] = L + 1;
-                    push = true;
-                }
-            }
-            stage_append(push, w, s_st[threadIdx.x >> 5], n_st, out, &cnt[C_Q]);
+        jump[i] = end ? make_int2((int32_t)n, 0) : make_int2((int32_t)nx, 1);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) jump[n] = make_int2((int32_t)n, 0);
+}
+
+__global__ void k_euler_double(const int2* in, int64_t n, int2* out) {
+    GRID_STRIDE(i, n + 1) {
+        const int2 a = in[i], b = in[a.x];
+        out[i] = make_int2(b.x, a.y + b.y);
+    }
+}
+
+// Arcs of every tree's tour, at its root (0 elsewhere): its first arc is the root's first.
+__global__ void k_tour_size(const uint64_t* arcs, int64_t n, const int32_t* scc, const int2* rank, int64_t* size) {
+    GRID_STRIDE(i, n) {
+        const int32_t x = (int32_t)(arcs[i] >> 32);
+        if (scc[x] == x && (i == 0 || (int32_t)(arcs[i - 1] >> 32) != x)) size[x] = (int64_t)rank[i].y + 1;
+    }
+}
+
+// Tour positions (trees back to back): the down arcs' flags, and every child's parent and subtree.
+__global__ void k_tour_down(const uint64_t* arcs, int64_t n, const int32_t* scc, const int32_t* twin, const int2* rank,
+                            const int64_t* tour, int64_t* down, int32_t* parent, int32_t* nd) {
+    GRID_STRIDE(i, n) {
+        const int32_t x = (int32_t)(arcs[i] >> 32), y = (int32_t)(arcs[i] & 0xffffffffULL);
+        const int32_t r = scc[x];
+        const int32_t d = rank[i].y, dt = rank[twin[i]].y;
+        down[tour[r + 1] - 1 - d] = d > dt;
+        if (d > dt) {
+            parent[y] = x;
+            nd[y] = (d - dt + 1) / 2;
         }
     }
-    stage_flush(s_st[threadIdx.x >> 5], n_st, out, &cnt[C_Q]);
+}
+
+// Preorder numbers (within the tree; roots have 0), all non-root vertices in preorder, and the roots'
+// subtree sizes. downs: exclusive scan of the down flags.
+__global__ void k_tour_pre(const uint64_t* arcs, int64_t n, const int32_t* scc, const int32_t* twin, const int2* rank,
+                           const int64_t* tour, const int64_t* downs, int32_t* pre, int32_t* at, int32_t* nd) {
+    GRID_STRIDE(i, n) {
+        const int32_t x = (int32_t)(arcs[i] >> 32), y = (int32_t)(arcs[i] & 0xffffffffULL);
+        const int32_t r = scc[x];
+        const int32_t d = rank[i].y, dt = rank[twin[i]].y;
+        if (d <= dt) continue;
+        const int64_t k = downs[tour[r + 1] - 1 - d];
+        pre[y] = (int32_t)(k - downs[tour[r]]) + 1;
+        at[k] = y;
+        if (x == r) nd[r] = (int32_t)((tour[r + 1] - tour[r]) / 2) + 1;
+    }
+}
+
+// Doubling windows over the preorder positions: win[k] = (min low, max high) of [k, k + len). A vertex
+// whose subtree is at least len and below 2 len long takes its interval from two of them.
+__global__ void k_win_first(const int32_t* at, int64_t n, const int32_t* low, const int32_t* high, int2* win) {
+    GRID_STRIDE(k, n) win[k] = make_int2(low[at[k]], high[at[k]]);
+}
+__global__ void k_win_step(const int32_t* at, int64_t n, int64_t len, const int32_t* nd, const int2* win, int2* next,
+                           int32_t* low, int32_t* high) {
+    GRID_STRIDE(k, n) {
+        const int2 a = win[k];
+        const int32_t v = at[k];
+        const int64_t s = nd[v];
+        if (s >= len && s < 2 * len) {
+            const int2 b = win[k + s - len];
+            low[v] = a.x < b.x ? a.x : b.x;
+            high[v] = a.y > b.y ? a.y : b.y;
+        }
+        const int2 b = k + len < n ? win[k + len] : a;
+        next[k] = make_int2(a.x < b.x ? a.x : b.x, a.y > b.y ? a.y : b.y);
+    }
+}
+
+// The smallest H neighbour of every tree root (a BFS forest's first child): it decides which of its
+// blocks is the root's parent block.
+__global__ void k_root_rows(int64_t V, const int32_t* scc, const int32_t* hdeg, int32_t* deg, int32_t* least) {
+    GRID_STRIDE(v, V) {
+        deg[v] = scc[v] == (int32_t)v ? hdeg[v] : 0;
+        least[v] = INT32_MAX;
+    }
+}
+__global__ void __launch_bounds__(kBlock) k_root_least(int64_t V, CSRView h, const int32_t* scc, int32_t* least) {
+    __shared__ int64_t s_excl[kBlock / 32][33];
+    __shared__ int32_t s_u[kBlock / 32][32];
+    const int wib = threadIdx.x >> 5;
+    warp_sweep_rows(h.beg, h.deg, h.adj, 0, V, s_excl[wib], s_u[wib], [&](int32_t u, int32_t w, int64_t) {
+        if (scc[w] == u && w < least[u]) atomicMin(&least[u], w);
+    });
+}
+__global__ void k_root_block_least(int64_t V, const int32_t* least, const int32_t* uf, const int32_t* id_of_rep,
+                                   int32_t* label) {
+    GRID_STRIDE(v, V) if (least[v] != INT32_MAX) label[v] = id_of_rep[uf[least[v]]];
 }
 
 __global__ void k_fill_i32(int32_t* p, int64_t n, int32_t v) { GRID_STRIDE(i, n) p[i] = v; }
@@ -167,28 +291,6 @@ __global__ void k_pre_level(const int32_t* q, int64_t n, const int32_t* parent, 
 }
 
 __global__ void k_pre_roots(const int32_t* q, int64_t n, int32_t* pre) { GRID_STRIDE(i, n) pre[q[i]] = 0; }
-
-// low / high from non-tree edges of H, and rule 1 unions.
-__device__ __forceinline__ int32_t uf_find(int32_t* uf, int32_t x) {
-    int32_t p = uf[x];
-    while (p != x) {
-        const int32_t gp = uf[p];
-        if (gp != p) uf[x] = gp;
-        x = p;
-        p = uf[x];
-    }
-    return x;
-}
-
-__device__ __forceinline__ void uf_union(int32_t* uf, int32_t a, int32_t b, unsigned long long* err) {
-    for (int iter = 0; iter < (1 << 22); ++iter) {
-        int32_t ra = uf_find(uf, a), rb = uf_find(uf, b);
-        if (ra == rb) return;
-        if (ra > rb) { const int32_t t = ra; ra = rb; rb = t; }
-        if (atomicCAS(&uf[rb], rb, ra) == rb) return;
-    }
-    atomicAdd(err, 1ull);
-}
 
 // Per-vertex tree data packed for the non-tree sweep: one 16-byte gather per neighbour instead of
 // four scattered 4-byte ones. x = pre, y = nd, z = parent, w = scc.
@@ -348,19 +450,98 @@ __global__ void k_bcnt_heads(const int32_t* head, int64_t nb, int32_t* bcnt) {
 
 }  // namespace
 
+// The rooted spanning forest of a deep H by union-find and Euler tours: parent, nd and pre of every
+// vertex of a non-singleton SCC (the callers' values stay elsewhere: parent = itself, nd = 1), and its
+// n_tree non-root vertices in preorder, tree after tree.
+static int euler_forest(gir_dev* g, const CSRView& h, const int32_t* scc, int32_t* parent, int32_t* nd, int32_t* pre,
+                        int32_t* at, int64_t* n_tree, unsigned long long* err) {
+    const int64_t V = g->V;
+    Temps t{g, {}};
+    uint64_t *edge = nullptr, *picked = nullptr;
+    int32_t* uf = nullptr;
+    uint8_t* flag = nullptr;
+    GIR_TRY(t.get(&edge, V));
+    GIR_TRY(t.get(&picked, V));
+    GIR_TRY(t.get(&uf, V));
+    GIR_TRY(t.get(&flag, V));
+    GIR_CUDA(g, cudaMemsetAsync(edge, 0xff, sizeof(uint64_t) * V, g->stream));
+    GIR_CUDA(g, cudaMemsetAsync(pre, 0, sizeof(int32_t) * V, g->stream));
+    k_uf_init<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(uf, V);
+    GIR_LAUNCH(g, "k_uf_init");
+    k_tree_link<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, h, scc, uf, edge, err);
+    GIR_LAUNCH(g, "k_tree_link");
+    k_tree_flags<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, edge, flag);
+    GIR_LAUNCH(g, "k_tree_flags");
+    int64_t m = 0;
+    GIR_TRY(select_flagged_u64(g, edge, flag, picked, V, &m));
+    *n_tree = m;
+    const int64_t n = 2 * m;  // arcs
+    uint64_t *arcs = nullptr, *atmp = nullptr;
+    int32_t* twin = nullptr;
+    int2 *ja = nullptr, *jb = nullptr;
+    int64_t *tour = nullptr, *down = nullptr;
+    GIR_TRY(t.get(&arcs, n + 1));
+    GIR_TRY(t.get(&atmp, n + 1));
+    GIR_TRY(t.get(&twin, n + 1));
+    GIR_TRY(t.get(&ja, n + 1));
+    GIR_TRY(t.get(&jb, n + 1));
+    GIR_TRY(t.get(&tour, V + 1));
+    GIR_TRY(t.get(&down, n + 1));
+    if (m == 0) return GIR_OK;
+    const int gn = grid_for(g, n + 1, kBlock);
+    k_tree_arcs<<<gn, kBlock, 0, g->stream>>>(picked, m, arcs);
+    GIR_LAUNCH(g, "k_tree_arcs");
+    GIR_TRY(sort_keys_u64(g, arcs, atmp, n, 64));
+    k_euler_next<<<gn, kBlock, 0, g->stream>>>(arcs, n, scc, twin, ja);
+    GIR_LAUNCH(g, "k_euler_next");
+    for (int64_t reach = 1; reach < n; reach *= 2) {
+        k_euler_double<<<gn, kBlock, 0, g->stream>>>(ja, n, jb);
+        GIR_LAUNCH(g, "k_euler_double");
+        std::swap(ja, jb);
+    }
+    GIR_CUDA(g, cudaMemsetAsync(tour, 0, sizeof(int64_t) * (V + 1), g->stream));
+    k_tour_size<<<gn, kBlock, 0, g->stream>>>(arcs, n, scc, ja, tour);
+    GIR_LAUNCH(g, "k_tour_size");
+    GIR_TRY(exclusive_scan_i64(g, tour, tour, V + 1));
+    GIR_CUDA(g, cudaMemsetAsync(down + n, 0, sizeof(int64_t), g->stream));
+    k_tour_down<<<gn, kBlock, 0, g->stream>>>(arcs, n, scc, twin, ja, tour, down, parent, nd);
+    GIR_LAUNCH(g, "k_tour_down");
+    GIR_TRY(exclusive_scan_i64(g, down, down, n + 1));
+    k_tour_pre<<<gn, kBlock, 0, g->stream>>>(arcs, n, scc, twin, ja, tour, down, pre, at, nd);
+    GIR_LAUNCH(g, "k_tour_pre");
+    return GIR_OK;
+}
+
+// low / high of every non-root vertex over its subtree (at: the n non-root vertices in preorder).
+static int subtree_windows(gir_dev* g, const int32_t* at, int64_t n, const int32_t* nd, int32_t* low, int32_t* high) {
+    if (n == 0) return GIR_OK;
+    Temps t{g, {}};
+    int2 *wa = nullptr, *wb = nullptr;
+    GIR_TRY(t.get(&wa, n));
+    GIR_TRY(t.get(&wb, n));
+    const int gn = grid_for(g, n, kBlock);
+    k_win_first<<<gn, kBlock, 0, g->stream>>>(at, n, low, high, wa);
+    GIR_LAUNCH(g, "k_win_first");
+    for (int64_t len = 1; len <= n; len *= 2) {
+        k_win_step<<<gn, kBlock, 0, g->stream>>>(at, n, len, nd, wa, wb, low, high);
+        GIR_LAUNCH(g, "k_win_step");
+        std::swap(wa, wb);
+    }
+    return GIR_OK;
+}
+
 int bct_build(gir_dev* g) {
     if (!g->scc_built) return fail(g, GIR_ERR_STATE, "buildBCT needs buildSCC_DAG first");
     const int64_t V = g->V;
     const int32_t* scc = static_cast<const int32_t*>(g->scc.p);
     HView h{view(g->sym), scc};  // (row lengths replaced by the H lengths below)
-    int32_t *parent = nullptr, *depth = nullptr, *order = nullptr, *nd = nullptr, *pre = nullptr, *off = nullptr;
+    int32_t *parent = nullptr, *order = nullptr, *nd = nullptr, *pre = nullptr, *off = nullptr;
     int32_t *low = nullptr, *high = nullptr, *uf = nullptr, *reps = nullptr, *id_of_rep = nullptr;
     uint64_t *keys = nullptr, *ktmp = nullptr;
     uint8_t* flag = nullptr;
     int64_t *scan = nullptr, *first = nullptr;
     unsigned long long* cnt = nullptr;
     GIR_TRY(ensure_n(g, g->scratch[0], V + 1, &parent));
-    GIR_TRY(ensure_n(g, g->scratch[1], V + 1, &depth));
     GIR_TRY(ensure_n(g, g->scratch[2], V + 1, &order));
     GIR_TRY(ensure_n(g, g->scratch[3], V + 1, &nd));
     GIR_TRY(ensure_n(g, g->scratch[4], V + 1, &pre));
@@ -403,57 +584,57 @@ int bct_build(gir_dev* g) {
     k_h_deg<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, scc, nontrivial, g->sym.deg, hdeg);
     GIR_LAUNCH(g, "k_h_deg");
     h.sym.deg = hdeg;
-    k_roots<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, scc, nontrivial, parent, depth, order, cnt);
+    Queue fq{order, nullptr};
+    unsigned long long* ctl = nullptr;
+    GIR_TRY(ensure_n(g, g->scratch[1], V + 1, &fq.off));
+    GIR_TRY(ensure_n(g, g->scratch[15], kLoopWords, &ctl));
+    GIR_CUDA(g, cudaMemsetAsync(ctl, 0, sizeof(unsigned long long) * kLoopWords, g->stream));
+    k_roots<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, scc, nontrivial, hdeg, parent, fq, ctl + W_Q);
     GIR_LAUNCH(g, "k_roots");
-    GIR_TRY(read());
-    std::vector<int64_t> lvl_off{0, (int64_t)hc[C_Q]};
-    for (int32_t L = 0;; ++L) {
-        const int64_t lo = lvl_off[L], n = lvl_off[L + 1] - lo;
-        if (n == 0) break;
-        GIR_CUDA(g, cudaMemsetAsync(&cnt[C_Q], 0, sizeof(unsigned long long), g->stream));
-        // (`scan` serves as the level's row-length prefix here; the preorder step reuses it later)
-        k_level_deg<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(order + lo, n, h.sym.deg, scan);
-        GIR_LAUNCH(g, "k_level_deg");
-        GIR_TRY(exclusive_scan_i64(g, scan, scan, n + 1));
-        k_forest_balanced<<<g->num_sms * 8, kBlock, 0, g->stream>>>(order + lo, n, scan, h, parent, depth, L,
-                                                                    order + lo + n, cnt);
-        GIR_LAUNCH(g, "k_forest_balanced");
-        GIR_TRY(read());
-        lvl_off.push_back(lvl_off.back() + (int64_t)hc[C_Q]);
-    }
-    const int D = (int)lvl_off.size() - 1;  // levels 0..D-1 (the last entry repeats the end)
-    trace_mark(g, "bct: forest");
-    // 2. subtree sizes, bottom-up
+    FrontierRun run;
+    GIR_TRY(run_frontier(g, ForestLevel{h.sym, scc, parent}, fq, ctl, run, V < kEulerMaxV ? deep_levels(V) : INT64_MAX));
+    const bool deep = !run.done();
+    trace_mark(g, deep ? "bct: forest levels (given up)" : "bct: forest");
+    std::vector<int64_t> lvl_off{0};
+    for (int64_t n : run.levels) lvl_off.push_back(lvl_off.back() + n);
+    const int D = deep ? 0 : (int)lvl_off.size() - 1;  // levels 0..D-1 (the last one may be empty)
+    int64_t n_tree = 0;
+    // 2. subtree sizes
     k_fill_i32<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(nd, V, 1);
     GIR_LAUNCH(g, "k_fill_i32");
-    for (int L = D - 1; L >= 1; --L) {
-        const int64_t n = lvl_off[L + 1] - lvl_off[L];
-        if (n == 0) continue;
-        k_nd_level<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(order + lvl_off[L], n, parent, nd);
-        GIR_LAUNCH(g, "k_nd_level");
-    }
-    //    preorder: children grouped by parent, sibling offsets, then levels top-down
-    k_child_keys<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, parent, keys, flag);
-    GIR_LAUNCH(g, "k_child_keys");
-    int64_t nc = 0;
-    GIR_TRY(select_flagged_u64(g, keys, flag, ktmp, V, &nc));
-    GIR_TRY(sort_keys_u64(g, ktmp, keys, nc, 64));
-    if (nc > 0) {
-        k_child_nd<<<grid_for(g, nc, kBlock), kBlock, 0, g->stream>>>(ktmp, nc, nd, scan);
-        GIR_LAUNCH(g, "k_child_nd");
-        GIR_TRY(exclusive_scan_i64(g, scan, scan, nc + 1));
-        k_group_first<<<grid_for(g, nc, kBlock), kBlock, 0, g->stream>>>(ktmp, nc, first);
-        GIR_LAUNCH(g, "k_group_first");
-        k_sibling_off<<<grid_for(g, nc, kBlock), kBlock, 0, g->stream>>>(ktmp, nc, scan, first, off);
-        GIR_LAUNCH(g, "k_sibling_off");
-    }
-    k_pre_roots<<<grid_for(g, lvl_off[1], kBlock), kBlock, 0, g->stream>>>(order, lvl_off[1], pre);
-    GIR_LAUNCH(g, "k_pre_roots");
-    for (int L = 1; L < D; ++L) {
-        const int64_t n = lvl_off[L + 1] - lvl_off[L];
-        if (n == 0) continue;
-        k_pre_level<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(order + lvl_off[L], n, parent, off, pre);
-        GIR_LAUNCH(g, "k_pre_level");
+    if (deep) {
+        GIR_TRY(euler_forest(g, h.sym, scc, parent, nd, pre, order, &n_tree, &cnt[C_ERR]));
+    } else {
+        //    levels bottom-up
+        for (int L = D - 1; L >= 1; --L) {
+            const int64_t n = lvl_off[L + 1] - lvl_off[L];
+            if (n == 0) continue;
+            k_nd_level<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(order + lvl_off[L], n, parent, nd);
+            GIR_LAUNCH(g, "k_nd_level");
+        }
+        //    preorder: children grouped by parent, sibling offsets, then levels top-down
+        k_child_keys<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, parent, keys, flag);
+        GIR_LAUNCH(g, "k_child_keys");
+        int64_t nc = 0;
+        GIR_TRY(select_flagged_u64(g, keys, flag, ktmp, V, &nc));
+        GIR_TRY(sort_keys_u64(g, ktmp, keys, nc, 64));
+        if (nc > 0) {
+            k_child_nd<<<grid_for(g, nc, kBlock), kBlock, 0, g->stream>>>(ktmp, nc, nd, scan);
+            GIR_LAUNCH(g, "k_child_nd");
+            GIR_TRY(exclusive_scan_i64(g, scan, scan, nc + 1));
+            k_group_first<<<grid_for(g, nc, kBlock), kBlock, 0, g->stream>>>(ktmp, nc, first);
+            GIR_LAUNCH(g, "k_group_first");
+            k_sibling_off<<<grid_for(g, nc, kBlock), kBlock, 0, g->stream>>>(ktmp, nc, scan, first, off);
+            GIR_LAUNCH(g, "k_sibling_off");
+        }
+        k_pre_roots<<<grid_for(g, lvl_off[1], kBlock), kBlock, 0, g->stream>>>(order, lvl_off[1], pre);
+        GIR_LAUNCH(g, "k_pre_roots");
+        for (int L = 1; L < D; ++L) {
+            const int64_t n = lvl_off[L + 1] - lvl_off[L];
+            if (n == 0) continue;
+            k_pre_level<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(order + lvl_off[L], n, parent, off, pre);
+            GIR_LAUNCH(g, "k_pre_level");
+        }
     }
     trace_mark(g, "bct: subtree sizes + preorder");
     // 3. low / high and rule 1
@@ -481,6 +662,7 @@ int bct_build(gir_dev* g) {
             GIR_LAUNCH(g, "k_nontree_heavy");
         }
     }
+    if (deep) GIR_TRY(subtree_windows(g, order, n_tree, nd, low, high));
     for (int L = D - 1; L >= 1; --L) {
         const int64_t n = lvl_off[L + 1] - lvl_off[L];
         if (n == 0) continue;
@@ -502,8 +684,20 @@ int bct_build(gir_dev* g) {
     k_block_ids<<<grid_for(g, nb, kBlock), kBlock, 0, g->stream>>>(reps, nb, id_of_rep);
     GIR_LAUNCH(g, "k_block_ids");
     GIR_TRY(ensure_n(g, g->blk_head, nb + 1, &head));
-    k_root_block<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, parent, pre, uf, id_of_rep, label);
-    GIR_LAUNCH(g, "k_root_block");
+    if (deep) {
+        int32_t *rdeg = pre, *least = high;  // (neither is read any more)
+        k_root_rows<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, scc, hdeg, rdeg, least);
+        GIR_LAUNCH(g, "k_root_rows");
+        CSRView rows = h.sym;
+        rows.deg = rdeg;
+        k_root_least<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, rows, scc, least);
+        GIR_LAUNCH(g, "k_root_least");
+        k_root_block_least<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, least, uf, id_of_rep, label);
+        GIR_LAUNCH(g, "k_root_block_least");
+    } else {
+        k_root_block<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, parent, pre, uf, id_of_rep, label);
+        GIR_LAUNCH(g, "k_root_block");
+    }
     k_block_assign<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, parent, nd, uf, id_of_rep, label, head);
     GIR_LAUNCH(g, "k_block_assign");
     k_bcnt<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, head, nb, bcnt);

@@ -226,8 +226,6 @@ int create_impl(const int32_t* fw_beg, const int32_t* fw_adj, const int32_t* bw_
     GIR_CUDA(g, cudaEventCreate(&g->ev3));
     GIR_CUDA(g, cudaEventCreate(&g->pev0));
     GIR_CUDA(g, cudaEventCreate(&g->pev1));
-    void* pin = nullptr;
-    GIR_TRY(pinned(g, kPinnedBytes, &pin));
     g->V = V;
     g->wrule_lo = 1;  // lo > hi: inserted edges get the hash weight of GIR::edgeWeight
     g->wrule_hi = 0;

@@ -231,8 +231,8 @@ void release(gir_dev* g, DevBuf& b);
 void release_scratch(gir_dev* g, size_t min_bytes);
 constexpr size_t kKeepScratchBelow = 64u << 20;
 
-// Pinned host scratch of at least `bytes` (kPinnedBytes are there from create on, so pointers to it
-// stay valid across calls that ask for no more).
+// Pinned host scratch of at least `bytes` (the first request gets kPinnedBytes, so pointers to it stay
+// valid across calls that ask for no more).
 constexpr size_t kPinnedBytes = 4096;
 int pinned(gir_dev* g, size_t bytes, void** out);
 
@@ -241,6 +241,21 @@ bool is_device_ptr(const void* p);
 // Copies `bytes` from a host or device pointer into device memory owned by the handle
 // (`stage`), or returns `p` itself when it is already device memory.
 int stage_input(gir_dev* g, DevBuf& stage, const void* p, size_t bytes, const void** dev);
+
+// Device arrays of one call, freed on return.
+struct Temps {
+    gir_dev* g;
+    std::vector<void*> held;
+    template <class T>
+    int get(T** p, size_t n) {
+        GIR_TRY(dev_alloc_n(g, p, n));
+        held.push_back(*p);
+        return GIR_OK;
+    }
+    ~Temps() {
+        for (void* p : held) dev_free(g, p);
+    }
+};
 
 // Grid size for a persistent/grid-stride kernel.
 inline int grid_for(gir_dev* g, int64_t work, int block) {

@@ -88,8 +88,9 @@ int pinned(gir_dev* g, size_t bytes, void** out) {
         if (g->pinned) cudaFreeHost(g->pinned);
         g->pinned = nullptr;
         g->pinned_bytes = 0;
-        GIR_CUDA(g, cudaMallocHost(&g->pinned, bytes));
-        g->pinned_bytes = bytes;
+        const size_t want = bytes < kPinnedBytes ? kPinnedBytes : bytes;
+        GIR_CUDA(g, cudaMallocHost(&g->pinned, want));
+        g->pinned_bytes = want;
     }
     *out = g->pinned;
     return GIR_OK;

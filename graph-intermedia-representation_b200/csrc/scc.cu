@@ -10,6 +10,8 @@
 //     unassigned in- (or out-) neighbour form an SCC of two;
 //  2. forward-backward from a pivot of maximal out-degree x in-degree (the giant SCC of a
 //     power-law graph): SCC(pivot) = forward reach ∩ backward reach over unassigned vertices;
+//     (a reach that is still growing after deep_levels(V) levels gives way to the reciprocal classes
+//     of a mostly undirected graph and the SCCs of their small quotient, where it has them);
 //  3. colour propagation for the rest, repeated until every vertex is assigned: every
 //     unassigned vertex starts with its own id as colour, colours spread along forward edges
 //     by max until stable, so colour(v) = largest id that reaches v; a vertex r with
@@ -21,6 +23,8 @@
 //     (level, label) order, so rank(a) < rank(b) for every DAG edge a -> b (the invariant of
 //     scc_rank, gir.h:54-57).
 #include "common.cuh"
+#include "frontier.cuh"
+#include "unionfind.cuh"
 
 namespace gir {
 
@@ -147,59 +151,46 @@ __global__ void k_pivot(int64_t V, const int32_t* label, const int32_t* indeg, c
     }
 }
 
-// Edge-balanced reach from the pivot, both directions in one level-synchronous traversal: a
-// queue entry e >= 0 is vertex e searched forward (out-rows), e < 0 is vertex ~e searched
-// backward (in-rows). The frontier's rows are cut into equal chunks after a scan of their
-// lengths, so hubs do not serialize a warp. An unassigned w joins a direction once (mark bit 1
-// forward, 2 backward); afterwards the vertices with both bits are SCC(pivot). Paths inside the
-// pivot's SCC never pass through trimmed (already labelled) vertices, so restricting both searches
-// to unassigned vertices keeps FW ∩ BW exact.
-__global__ void k_frontier_deg(const int32_t* q, int64_t n, const int32_t* fdeg, const int32_t* bdeg, int64_t* pref) {
-    GRID_STRIDE(i, n) {
-        const int32_t e = q[i];
-        pref[i] = e >= 0 ? fdeg[e] : bdeg[~e];
+// Reach from the pivot, both directions in one level-synchronous traversal (frontier.cuh): a queue
+// entry e >= 0 is vertex e searched forward (out-rows), e < 0 is vertex ~e searched backward
+// (in-rows). An unassigned w joins a direction once (mark bit 1 forward, 2 backward; an assigned
+// vertex starts with both, so one load tells both apart); afterwards the unassigned vertices with
+// both bits are SCC(pivot). Paths inside the pivot's SCC never pass through trimmed (already labelled)
+// vertices, so restricting both searches to unassigned vertices keeps FW and BW exact.
+// Bound by the latency of the marks' random accesses; a level was a degree pass, a scan and a launch
+// whose warps took 512 edges each, so on a lattice four warps worked: 46 us a level, now about 8.
+struct ReachBoth {
+    CSRView fw, bw;
+    int32_t* mark;
+    __device__ __forceinline__ int32_t deg(int32_t e) const { return e >= 0 ? fw.deg[e] : bw.deg[~e]; }
+    __device__ __forceinline__ void row(int32_t e, int64_t& beg, unsigned long long& back) const {
+        back = e < 0;
+        beg = back ? bw.beg[~e] : fw.beg[e];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) pref[n] = 0;
-}
-
-constexpr int kReachChunk = 32 * 16;
-
-__global__ void __launch_bounds__(kBlock) k_reach_both(const int32_t* q, int64_t nq, const int64_t* pref, CSRView fw,
-                                                       CSRView bw, const int32_t* label, int32_t* mark, int32_t* out,
-                                                       unsigned long long* cnt) {
-    __shared__ int32_t s_st[kBlock / 32][kStage];
-    int n_st = 0;
-    const int64_t total = pref[nq];
-    const int lane = lane_id();
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t c0 = warp * kReachChunk; c0 < total; c0 += nwarps * kReachChunk) {
-        const int64_t c1 = c0 + kReachChunk < total ? c0 + kReachChunk : total;
-        const int64_t key = c0 + lane < total ? c0 + lane : total - 1;
-        int64_t lo = 0, hi = nq - 1;
-        while (lo < hi) {
-            const int64_t m = (lo + hi + 1) >> 1;
-            if (pref[m] <= key) lo = m; else hi = m - 1;
-        }
-        int64_t i = lo;
-        for (int64_t base = c0; base < c1; base += 32) {
-            const int64_t p = base + lane;
-            bool push = false;
-            int32_t ent = 0;
-            if (p < c1) {
-                while (pref[i + 1] <= p) ++i;
-                const int32_t e = q[i];
-                const bool back = e < 0;
-                const int32_t u = back ? ~e : e;
-                const int32_t w = back ? bw.adj[bw.beg[u] + (p - pref[i])] : fw.adj[fw.beg[u] + (p - pref[i])];
-                const int32_t bit = back ? 2 : 1;
-                if (label[w] == -1 && (mark[w] & bit) == 0) push = (atomicOr(&mark[w], bit) & bit) == 0;
-                ent = back ? ~w : w;
-            }
-            stage_append(push, ent, s_st[threadIdx.x >> 5], n_st, out, &cnt[C_Q]);
-        }
+    __device__ __forceinline__ int32_t adj(int64_t i, unsigned long long back) const {
+        return back ? bw.adj[i] : fw.adj[i];
     }
-    stage_flush(s_st[threadIdx.x >> 5], n_st, out, &cnt[C_Q]);
+    __device__ __forceinline__ unsigned long long want(int32_t w, unsigned long long back) const {
+        const int bit = back ? 2 : 1;
+        return __ldcg(mark + w) & bit ? 0ull : bit;
+    }
+    __device__ __forceinline__ bool apply(int32_t w, unsigned long long back, unsigned long long bit, int32_t& e) {
+        e = back ? ~w : w;
+        return (atomicOr(&mark[w], (int)bit) & (int)bit) == 0;
+    }
+};
+
+// Marks of the assigned vertices, and the pivot in both directions as the first frontier.
+__global__ void k_reach_init(int64_t V, const int32_t* label, int32_t pivot, CSRView fw, CSRView bw, int32_t* mark,
+                             Queue q, unsigned long long* ctl) {
+    GRID_STRIDE(v, V) mark[v] = label[v] != -1 || v == pivot ? 3 : 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        q.v[0] = pivot;
+        q.v[1] = ~pivot;
+        q.off[0] = 0;
+        q.off[1] = (uint64_t)fw.deg[pivot];
+        ctl[W_Q] = (2ull << kQShift) | (unsigned long long)((int64_t)fw.deg[pivot] + bw.deg[pivot]);
+    }
 }
 
 // SCC(pivot): the unassigned vertices reached both ways.
@@ -348,6 +339,95 @@ __global__ void k_rank_gather(int64_t V, const int32_t* label, const int32_t* ra
     GRID_STRIDE(v, V) rank[v] = rank_of[label[v]];
 }
 
+// ---- Reciprocal classes ------------------------------------------------------------------------
+// The ends of a reciprocal pair of edges (u -> v and v -> u) share an SCC. A vertex whose in- and
+// out-rows (without a self-loop) are as long as its symmetrized row has reciprocal edges only, so
+// that test per vertex finds them without a search per edge. Joining every such vertex with its
+// neighbours by union-find leaves, on a graph that is undirected or nearly so (a road network), a few
+// classes and only the edges between the other vertices; the SCCs of that small quotient graph are
+// the SCCs of the graph.
+__global__ void k_reciprocal(int64_t V, CSRView fw, CSRView bw, CSRView sym, uint8_t* full, int32_t* cls,
+                             unsigned long long* n_full) {
+    unsigned long long c = 0;
+    GRID_STRIDE(v, V) {
+        const int32_t o = fw.deg[v];
+        const int64_t fb = fw.beg[v];
+        const int64_t p = lower_bound_dev(fw.adj, fb, fb + o, (int32_t)v);
+        const int32_t self = p < fb + o && fw.adj[p] == (int32_t)v;
+        const bool f = o - self == sym.deg[v] && bw.deg[v] - self == sym.deg[v];
+        full[v] = f;
+        cls[v] = (int32_t)v;
+        c += f;
+    }
+    c = warp_sum_u64(c);
+    if (lane_id() == 0 && c) atomicAdd(n_full, c);
+}
+
+// Row lengths of the vertices with full[v] == want, 0 for the others.
+__global__ void k_mask_deg(int64_t V, const int32_t* deg, const uint8_t* full, int want, int32_t* out) {
+    GRID_STRIDE(v, V) out[v] = (full[v] != 0) == (want != 0) ? deg[v] : 0;
+}
+
+__global__ void __launch_bounds__(kBlock) k_class_link(int64_t V, CSRView sym, int32_t* cls, unsigned long long* err) {
+    __shared__ int64_t s_excl[kWarps][33];
+    __shared__ int32_t s_u[kWarps][32];
+    const int wib = threadIdx.x >> 5;
+    warp_sweep_rows(sym.beg, sym.deg, sym.adj, 0, V, s_excl[wib], s_u[wib],
+                    [&](int32_t u, int32_t w, int64_t) { uf_union(cls, u, w, err); });
+}
+
+__global__ void k_class_flatten(int64_t V, int32_t* cls) {
+    GRID_STRIDE(v, V) {
+        int32_t x = cls[v];
+        while (cls[x] != x) x = cls[x];
+        cls[v] = x;
+    }
+}
+
+// Keys (class(u) << 32 | class(w)) of the edges between classes; counted only while keys is null.
+__global__ void __launch_bounds__(kBlock) k_quotient_keys(int64_t V, CSRView fw, const int32_t* cls, uint64_t* keys,
+                                                          unsigned long long* n) {
+    __shared__ int64_t s_excl[kWarps][33];
+    __shared__ int32_t s_u[kWarps][32];
+    const int wib = threadIdx.x >> 5;
+    warp_sweep_rows(fw.beg, fw.deg, fw.adj, 0, V, s_excl[wib], s_u[wib], [&](int32_t u, int32_t w, int64_t) {
+        const int32_t a = cls[u], b = cls[w];
+        if (a == b) return;
+        const unsigned m = __activemask();  // (one atomic for the threads that are here together)
+        const int leader = __ffs(m) - 1;
+        unsigned long long at = 0;
+        if (lane_id() == leader) at = atomicAdd(n, (unsigned long long)__popc(m));
+        at = __shfl_sync(m, at, leader) + __popc(m & ((1u << lane_id()) - 1));
+        if (keys) keys[at] = ((uint64_t)(uint32_t)a << 32) | (uint32_t)b;
+    });
+}
+
+__global__ void k_flip_keys(const uint64_t* in, int64_t n, uint64_t* out) {
+    GRID_STRIDE(i, n) out[i] = (in[i] << 32) | (in[i] >> 32);
+}
+
+// Compact CSR of sorted keys.
+__global__ void k_keys_csr(const uint64_t* keys, int64_t n, int64_t V, int64_t* beg, int32_t* deg, int32_t* adj) {
+    GRID_STRIDE(v, V) {
+        const int64_t a = lower_bound_dev(keys, (int64_t)0, n, (uint64_t)v << 32);
+        beg[v] = a;
+        deg[v] = (int32_t)(lower_bound_dev(keys, a, n, ((uint64_t)v + 1) << 32) - a);
+    }
+    GRID_STRIDE(i, n) adj[i] = (int32_t)(keys[i] & 0xffffffffULL);
+}
+
+__global__ void k_quotient_labels(int64_t V, const int32_t* cls, const int32_t* qlabel, int32_t* label,
+                                  unsigned long long* n_classes) {
+    unsigned long long c = 0;
+    GRID_STRIDE(v, V) {
+        const int32_t l = qlabel ? qlabel[cls[v]] : cls[v];
+        label[v] = l;
+        c += l == (int32_t)v;
+    }
+    c = warp_sum_u64(c);
+    if (lane_id() == 0 && c) atomicAdd(n_classes, c);
+}
+
 struct Loop {
     gir_dev* g;
     unsigned long long* cnt;
@@ -362,9 +442,96 @@ struct Loop {
 
 }  // namespace
 
-int scc_labels(gir_dev* g, int32_t* label, int64_t* n_scc) {
+static int scc_labels(gir_dev* g, const CSRView fw, const CSRView bw, bool whole, int32_t* label, int64_t* n_scc);
+
+// SCC labels of the handle's graph through its reciprocal classes (above), where at least half of the
+// vertices have reciprocal edges only; *used says whether it was done.
+static int scc_by_quotient(gir_dev* g, int32_t* label, int64_t* n_scc, bool* used) {
     const int64_t V = g->V;
-    const CSRView fw = view(g->fw), bw = view(g->bw);
+    *used = false;
+    Temps t{g, {}};
+    uint8_t* full = nullptr;
+    int32_t *cls = nullptr, *mdeg = nullptr;
+    unsigned long long* cnt = nullptr;  // [0] full vertices, [1] union-find errors, [2] keys, [3] keys, [4] classes
+    GIR_TRY(t.get(&full, V));
+    GIR_TRY(t.get(&cls, V));
+    GIR_TRY(t.get(&mdeg, V));
+    GIR_TRY(t.get(&cnt, 8));
+    void* hp = nullptr;
+    GIR_TRY(pinned(g, 256, &hp));
+    unsigned long long* hc = static_cast<unsigned long long*>(hp);
+    auto read = [&]() -> int {
+        GIR_CUDA(g, cudaMemcpyAsync(hc, cnt, sizeof(unsigned long long) * 8, cudaMemcpyDeviceToHost, g->stream));
+        GIR_CUDA(g, cudaStreamSynchronize(g->stream));
+        return GIR_OK;
+    };
+    GIR_CUDA(g, cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * 8, g->stream));
+    k_reciprocal<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, view(g->fw), view(g->bw), view(g->sym), full, cls, cnt);
+    GIR_LAUNCH(g, "k_reciprocal");
+    GIR_TRY(read());
+    if ((int64_t)hc[0] * 2 < V) return GIR_OK;
+    CSRView sym = view(g->sym), fw = view(g->fw);
+    sym.deg = mdeg;
+    k_mask_deg<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, g->sym.deg, full, 1, mdeg);
+    GIR_LAUNCH(g, "k_mask_deg");
+    k_class_link<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, sym, cls, cnt + 1);
+    GIR_LAUNCH(g, "k_class_link");
+    k_class_flatten<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, cls);
+    GIR_LAUNCH(g, "k_class_flatten");
+    // (an edge between classes has two ends that are not full)
+    fw.deg = mdeg;
+    k_mask_deg<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, g->fw.deg, full, 0, mdeg);
+    GIR_LAUNCH(g, "k_mask_deg");
+    k_quotient_keys<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, fw, cls, nullptr, cnt + 2);
+    GIR_LAUNCH(g, "k_quotient_keys");
+    GIR_TRY(read());
+    if (hc[1]) return fail(g, GIR_ERR_TIMEOUT, "scc: union-find exceeded its retry bound");
+    const int64_t n = (int64_t)hc[2];
+    int32_t* qlabel = nullptr;
+    if (n > 0) {
+        uint64_t *keys = nullptr, *flip = nullptr, *tmp = nullptr;
+        uint8_t* flag = nullptr;
+        GIR_TRY(t.get(&keys, n));
+        GIR_TRY(t.get(&flip, n));
+        GIR_TRY(t.get(&tmp, n));
+        GIR_TRY(t.get(&flag, n));
+        k_quotient_keys<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, fw, cls, keys, cnt + 3);
+        GIR_LAUNCH(g, "k_quotient_keys");
+        GIR_TRY(sort_keys_u64(g, keys, tmp, n, 64));
+        k_distinct_u64<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(keys, n, flag);
+        GIR_LAUNCH(g, "k_distinct_u64");
+        int64_t m = 0;
+        GIR_TRY(select_flagged_u64(g, keys, flag, tmp, n, &m));
+        k_flip_keys<<<grid_for(g, m, kBlock), kBlock, 0, g->stream>>>(tmp, m, flip);
+        GIR_LAUNCH(g, "k_flip_keys");
+        GIR_TRY(sort_keys_u64(g, flip, keys, m, 64));
+        int64_t* beg[2];
+        int32_t *deg[2], *adj[2];
+        for (int i = 0; i < 2; ++i) {
+            GIR_TRY(t.get(&beg[i], V));
+            GIR_TRY(t.get(&deg[i], V));
+            GIR_TRY(t.get(&adj[i], m));
+            k_keys_csr<<<grid_for(g, V > m ? V : m, kBlock), kBlock, 0, g->stream>>>(i ? flip : tmp, m, V, beg[i], deg[i],
+                                                                                   adj[i]);
+            GIR_LAUNCH(g, "k_keys_csr");
+        }
+        GIR_TRY(t.get(&qlabel, V));
+        int64_t n_q = 0;
+        GIR_TRY(scc_labels(g, CSRView{beg[0], deg[0], adj[0], nullptr}, CSRView{beg[1], deg[1], adj[1], nullptr}, false,
+                           qlabel, &n_q));
+    }
+    // (class roots and SCC labels are smallest members: the composition is canonical)
+    k_quotient_labels<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, cls, qlabel, label, cnt + 4);
+    GIR_LAUNCH(g, "k_quotient_labels");
+    GIR_TRY(read());
+    *n_scc = (int64_t)hc[4];
+    *used = true;
+    return GIR_OK;
+}
+
+// SCC labels of the graph with rows fw / bw; `whole`: it is the handle's graph.
+static int scc_labels(gir_dev* g, const CSRView fw, const CSRView bw, bool whole, int32_t* label, int64_t* n_scc) {
+    const int64_t V = g->V;
     int32_t *indeg = nullptr, *outdeg = nullptr, *qa = nullptr, *qb = nullptr, *mark = nullptr, *color = nullptr;
     unsigned long long* cnt = nullptr;
     GIR_TRY(ensure_n(g, g->scratch[0], V + 1, &indeg));
@@ -434,7 +601,6 @@ int scc_labels(gir_dev* g, int32_t* label, int64_t* n_scc) {
 
     trace_mark(g, "scc: trim");
     // 2. forward-backward from the max-degree pivot
-    GIR_CUDA(g, cudaMemsetAsync(mark, 0, sizeof(int32_t) * V, g->stream));
     GIR_CUDA(g, cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * C_N, g->stream));
     k_pivot<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, label, indeg, outdeg, 0, cnt);
     GIR_LAUNCH(g, "k_pivot");
@@ -452,9 +618,11 @@ int scc_labels(gir_dev* g, int32_t* label, int64_t* n_scc) {
             rule = 0;
             if (g->schedule == GIR_SCHEDULE_LEARNED && g->sched_loaded) GIR_TRY(sched_choose_pivot(g, feat, &rule));
         }
-        g->trace_x.clear();
-        g->trace_y.clear();
-        sched_trace(g, feat, 8 + rule);
+        if (whole) {
+            g->trace_x.clear();
+            g->trace_y.clear();
+            sched_trace(g, feat, 8 + rule);
+        }
     }
     if (rule == 1 || rule == 2) {
         GIR_CUDA(g, cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * C_N, g->stream));
@@ -465,24 +633,23 @@ int scc_labels(gir_dev* g, int32_t* label, int64_t* n_scc) {
     }
     if (rule != 3 && lp.hc[C_PIV] != 0) {
         const int32_t pivot = (int32_t)((lp.hc[C_PIV] - 1) & 0xffffffffULL);
-        // both searches seeded with the pivot (marked both ways)
-        int32_t *fa = qa, *fb = qb;
-        int64_t* pref = nullptr;
-        GIR_TRY(ensure_n(g, g->scratch[7], 2 * V + 2, &pref));
-        const int32_t seed[2] = {pivot, ~pivot}, both = 3;
-        GIR_CUDA(g, cudaMemcpyAsync(mark + pivot, &both, sizeof(int32_t), cudaMemcpyHostToDevice, g->stream));
-        GIR_CUDA(g, cudaMemcpyAsync(fa, seed, sizeof(seed), cudaMemcpyHostToDevice, g->stream));
-        GIR_CUDA(g, cudaStreamSynchronize(g->stream));  // (seed is a host stack array)
-        int64_t n = 2;
-        while (n > 0) {
-            k_frontier_deg<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(fa, n, fw.deg, bw.deg, pref);
-            GIR_LAUNCH(g, "k_frontier_deg");
-            GIR_TRY(exclusive_scan_i64(g, pref, pref, n + 1));
-            GIR_CUDA(g, cudaMemsetAsync(&cnt[C_Q], 0, sizeof(unsigned long long), g->stream));
-            k_reach_both<<<grid, kBlock, 0, g->stream>>>(fa, n, pref, fw, bw, label, mark, fb, cnt);
-            GIR_LAUNCH(g, "k_reach_both");
-            std::swap(fa, fb);
-            GIR_TRY(lp.read(&n));
+        // both searches start from the pivot (marked both ways)
+        Queue q{qa, nullptr};
+        unsigned long long* ctl = nullptr;
+        GIR_TRY(ensure_n(g, g->scratch[7], 2 * V + 2, &q.off));
+        GIR_TRY(ensure_n(g, g->scratch[10], kLoopWords, &ctl));
+        GIR_CUDA(g, cudaMemsetAsync(ctl, 0, sizeof(unsigned long long) * kLoopWords, g->stream));
+        k_reach_init<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, label, pivot, fw, bw, mark, q, ctl);
+        GIR_LAUNCH(g, "k_reach_init");
+        const ReachBoth op{fw, bw, mark};
+        FrontierRun run;
+        GIR_TRY(run_frontier(g, op, q, ctl, run, whole ? deep_levels(V) : INT64_MAX));
+        if (!run.done()) {
+            bool used = false;
+            GIR_TRY(scc_by_quotient(g, label, n_scc, &used));
+            trace_mark(g, "scc: reciprocal classes");
+            if (used) return GIR_OK;
+            GIR_TRY(run_frontier(g, op, q, ctl, run, INT64_MAX));
         }
         k_reach_label<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, mark, pivot, label);
         GIR_LAUNCH(g, "k_reach_label");
@@ -535,7 +702,7 @@ int scc_build(gir_dev* g) {
     const int64_t V = g->V;
     int32_t* label = nullptr;
     GIR_TRY(ensure_n(g, g->scc, V + 1, &label));
-    GIR_TRY(scc_labels(g, label, &g->n_scc));
+    GIR_TRY(scc_labels(g, view(g->fw), view(g->bw), true, label, &g->n_scc));
     trace_mark(g, "scc: labels");
     return scc_build_dag(g);
 }

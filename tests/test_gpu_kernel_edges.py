@@ -76,3 +76,56 @@ def test_bfs_of_a_graph_whose_bottom_up_levels_leave_the_launch(pkg, orc):
         assert 0 < st["persistent_levels"] < st["iterations"]
         assert (st["bottom_up"] > 0) == (alpha > 1)
     d.close()
+
+
+def _deep_shapes():
+    """(name, V, u, v): graphs whose searches run past the level counts at which the builds change to the
+    reciprocal classes (SCC) and to the forest without levels (blocks), and just below them."""
+    rng = np.random.default_rng(3)
+    for n in (24, 25, 26, 64, 65, 66, 129, 700):  # paths: eccentricity n - 1 from the smallest vertex
+        a = np.arange(n - 1)
+        yield f"path {n}", n, np.r_[a, a + 1], np.r_[a + 1, a]
+    side = 90
+    at = np.arange(side * side).reshape(side, side)
+    a = np.r_[at[:, :-1].ravel(), at[:-1, :].ravel()]
+    b = np.r_[at[:, 1:].ravel(), at[1:, :].ravel()]
+    keep = rng.random(len(a)) > 0.25  # holes: bridges, small components, many blocks
+    a, b = a[keep], b[keep]
+    V = side * side
+    perm = rng.permutation(V)
+    yield "lattice", V, perm[np.r_[a, b]], perm[np.r_[b, a]]
+    # one-way streets: classes joined into one SCC by one-way cycles, others left one-way between SCCs
+    one = rng.random(len(a)) < 0.3
+    yield "one-way", V, perm[np.r_[a, b[~one]]], perm[np.r_[b, a[~one]]]
+    extra = rng.integers(0, V, (2, 60))
+    loops = rng.integers(0, V, 50)
+    yield "one-way, long range, loops", V, np.r_[perm[np.r_[a, b[~one]]], extra[0], loops], np.r_[
+        perm[np.r_[b, a[~one]]], extra[1], loops]
+    n = 2000  # two long reciprocal paths joined by one-way edges both ways (one SCC), a third only one way
+    p = np.arange(n - 1)
+    parts = [(p + k * n, p + 1 + k * n) for k in range(3)]
+    u = np.concatenate([np.r_[x, y] for x, y in parts] + [[5, n + 900, 2 * n + 7]])
+    v = np.concatenate([np.r_[y, x] for x, y in parts] + [[n + 3, 1500, 12]])
+    yield "joined paths", 3 * n, u, v
+    c = np.arange(1500)  # directed rings sharing single vertices, a hub with every tenth vertex
+    yield "rings", 4500, np.r_[c, c + 1500, 1500 * 2 + c, c[::10], np.full(150, 7)], np.r_[
+        (c + 1) % 1500, np.where(c == 1499, 0, c + 1501), 3000 + (c + 1) % 1500, np.full(150, 7), c[::10]]
+
+
+def test_layers_of_deep_graphs(pkg, orc):
+    from test_gpu_layers import _oracle_match
+    for name, V, u, v in _deep_shapes():
+        keep = (u != v) | ("loops" in name)
+        g = _graph(pkg, V, u[keep], v[keep])
+        fb, fa = orc.normalize(V, g.fw_beg, g.fw_adj)
+        d = pkg.DeviceGraph.from_graph(g, weights=False)
+        d.build()
+        _oracle_match(pkg, orc, d, V, fb, fa, name)
+        if V > 1000:  # one-way inserts and deletions: fewer vertices with reciprocal edges only
+            for step in range(2):
+                cb, ca = d.csr(0)
+                bu, bv, ins = pkg.graphs.updates(pkg.graphs.Graph(V, cb.astype(np.int32), ca, None, None), 40, 40, 9 + step)
+                d.apply_batch(bu, bv, ins)
+                fb, fa, _, _ = orc.apply_batch(V, fb, fa, bu, bv, ins)
+                _oracle_match(pkg, orc, d, V, fb, fa, f"{name}, batch {step}")
+        d.close()
