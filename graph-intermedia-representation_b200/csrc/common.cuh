@@ -147,10 +147,11 @@ struct gir_dev {
     gir::DevBuf stage_in, stage_out;  // device staging for host pointers
     gir::DevBuf work[8];              // buffers of the create / batch pipelines (not used by store ops)
     gir::DevBuf lane_dist;            // lane-interleaved SSSP distances (V x lanes)
-    gir::DevBuf qitems[5];            // per-queue-entry work items of the SSSP relaxation
+    gir::DevBuf qitems[5];            // SSSP: queue offsets and the row records
     gir::DevBuf sssp_sets;            // SSSP: every set's source range and lane-order key
     gir::DevBuf sssp_lanes;           // SSSP: one lane group's source ranges and output rows
     gir::DevBuf sssp_done;            // SSSP: per vertex, the lanes whose distance is final
+    gir::DevBuf sssp_ctl;             // SSSP: counters and the state of the bucket loop
     void* pinned = nullptr;           // small pinned host buffer for counters
     size_t pinned_bytes = 0;
 

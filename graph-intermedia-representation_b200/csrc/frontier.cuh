@@ -73,14 +73,14 @@ __device__ __forceinline__ void queue_flush(int32_t* s_buf, int& s_n, const Queu
     s_n = 0;
 }
 
-// Staged append (warp-uniform call): collects in shared memory, one reservation per kStage entries.
-template <class Deg>
+// Staged append (warp-uniform call): collects in shared memory, one reservation per kSlots entries.
+template <int kSlots = kStage, class Deg>
 __device__ __forceinline__ void queue_push(bool pred, int32_t v, int32_t* s_buf, int& s_n, const Queue& q, const Deg& deg,
                                            unsigned long long* cnt) {
     const unsigned m = __ballot_sync(0xffffffffu, pred);
     if (!m) return;
     const int k = __popc(m);
-    if (s_n + k > kStage) queue_flush(s_buf, s_n, q, deg, cnt);
+    if (s_n + k > kSlots) queue_flush(s_buf, s_n, q, deg, cnt);
     if (pred) s_buf[s_n + __popc(m & ((1u << lane_id()) - 1))] = v;
     __syncwarp();
     s_n += k;
@@ -134,9 +134,9 @@ __device__ __forceinline__ void block_publish(LevelShared<kWarps>& sh, const int
     }
 }
 
-// Largest i in [0, n) with off[i] <= key (off[0] = 0): one warp, 32 probes a round.
-__device__ __forceinline__ int64_t queue_find(const uint64_t* off, int64_t n, uint64_t key) {
-    int64_t lo = 0, hi = n - 1;
+// Largest i in [lo, n) with off[i] <= key (off[lo] <= key): one warp, 32 probes a round.
+__device__ __forceinline__ int64_t queue_find(const uint64_t* off, int64_t lo, int64_t n, uint64_t key) {
+    int64_t hi = n - 1;
     while (hi > lo) {
         const int64_t step = (hi - lo + 31) / 32;
         const int64_t i = lo + (int64_t)(lane_id() + 1) * step;
@@ -218,7 +218,7 @@ __device__ __forceinline__ void walk_level(const Queue& q, int64_t nq, int64_t t
     run = run < kRun ? run : kRun;
     for (int64_t c0 = warp * run; c0 < total; c0 += nwarps * run) {
         const int64_t c1 = c0 + run < total ? c0 + run : total;
-        walk_rows(q, nq, total, c0, c1, queue_find(q.off, nq, (uint64_t)c0), op, out, cnt, s_buf, s_n);
+        walk_rows(q, nq, total, c0, c1, queue_find(q.off, 0, nq, (uint64_t)c0), op, out, cnt, s_buf, s_n);
     }
 }
 

@@ -3,8 +3,8 @@
 //
 // Up to 64 queries run as one traversal (lanes), like the BFS: every vertex carries 64-bit lane
 // masks for the work of the current bucket (near), for relaxations beyond it (far) and for the
-// lanes settled in the bucket; distances are stored lane-interleaved (dist[v * lanes + s]) so a
-// warp relaxing one edge for many lanes touches one contiguous row. All lanes step through the
+// lanes settled in the bucket; distances are stored lane-interleaved (dist[v * ld + s]) so a
+// relaxation of one edge for many lanes touches one contiguous row. All lanes step through the
 // buckets together, each lane running exact Delta-stepping:
 //  - bucket k = [k*Delta, (k+1)*Delta): the near vertices relax their light edges
 //    (weight < Delta) round after round until no lane re-enters the bucket;
@@ -18,6 +18,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "frontier.cuh"
 
 namespace gir {
 
@@ -29,12 +30,15 @@ constexpr uint64_t kInf = ~0ull;
 #define GRID_STRIDE(i, n) \
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (n); i += (int64_t)gridDim.x * blockDim.x)
 
-// counters: [0] next near queue length, [1] far queue length, [2] settled queue length,
-// [3] min live far distance, [4] far queue length after a split, [5] relaxation items,
-// [6] set when a 16-bit lane distance could not hold a tentative distance;
-// accumulated over the call: [16] reached (vertex, lane) pairs, [17] their out-edges
-enum { S_NEAR = 0, S_FAR = 1, S_SET = 2, S_MIN = 3, S_FAR2 = 4, S_ITEMS = 5, S_OVF = 6, S_REACHED = 16, S_EDGES = 17,
-       S_N = 32 };
+// Device words of a call. Counters that one phase reads and a later one fills come in threes, used in
+// turn (a slot is cleared while no phase can touch it): the near queues (entries << 33 | their light
+// edges), the far queue's entries, the smallest distance a far split kept.
+// X_SET: the settled queue (entries << 33 | their heavy edges); X_OVF: set when a 16-bit lane distance
+// could not hold a tentative distance; X_PHASE .. X_PASSES: where the buckets stand (Bucket);
+// X_REACHED, X_EDGES: accumulated over the call, reached (vertex, lane) pairs and their out-edges;
+// X_TMP: scratch of the lane order; X_BAR: the loop's grid barrier (its own 128-byte line).
+enum { X_NEAR = 0, X_SET = 3, X_FAR = 4, X_MIN = 7, X_OVF = 10, X_ERR = 11, X_PHASE = 12, X_LO, X_ROT, X_SPL, X_FQ,
+       X_NCLEAR, X_NSETCLEAR, X_PASSES, X_GROUP = 24, X_REACHED = 24, X_EDGES = 25, X_TMP = 26, X_BAR = 32, X_N = 64 };
 
 // Sort keys (row << 32 | weight) and columns of every entry of the compact copy of `c`. For the
 // forward CSR the weight of entry (u, v) is that of edge u -> v. With `reverse` the rows are
@@ -95,21 +99,6 @@ __global__ void k_deg_i64(int64_t V, const int32_t* deg, int64_t* out) {
     if (blockIdx.x == 0 && threadIdx.x == 0) out[V] = 0;
 }
 
-// Lane s of the group starts at every vertex of srcs[lane_rng[2s] .. lane_rng[2s + 1]) (one
-// CTA row per lane: blockIdx.y = s).
-template <class D>
-__global__ void k_sssp_init(const int64_t* lane_rng, const int32_t* srcs, int64_t V, int nl, D* dist,
-                            unsigned long long* nearmask, int32_t* nearq, unsigned long long* cnt) {
-    const int s = blockIdx.y;
-    const int64_t lo = lane_rng[2 * s], hi = lane_rng[2 * s + 1];
-    for (int64_t e = lo + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < hi; e += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t v = srcs[e];
-        if (v < 0 || v >= V) continue;
-        dist[(int64_t)v * nl + s] = 0;
-        if (atomicOr(&nearmask[v], 1ull << s) == 0ull) nearq[atomicAdd(&cnt[S_NEAR], 1ull)] = v;
-    }
-}
-
 // Distances inside a lane group are uint32 when every finite distance fits ((V - 1) * max weight
 // < 2^32 - 1): half the bytes, eight lanes per 32-byte sector, 32-bit atomics. Output is uint64.
 template <class D>
@@ -117,14 +106,14 @@ struct DistT;
 template <>
 struct DistT<uint64_t> {
     static constexpr uint64_t inf = ~0ull;
-    __device__ static uint64_t atomic_min(uint64_t* p, uint64_t v) {
-        return atomicMin((unsigned long long*)p, (unsigned long long)v);
-    }
+    using acc = uint64_t;  // what tentative distances are added up in
+    __device__ static void atomic_min(uint64_t* p, uint64_t v) { atomicMin((unsigned long long*)p, (unsigned long long)v); }
 };
 template <>
 struct DistT<uint32_t> {
     static constexpr uint32_t inf = ~0u;
-    __device__ static uint32_t atomic_min(uint32_t* p, uint32_t v) { return atomicMin((unsigned int*)p, v); }
+    using acc = uint32_t;
+    __device__ static void atomic_min(uint32_t* p, uint32_t v) { atomicMin((unsigned int*)p, v); }
 };
 // 16-bit lane distances (64 lanes in one 128-byte line) when the distances are small: the
 // minimum is taken by compare-and-swap on the aligned 32-bit word holding the lane. Every failed
@@ -132,67 +121,60 @@ struct DistT<uint32_t> {
 template <>
 struct DistT<uint16_t> {
     static constexpr uint16_t inf = 0xffffu;
-    __device__ static uint16_t atomic_min(uint16_t* p, uint16_t v) {
+    using acc = uint32_t;
+    __device__ static void atomic_min(uint16_t* p, uint16_t v) {
         const uintptr_t a = reinterpret_cast<uintptr_t>(p);
         unsigned int* wp = reinterpret_cast<unsigned int*>(a & ~(uintptr_t)3);
         const int sh = (a & 2) ? 16 : 0;
         unsigned int old = *(volatile unsigned int*)wp;
         while (true) {
             const uint16_t cur = (uint16_t)(old >> sh);
-            if (cur <= v) return cur;
+            if (cur <= v) return;
             const unsigned int nw = (old & ~(0xffffu << sh)) | ((unsigned int)v << sh);
             const unsigned int prev = atomicCAS(wp, old, nw);
-            if (prev == old) return cur;
+            if (prev == old) return;
             old = prev;
         }
     }
 };
 
-// Index of the k-th set bit of a 64-bit mask (k < popcount).
-__device__ __forceinline__ int nth_bit(uint64_t m, int k) {
-    const unsigned lo = (unsigned)m;
-    const int cl = __popc(lo);
-    if (k < cl) return __fns(lo, 0, k + 1);
-    return 32 + __fns((unsigned)(m >> 32), 0, k - cl + 1);
+// Sixteen bytes of a distance row: kVec neighbouring lanes. Rows are padded to a multiple of it (`ld`;
+// a single lane is not), so they can be read this way.
+template <class D>
+struct alignas(16) Vec {
+    static constexpr int n = 16 / sizeof(D);
+    D v[n];
+};
+// Past the L1 (kCg) or through it.
+template <bool kCg, class D>
+__device__ __forceinline__ Vec<D> load_vec(const D* p) {
+    const uint4 r = kCg ? __ldcg(reinterpret_cast<const uint4*>(p)) : *reinterpret_cast<const uint4*>(p);
+    return *reinterpret_cast<const Vec<D>*>(&r);
 }
 
-struct Relax {
-    const int64_t* wb;       // weight-sorted rows (compact offsets)
-    const int32_t* wdeg;
-    const int32_t* wadj;
-    const uint32_t* ww;
-    uint64_t delta, kend;    // bucket width; end of the current bucket
-    int nl;                  // lanes (row stride of dist)
-    void* dist;              // lane distances (uint32 or uint64, see DistT)
-    unsigned long long* curmask;   // lanes of each queued vertex to process (read and cleared)
-    unsigned long long* nextmask;  // lanes re-entering the bucket
-    int32_t* nextq;
-    unsigned long long* farmask;
-    int32_t* farq;
-    unsigned long long* setmask;   // lanes settled in this bucket
-    int32_t* setq;
-    // Lanes whose distance is final: those settled in buckets whose light phase is over (their
-    // heavy pass ORs them in). k_far_split drops such lanes from the far set without reading
-    // their distances. (k_relax does not test it: on R-MAT graphs the extra 8-byte load per edge
-    // cost more than the distance reads and atomics it saved.)
-    unsigned long long* done;
-    unsigned long long* cnt;
-};
+// OR over the eight threads of a row group.
+__device__ __forceinline__ unsigned long long or8(unsigned long long x) {
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) x |= __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
 
-// Work-balanced relaxation: k_relax_prep turns the queue into items (one per vertex with work),
-// an exclusive scan of the items' work (edges x lanes) numbers all (edge, lane) pairs, and
-// k_relax processes them in equal runs, so a hub with many lanes is spread over the grid.
-struct Items {
-    int32_t* u;
-    int64_t* eb;
-    unsigned long long* m;
-    int64_t* pref;  // work per item, then its exclusive scan (n + 1 entries)
-};
+// Staged append to a far queue (warp-uniform call).
+template <int kSlots>
+__device__ __forceinline__ void far_push(bool pred, int32_t v, int32_t* s_buf, int& s_n, int32_t* q,
+                                         unsigned long long* cnt) {
+    const unsigned m = __ballot_sync(0xffffffffu, pred);
+    if (!m) return;
+    const int k = __popc(m);
+    if (s_n + k > kSlots) stage_flush(s_buf, s_n, q, cnt);
+    if (pred) s_buf[s_n + __popc(m & ((1u << lane_id()) - 1))] = v;
+    __syncwarp();
+    s_n += k;
+}
 
-// Number of light edges (weight < delta) of every weight-sorted row, once per query group.
-// Written with it, one 16-byte record per vertex for the queue bookkeeping of every pass: the
-// row start (two halves), its length and its light-edge count, so a queued vertex costs one
-// scattered load instead of three.
+// One 16-byte record per vertex for every queue entry a pass handles: the start of its weight-sorted
+// row (two halves), its length and its light edges (weight < delta), which are the row's prefix. Once
+// per query group.
 __global__ void k_light_split(int64_t V, const int64_t* wb, const int32_t* wdeg, const uint32_t* ww, uint64_t delta,
                               int4* rows) {
     GRID_STRIDE(v, V) {
@@ -207,340 +189,542 @@ __global__ void k_light_split(int64_t V, const int64_t* wb, const int32_t* wdeg,
     }
 }
 
-// Takes every queued vertex's lanes (clearing them), does the settle bookkeeping and writes queue
-// entry i's item (vertex, first edge, lane mask, work = edges x lanes) into slot i; cnt[S_ITEMS]
-// = n and pref[n] = 0, so the scan of the n + 1 slots needs nothing cleared beforehand (and the
-// near-queue counter starts the pass at zero). Items
-// without work stay in place: the relaxation's searches take the largest item whose prefix is at
-// most the pair's index, which is never a zero-work item (its prefix equals the next item's).
-// A vertex is queued once per pass, so its setmask word is touched by one thread only.
-__global__ void k_relax_prep(const int32_t* q, int64_t n, int heavy, Relax a, const int4* rows, Items it) {
-    __shared__ int s_w[kBlock / 32];
-    __shared__ unsigned long long s_base;
-    for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t i = base + threadIdx.x;
-        int32_t u = 0;
-        unsigned long long m = 0;
-        int64_t eb = 0, work = 0;
-        bool settles = false;
-        if (i < n) {
-            // (every load of the vertex's words is issued before any store: the stores may alias
-            // them for all the compiler knows, and would otherwise serialize three DRAM latencies)
-            u = q[i];
-            const int4 r = rows[u];
-            if (heavy) {
-                m = a.setmask[u];
-                const unsigned long long dn = a.done[u];
-                a.setmask[u] = 0ull;
-                a.done[u] = dn | m;  // (u appears once in a heavy pass)
-            } else {
-                m = a.curmask[u];
-                const unsigned long long old = a.setmask[u];
-                a.curmask[u] = 0ull;
-                a.setmask[u] = old | m;
-                settles = m && old == 0ull;
-            }
-            const int64_t b = (int64_t)(((uint64_t)(uint32_t)r.y << 32) | (uint32_t)r.x);
-            const int32_t nlu = r.w;
-            eb = heavy ? b + nlu : b;
-            work = (int64_t)(heavy ? r.z - nlu : nlu) * __popcll(m);
-            it.u[i] = u;
-            it.eb[i] = eb;
-            it.m[i] = m;
-            it.pref[i] = work;
-        }
-        const unsigned long long ss = block_slot(settles, &a.cnt[S_SET], s_w, &s_base);
-        if (settles) a.setq[ss] = u;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        it.pref[n] = 0;
-        a.cnt[S_ITEMS] = (unsigned long long)n;
-        a.cnt[S_NEAR] = 0ull;  // the pass's near appends count from zero (the host read the last count)
-    }
+__device__ __forceinline__ int64_t row_start(const int4& r) {
+    return (int64_t)(((uint64_t)(uint32_t)r.y << 32) | (uint32_t)r.x);
 }
 
-constexpr int kRelaxThreads = 256;
-// Pairs per thread per step, and CTAs per SM: latency-bound, so occupancy wins. Measured on the
-// 4.8M-vertex R-MAT (64 lanes): 1 pair at 8 CTAs (32 registers) 71 ms per call, 7 CTAs the same,
-// 6 CTAs 75 ms, 4 CTAs 83 ms; 2 pairs at 6 CTAs 74 ms, at 5 CTAs 76 ms. (With the later changes:
-// 256-thread CTAs 66.3 ms, 128-thread CTAs at 16 per SM 66.8 ms.)
-constexpr int kPairs = 1;
-constexpr int kRelaxMinBlocks = 8;
-constexpr int kDeal = 8;  // chunks of pairs per warp and launch, at least 32 pairs each (measured on
-                          // the 4.8M-vertex R-MAT: 4 or 8 68.4 ms per call, 16 69.5, 32 72.0)
-
-// Largest e in [lo, hi] with pref[e] <= key, for a non-decreasing pref with pref[lo] <= key
-// (the probes at or below the key are a prefix of each round's 32). One warp, 32 probes a round:
-// the window shrinks 32-fold per dependent load.
-__device__ __forceinline__ int64_t warp_search(const int64_t* pref, int64_t lo, int64_t hi, int64_t key) {
-    const int ln = lane_id();
-    while (hi > lo) {
-        const int64_t step = (hi - lo + 31) / 32;
-        const int64_t p = lo + (int64_t)(ln + 1) * step;
-        const bool c = p <= hi && pref[p] <= key;
-        const int t = __popc(__ballot_sync(0xffffffffu, c));
-        if (t > 0) lo += (int64_t)t * step;
-        hi = lo + step - 1 < hi ? lo + step - 1 : hi;
+// Light / heavy edges of a queued vertex (the lengths the queues' offsets add up).
+struct LightLen {
+    const int4* rows;
+    __device__ __forceinline__ int32_t operator()(int32_t v) const { return rows[v].w; }
+};
+struct HeavyLen {
+    const int4* rows;
+    __device__ __forceinline__ int32_t operator()(int32_t v) const {
+        const int4 r = rows[v];
+        return r.z - r.w;
     }
-    return lo;
-}
+};
 
-// Relaxes the pairs this thread holds (pair j: on[j], target w[j], lane sl[j], the source's lane
-// distance du[j], edge weight wt[j]); the queue appends are staged per warp (warp-uniform call).
+// The lane at position p of the group starts at every vertex of srcs[lane_rng[2p] .. lane_rng[2p + 1])
+// (one CTA row per lane: blockIdx.y = p).
 template <class D>
-__device__ __forceinline__ void relax_held(D* dist, const Relax& a, const bool (&on)[kPairs], const int32_t (&w)[kPairs],
-                                           const int32_t (&sl)[kPairs], const uint64_t (&du)[kPairs],
-                                           const uint32_t (&wt)[kPairs], int32_t* s_near, int& n_near, int32_t* s_far,
-                                           int& n_far) {
-    uint64_t cur[kPairs];
-#pragma unroll
-    for (int j = 0; j < kPairs; ++j)
-        cur[j] = on[j] ? *(volatile D*)&dist[(int64_t)w[j] * a.nl + sl[j]] : (D)0;
-#pragma unroll
-    for (int j = 0; j < kPairs; ++j) {
-        bool to_near = false, to_far = false;
-        if (on[j]) {
-            const uint64_t nd = du[j] + (uint64_t)wt[j];
-            if (sizeof(D) == 2 && nd >= (uint64_t)DistT<D>::inf) {
-                // a 16-bit lane cannot hold it: the group is run again with 32-bit lanes
-                if (cur[j] == (uint64_t)DistT<D>::inf) a.cnt[S_OVF] = 1ull;
-            } else if (nd < cur[j]) {  // plain pre-check: most relaxations lose
-                const uint64_t old = DistT<D>::atomic_min(&dist[(int64_t)w[j] * a.nl + sl[j]], (D)nd);
-                if (nd < old) {
-                    const unsigned long long bit = 1ull << sl[j];
-                    if (nd < a.kend) to_near = atomicOr(&a.nextmask[w[j]], bit) == 0ull;
-                    else to_far = atomicOr(&a.farmask[w[j]], bit) == 0ull;
-                }
-            }
+__global__ void k_sssp_init(const int64_t* lane_rng, const int32_t* srcs, int64_t V, int ld, D* dist,
+                            unsigned long long* mask, Queue q, const int4* rows, unsigned long long* cnt) {
+    __shared__ int32_t s_stage[kBlock / 32][kStage];
+    int32_t* s_buf = s_stage[threadIdx.x >> 5];
+    int n_st = 0;
+    const LightLen light{rows};
+    const int p = blockIdx.y;
+    const int64_t lo = lane_rng[2 * p], hi = lane_rng[2 * p + 1];
+    for (int64_t base = lo + blockIdx.x * (int64_t)blockDim.x; base < hi; base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t e = base + threadIdx.x;
+        const int32_t v = e < hi ? srcs[e] : -1;
+        bool on = false;
+        if (v >= 0 && v < V) {
+            dist[(int64_t)v * ld + p] = 0;
+            on = atomicOr(&mask[v], 1ull << p) == 0ull;
         }
-        stage_append(to_near, w[j], s_near, n_near, a.nextq, &a.cnt[S_NEAR]);
-        stage_append(to_far, w[j], s_far, n_far, a.farq, &a.cnt[S_FAR]);
+        queue_push(on, v, s_buf, n_st, q, light, cnt);
+    }
+    queue_flush(s_buf, n_st, q, light, cnt);
+}
+
+// What a group's passes work on. The near masks and queues rotate: a light pass reads one pair, fills
+// the next and clears the masks of the one before, so a queued vertex's mask can be read by every
+// warp that holds a piece of its row.
+struct Group {
+    const int4* rows;
+    const int32_t* wadj;          // weight-sorted rows
+    const uint32_t* ww;
+    uint64_t delta;
+    int nl, ld;                   // lanes, row stride of dist
+    void* dist;                   // lane distances (see DistT)
+    unsigned long long* mask[3];  // near lanes
+    Queue q[3];
+    unsigned long long* farmask;
+    int32_t* farq[2];             // filled by the passes, rewritten into the other one by a far split
+    unsigned long long* setmask;  // lanes settled in this bucket
+    Queue setq;
+    // Lanes whose distance is final: those settled in buckets whose light phase is over (their heavy
+    // pass ORs them in). A relaxation drops such lanes of its target without reading their distances,
+    // and so does the far split.
+    unsigned long long* done;
+    unsigned long long* ctl;
+};
+
+// Where the buckets stand: the phase to run next and the start of its bucket, which near queue (rot),
+// far counter (spl) and far queue (fq) it uses, and the entries of the last near queue and of the
+// settled queue whose masks are still to be cleared.
+enum { PH_LIGHT = 0, PH_HEAVY = 1, PH_SPLIT = 2, PH_DONE = 3 };
+struct Bucket {
+    int phase, rot, spl, fq;
+    uint64_t lo;
+    int64_t n_clear, n_setclear;
+    int64_t passes;  // light passes so far
+};
+
+// End of the bucket that holds `lo` (saturating).
+__host__ __device__ inline uint64_t bucket_end(uint64_t lo, uint64_t delta) {
+    const uint64_t b = lo / delta * delta;
+    return b + delta < b ? ~0ull : b + delta;
+}
+
+// The phase that follows, from the counters the phase left in ctl (rd reads a word).
+template <class Read>
+__host__ __device__ inline void next_phase(Bucket& s, uint64_t delta, int64_t entries, Read&& rd) {
+    if (s.phase == PH_LIGHT) {
+        s.n_clear = entries;
+        s.rot = (s.rot + 1) % 3;
+        ++s.passes;
+        if ((rd(X_NEAR + s.rot) >> kQShift) == 0) s.phase = PH_HEAVY;
+    } else if (s.phase == PH_HEAVY) {
+        s.n_clear = 0;
+        s.n_setclear = entries;
+        s.lo = bucket_end(s.lo, delta);
+        s.phase = rd(X_FAR + s.spl) != 0 ? PH_SPLIT : PH_DONE;
+    } else {
+        s.n_setclear = 0;
+        s.fq ^= 1;
+        s.rot = (s.rot + 1) % 3;
+        const unsigned long long least = rd(X_MIN + s.spl);
+        s.spl = (s.spl + 1) % 3;
+        if ((rd(X_NEAR + s.rot) >> kQShift) != 0) {
+            s.phase = PH_LIGHT;
+        } else if (least == kInf) {
+            s.phase = PH_DONE;
+        } else {
+            s.lo = least;  // an empty bucket: on to the one of the smallest distance still far
+        }
     }
 }
 
-// Load-balanced relaxation over all (edge, lane) pairs of the item list, numbered by the
-// exclusive scan of the items' work. Every warp takes one contiguous run of pairs and finds the
-// item holding its first pair with one warp search. It then walks windows of 32 consecutive
-// items, one item per lane in registers: a pair finds its item by a binary search over the
-// window through shuffles, so no shared memory and no block barrier is involved and warps
-// proceed independently. Pairs are enumerated edge-major within an item: with many lanes
-// active, consecutive threads update consecutive lanes of one distance row.
-//
-// Where the warp's next steps (32 * kPairs pairs each) all lie inside one item (a hub's row,
-// settled in many lanes at once: a few such items hold most of the pairs of the early heavy
-// passes), the warp leaves the per-pair search: each thread divides its first pair's rank once,
-// then steps its (edge, lane rank) position by the constant 32 * kPairs, and takes the lane from
-// a table of the item's set lanes held one per thread (two shuffles instead of a search, a divide
-// and a find-n-th-bit per pair). The pairs relaxed are the same either way.
-template <class D>
-__global__ void __launch_bounds__(kRelaxThreads, kRelaxMinBlocks) k_relax(const unsigned long long* n_items, Items it, Relax a) {
+// A warp's staged appends: near (or settled-next) entries, settled entries, far entries.
+struct Stage {
+    int32_t *near, *set, *far;
+    unsigned char* map;  // 64 slots: the threads that hold the live edges of a step (relax_edges)
+    int n_near, n_set, n_far;
+};
+
+// Lane distances are read past the L1 where other CTAs may have written them during this launch (kCg:
+// the bucket loop; a pass of its own starts with a clean L1).
+template <bool kCg, class D>
+__device__ __forceinline__ D load_dist(const D* p) {
+    return kCg ? __ldcg(p) : *p;
+}
+
+// Relaxes one edge per thread, u -> w of weight wt, in the lanes `need` (0: no edge), and queues what
+// improved. A warp takes the cheaper of two ways, by the work in front of it:
+//  - every thread steps through the lanes of its own edge (few lanes an edge);
+//  - eight threads take an edge, so four edges at once, each thread 16 bytes of the two distance rows at
+//    a time (many lanes an edge: the passes of a power-law graph, whose vertices are reached in most
+//    lanes at once). kU such steps are in flight: the rows come from L2 and HBM.
+// The minimum is taken without waiting for its result: a lane counts as improved by the plain read
+// before it. Where another thread lowered the lane in between, that thread queued it as well, and a far
+// entry that is no longer far is dropped by the far split, so the queues stay supersets of the lanes
+// whose distance changed. Either way an edge's improved lanes go out with one atomicOr per mask.
+constexpr int kThreadShare = 4;
+template <class D, bool kCg, bool kHeavy, int kSlots>
+__device__ __forceinline__ void relax_edges(const Group& a, uint64_t kend, int32_t u, int32_t w, uint32_t wt,
+                                            unsigned long long need, unsigned long long* next, const Queue& outq,
+                                            unsigned long long* near_cnt, int32_t* farq, unsigned long long* far_cnt,
+                                            Stage& st) {
+    using A = typename DistT<D>::acc;
+    const unsigned any = __ballot_sync(0xffffffffu, need != 0ull);
+    if (!any) return;
     D* const dist = static_cast<D*>(a.dist);
-    const int64_t n = (int64_t)*n_items;
-    if (n == 0) return;
-    const int64_t total = it.pref[n];
-    __shared__ int32_t s_near[kRelaxThreads / 32][kStage], s_far[kRelaxThreads / 32][kStage];
-    int32_t* const my_near = s_near[threadIdx.x >> 5];
-    int32_t* const my_far = s_far[threadIdx.x >> 5];
-    int n_near = 0, n_far = 0;
+    const A kend_a = kend < (uint64_t)(A)~(A)0 ? (A)kend : (A)~(A)0;
     const int ln = lane_id();
-    const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    constexpr int kStep = 32 * kPairs;
-    // The pairs are dealt in chunks, round-robin over the warps (about kDeal chunks per warp), so
-    // every warp gets a mix of cheap pairs (long items, the fast path below) and costly ones
-    // (short items): one contiguous run per warp left the warps inside short items running
-    // 1.75x longer than the average SM in the first heavy passes.
-    const int64_t chunk = (((total + nw * kDeal - 1) / (nw * kDeal)) + 31) & ~(int64_t)31;
-    int64_t e_from = 0;  // (a warp's chunks ascend: each search starts at the previous chunk's item)
-    for (int64_t c0 = gw * chunk; c0 < total; c0 += nw * chunk) {
-        const int64_t c1 = c0 + chunk < total ? c0 + chunk : total;
-        int64_t e0 = warp_search(it.pref, e_from, n - 1, c0);
-        e_from = e0;
+    unsigned long long near = 0, far = 0;
+    // takes one lane of a target from its tentative distance: 0 no gain, 1 near, 2 far
+    auto take = [&](D* at, A du, A dw, uint32_t weight) -> int {
+        const A nd = du + weight;
+        if (sizeof(D) == 2 && nd >= (A)DistT<D>::inf) {
+            // a 16-bit lane cannot hold it: the group is run again with 32-bit lanes
+            if (dw == (A)DistT<D>::inf) a.ctl[X_OVF] = 1ull;
+            return 0;
+        }
+        if (nd >= dw) return 0;  // (most relaxations lose)
+        DistT<D>::atomic_min(at, (D)nd);
+        return !kHeavy && nd < kend_a ? 1 : 2;
+    };
+    const int lanes_max = __reduce_max_sync(0xffffffffu, __popcll(need)), live = __popc(any);
+    if (a.ld == 1 || kThreadShare * lanes_max <= live) {
+        const D* du_row = dist + (int64_t)u * a.ld;
+        D* dw_row = dist + (int64_t)w * a.ld;
+        while (need) {
+            const int b0 = __ffsll((long long)need) - 1;
+            need &= need - 1;
+            const int b1 = need ? __ffsll((long long)need) - 1 : b0;
+            const bool two = need != 0ull;
+            need &= need - 1;
+            const A du0 = load_dist<kCg>(du_row + b0), dw0 = __ldcg(dw_row + b0);
+            A du1 = 0, dw1 = 0;
+            if (two) {
+                du1 = load_dist<kCg>(du_row + b1);
+                dw1 = __ldcg(dw_row + b1);
+            }
+            const int t0 = take(dw_row + b0, du0, dw0, wt), t1 = two ? take(dw_row + b1, du1, dw1, wt) : 0;
+            if (t0 == 1) near |= 1ull << b0;
+            if (t0 == 2) far |= 1ull << b0;
+            if (t1 == 1) near |= 1ull << b1;
+            if (t1 == 2) far |= 1ull << b1;
+        }
+    } else {
+        constexpr int kV = Vec<D>::n;
+        const int sub = ln >> 3, k = ln & 7;
+        const int rank = __popc(any & ((1u << ln) - 1));  // this thread's edge among the live ones
+        st.map[rank | (need ? 0 : 32)] = (unsigned char)ln;  // (dead edges write past the live ones)
+        __syncwarp();
+        for (int r0 = 0; r0 < live; r0 += 4) {
+            const bool on = r0 + sub < live;
+            const int src = on ? st.map[r0 + sub] : 0;
+            unsigned long long nj = __shfl_sync(0xffffffffu, need, src);
+            nj = on ? nj : 0ull;
+            const D* du_row = dist + (int64_t)__shfl_sync(0xffffffffu, u, src) * a.ld;
+            D* dw_row = dist + (int64_t)__shfl_sync(0xffffffffu, w, src) * a.ld;
+            const uint32_t weight = __shfl_sync(0xffffffffu, wt, src);
+            unsigned long long n = 0, f = 0;
+            for (int at = k * kV; at < a.ld; at += 8 * kV) {
+                const unsigned m = (unsigned)(nj >> at) & ((1u << kV) - 1);
+                if (!m) continue;
+                const Vec<D> du = load_vec<kCg>(du_row + at), dw = load_vec<true>(dw_row + at);
+                unsigned mn = 0, mf = 0;
+#pragma unroll
+                for (int e = 0; e < kV; ++e) {
+                    if ((m >> e) & 1u) {
+                        const int t = take(dw_row + at + e, du.v[e], dw.v[e], weight);
+                        mn |= (unsigned)(t & 1) << e;
+                        mf |= (unsigned)(t >> 1) << e;
+                    }
+                }
+                n |= (unsigned long long)mn << at;
+                f |= (unsigned long long)mf << at;
+            }
+            if (!__any_sync(0xffffffffu, (n | f) != 0ull)) continue;
+            // every edge's masks go to the thread that holds it
+            const int from = 8 * (rank & 3);
+            if (!kHeavy) n = __shfl_sync(0xffffffffu, or8(n), from);
+            f = __shfl_sync(0xffffffffu, or8(f), from);
+            if (need != 0ull && (rank & ~3) == r0) {
+                near = n;
+                far = f;
+            }
+        }
+        __syncwarp();  // (the map is rewritten by the next edges)
+    }
+    if (!__any_sync(0xffffffffu, (near | far) != 0ull)) return;
+    if (!kHeavy) {
+        const bool to_near = near != 0ull && atomicOr(&next[w], near) == 0ull;
+        queue_push<kSlots>(to_near, w, st.near, st.n_near, outq, LightLen{a.rows}, near_cnt);
+    }
+    const bool to_far = far != 0ull && atomicOr(&a.farmask[w], far) == 0ull;
+    far_push<kSlots>(to_far, w, st.far, st.n_far, farq, far_cnt);
+}
+
+// A warp's share of a pass over the queue's rows (light prefixes or heavy rests), cut into equal runs of
+// edges by the queue's offsets; `mask` holds every entry's lanes. The search for a run's first entry and
+// the shuffles that find an edge's entry are per edge, not per (edge, lane) pair.
+// The runs are dealt round-robin, about kDeal per warp and at most 512 edges long, so every warp gets a
+// mix of cheap edges (targets already final) and costly ones; a pass of fewer edges than threads is cut
+// finer than a warp's width, since an edge of many lanes is a chain of its own.
+constexpr int kDeal = 8;
+template <class D, bool kCg, bool kHeavy, int kSlots>
+__device__ __forceinline__ void relax_rows(const Group& a, const Bucket& b, const Queue& q, const unsigned long long* mask,
+                                           unsigned long long packed, int64_t warp, int64_t nwarps, Stage& st) {
+    const int64_t nq = (int64_t)(packed >> kQShift), total = (int64_t)(packed & kQEdges);
+    const uint64_t kend = bucket_end(b.lo, a.delta);
+    const int nx = (b.rot + 1) % 3;
+    const int ln = lane_id();
+    int64_t run = (total + nwarps - 1) / nwarps;
+    if (run > 32) run = ((total + nwarps * kDeal - 1) / (nwarps * kDeal) + 31) & ~(int64_t)31;
+    run = run < kRun ? run : kRun;
+    for (int64_t c0 = warp * run; c0 < total; c0 += nwarps * run) {
+        const int64_t c1 = c0 + run < total ? c0 + run : total;
+        int64_t i0 = queue_find(q.off, 0, nq, (uint64_t)c0);
         int64_t p = c0;
         while (p < c1) {
-            // window: items e0 .. e0+31, lane j holding item e0+j
-            const int64_t ej = e0 + ln;
-            int64_t pj = INT64_MAX, ebj = 0;
+            // 32 queue entries, one per thread: where its edges start in the run, its row, its lanes
+            const int64_t ij = i0 + ln;
+            uint32_t relj = 0xffffffffu;
+            int64_t begj = 0;
             unsigned long long mj = 0;
             int32_t uj = 0;
-            if (ej < n) {
-                pj = it.pref[ej];
-                ebj = it.eb[ej];
-                mj = it.m[ej];
-                uj = it.u[ej];
+            if (ij < nq) {
+                uj = __ldcg(q.v + ij);
+                const int64_t off = (int64_t)__ldcg((const unsigned long long*)q.off + ij) - c0;
+                relj = off <= 0 ? 0u : (off < 0x7fffffff ? (uint32_t)off : 0x7fffffffu);
+                const int4 r = a.rows[uj];
+                begj = row_start(r) + (kHeavy ? r.w : 0) - off;
+                mj = __ldcg(mask + uj);
             }
-            const int64_t wnext = e0 + 32 < n ? it.pref[e0 + 32] : total;
+            const int64_t wnext = i0 + 32 < nq ? (int64_t)__ldcg((const unsigned long long*)q.off + i0 + 32) : total;
             const int64_t wend = wnext < c1 ? wnext : c1;
-            while (p < wend) {
-                {
-                    // the item holding pair p (the same for every thread) and where its run ends
-                    int x = 0;
-    #pragma unroll
-                    for (int b = 16; b; b >>= 1) {
-                        const int64_t v = __shfl_sync(0xffffffffu, pj, x + b);
-                        if (v <= p) x += b;
-                    }
-                    const int64_t pn = __shfl_sync(0xffffffffu, pj, (x + 1) & 31);
-                    const int64_t xend = x < 31 ? (pn < wend ? pn : wend) : wend;
-                    if (xend - p >= 2 * kStep) {
-                        const int64_t px = __shfl_sync(0xffffffffu, pj, x);
-                        const int64_t ebx = __shfl_sync(0xffffffffu, ebj, x);
-                        const unsigned long long mx = __shfl_sync(0xffffffffu, mj, x);
-                        const int64_t urow = (int64_t)__shfl_sync(0xffffffffu, uj, x) * a.nl;
-                        const int pc = __popcll(mx);
-                        const int32_t sel_lo = ln < pc ? nth_bit(mx, ln) : 0;
-                        const int32_t sel_hi = ln + 32 < pc ? nth_bit(mx, ln + 32) : 0;
-                        const int da = kStep / pc, db = kStep % pc;
-                        int64_t e[kPairs];  // the pair's entry of the weight-sorted rows (ebx + edge)
-                        int r[kPairs];
-    #pragma unroll
-                        for (int j = 0; j < kPairs; ++j) {
-                            const int64_t q2 = p + j * 32 + ln - px;
-                            const int64_t ed = q2 / pc;
-                            r[j] = (int)(q2 - ed * pc);
-                            e[j] = ebx + ed;
-                        }
-                        for (; p + kStep <= xend; p += kStep) {
-                            bool on[kPairs];
-                            int32_t w[kPairs], sl[kPairs];
-                            uint64_t du[kPairs];
-                            uint32_t wt[kPairs];
-    #pragma unroll
-                            for (int j = 0; j < kPairs; ++j) {
-                                const int32_t lo = __shfl_sync(0xffffffffu, sel_lo, r[j] & 31);
-                                const int32_t hi = __shfl_sync(0xffffffffu, sel_hi, r[j] & 31);
-                                sl[j] = r[j] < 32 ? lo : hi;
-                                on[j] = true;
-                                w[j] = __ldcs(&a.wadj[e[j]]);
-                                wt[j] = __ldcs(&a.ww[e[j]]);
-                                du[j] = dist[urow + sl[j]];
-                                e[j] += da;
-                                r[j] += db;
-                                if (r[j] >= pc) {
-                                    r[j] -= pc;
-                                    e[j] += 1;
-                                }
-                            }
-                            relax_held<D>(dist, a, on, w, sl, du, wt, my_near, n_near, my_far, n_far);
-                        }
-                        continue;  // (what is left of the item, under one step, goes the general way)
-                    }
+            for (; p < wend; p += 32) {
+                const int64_t pos = p + ln;
+                const uint32_t rel = (uint32_t)(pos - c0);
+                int x = 0;
+#pragma unroll
+                for (int s = 16; s; s >>= 1)
+                    if (__shfl_sync(0xffffffffu, relj, x + s) <= rel) x += s;
+                const int64_t bx = __shfl_sync(0xffffffffu, begj, x);
+                unsigned long long need = __shfl_sync(0xffffffffu, mj, x);
+                const int32_t u = __shfl_sync(0xffffffffu, uj, x);
+                int32_t w = 0;
+                uint32_t wt = 0;
+                if (pos < wend) {
+                    w = __ldcs(a.wadj + bx + rel);
+                    wt = __ldcs(a.ww + bx + rel);
+                    if (a.nl > 1) need &= ~__ldcg(a.done + w);
+                } else {
+                    need = 0;
                 }
-                int32_t w[kPairs], sl[kPairs];
-                int64_t k[kPairs];
-                uint64_t du[kPairs];
-                bool on[kPairs];
-    #pragma unroll
-                for (int j = 0; j < kPairs; ++j) {
-                    const int64_t q = p + j * 32 + ln;
-                    on[j] = q < wend;
-                    int x = 0;  // largest x with pref(x) <= q
-    #pragma unroll
-                    for (int b = 16; b; b >>= 1) {
-                        const int64_t v = __shfl_sync(0xffffffffu, pj, x + b);
-                        if (v <= q) x += b;
-                    }
-                    const int64_t px = __shfl_sync(0xffffffffu, pj, x);
-                    const int64_t ebx = __shfl_sync(0xffffffffu, ebj, x);
-                    const unsigned long long mx = __shfl_sync(0xffffffffu, mj, x);
-                    const int32_t ux = __shfl_sync(0xffffffffu, uj, x);
-                    if (on[j]) {
-                        const int pc = __popcll(mx);
-                        const int64_t q2 = q - px;
-                        // (an item of 2^31 pairs or more, a row of over 2^25 entries, takes the wide divide)
-                        const int64_t ed = q2 <= INT32_MAX ? (int64_t)((uint32_t)q2 / (uint32_t)pc) : q2 / pc;
-                        k[j] = ebx + ed;
-                        sl[j] = nth_bit(mx, (int)(q2 - ed * pc));
-                        du[j] = dist[(int64_t)ux * a.nl + sl[j]];
-                    }
-                }
-                uint32_t wt[kPairs];
-    #pragma unroll
-                for (int j = 0; j < kPairs; ++j) {
-                    if (on[j]) { w[j] = __ldcs(&a.wadj[k[j]]); wt[j] = __ldcs(&a.ww[k[j]]); } else { w[j] = 0; wt[j] = 0; }
-                }
-                relax_held<D>(dist, a, on, w, sl, du, wt, my_near, n_near, my_far, n_far);
-                p += kStep;
+                relax_edges<D, kCg, kHeavy, kSlots>(a, kend, u, w, wt, need, a.mask[nx], a.q[nx], a.ctl + X_NEAR + nx,
+                                                    a.farq[b.fq], a.ctl + X_FAR + b.spl, st);
             }
-            p = wend;  // (the pairs of this window end exactly where item e0+32 begins)
+            p = wend;
             if (p >= c1) break;
-            // Items without work keep their slots (their prefix equals the next item's): where the
-            // whole next window is such items, jump past the run with one search instead of
-            // walking it 32 items at a time (a heavy pass on a lattice can hold millions of them).
-            const int64_t nx = e0 + 32;
-            e0 = nx + 32 < n && it.pref[nx + 32] <= p ? warp_search(it.pref, nx, n - 1, p) : nx;
+            i0 += 32;
+            // Entries without edges keep their slots (a road network's settled queue holds a heavy edge
+            // in every thousandth): where the next window has none, jump past the run of such entries.
+            if (i0 + 32 < nq && (int64_t)__ldcg((const unsigned long long*)q.off + i0 + 32) <= p)
+                i0 = queue_find(q.off, i0 + 32, nq, (uint64_t)p);
         }
     }
-    stage_flush(my_near, n_near, a.nextq, &a.cnt[S_NEAR]);
-    stage_flush(my_far, n_far, a.farq, &a.cnt[S_FAR]);
 }
 
-// Splits the far entries at the bucket [lo, hi): lanes inside it become near work, later lanes
-// stay far (queued in farq2) and their smallest distance goes to cnt[S_MIN] (the bucket to jump
-// to when this one turns out empty); settled lanes are dropped.
-template <class D>
-__global__ void k_far_split(const int32_t* farq, const unsigned long long* nfar, unsigned long long* farmask,
-                            const D* dist, int nl, uint64_t lo, uint64_t hi, unsigned long long* nearmask,
-                            int32_t* nearq, int32_t* farq2, const unsigned long long* done, unsigned long long* cnt) {
-    const int64_t n = (int64_t)*nfar;
-    __shared__ int32_t s_near[kBlock / 32][kStage], s_far[kBlock / 32][kStage];
-    int n_near = 0, n_far = 0;
-    const int ln = lane_id();
-    for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t i = base + threadIdx.x;
+// A light pass: the near lanes relax their light edges; lanes entering the bucket are settled.
+template <class D, bool kCg, int kSlots>
+__device__ __forceinline__ void phase_light(const Group& a, const Bucket& b, unsigned long long packed, int64_t tid,
+                                            int64_t nthreads, int64_t warp, int64_t nwarps, Stage& st) {
+    const int64_t nq = (int64_t)(packed >> kQShift);
+    const Queue& q = a.q[b.rot];
+    const unsigned long long* mask = a.mask[b.rot];
+    const int old = (b.rot + 2) % 3;
+    if (tid == 0) a.ctl[X_NEAR + old] = 0ull;
+    for (int64_t i = tid; i < b.n_clear; i += nthreads) a.mask[old][__ldcg(a.q[old].v + i)] = 0ull;
+    for (int64_t base = tid & ~(int64_t)31; base < nq; base += nthreads) {
+        const int64_t i = base + lane_id();
+        int32_t u = 0;
+        bool settles = false;
+        if (i < nq) {  // (a vertex is queued once per pass: its settled mask is this thread's)
+            u = __ldcg(q.v + i);
+            const unsigned long long m = __ldcg(mask + u), s = __ldcg(a.setmask + u);
+            if (m & ~s) a.setmask[u] = s | m;
+            settles = m != 0ull && s == 0ull;
+        }
+        queue_push<kSlots>(settles, u, st.set, st.n_set, a.setq, HeavyLen{a.rows}, a.ctl + X_SET);
+    }
+    relax_rows<D, kCg, false, kSlots>(a, b, q, mask, packed, warp, nwarps, st);
+}
+
+// The heavy pass of a bucket: its settled lanes are final and relax their heavy edges once, into later
+// buckets only. (A target lane that becomes final while this runs was settled in this bucket too, so no
+// heavy edge improves it: it does not matter whether the relaxation sees its bit.)
+template <class D, bool kCg, int kSlots>
+__device__ __forceinline__ void phase_heavy(const Group& a, const Bucket& b, unsigned long long packed, int64_t tid,
+                                            int64_t nthreads, int64_t warp, int64_t nwarps, Stage& st) {
+    const int64_t nset = (int64_t)(packed >> kQShift);
+    const int old = (b.rot + 2) % 3;
+    for (int64_t i = tid; i < b.n_clear; i += nthreads) a.mask[old][__ldcg(a.q[old].v + i)] = 0ull;
+    for (int64_t i = tid; i < nset; i += nthreads) {
+        const int32_t u = __ldcg(a.setq.v + i);
+        a.done[u] = __ldcg(a.done + u) | __ldcg(a.setmask + u);
+    }
+    relax_rows<D, kCg, true, kSlots>(a, b, a.setq, a.setmask, packed, warp, nwarps, st);
+}
+
+// Splits the far entries at the bucket of b.lo: lanes inside it become near work, later lanes stay far
+// (queued in the other far queue) and their smallest distance goes to X_MIN (the bucket to jump to when
+// this one turns out empty); settled lanes are dropped. n: the far entries.
+template <class D, bool kCg, int kSlots>
+__device__ __forceinline__ void phase_split(const Group& a, const Bucket& b, int64_t n, int64_t tid, int64_t nthreads,
+                                            Stage& st) {
+    const D* dist = static_cast<const D*>(a.dist);
+    const uint64_t lo = b.lo / a.delta * a.delta, hi = bucket_end(b.lo, a.delta);
+    const int nx = (b.rot + 1) % 3, ln = lane_id();
+    if (tid == 0) {
+        a.ctl[X_NEAR + (b.rot + 2) % 3] = 0ull;
+        a.ctl[X_FAR + (b.spl + 2) % 3] = 0ull;
+        a.ctl[X_MIN + (b.spl + 1) % 3] = kInf;
+        a.ctl[X_SET] = 0ull;
+    }
+    for (int64_t i = tid; i < b.n_setclear; i += nthreads) a.setmask[__ldcg(a.setq.v + i)] = 0ull;
+    unsigned long long mn = kInf;
+    for (int64_t base = tid & ~(int64_t)31; base < n; base += nthreads) {
+        const int64_t i = base + ln;
         int32_t w = 0;
         unsigned long long m = 0;
         if (i < n) {
-            w = farq[i];
+            w = __ldcg(a.farq[b.fq] + i);
             // (lanes already final were reached by a shorter path since: dropped unread)
-            m = farmask[w] & ~done[w];
+            m = __ldcg(a.farmask + w) & ~__ldcg(a.done + w);
         }
-        // The warp takes its 32 entries in turn and reads each entry's distance row once, lanes
-        // ln and ln + 32 per thread (coalesced); ballots give the entry's near and kept lanes.
-        unsigned long long mn = kInf, my_near = 0, my_keep = 0;
-#pragma unroll 4
-        for (int j = 0; j < 32; ++j) {
-            const unsigned long long mj = __shfl_sync(0xffffffffu, m, j);
-            if (mj == 0ull) continue;  // (warp-uniform)
-            const int64_t row = (int64_t)__shfl_sync(0xffffffffu, w, j) * nl;
-            bool n0 = false, n1 = false, k0 = false, k1 = false;
-            if ((mj >> ln) & 1ull) {
-                const uint64_t d = dist[row + ln];
-                n0 = d >= lo && d < hi;
-                k0 = d >= hi;
-                if (k0) mn = d < mn ? d : mn;
+        // Eight threads take an entry, so four at once, 16 bytes of its distance row per thread.
+        unsigned long long my_near = 0, my_keep = 0;
+        constexpr int kV = Vec<D>::n;
+        const int sub = ln >> 3, k = ln & 7;
+#pragma unroll 2
+        for (int j0 = 0; j0 < 32; j0 += 4) {
+            const unsigned long long mj = __shfl_sync(0xffffffffu, m, j0 + sub);
+            if (!__any_sync(0xffffffffu, mj != 0ull)) continue;
+            const D* row = dist + (int64_t)__shfl_sync(0xffffffffu, w, j0 + sub) * a.ld;
+            unsigned long long nm = 0, kp = 0;
+            for (int at = k * kV; at < a.ld; at += 8 * kV) {
+                const unsigned mk = (unsigned)(mj >> at) & ((1u << kV) - 1);
+                if (!mk) continue;
+                Vec<D> d;
+                if (a.ld == 1) d.v[0] = load_dist<kCg>(row);
+                else d = load_vec<kCg>(row + at);
+#pragma unroll
+                for (int e = 0; e < kV; ++e) {
+                    const uint64_t x = d.v[e];
+                    if (!((mk >> e) & 1u) || x < lo) continue;
+                    if (x < hi) {
+                        nm |= 1ull << (at + e);
+                    } else {
+                        kp |= 1ull << (at + e);
+                        mn = x < mn ? x : mn;
+                    }
+                }
             }
-            if ((mj >> 32 >> ln) & 1ull) {
-                const uint64_t d = dist[row + 32 + ln];
-                n1 = d >= lo && d < hi;
-                k1 = d >= hi;
-                if (k1) mn = d < mn ? d : mn;
-            }
-            const unsigned long long nm = (unsigned long long)__ballot_sync(0xffffffffu, n0) |
-                                          ((unsigned long long)__ballot_sync(0xffffffffu, n1) << 32);
-            const unsigned long long kp = (unsigned long long)__ballot_sync(0xffffffffu, k0) |
-                                          ((unsigned long long)__ballot_sync(0xffffffffu, k1) << 32);
-            if (ln == j) {
+            nm = __shfl_sync(0xffffffffu, or8(nm), 8 * (ln & 3));
+            kp = __shfl_sync(0xffffffffu, or8(kp), 8 * (ln & 3));
+            if ((ln & ~3) == j0) {
                 my_near = nm;
                 my_keep = kp;
             }
         }
-        bool to_near = false, to_far = false;
         if (i < n) {
-            farmask[w] = my_keep;
-            to_far = my_keep != 0ull;
-            if (my_near) to_near = atomicOr(&nearmask[w], my_near) == 0ull;
+            a.farmask[w] = my_keep;
+            if (my_near) a.mask[nx][w] = my_near;
         }
-        stage_append(to_near, w, s_near[threadIdx.x >> 5], n_near, nearq, &cnt[S_NEAR]);
-        stage_append(to_far, w, s_far[threadIdx.x >> 5], n_far, farq2, &cnt[S_FAR2]);
-        for (int o = 16; o; o >>= 1) {
-            const unsigned long long t = __shfl_xor_sync(0xffffffffu, mn, o);
-            mn = t < mn ? t : mn;
-        }
-        if (ln == 0 && mn != kInf) atomicMin(&cnt[S_MIN], mn);
+        queue_push<kSlots>(my_near != 0ull, w, st.near, st.n_near, a.q[nx], LightLen{a.rows}, a.ctl + X_NEAR + nx);
+        far_push<kSlots>(my_keep != 0ull, w, st.far, st.n_far, a.farq[b.fq ^ 1], a.ctl + X_FAR + (b.spl + 1) % 3);
     }
-    stage_flush(s_near[threadIdx.x >> 5], n_near, nearq, &cnt[S_NEAR]);
-    stage_flush(s_far[threadIdx.x >> 5], n_far, farq2, &cnt[S_FAR2]);
+    for (int o = 16; o; o >>= 1) {
+        const unsigned long long t = __shfl_xor_sync(0xffffffffu, mn, o);
+        mn = t < mn ? t : mn;
+    }
+    if (ln == 0 && mn != kInf) atomicMin(&a.ctl[X_MIN + b.spl], mn);
+}
+
+// ---- A phase launched from the host ------------------------------------------------------------
+// Bound by the latency of the distance rows' accesses, so occupancy counts: six CTAs an SM (40 registers)
+// 16.1 ms a call of 64 sources on the 4.8M-vertex R-MAT, four CTAs (64 registers) 16.6. Pairs of edge and
+// lane dealt one to a thread, numbered by a scan, had taken 26.4 of 35 ms: about 140 instructions a pair
+// to find it, and every pair's distance read; now final lanes are dropped by one mask per edge (8 of 10
+// edges of the heavy passes have none left) and a row of 64 lanes costs about 20 instructions.
+constexpr int kPassThreads = 256;
+
+template <class D, int kPhase>
+__global__ void __launch_bounds__(kPassThreads, 6) k_relax(Group a, Bucket b) {
+    constexpr int kWarpsPer = kPassThreads / 32;
+    __shared__ int32_t s_near[kWarpsPer][kStage], s_set[kWarpsPer][kStage], s_far[kWarpsPer][kStage];
+    const int wib = threadIdx.x >> 5;
+    __shared__ unsigned char s_map[kWarpsPer][64];
+    Stage st{s_near[wib], s_set[wib], s_far[wib], s_map[wib], 0, 0, 0};
+    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nthreads = (int64_t)gridDim.x * blockDim.x;
+    const int nx = (b.rot + 1) % 3;
+    if (kPhase == PH_LIGHT) phase_light<D, false, kStage>(a, b, a.ctl[X_NEAR + b.rot], tid, nthreads, tid >> 5, nthreads >> 5, st);
+    if (kPhase == PH_HEAVY) phase_heavy<D, false, kStage>(a, b, a.ctl[X_SET], tid, nthreads, tid >> 5, nthreads >> 5, st);
+    if (kPhase == PH_SPLIT) phase_split<D, false, kStage>(a, b, (int64_t)a.ctl[X_FAR + b.spl], tid, nthreads, st);
+    if (kPhase != PH_HEAVY) queue_flush(st.near, st.n_near, a.q[nx], LightLen{a.rows}, a.ctl + X_NEAR + nx);
+    if (kPhase == PH_LIGHT) queue_flush(st.set, st.n_set, a.setq, HeavyLen{a.rows}, a.ctl + X_SET);
+    const int fq = kPhase == PH_SPLIT ? b.fq ^ 1 : b.fq, spl = kPhase == PH_SPLIT ? (b.spl + 1) % 3 : b.spl;
+    stage_flush(st.far, st.n_far, a.farq[fq], a.ctl + X_FAR + spl);
+}
+
+// ---- The bucket loop ---------------------------------------------------------------------------
+// Phase after phase in one cooperative launch (a CTA of 1,024 threads per SM, one grid barrier a phase)
+// while the phases are small: on a road network, or for a single source, a pass has a few thousand
+// edges and was four launches and a host read. It hands back when a pass has more than max_edges edges
+// or the far queue more than max_far entries; the host launches such a phase at full occupancy and
+// comes back. Bound by latency, about 17 us a pass: 16 sources on a 901 x 901 lattice (1,600 passes)
+// 71 -> 25 ms, one source on 65,536 vertices 4.4 -> 1.5 ms.
+constexpr int kLoopSlots = 64;
+constexpr int kMaxPhases = 1 << 23;  // of one launch (its barrier's counter is 32 bits wide)
+
+template <class D>
+__global__ void __launch_bounds__(kLoopThreads, 1) k_bucket_loop(Group a, int64_t max_edges, int64_t max_far) {
+    __shared__ int32_t s_near[32][kLoopSlots], s_set[32][kLoopSlots], s_far[32][kLoopSlots];
+    __shared__ unsigned char s_map[32][64];
+    __shared__ uint32_t s_n[3][32];
+    __shared__ uint64_t s_e[2][32];
+    __shared__ unsigned long long s_base[3];
+    unsigned int* bar = reinterpret_cast<unsigned int*>(a.ctl + X_BAR);
+    const int wib = threadIdx.x >> 5, ln = lane_id();
+    // (warps and threads numbered across the CTAs first, so that a short queue spreads over the SMs)
+    const int64_t warp = (int64_t)wib * gridDim.x + blockIdx.x, nwarps = (int64_t)gridDim.x * 32;
+    const int64_t tid = warp * 32 + ln, nthreads = nwarps * 32;
+    auto rd = [&](int i) { return __ldcg(a.ctl + i); };
+    Bucket b{(int)rd(X_PHASE), (int)rd(X_ROT), (int)rd(X_SPL), (int)rd(X_FQ), rd(X_LO), (int64_t)rd(X_NCLEAR),
+             (int64_t)rd(X_NSETCLEAR), (int64_t)rd(X_PASSES)};
+    for (int ph = 0; ph < kMaxPhases && b.phase != PH_DONE; ++ph) {
+        Stage st{s_near[wib], s_set[wib], s_far[wib], s_map[wib], 0, 0, 0};
+        const int nx = (b.rot + 1) % 3;
+        int64_t entries = 0;
+        int fq = b.fq, spl = b.spl;
+        if (b.phase == PH_LIGHT) {
+            const unsigned long long packed = rd(X_NEAR + b.rot);
+            if ((int64_t)(packed & kQEdges) > max_edges) break;
+            entries = (int64_t)(packed >> kQShift);
+            phase_light<D, true, kLoopSlots>(a, b, packed, tid, nthreads, warp, nwarps, st);
+        } else if (b.phase == PH_HEAVY) {
+            const unsigned long long packed = rd(X_SET);
+            if ((int64_t)(packed & kQEdges) > max_edges) break;
+            entries = (int64_t)(packed >> kQShift);
+            phase_heavy<D, true, kLoopSlots>(a, b, packed, tid, nthreads, warp, nwarps, st);
+        } else {
+            entries = (int64_t)rd(X_FAR + b.spl);
+            if (entries > max_far) break;
+            fq ^= 1;
+            spl = (spl + 1) % 3;
+            phase_split<D, true, kLoopSlots>(a, b, entries, tid, nthreads, st);
+        }
+        // the CTA's staged entries go out with one reservation per queue
+        const uint64_t e_near = staged_edges(st.near, st.n_near, LightLen{a.rows});
+        const uint64_t e_set = staged_edges(st.set, st.n_set, HeavyLen{a.rows});
+        if (ln == 0) {
+            s_n[0][wib] = (uint32_t)st.n_near;
+            s_n[1][wib] = (uint32_t)st.n_set;
+            s_n[2][wib] = (uint32_t)st.n_far;
+            s_e[0][wib] = e_near;
+            s_e[1][wib] = e_set;
+        }
+        __syncthreads();
+        if (wib < 3) {  // warp 0 near, warp 1 settled, warp 2 far
+            const uint32_t n = s_n[wib][ln];
+            const uint64_t e = wib < 2 ? s_e[wib][ln] : 0ull;
+            const uint64_t n_in = warp_incl_u64(n), e_in = warp_incl_u64(e);
+            s_n[wib][ln] = (uint32_t)n_in - n;
+            if (wib < 2) s_e[wib][ln] = e_in - e;
+            if (ln == 31) {
+                unsigned long long* c = a.ctl + (wib == 0 ? X_NEAR + nx : wib == 1 ? X_SET : X_FAR + spl);
+                s_base[wib] = n_in ? atomicAdd(c, wib < 2 ? ((unsigned long long)n_in << kQShift) | e_in : n_in) : 0ull;
+            }
+        }
+        __syncthreads();
+        if (st.n_near)
+            queue_write(st.near, st.n_near, a.q[nx], LightLen{a.rows}, (s_base[0] >> kQShift) + s_n[0][wib],
+                        (s_base[0] & kQEdges) + s_e[0][wib]);
+        if (st.n_set)
+            queue_write(st.set, st.n_set, a.setq, HeavyLen{a.rows}, (s_base[1] >> kQShift) + s_n[1][wib],
+                        (s_base[1] & kQEdges) + s_e[1][wib]);
+        for (int i = ln; i < st.n_far; i += 32) a.farq[fq][s_base[2] + s_n[2][wib] + i] = st.far[i];
+        if (!grid_barrier(bar, a.ctl + X_ERR, kLoopSpins)) return;
+        next_phase(b, a.delta, entries, rd);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.ctl[X_PHASE] = (unsigned long long)b.phase;
+        a.ctl[X_ROT] = (unsigned long long)b.rot;
+        a.ctl[X_SPL] = (unsigned long long)b.spl;
+        a.ctl[X_FQ] = (unsigned long long)b.fq;
+        a.ctl[X_LO] = b.lo;
+        a.ctl[X_NCLEAR] = (unsigned long long)b.n_clear;
+        a.ctl[X_NSETCLEAR] = (unsigned long long)b.n_setclear;
+        a.ctl[X_PASSES] = (unsigned long long)b.passes;
+    }
 }
 
 // Reached (vertex, lane) pairs and their out-degrees (the traversed edges of the GTEPS figure).
@@ -559,16 +743,16 @@ __global__ void k_sssp_reached(const D* dist, int64_t V, int nl, const int32_t* 
         e += __shfl_xor_sync(0xffffffffu, e, o);
     }
     if (lane_id() == 0) {
-        if (r) atomicAdd(&cnt[S_REACHED], r);
-        if (e) atomicAdd(&cnt[S_EDGES], e);
+        if (r) atomicAdd(&cnt[X_REACHED], r);
+        if (e) atomicAdd(&cnt[X_EDGES], e);
     }
 }
 
-// dist[v * nl + s] -> out[row[s] * V + v], through 32 x 32 shared-memory tiles, a fixed grid
+// dist[v * ld + s] -> out[row[s] * V + v], through 32 x 32 shared-memory tiles, a fixed grid
 // striding over the tiles. On the way it counts what k_sssp_reached counts (reached (vertex, lane)
 // pairs and their out-edges) from the same coalesced loads, with one atomicAdd per CTA.
 template <class D>
-__global__ void k_transpose(const D* dist, int64_t V, int nl, const int64_t* row, const int32_t* outdeg,
+__global__ void k_transpose(const D* dist, int64_t V, int nl, int ld, const int64_t* row, const int32_t* outdeg,
                             uint64_t* out, unsigned long long* cnt) {
     __shared__ uint64_t tile[32][33];
     __shared__ unsigned long long s_r[8], s_e[8];
@@ -582,7 +766,7 @@ __global__ void k_transpose(const D* dist, int64_t V, int nl, const int64_t* row
             const int64_t v = v0 + r;
             const int s = s0 + tx;
             if (v < V && s < nl) {
-                const D d = dist[v * nl + s];
+                const D d = dist[v * ld + s];
                 const bool fin = d != DistT<D>::inf;
                 tile[r][tx] = fin ? (uint64_t)d : kInf;
                 if (fin) {
@@ -614,8 +798,8 @@ __global__ void k_transpose(const D* dist, int64_t V, int nl, const int64_t* row
             rr += s_r[k];
             ee += s_e[k];
         }
-        if (rr) atomicAdd(&cnt[S_REACHED], rr);
-        if (ee) atomicAdd(&cnt[S_EDGES], ee);
+        if (rr) atomicAdd(&cnt[X_REACHED], rr);
+        if (ee) atomicAdd(&cnt[X_EDGES], ee);
     }
 }
 
@@ -706,41 +890,64 @@ namespace {
 
 // Working arrays of one SSSP call, sized for V vertices and up to 64 lanes.
 struct Work {
-    int32_t *nearq, *nextq, *farq, *farq2, *setq;
-    unsigned long long *curmask, *nextmask, *farmask, *setmask, *done, *cnt;
+    Group a;
     int4* rows;
-    Items items;
-    unsigned long long* hc;  // pinned host copy of the counters
+    unsigned long long *ctl, *hc;  // device words (X_*), their pinned host copy
 };
 
 int sssp_work(gir_dev* g, Work& w) {
     const int64_t V = g->V;
-    GIR_TRY(ensure_n(g, g->scratch[0], V + 1, &w.nearq));
-    GIR_TRY(ensure_n(g, g->scratch[1], V + 1, &w.nextq));
-    GIR_TRY(ensure_n(g, g->scratch[2], V + 1, &w.farq));
-    GIR_TRY(ensure_n(g, g->scratch[3], V + 1, &w.farq2));
-    GIR_TRY(ensure_n(g, g->scratch[4], V + 1, &w.setq));
-    GIR_TRY(ensure_n(g, g->scratch[5], V + 1, &w.curmask));
-    GIR_TRY(ensure_n(g, g->scratch[6], V + 1, &w.nextmask));
-    GIR_TRY(ensure_n(g, g->scratch[7], V + 1, &w.farmask));
-    GIR_TRY(ensure_n(g, g->scratch[12], V + 1, &w.setmask));
-    GIR_TRY(ensure_n(g, g->sssp_done, V + 1, &w.done));
-    GIR_TRY(ensure_n(g, g->scratch[13], S_N, &w.cnt));
+    Group& a = w.a;
+    const int mask_slots[3] = {5, 6, 13}, q_slots[3] = {0, 1, 14};
+    for (int i = 0; i < 3; ++i) {
+        GIR_TRY(ensure_n(g, g->scratch[mask_slots[i]], V + 1, &a.mask[i]));
+        GIR_TRY(ensure_n(g, g->scratch[q_slots[i]], V + 1, &a.q[i].v));
+        GIR_TRY(ensure_n(g, g->qitems[i], V + 1, &a.q[i].off));
+    }
+    GIR_TRY(ensure_n(g, g->scratch[2], V + 1, &a.farq[0]));
+    GIR_TRY(ensure_n(g, g->scratch[3], V + 1, &a.farq[1]));
+    GIR_TRY(ensure_n(g, g->scratch[4], V + 1, &a.setq.v));
+    GIR_TRY(ensure_n(g, g->qitems[4], V + 1, &a.setq.off));
+    GIR_TRY(ensure_n(g, g->scratch[7], V + 1, &a.farmask));
+    GIR_TRY(ensure_n(g, g->scratch[12], V + 1, &a.setmask));
+    GIR_TRY(ensure_n(g, g->sssp_done, V + 1, &a.done));
     GIR_TRY(ensure_n(g, g->qitems[3], V + 1, &w.rows));
-    GIR_TRY(ensure_n(g, g->qitems[0], V + 1, &w.items.u));
-    GIR_TRY(ensure_n(g, g->qitems[1], V + 1, &w.items.eb));
-    GIR_TRY(ensure_n(g, g->qitems[2], V + 1, &w.items.m));
-    GIR_TRY(ensure_n(g, g->qitems[4], V + 2, &w.items.pref));
+    GIR_TRY(ensure_n(g, g->sssp_ctl, X_N, &w.ctl));
+    a.rows = w.rows;
+    a.ctl = w.ctl;
     void* h = nullptr;
-    GIR_TRY(pinned(g, 256, &h));
+    GIR_TRY(pinned(g, kPinnedBytes, &h));
     w.hc = static_cast<unsigned long long*>(h);
     return GIR_OK;
 }
 
-// One group of nl lanes (1..64) over the weight-sorted rows `ws`: lane s starts from
-// srcs[lane_rng[2s] .. lane_rng[2s + 1]) (device arrays, n_entries sources in all). Lane
+// Phases of more edges (far entries) than these run as launches of their own at full occupancy.
+constexpr int64_t kLoopMaxRelax = 1ll << 18;
+constexpr int64_t kLoopMaxFar = 1ll << 18;
+
+template <class D>
+int launch_phase(gir_dev* g, const Group& a, const Bucket& b, int64_t edges, int64_t entries) {
+    auto grid = [&](const void* f, int64_t threads) -> int {
+        int per_sm = 1;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, kPassThreads, 0);
+        const int64_t cap = (int64_t)g->num_sms * (per_sm > 0 ? per_sm : 1), want = (threads + kPassThreads - 1) / kPassThreads;
+        return (int)(want < 1 ? 1 : (want < cap ? want : cap));
+    };
+    const int64_t threads = edges > entries ? edges : entries;
+    if (b.phase == PH_LIGHT)
+        k_relax<D, PH_LIGHT><<<grid((const void*)k_relax<D, PH_LIGHT>, threads), kPassThreads, 0, g->stream>>>(a, b);
+    else if (b.phase == PH_HEAVY)
+        k_relax<D, PH_HEAVY><<<grid((const void*)k_relax<D, PH_HEAVY>, threads), kPassThreads, 0, g->stream>>>(a, b);
+    else
+        k_relax<D, PH_SPLIT><<<grid((const void*)k_relax<D, PH_SPLIT>, threads), kPassThreads, 0, g->stream>>>(a, b);
+    GIR_LAUNCH(g, "k_relax");
+    return GIR_OK;
+}
+
+// One group of nl lanes (1..64) over the weight-sorted rows `ws`: the lane at
+// position p starts from srcs[lane_rng[2p] .. lane_rng[2p + 1]) (device arrays, n_entries sources in all). Lane
 // distances have the type D. With nl == 1 and 64-bit lanes the result is written straight into
-// `out` (V entries); otherwise lane s ends in row lane_row[s] of `out` (rows of V). A 16-bit run
+// `out` (V entries); otherwise position p ends in row lane_row[p] of `out` (rows of V). A 16-bit run
 // that met a distance it cannot hold sets *overflow and writes nothing.
 template <class D>
 int sssp_group(gir_dev* g, Work& wk, const DevCSR& ws, int nl, const int64_t* lane_rng_d, const int32_t* srcs_d,
@@ -748,137 +955,96 @@ int sssp_group(gir_dev* g, Work& wk, const DevCSR& ws, int nl, const int64_t* la
     const int64_t V = g->V;
     QueryStats& st = g->qstats;
     *overflow = false;
-    unsigned long long* cnt = wk.cnt;
-    unsigned long long* hc = wk.hc;
-    auto read = [&]() -> int {
-        GIR_CUDA(g, cudaMemcpyAsync(hc, cnt, sizeof(unsigned long long) * S_N, cudaMemcpyDeviceToHost, g->stream));
-        GIR_CUDA(g, cudaStreamSynchronize(g->stream));
-        return GIR_OK;
-    };
+    Group& a = wk.a;
+    unsigned long long *ctl = wk.ctl, *hc = wk.hc;
     const bool direct = nl == 1 && sizeof(D) == sizeof(uint64_t);
+    const int ld = nl == 1 ? 1 : (nl + Vec<D>::n - 1) / Vec<D>::n * Vec<D>::n;
     D* dist = nullptr;
     if (direct) {
         dist = reinterpret_cast<D*>(out);
     } else {
-        GIR_TRY(ensure_n(g, g->lane_dist, (size_t)V * nl * sizeof(D) / sizeof(uint64_t) + 1,
+        GIR_TRY(ensure_n(g, g->lane_dist, (size_t)V * ld * sizeof(D) / sizeof(uint64_t) + 1,
                          reinterpret_cast<uint64_t**>(&dist)));
     }
-    int per_sm = 0;
-    GIR_CUDA(g, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_relax<D>, kRelaxThreads, 0));
-    const int run_grid = g->num_sms * (per_sm > 0 ? per_sm : 1);
+    a.wadj = ws.adj; a.ww = ws.w; a.delta = Dw; a.nl = nl; a.ld = ld; a.dist = dist;
     MainTimer timer{g, g->params[GIR_PARAM_PROFILE] != 0.0};
-    int32_t *nearq = wk.nearq, *nextq = wk.nextq, *farq = wk.farq, *farq2 = wk.farq2;
-    unsigned long long *curmask = wk.curmask, *nextmask = wk.nextmask;
     // (a group that ends on settled-only far entries leaves their lane bits behind)
-    GIR_CUDA(g, cudaMemsetAsync(curmask, 0, sizeof(unsigned long long) * V, g->stream));
-    GIR_CUDA(g, cudaMemsetAsync(nextmask, 0, sizeof(unsigned long long) * V, g->stream));
-    GIR_CUDA(g, cudaMemsetAsync(wk.farmask, 0, sizeof(unsigned long long) * V, g->stream));
-    GIR_CUDA(g, cudaMemsetAsync(wk.setmask, 0, sizeof(unsigned long long) * V, g->stream));
-    GIR_CUDA(g, cudaMemsetAsync(wk.done, 0, sizeof(unsigned long long) * V, g->stream));
-    GIR_CUDA(g, cudaMemsetAsync(dist, 0xff, sizeof(D) * V * nl, g->stream));
-    for (int k = 0; k < S_N; ++k)
-        if (k != S_REACHED && k != S_EDGES) hc[k] = 0;
-    GIR_CUDA(g, cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * 16, g->stream));
-    if (n_entries > 0) {
-        const int gx = (int)((n_entries / nl + kBlock - 1) / kBlock > 0 ? (n_entries / nl + kBlock - 1) / kBlock : 1);
-        k_sssp_init<D><<<dim3(gx < 1024 ? gx : 1024, nl), kBlock, 0, g->stream>>>(lane_rng_d, srcs_d, V, nl, dist,
-                                                                                  curmask, nearq, cnt);
-        GIR_LAUNCH(g, "k_sssp_init");
-    }
-    GIR_TRY(read());
-    int64_t n_near = (int64_t)hc[S_NEAR], n_far = 0;
-    Relax a;
-    a.wb = ws.beg; a.wdeg = ws.deg; a.wadj = ws.adj; a.ww = ws.w; a.delta = Dw; a.nl = nl; a.dist = dist;
-    a.farmask = wk.farmask; a.setmask = wk.setmask; a.setq = wk.setq; a.done = wk.done; a.cnt = cnt;
-    uint64_t k = 0;
-    int64_t trace_pairs = 0, trace_passes = 0;
+    for (unsigned long long* m : {a.mask[0], a.mask[1], a.mask[2], a.farmask, a.setmask, a.done})
+        GIR_CUDA(g, cudaMemsetAsync(m, 0, sizeof(unsigned long long) * V, g->stream));
+    GIR_CUDA(g, cudaMemsetAsync(dist, 0xff, sizeof(D) * V * ld, g->stream));
+    GIR_CUDA(g, cudaMemsetAsync(ctl, 0, sizeof(unsigned long long) * X_GROUP, g->stream));
+    GIR_CUDA(g, cudaMemsetAsync(ctl + X_MIN, 0xff, sizeof(unsigned long long), g->stream));
     k_light_split<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, ws.beg, ws.deg, ws.w, Dw, wk.rows);
     GIR_LAUNCH(g, "k_light_split");
-    Items items = wk.items;
-    // one relaxation pass over queue q (n entries): prep, scan of the work, balanced run
-    auto relax = [&](const int32_t* q, int64_t n, int heavy) -> int {
-        k_relax_prep<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(q, n, heavy, a, wk.rows, items);
-        GIR_LAUNCH(g, "k_relax_prep");
-        GIR_TRY(exclusive_scan_i64(g, items.pref, items.pref, n + 1));
-        if (g->trace_marks) {
-            int64_t tot = 0;
-            GIR_CUDA(g, cudaMemcpyAsync(&tot, items.pref + n, sizeof(int64_t), cudaMemcpyDeviceToHost, g->stream));
-            GIR_CUDA(g, cudaStreamSynchronize(g->stream));
-            trace_pairs += tot;
-            ++trace_passes;
-        }
-        GIR_TRY(timer.run([&]() -> int {
-            k_relax<D><<<run_grid, kRelaxThreads, 0, g->stream>>>(cnt + S_ITEMS, items, a);
-            GIR_LAUNCH(g, "k_relax");
-            return GIR_OK;
-        }));
-        st.launches += 4;  // prep, the scan's two kernels, the relaxation
+    if (n_entries > 0) {
+        const int gx = (int)((n_entries / nl + kBlock - 1) / kBlock > 0 ? (n_entries / nl + kBlock - 1) / kBlock : 1);
+        k_sssp_init<D><<<dim3(gx < 1024 ? gx : 1024, nl), kBlock, 0, g->stream>>>(lane_rng_d, srcs_d, V, ld, dist,
+                                                                                  a.mask[0], a.q[0], wk.rows, ctl + X_NEAR);
+        GIR_LAUNCH(g, "k_sssp_init");
+    }
+    // (bucket 0 starts with a light pass, of no entries where no source is in range)
+    Bucket b{PH_LIGHT, 0, 0, 0, 0, 0, 0, 0};
+    auto rd = [&](int i) { return hc[i]; };
+    auto read = [&]() -> int {
+        GIR_CUDA(g, cudaMemcpyAsync(hc, ctl, sizeof(unsigned long long) * X_GROUP, cudaMemcpyDeviceToHost, g->stream));
+        GIR_CUDA(g, cudaStreamSynchronize(g->stream));
         return GIR_OK;
     };
-    while (true) {
-        a.kend = (k + 1) * Dw;
-        GIR_CUDA(g, cudaMemsetAsync(cnt + S_SET, 0, sizeof(unsigned long long), g->stream));
-        // light rounds: nearq (lanes in curmask) -> nextq (lanes in nextmask)
-        while (n_near > 0) {
-            a.curmask = curmask; a.nextmask = nextmask; a.nextq = nextq; a.farq = farq;
-            GIR_TRY(relax(nearq, n_near, 0));
-            st.iterations++;
-            std::swap(nearq, nextq);
-            std::swap(curmask, nextmask);
-            GIR_TRY(read());
-            n_near = (int64_t)hc[S_NEAR];
+    bool fresh = true;  // the first phase's size was not read: the loop looks at it
+    while (b.phase != PH_DONE) {
+        int64_t edges = 0, entries = 0;
+        if (!fresh) {
+            const unsigned long long packed = b.phase == PH_LIGHT ? hc[X_NEAR + b.rot]
+                                              : b.phase == PH_HEAVY ? hc[X_SET] : hc[X_FAR + b.spl] << kQShift;
+            edges = (int64_t)(packed & kQEdges);
+            entries = b.phase == PH_SPLIT ? (int64_t)hc[X_FAR + b.spl] : (int64_t)(packed >> kQShift);
         }
-        // heavy edges of the (vertex, lane) pairs settled in this bucket
-        const int64_t n_set = (int64_t)hc[S_SET];
-        if (n_set > 0) {
-            a.curmask = curmask; a.nextmask = nextmask; a.nextq = nextq; a.farq = farq;
-            GIR_TRY(relax(wk.setq, n_set, 1));
-        }
-        // next bucket: split the far entries at bucket k + 1; when that one is empty, jump to
-        // the bucket of the smallest distance still far
-        GIR_TRY(read());
-        n_far = (int64_t)hc[S_FAR];
-        if (n_far == 0) break;
-        uint64_t lo = a.kend;
-        bool finished = false;
-        while (true) {
-            k = lo / Dw;
-            GIR_CUDA(g, cudaMemsetAsync(cnt + S_MIN, 0xff, sizeof(unsigned long long), g->stream));
-            GIR_CUDA(g, cudaMemsetAsync(cnt + S_FAR2, 0, sizeof(unsigned long long), g->stream));
-            k_far_split<D><<<grid_for(g, n_far, kBlock), kBlock, 0, g->stream>>>(
-                farq, cnt + S_FAR, wk.farmask, dist, nl, k * Dw, (k + 1) * Dw, curmask, nearq, farq2, wk.done, cnt);
-            GIR_LAUNCH(g, "k_far_split");
-            st.launches++;
-            std::swap(farq, farq2);
-            GIR_CUDA(g, cudaMemcpyAsync(cnt + S_FAR, cnt + S_FAR2, sizeof(unsigned long long), cudaMemcpyDeviceToDevice,
-                                        g->stream));
-            GIR_TRY(read());
-            n_near = (int64_t)hc[S_NEAR];
-            n_far = (int64_t)hc[S_FAR];
-            if (n_near > 0) break;
-            if (hc[S_MIN] == kInf) {  // nothing live is left far
-                finished = true;
-                break;
+        if (fresh || (edges <= kLoopMaxRelax && (b.phase != PH_SPLIT || entries <= kLoopMaxFar))) {
+            if (!fresh) {
+                hc[X_PHASE] = (unsigned long long)b.phase;
+                hc[X_ROT] = (unsigned long long)b.rot;
+                hc[X_SPL] = (unsigned long long)b.spl;
+                hc[X_FQ] = (unsigned long long)b.fq;
+                hc[X_LO] = b.lo;
+                hc[X_NCLEAR] = (unsigned long long)b.n_clear;
+                hc[X_NSETCLEAR] = (unsigned long long)b.n_setclear;
+                hc[X_PASSES] = (unsigned long long)b.passes;
+                GIR_CUDA(g, cudaMemcpyAsync(ctl + X_PHASE, hc + X_PHASE, sizeof(unsigned long long) * (X_PASSES + 1 - X_PHASE),
+                                            cudaMemcpyHostToDevice, g->stream));
             }
-            lo = hc[S_MIN];
+            GIR_CUDA(g, cudaMemsetAsync(ctl + X_BAR, 0, sizeof(unsigned long long), g->stream));
+            int64_t max_edges = kLoopMaxRelax, max_far = kLoopMaxFar;
+            void* args[] = {&a, &max_edges, &max_far};
+            GIR_TRY(timer.run([&]() -> int {
+                GIR_CUDA(g, cudaLaunchCooperativeKernel((const void*)k_bucket_loop<D>, g->num_sms, kLoopThreads, args, 0,
+                                                        g->stream));
+                return GIR_OK;
+            }));
+            GIR_TRY(read());
+            if (hc[X_ERR]) return fail(g, GIR_ERR_TIMEOUT, "sssp: the bucket loop ran out its barrier bound");
+            b = Bucket{(int)hc[X_PHASE], (int)hc[X_ROT], (int)hc[X_SPL], (int)hc[X_FQ], hc[X_LO], (int64_t)hc[X_NCLEAR],
+                       (int64_t)hc[X_NSETCLEAR], (int64_t)hc[X_PASSES]};
+            fresh = false;
+        } else {
+            GIR_TRY(timer.run([&]() -> int { return launch_phase<D>(g, a, b, edges, entries); }));
+            GIR_TRY(read());
+            next_phase(b, a.delta, entries, rd);
         }
-        if (finished) break;
+        st.launches++;
     }
+    st.iterations += b.passes;
     if (g->trace_marks)
-        std::fprintf(stderr, "[gir] sssp group of %d lanes, %d-bit distances, delta %llu: %lld passes, %lld (edge, lane) pairs\n",
-                     nl, (int)(8 * sizeof(D)), (unsigned long long)Dw, (long long)trace_passes, (long long)trace_pairs);
-    if (sizeof(D) == sizeof(uint16_t)) {
-        GIR_TRY(read());
-        if (hc[S_OVF]) {
-            *overflow = true;
-            return GIR_OK;
-        }
+        std::fprintf(stderr, "[gir] sssp group of %d lanes, %d-bit distances, delta %llu: %lld light passes\n", nl,
+                     (int)(8 * sizeof(D)), (unsigned long long)Dw, (long long)b.passes);
+    if (sizeof(D) == sizeof(uint16_t) && hc[X_OVF]) {
+        *overflow = true;
+        return GIR_OK;
     }
     if (!direct) {  // (the transpose also counts the reached pairs and their edges)
-        k_transpose<D><<<g->num_sms * 8, 256, 0, g->stream>>>(dist, V, nl, lane_row_d, g->fw.deg, out, cnt);
+        k_transpose<D><<<g->num_sms * 8, 256, 0, g->stream>>>(dist, V, nl, ld, lane_row_d, g->fw.deg, out, ctl);
         GIR_LAUNCH(g, "k_transpose");
     } else {
-        k_sssp_reached<D><<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(dist, V, nl, g->fw.deg, cnt);
+        k_sssp_reached<D><<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(dist, V, nl, g->fw.deg, ctl);
         GIR_LAUNCH(g, "k_sssp_reached");
     }
     return GIR_OK;
@@ -903,12 +1069,12 @@ static int hub_order(gir_dev* g, int hash) {
     int64_t* lanes = nullptr;
     if (!rc) rc = ensure_n(g, g->sssp_lanes, 4, &lanes);
     unsigned long long st[2] = {0, 0};
-    if (!rc) rc = cuda_check(g, cudaMemsetAsync(wk.cnt + 24, 0, 2 * sizeof(unsigned long long), g->stream), "memset");
+    if (!rc) rc = cuda_check(g, cudaMemsetAsync(wk.ctl + X_TMP, 0, 2 * sizeof(unsigned long long), g->stream), "memset");
     if (!rc) {
-        k_argmax_deg<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, g->bw.deg, wk.cnt + 24);
+        k_argmax_deg<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, g->bw.deg, wk.ctl + X_TMP);
         rc = cuda_check(g, cudaGetLastError(), "k_argmax_deg");
     }
-    if (!rc) rc = cuda_check(g, cudaMemcpyAsync(st, wk.cnt + 24, sizeof(st), cudaMemcpyDeviceToHost, g->stream), "copy");
+    if (!rc) rc = cuda_check(g, cudaMemcpyAsync(st, wk.ctl + X_TMP, sizeof(st), cudaMemcpyDeviceToHost, g->stream), "copy");
     if (!rc) rc = cuda_check(g, cudaStreamSynchronize(g->stream), "sync");
     if (!rc) {
         const int32_t hub = (int32_t)~(uint32_t)(st[0] & 0xffffffffull);
@@ -918,12 +1084,12 @@ static int hub_order(gir_dev* g, int hash) {
         if (!rc) rc = cuda_check(g, cudaMemcpyAsync(src_d, &hub, sizeof(hub), cudaMemcpyHostToDevice, g->stream), "copy");
         bool ovf = false;
         if (!rc) rc = sssp_group<uint64_t>(g, wk, wsb, 1, lanes, src_d, 1, nullptr, hd, 16, &ovf);
-        if (!rc) rc = cuda_check(g, cudaMemsetAsync(wk.cnt + 25, 0, sizeof(unsigned long long), g->stream), "memset");
+        if (!rc) rc = cuda_check(g, cudaMemsetAsync(wk.ctl + X_TMP + 1, 0, sizeof(unsigned long long), g->stream), "memset");
         if (!rc) {
-            k_max_finite<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, hd, wk.cnt + 24);
+            k_max_finite<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, hd, wk.ctl + X_TMP);
             rc = cuda_check(g, cudaGetLastError(), "k_max_finite");
         }
-        if (!rc) rc = cuda_check(g, cudaMemcpyAsync(st, wk.cnt + 24, sizeof(st), cudaMemcpyDeviceToHost, g->stream), "copy");
+        if (!rc) rc = cuda_check(g, cudaMemcpyAsync(st, wk.ctl + X_TMP, sizeof(st), cudaMemcpyDeviceToHost, g->stream), "copy");
         if (!rc) rc = cuda_check(g, cudaStreamSynchronize(g->stream), "sync");
         if (!rc) {
             g->hub_max[mi] = st[1];
@@ -945,9 +1111,7 @@ int sssp_run(gir_dev* g, const int64_t* set_beg_h, const int32_t* srcs_d, int64_
     st = QueryStats{};
     g->trace_x.clear();
     g->trace_y.clear();
-    if (n_sets <= 0) return GIR_OK;
-    GIR_CUDA(g, cudaMemsetAsync(dist_d, 0xff, sizeof(uint64_t) * V * n_sets, g->stream));
-    if (V == 0) return GIR_OK;
+    if (n_sets <= 0 || V == 0) return GIR_OK;  // (every row of dist_d is written whole by its group)
     const int hash = weight_mode == GIR_WEIGHT_HASH;
     const int mi = hash ? 0 : 1;
     if (!hash && !g->has_weights) return fail(g, GIR_ERR_STATE, "sssp: the graph has no stored weights");
@@ -990,7 +1154,7 @@ int sssp_run(gir_dev* g, const int64_t* set_beg_h, const int32_t* srcs_d, int64_
     const bool fits32 = bits != 64 && (double)V * wmax < 4294967295.0;
     const bool try16 = bits == 16 && !g->narrow16_failed[mi];
     GIR_CUDA(g, cudaEventRecord(g->ev0, g->stream));
-    GIR_CUDA(g, cudaMemsetAsync(wk.cnt, 0, sizeof(unsigned long long) * S_N, g->stream));
+    GIR_CUDA(g, cudaMemsetAsync(wk.ctl, 0, sizeof(unsigned long long) * X_N, g->stream));
     std::vector<int64_t> lh(3 * 64);
     for (int64_t g0 = 0; g0 < n_sets; g0 += 64) {
         const int nl = (int)((n_sets - g0) < 64 ? (n_sets - g0) : 64);
@@ -1033,11 +1197,11 @@ int sssp_run(gir_dev* g, const int64_t* set_beg_h, const int32_t* srcs_d, int64_
             GIR_TRY(sssp_group<uint64_t>(g, wk, ws, nl, lanes, srcs_d, n_entries, rows_d, dist_d, D, &ovf));
     }
     unsigned long long* hc = wk.hc;
-    GIR_CUDA(g, cudaMemcpyAsync(hc, wk.cnt, sizeof(unsigned long long) * S_N, cudaMemcpyDeviceToHost, g->stream));
+    GIR_CUDA(g, cudaMemcpyAsync(hc, wk.ctl, sizeof(unsigned long long) * X_N, cudaMemcpyDeviceToHost, g->stream));
     GIR_CUDA(g, cudaEventRecord(g->ev1, g->stream));
     GIR_CUDA(g, cudaEventSynchronize(g->ev1));
-    st.reached = (int64_t)hc[S_REACHED];
-    st.edges = (int64_t)hc[S_EDGES];
+    st.reached = (int64_t)hc[X_REACHED];
+    st.edges = (int64_t)hc[X_EDGES];
     float ms = 0;
     GIR_CUDA(g, cudaEventElapsedTime(&ms, g->ev0, g->ev1));
     st.kernel_ms = ms;

@@ -129,3 +129,70 @@ def test_layers_of_deep_graphs(pkg, orc):
                 fb, fa, _, _ = orc.apply_batch(V, fb, fa, bu, bv, ins)
                 _oracle_match(pkg, orc, d, V, fb, fa, f"{name}, batch {step}")
         d.close()
+
+
+def _weighted(pkg, V, u, v, w):
+    key, first = np.unique(np.asarray(u, np.int64) * V + np.asarray(v, np.int64), return_index=True)
+    return pkg.graphs.from_edges(V, key // V, key % V, np.asarray(w, np.uint32)[first])
+
+
+@pytest.mark.parametrize("lanes", [1, 2, 3, 5, 8, 17, 33, 63, 64, 65])
+def test_sssp_lane_counts_widths_and_buckets(pkg, orc, lanes):
+    """Rows of every padding, lane widths of 16, 32 and 64 bits, bucket widths from one (every edge heavy)
+    to wider than any path (every edge light), weights of zero, sources repeated and out of range; hubs
+    whose rows are cut into runs, and long stretches of settled vertices without a heavy edge."""
+    rng = np.random.default_rng(lanes)
+    V = 3000
+    u = np.concatenate([rng.integers(0, V, 3 * V), np.zeros(2500, np.int64), np.full(900, 7), np.arange(V - 1)])
+    v = np.concatenate([rng.integers(0, V, 3 * V), 1 + np.arange(2500), V - 1 - np.arange(900), 1 + np.arange(V - 1)])
+    w = rng.integers(0, 60, len(u))
+    w[rng.random(len(u)) < 0.002] = 5000
+    w[-(V - 1):] = 3
+    keep = u != v
+    g = _weighted(pkg, V, u[keep], v[keep], w[keep])
+    fb, fa = orc.normalize(V, g.fw_beg, g.fw_adj)
+    d = pkg.DeviceGraph.from_graph(g)
+    src = rng.integers(0, V, lanes).astype(np.int32)
+    src[-1] = src[0]
+    if lanes > 4:
+        src[2], src[3] = -1, V
+    exp = np.stack([orc.sssp(V, fb, fa, [int(s)], w=g.w) for s in src])
+    exp_hash = np.stack([orc.sssp(V, fb, fa, [int(s)]) for s in src[:4]])
+    for bits in (0, 16, 32, 64):
+        d.set_param(pkg.native.PARAM_LANE_BITS, bits)
+        for delta in (1, 16, 61, 1000, 1 << 40):
+            got = d.sssp(src, delta=delta, weights=pkg.native.WEIGHT_STORED)
+            np.testing.assert_array_equal(got, exp, err_msg=f"{bits} bits, delta {delta}")
+            st = d.query_stats()
+            fin = exp != np.uint64(2**64 - 1)
+            assert st["reached"] == fin.sum() and st["edges"] == (fin * np.diff(fb)).sum()
+    np.testing.assert_array_equal(d.sssp(src, delta=16)[:4], exp_hash)
+    sets = [rng.integers(0, V, n).astype(np.int32) for n in (1, 700, 0, 3)]
+    got = d.sssp_sets(sets, delta=20, weights=pkg.native.WEIGHT_STORED)
+    for row, s in zip(got, sets):
+        np.testing.assert_array_equal(row, orc.sssp(V, fb, fa, [int(x) for x in s], w=g.w) if len(s)
+                                      else np.full(V, 2**64 - 1, np.uint64))
+    d.close()
+
+
+def test_sssp_phases_inside_and_outside_the_bucket_loop(pkg, orc):
+    """Passes of over 2^18 edges and far queues of over 2^18 entries leave the device-resident loop for
+    launches of their own, and the loop takes over again for a long tail; 32- and 64-bit lanes."""
+    V = 400_000
+    rng = np.random.default_rng(8)
+    tail = np.arange(V - 400, V - 1)
+    u = np.concatenate([rng.integers(0, V - 400, 8 * V), tail, [11], np.zeros(9000, np.int64)])
+    v = np.concatenate([rng.integers(0, V - 400, 8 * V), tail + 1, [V - 400], rng.integers(0, V - 400, 9000)])
+    w = rng.integers(1, 200, len(u))
+    keep = u != v
+    for scale in (1, 300):  # the larger weights do not fit 32-bit lanes
+        g = _weighted(pkg, V, u[keep], v[keep], w[keep] * scale)
+        fb, fa = orc.normalize(V, g.fw_beg, g.fw_adj)
+        d = pkg.DeviceGraph.from_graph(g)
+        src = np.concatenate([rng.integers(0, V, 38), [0, V - 1]]).astype(np.int32)
+        got = d.sssp(src, delta=40 * scale, weights=pkg.native.WEIGHT_STORED)
+        for i in (0, 5, 38, 39):
+            np.testing.assert_array_equal(got[i], orc.sssp(V, fb, fa, [int(src[i])], w=g.w))
+        one = d.sssp(src[:1], delta=7 * scale, weights=pkg.native.WEIGHT_STORED)
+        np.testing.assert_array_equal(one[0], got[0])
+        d.close()
