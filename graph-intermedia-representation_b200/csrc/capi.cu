@@ -33,17 +33,12 @@ __global__ void k_validate(const int32_t* beg, const int32_t* adj, int64_t V, in
 
 // Edge keys (row << 32 | col) of an int32 CSR; `unsorted` is set if some row is not strictly
 // increasing (then the keys need sorting and de-duplication).
-__global__ void k_csr_keys(const int32_t* beg, const int32_t* adj, int64_t V, int64_t E, uint64_t* keys,
-                           int32_t* unsorted) {
-    GRID_STRIDE(i, E) {
-        int64_t lo = 0, hi = V - 1;  // row: largest r with beg[r] <= i
-        while (lo < hi) {
-            const int64_t m = (lo + hi + 1) >> 1;
-            if ((int64_t)beg[m] <= i) lo = m; else hi = m - 1;
-        }
-        keys[i] = ((uint64_t)lo << 32) | (uint32_t)adj[i];
-        if (i > beg[lo] && adj[i - 1] >= adj[i]) atomicExch(unsorted, 1);
-    }
+__global__ void k_csr_keys(const int32_t* beg, const int32_t* adj, int64_t V, uint64_t* keys, int32_t* unsorted) {
+    walk_segments(beg, V, [&](int64_t r, int64_t j) {
+        const int64_t i = beg[r] + j;
+        keys[i] = ((uint64_t)r << 32) | (uint32_t)adj[i];
+        if (j > 0 && adj[i - 1] >= adj[i]) atomicExch(unsorted, 1);
+    });
 }
 
 __global__ void k_distinct(const uint64_t* keys, int64_t n, uint8_t* flag) {
@@ -175,7 +170,7 @@ int build_direction(gir_dev* g, DevCSR& c, const int32_t* beg, const int32_t* ad
     }
     GIR_CUDA(g, cudaMemsetAsync(unsorted, 0, sizeof(int32_t), g->stream));
     if (E > 0) {
-        k_csr_keys<<<grid_for(g, E, kBlock), kBlock, 0, g->stream>>>(beg, adj, V, E, keys, unsorted);
+        k_csr_keys<<<grid_for(g, E, kBlock), kBlock, 0, g->stream>>>(beg, adj, V, keys, unsorted);
         GIR_LAUNCH(g, "k_csr_keys");
     }
     int32_t h_unsorted = 0;

@@ -127,34 +127,37 @@ int sort_keys_u64(gir_dev* g, uint64_t* keys, uint64_t* tmp, int64_t n, int end_
     return GIR_OK;
 }
 
-int sort_pairs_u64(gir_dev* g, uint64_t* keys, uint64_t* ktmp, uint32_t* vals, uint32_t* vtmp, int64_t n, int end_bit) {
+namespace {
+
+// Pairs sorted by key; the result is in keys / vals.
+template <class K, class T>
+int sort_pairs(gir_dev* g, K* keys, K* ktmp, T* vals, T* vtmp, int64_t n, int end_bit) {
     if (n <= 1) return GIR_OK;
-    cub::DoubleBuffer<uint64_t> kb(keys, ktmp);
-    cub::DoubleBuffer<uint32_t> vb(vals, vtmp);
+    cub::DoubleBuffer<K> kb(keys, ktmp);
+    cub::DoubleBuffer<T> vb(vals, vtmp);
     size_t bytes = 0;
     GIR_CUDA(g, cub::DeviceRadixSort::SortPairs(nullptr, bytes, kb, vb, n, 0, end_bit, g->stream));
     GIR_TRY(ensure(g, g->cub_tmp, bytes));
     GIR_CUDA(g, cub::DeviceRadixSort::SortPairs(g->cub_tmp.p, bytes, kb, vb, n, 0, end_bit, g->stream));
     if (kb.Current() != keys)
-        GIR_CUDA(g, cudaMemcpyAsync(keys, kb.Current(), sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, g->stream));
+        GIR_CUDA(g, cudaMemcpyAsync(keys, kb.Current(), sizeof(K) * n, cudaMemcpyDeviceToDevice, g->stream));
     if (vb.Current() != vals)
-        GIR_CUDA(g, cudaMemcpyAsync(vals, vb.Current(), sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, g->stream));
+        GIR_CUDA(g, cudaMemcpyAsync(vals, vb.Current(), sizeof(T) * n, cudaMemcpyDeviceToDevice, g->stream));
     return GIR_OK;
 }
 
+}  // namespace
+
+int sort_pairs_u64(gir_dev* g, uint64_t* keys, uint64_t* ktmp, uint32_t* vals, uint32_t* vtmp, int64_t n, int end_bit) {
+    return sort_pairs(g, keys, ktmp, vals, vtmp, n, end_bit);
+}
+
+int sort_pairs_u32(gir_dev* g, uint32_t* keys, uint32_t* ktmp, uint32_t* vals, uint32_t* vtmp, int64_t n, int end_bit) {
+    return sort_pairs(g, keys, ktmp, vals, vtmp, n, end_bit);
+}
+
 int sort_pairs_u64_i64(gir_dev* g, uint64_t* keys, uint64_t* ktmp, int64_t* vals, int64_t* vtmp, int64_t n, int end_bit) {
-    if (n <= 1) return GIR_OK;
-    cub::DoubleBuffer<uint64_t> kb(keys, ktmp);
-    cub::DoubleBuffer<int64_t> vb(vals, vtmp);
-    size_t bytes = 0;
-    GIR_CUDA(g, cub::DeviceRadixSort::SortPairs(nullptr, bytes, kb, vb, n, 0, end_bit, g->stream));
-    GIR_TRY(ensure(g, g->cub_tmp, bytes));
-    GIR_CUDA(g, cub::DeviceRadixSort::SortPairs(g->cub_tmp.p, bytes, kb, vb, n, 0, end_bit, g->stream));
-    if (kb.Current() != keys)
-        GIR_CUDA(g, cudaMemcpyAsync(keys, kb.Current(), sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, g->stream));
-    if (vb.Current() != vals)
-        GIR_CUDA(g, cudaMemcpyAsync(vals, vb.Current(), sizeof(int64_t) * n, cudaMemcpyDeviceToDevice, g->stream));
-    return GIR_OK;
+    return sort_pairs(g, keys, ktmp, vals, vtmp, n, end_bit);
 }
 
 int exclusive_scan_i64(gir_dev* g, const int64_t* in, int64_t* out, int64_t n) {

@@ -40,20 +40,15 @@ constexpr uint64_t kInf = ~0ull;
 enum { X_NEAR = 0, X_SET = 3, X_FAR = 4, X_MIN = 7, X_OVF = 10, X_ERR = 11, X_PHASE = 12, X_LO, X_ROT, X_SPL, X_FQ,
        X_NCLEAR, X_NSETCLEAR, X_PASSES, X_GROUP = 24, X_REACHED = 24, X_EDGES = 25, X_TMP = 26, X_BAR = 32, X_N = 64 };
 
-// Sort keys (row << 32 | weight) and columns of every entry of the compact copy of `c`. For the
-// forward CSR the weight of entry (u, v) is that of edge u -> v. With `reverse` the rows are
-// those of the backward CSR: row v holds the u of every edge u -> v, whose weight is the hash
-// weight of (u, v) or the stored weight found in the forward row of u (`f`).
-__global__ void k_ws_keys(int64_t V, int64_t E, const int64_t* cb, CSRView c, int hash, int reverse, CSRView f,
-                          uint64_t* keys, uint32_t* cols) {
-    GRID_STRIDE(i, E) {
-        int64_t lo = 0, hi = V - 1;
-        while (lo < hi) {
-            const int64_t m = (lo + hi + 1) >> 1;
-            if (cb[m] <= i) lo = m; else hi = m - 1;
-        }
-        const int64_t u = lo;
-        const int64_t p = c.beg[u] + (i - cb[u]);
+// Columns and weights of every entry of the compact copy of `c`, in row order, and the weights' sum and
+// maximum (st[0], st[1]). For the forward CSR the weight of entry (u, v) is that of edge u -> v. With
+// `reverse` the rows are those of the backward CSR: row v holds the u of every edge u -> v, whose
+// weight is the hash weight of (u, v) or the stored weight found in the forward row of u (`f`).
+__global__ void k_ws_gather(int64_t V, const int64_t* cb, CSRView c, int hash, int reverse, CSRView f, uint32_t* cols,
+                            uint32_t* weights, unsigned long long* st) {
+    unsigned long long s = 0, m = 0;
+    walk_segments(cb, V, [&](int64_t u, int64_t j) {
+        const int64_t i = cb[u] + j, p = c.beg[u] + j;
         const int32_t v = c.adj[p];
         uint32_t w;
         if (!reverse) {
@@ -64,33 +59,33 @@ __global__ void k_ws_keys(int64_t V, int64_t E, const int64_t* cb, CSRView c, in
             const int64_t b = f.beg[v];
             w = f.w[lower_bound_dev(f.adj, b, b + f.deg[v], (int32_t)u)];
         }
-        keys[i] = ((uint64_t)u << 32) | w;
         cols[i] = (uint32_t)v;
-    }
-}
-
-__global__ void k_ws_split(int64_t E, const uint64_t* keys, const uint32_t* cols, int32_t* adj, uint32_t* w) {
-    GRID_STRIDE(i, E) {
-        adj[i] = (int32_t)cols[i];
-        w[i] = (uint32_t)(keys[i] & 0xffffffffULL);
-    }
-}
-
-// Sum and maximum of the weights (st[0], st[1]).
-__global__ void k_wstat(const uint32_t* w, int64_t E, unsigned long long* st) {
-    unsigned long long s = 0, m = 0;
-    GRID_STRIDE(i, E) {
-        s += w[i];
-        m = w[i] > m ? w[i] : m;
-    }
+        weights[i] = w;
+        s += w;
+        m = w > m ? w : m;
+    });
+    s = warp_sum_u64(s);
     for (int o = 16; o; o >>= 1) {
-        s += __shfl_xor_sync(0xffffffffu, s, o);
         const unsigned long long t = __shfl_xor_sync(0xffffffffu, m, o);
         m = t > m ? t : m;
     }
-    if (lane_id() == 0) {
+    if (lane_id() == 0 && (s | m)) {
         atomicAdd(&st[0], s);
         atomicMax(&st[1], m);
+    }
+}
+
+// Sort keys: row << wbits | weight.
+template <class K>
+__global__ void k_ws_keys(int64_t V, const int64_t* cb, const uint32_t* weights, int wbits, K* keys) {
+    walk_segments(cb, V, [&](int64_t u, int64_t j) { keys[cb[u] + j] = ((K)u << wbits) | (K)weights[cb[u] + j]; });
+}
+
+template <class K>
+__global__ void k_ws_split(int64_t E, const K* keys, const uint32_t* cols, int wbits, int32_t* adj, uint32_t* w) {
+    GRID_STRIDE(i, E) {
+        adj[i] = (int32_t)cols[i];
+        w[i] = (uint32_t)(keys[i] & (((K)1 << wbits) - 1));
     }
 }
 
@@ -849,8 +844,6 @@ static int build_weight_sorted(gir_dev* g, int hash, int reverse, DevCSR& ws) {
     const DevCSR& c = reverse ? g->bw : g->fw;
     const int64_t V = g->V, E = c.E;
     store_free(g, ws);
-    uint64_t *keys = nullptr, *ktmp = nullptr;
-    uint32_t *cols = nullptr, *ctmp = nullptr;
     GIR_TRY(dev_alloc_n(g, &ws.beg, V + 1));
     GIR_TRY(dev_alloc_n(g, &ws.deg, V > 0 ? V : 1));
     GIR_TRY(dev_alloc_n(g, &ws.adj, E > 0 ? E : 1));
@@ -862,25 +855,47 @@ static int build_weight_sorted(gir_dev* g, int hash, int reverse, DevCSR& ws) {
     GIR_TRY(exclusive_scan_i64(g, cb, cb, V + 1));
     GIR_CUDA(g, cudaMemcpyAsync(ws.deg, c.deg, sizeof(int32_t) * V, cudaMemcpyDeviceToDevice, g->stream));
     if (E == 0) return GIR_OK;
-    GIR_TRY(ensure_n(g, g->scratch[8], E, &keys));
-    GIR_TRY(ensure_n(g, g->scratch[9], E, &ktmp));
+    uint32_t *cols = nullptr, *ctmp = nullptr;
+    unsigned long long* st = nullptr;
     GIR_TRY(ensure_n(g, g->scratch[10], E, &cols));
     GIR_TRY(ensure_n(g, g->scratch[11], E, &ctmp));
-    k_ws_keys<<<grid_for(g, E, kBlock), kBlock, 0, g->stream>>>(V, E, cb, view(c), hash, reverse, view(g->fw), keys,
-                                                                 cols);
-    GIR_LAUNCH(g, "k_ws_keys");
-    GIR_TRY(sort_pairs_u64(g, keys, ktmp, cols, ctmp, E, 64));
-    k_ws_split<<<grid_for(g, E, kBlock), kBlock, 0, g->stream>>>(E, keys, cols, ws.adj, ws.w);
+    GIR_TRY(ensure_n(g, g->sssp_ctl, X_N, &st));
+    GIR_CUDA(g, cudaMemsetAsync(st, 0, 2 * sizeof(unsigned long long), g->stream));
+    k_ws_gather<<<grid_for(g, E, kBlock), kBlock, 0, g->stream>>>(V, cb, view(c), hash, reverse, view(g->fw), cols, ws.w, st);
+    GIR_LAUNCH(g, "k_ws_gather");
+    // The sort key holds no more bits than rows and weights have (4.8M vertices, hash weights: 30, so
+    // 32-bit keys and four radix passes instead of eight over 64-bit ones).
+    unsigned long long h[2] = {0, 100};
+    if (!hash || !reverse) {
+        GIR_CUDA(g, cudaMemcpyAsync(h, st, sizeof(h), cudaMemcpyDeviceToHost, g->stream));
+        GIR_CUDA(g, cudaStreamSynchronize(g->stream));
+    }
+    auto bits_of = [](uint64_t x) {
+        int n = 0;
+        while (x >> n) ++n;
+        return n;
+    };
+    const int wbits = bits_of(h[1]), bits = std::max(1, wbits + bits_of((uint64_t)(V - 1)));
+    if (bits <= 32 && wbits < 32) {
+        uint32_t *keys = nullptr, *ktmp = nullptr;
+        GIR_TRY(ensure_n(g, g->scratch[8], E, &keys));
+        GIR_TRY(ensure_n(g, g->scratch[9], E, &ktmp));
+        k_ws_keys<uint32_t><<<grid_for(g, E, kBlock), kBlock, 0, g->stream>>>(V, cb, ws.w, wbits, keys);
+        GIR_LAUNCH(g, "k_ws_keys");
+        GIR_TRY(sort_pairs_u32(g, keys, ktmp, cols, ctmp, E, bits));
+        k_ws_split<uint32_t><<<grid_for(g, E, kBlock), kBlock, 0, g->stream>>>(E, keys, cols, wbits, ws.adj, ws.w);
+    } else {
+        uint64_t *keys = nullptr, *ktmp = nullptr;
+        GIR_TRY(ensure_n(g, g->scratch[8], E, &keys));
+        GIR_TRY(ensure_n(g, g->scratch[9], E, &ktmp));
+        k_ws_keys<uint64_t><<<grid_for(g, E, kBlock), kBlock, 0, g->stream>>>(V, cb, ws.w, wbits, keys);
+        GIR_LAUNCH(g, "k_ws_keys");
+        GIR_TRY(sort_pairs_u64(g, keys, ktmp, cols, ctmp, E, bits));
+        k_ws_split<uint64_t><<<grid_for(g, E, kBlock), kBlock, 0, g->stream>>>(E, keys, cols, wbits, ws.adj, ws.w);
+    }
     GIR_LAUNCH(g, "k_ws_split");
     if (reverse) return GIR_OK;
     // weight statistics for the schedule's features
-    unsigned long long* st = reinterpret_cast<unsigned long long*>(ktmp);
-    GIR_CUDA(g, cudaMemsetAsync(st, 0, 2 * sizeof(unsigned long long), g->stream));
-    k_wstat<<<grid_for(g, E, kBlock), kBlock, 0, g->stream>>>(ws.w, E, st);
-    GIR_LAUNCH(g, "k_wstat");
-    unsigned long long h[2] = {0, 0};
-    GIR_CUDA(g, cudaMemcpyAsync(h, st, sizeof(h), cudaMemcpyDeviceToHost, g->stream));
-    GIR_CUDA(g, cudaStreamSynchronize(g->stream));
     g->wstat[hash ? 0 : 1][0] = (double)h[0] / (double)E;
     g->wstat[hash ? 0 : 1][1] = (double)h[1];
     return GIR_OK;
@@ -1082,8 +1097,11 @@ static int hub_order(gir_dev* g, int hash) {
         int32_t* src_d = reinterpret_cast<int32_t*>(lanes + 2);
         rc = cuda_check(g, cudaMemcpyAsync(lanes, h_lane, sizeof(h_lane), cudaMemcpyHostToDevice, g->stream), "copy");
         if (!rc) rc = cuda_check(g, cudaMemcpyAsync(src_d, &hub, sizeof(hub), cudaMemcpyHostToDevice, g->stream), "copy");
+        // One lane's passes are short, so wide buckets win (fewer phases): 32 mean weights took a 901 x 901
+        // lattice's run from 280 ms (a width of 16, 27,000 phases) to 15.
+        const uint64_t width = 16 + (uint64_t)(32.0 * g->wstat[mi][0]);
         bool ovf = false;
-        if (!rc) rc = sssp_group<uint64_t>(g, wk, wsb, 1, lanes, src_d, 1, nullptr, hd, 16, &ovf);
+        if (!rc) rc = sssp_group<uint64_t>(g, wk, wsb, 1, lanes, src_d, 1, nullptr, hd, width, &ovf);
         if (!rc) rc = cuda_check(g, cudaMemsetAsync(wk.ctl + X_TMP + 1, 0, sizeof(unsigned long long), g->stream), "memset");
         if (!rc) {
             k_max_finite<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, hd, wk.ctl + X_TMP);

@@ -20,16 +20,6 @@ __device__ __forceinline__ int64_t row_capacity(int64_t d) {
     return (c + 3) & ~(int64_t)3;
 }
 
-// Row of compact position `i`, given the exclusive scan `cb` of row lengths (V+1 entries).
-__device__ __forceinline__ int64_t row_of(const int64_t* cb, int64_t V, int64_t i) {
-    int64_t lo = 0, hi = V - 1;  // largest r with cb[r] <= i
-    while (lo < hi) {
-        const int64_t m = (lo + hi + 1) >> 1;
-        if (cb[m] <= i) lo = m; else hi = m - 1;
-    }
-    return lo;
-}
-
 #define GRID_STRIDE(i, n) \
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (n); i += (int64_t)gridDim.x * blockDim.x)
 
@@ -81,26 +71,25 @@ __global__ void k_deg_to_i64(int64_t V, const int32_t* deg, int64_t* out) {
     if (blockIdx.x == 0 && threadIdx.x == 0) out[V] = 0;
 }
 
-__global__ void k_sym_keys(int64_t V, int64_t E, const int64_t* cb, CSRView c, uint64_t* keys, uint8_t* keep) {
-    GRID_STRIDE(i, E) {
-        const int64_t u = row_of(cb, V, i);
-        const int32_t v = c.adj[c.beg[u] + (i - cb[u])];
+__global__ void k_sym_keys(int64_t V, const int64_t* cb, CSRView c, uint64_t* keys, uint8_t* keep) {
+    walk_segments(cb, V, [&](int64_t u, int64_t j) {
+        const int64_t i = cb[u] + j;
+        const int32_t v = c.adj[c.beg[u] + j];
         keys[2 * i] = ((uint64_t)u << 32) | (uint32_t)v;
         keys[2 * i + 1] = ((uint64_t)(uint32_t)v << 32) | (uint64_t)u;
         keep[2 * i] = keep[2 * i + 1] = (v != (int32_t)u);
-    }
+    });
 }
 
 __global__ void k_distinct_flags(const uint64_t* keys, int64_t n, uint8_t* flag) {
     GRID_STRIDE(i, n) flag[i] = (i == 0 || keys[i] != keys[i - 1]);
 }
 
-__global__ void k_compact_copy(int64_t V, int64_t E, const int64_t* cb, CSRView c, int32_t* adj_out, int64_t cap) {
-    GRID_STRIDE(i, E) {
-        if (i >= cap) continue;
-        const int64_t u = row_of(cb, V, i);
-        adj_out[i] = c.adj[c.beg[u] + (i - cb[u])];
-    }
+__global__ void k_compact_copy(int64_t V, const int64_t* cb, CSRView c, int32_t* adj_out, int64_t cap) {
+    walk_segments(cb, V, [&](int64_t u, int64_t j) {
+        const int64_t i = cb[u] + j;
+        if (i < cap) adj_out[i] = c.adj[c.beg[u] + j];
+    });
 }
 
 __global__ void k_has_edges(CSRView c, int64_t V, const int32_t* u, const int32_t* v, int64_t n, uint8_t* out) {
@@ -118,111 +107,106 @@ __global__ void k_has_edges(CSRView c, int64_t V, const int32_t* u, const int32_
 
 // ---- batched row updates -------------------------------------------------------------------
 // Ops are sorted, distinct keys (row << 32 | col): `ins` are absent edges to add, `del` present
-// edges to remove. For each touched row r: new length = deg - |del_r| + |ins_r|. When every
-// touched row still fits its capacity the rows are rewritten in place; otherwise the whole CSR
-// is re-laid-out with fresh slack.
+// edges to remove. For each touched row r: new length = deg - |del_r| + |ins_r|. The entries before
+// its first changed position stay where they are; the rest is merged into `tmp`. When every
+// touched row still fits its capacity the merged rests are copied back in place; otherwise the whole
+// CSR is re-laid-out with fresh slack.
 
-// Per touched row (from the merged op list `rows`, sorted distinct): op ranges and new length.
+// A touched row: its op ranges, its first changed position and its new length.
+struct Touched {
+    int64_t beg, ib, ie, db, de;
+    int32_t row, deg, keep, newdeg;
+};
+
+// Per touched row (from the merged op list `rows`, sorted distinct); elen / nlen = entries of its rest
+// before (old ones and inserts) and after the merge.
 __global__ void k_touched_rows(const uint64_t* ins, int64_t n_ins, const uint64_t* del, int64_t n_del,
-                               const int32_t* rows, int64_t n_rows, CSRView c, int64_t* i_lo, int64_t* d_lo,
-                               int32_t* newdeg, int32_t* overflow) {
+                               const int32_t* rows, int64_t n_rows, CSRView c, Touched* touched, int64_t* elen,
+                               int64_t* nlen, int32_t* overflow) {
     GRID_STRIDE(k, n_rows) {
-        const uint64_t r = (uint64_t)(uint32_t)rows[k];
-        const int64_t a = lower_bound_dev(ins, (int64_t)0, n_ins, r << 32);
-        const int64_t b = lower_bound_dev(ins, a, n_ins, (r + 1) << 32);
-        const int64_t x = lower_bound_dev(del, (int64_t)0, n_del, r << 32);
-        const int64_t y = lower_bound_dev(del, x, n_del, (r + 1) << 32);
-        i_lo[k] = a; i_lo[n_rows + k] = b;
-        d_lo[k] = x; d_lo[n_rows + k] = y;
-        const int64_t nd = (int64_t)c.deg[r] - (y - x) + (b - a);
-        if (nd < 0) {  // more deletions than entries: the ops do not match this CSR
+        Touched t;
+        t.row = rows[k];
+        const uint64_t r = (uint64_t)(uint32_t)t.row;
+        t.ib = lower_bound_dev(ins, (int64_t)0, n_ins, r << 32);
+        t.ie = lower_bound_dev(ins, t.ib, n_ins, (r + 1) << 32);
+        t.db = lower_bound_dev(del, (int64_t)0, n_del, r << 32);
+        t.de = lower_bound_dev(del, t.db, n_del, (r + 1) << 32);
+        t.beg = c.beg[r];
+        t.deg = c.deg[r];
+        const int64_t nd = (int64_t)t.deg - (t.de - t.db) + (t.ie - t.ib);
+        uint32_t first = 0xffffffffu;  // smallest column of an op
+        if (t.ib < t.ie) first = (uint32_t)ins[t.ib];
+        if (t.db < t.de && (uint32_t)del[t.db] < first) first = (uint32_t)del[t.db];
+        t.keep = (int32_t)(lower_bound_dev(c.adj, t.beg, t.beg + t.deg, (int32_t)first) - t.beg);
+        t.newdeg = (int32_t)nd;
+        if (nd < t.keep) {  // more deletions than entries: the ops do not match this CSR
             atomicExch(overflow + 1, 1);
-            newdeg[k] = 0;
-            continue;
+            t.newdeg = t.keep;
         }
-        newdeg[k] = (int32_t)nd;
-        if (c.beg[r] + nd > c.beg[r + 1]) atomicExch(overflow, 1);
+        if (t.beg + nd > c.beg[r + 1]) atomicExch(overflow, 1);
+        touched[k] = t;
+        elen[k] = t.deg - t.keep + (t.ie - t.ib);
+        nlen[k] = t.newdeg - t.keep;
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0) elen[n_rows] = nlen[n_rows] = 0;
 }
 
-// Writes the new content of every touched row into `tmp` (at toff[k]): surviving old entries
-// and inserted entries, merged in sorted order. Element-parallel: each element computes its
-// output slot with two binary searches.
-__global__ void k_merge_rows(const uint64_t* ins, const uint64_t* del, const int32_t* rows, int64_t n_rows,
-                             const int64_t* i_lo, const int64_t* d_lo, const int64_t* eoff, int64_t n_elems,
-                             const int64_t* toff, const int32_t* newdeg, CSRView c, int32_t* tmp, uint32_t* tmpw,
+// Merges the rest of every touched row into `tmp` (at noff[k]): surviving old entries and inserted
+// entries in sorted order. Element-parallel: each element computes its output slot with two binary
+// searches of its row's few ops. eoff: exclusive scan of elen. (100K ops on the 4.8M-vertex R-MAT, the
+// three CSRs together: 2.8 ms with a binary search of the rows per entry and every touched row copied
+// whole, 0.7 ms with walk_segments and the rests only; the copy back 2.1 -> 0.35 ms.)
+__global__ void k_merge_rows(const uint64_t* ins, const uint64_t* del, const Touched* touched, int64_t n_rows,
+                             const int64_t* eoff, const int64_t* noff, CSRView c, int32_t* tmp, uint32_t* tmpw,
                              bool weights, uint64_t wseed, uint32_t wlo, uint32_t whi, int32_t* bad) {
-    GRID_STRIDE(e, n_elems) {
-        // row k of element e: eoff is the exclusive scan of (deg + |ins|) over touched rows
-        int64_t lo = 0, hi = n_rows - 1;
-        while (lo < hi) {
-            const int64_t m = (lo + hi + 1) >> 1;
-            if (eoff[m] <= e) lo = m; else hi = m - 1;
-        }
-        const int64_t k = lo, j = e - eoff[k];
-        const int64_t r = rows[k];
-        const int64_t ib = i_lo[k], ie = i_lo[n_rows + k], db = d_lo[k], de = d_lo[n_rows + k];
-        const int64_t rb = c.beg[r], rd = c.deg[r];
-        if (j < rd) {
-            const int32_t x = c.adj[rb + j];
-            const uint64_t key = ((uint64_t)r << 32) | (uint32_t)x;
-            const int64_t pd = lower_bound_dev(del, db, de, key);
-            if (pd < de && del[pd] == key) continue;  // deleted
-            const int64_t pi = lower_bound_dev(ins, ib, ie, key);
-            const int64_t slot = j - (pd - db) + (pi - ib);
-            if (slot < 0 || slot >= newdeg[k]) { atomicExch(bad, 1); continue; }  // ops not consistent with the row
-            tmp[toff[k] + slot] = x;
-            if (weights) tmpw[toff[k] + slot] = c.w[rb + j];
+    walk_segments(eoff, n_rows, [&](int64_t k, int64_t e) {
+        const Touched t = touched[k];
+        const int64_t j = e + t.keep;
+        const uint64_t row_key = (uint64_t)(uint32_t)t.row << 32;
+        if (j < t.deg) {
+            const int32_t x = c.adj[t.beg + j];
+            const uint64_t key = row_key | (uint32_t)x;
+            const int64_t pd = lower_bound_dev(del, t.db, t.de, key);
+            if (pd < t.de && del[pd] == key) return;  // deleted
+            const int64_t pi = lower_bound_dev(ins, t.ib, t.ie, key);
+            const int64_t slot = j - (pd - t.db) + (pi - t.ib);
+            if (slot < t.keep || slot >= t.newdeg) { atomicExch(bad, 1); return; }  // ops not consistent with the row
+            tmp[noff[k] + slot - t.keep] = x;
+            if (weights) tmpw[noff[k] + slot - t.keep] = c.w[t.beg + j];
         } else {
-            const int64_t q = j - rd;  // insert index within the row
-            const uint64_t key = ins[ib + q];
+            const int64_t q = j - t.deg;  // insert index within the row
+            const uint64_t key = ins[t.ib + q];
             const int32_t x = (int32_t)(key & 0xffffffffULL);
-            const int64_t po = lower_bound_dev(c.adj, rb, rb + rd, x) - rb;
-            const int64_t pd = lower_bound_dev(del, db, de, key);
-            const int64_t slot = q + po - (pd - db);
-            if (slot < 0 || slot >= newdeg[k]) { atomicExch(bad, 1); continue; }
-            tmp[toff[k] + slot] = x;
-            if (weights) tmpw[toff[k] + slot] = new_edge_weight((int32_t)r, x, wseed, wlo, whi);
+            const int64_t po = lower_bound_dev(c.adj, t.beg + t.keep, t.beg + t.deg, x) - t.beg;
+            const int64_t pd = lower_bound_dev(del, t.db, t.de, key);
+            const int64_t slot = q + po - (pd - t.db);
+            if (slot < t.keep || slot >= t.newdeg) { atomicExch(bad, 1); return; }
+            tmp[noff[k] + slot - t.keep] = x;
+            if (weights) tmpw[noff[k] + slot - t.keep] = new_edge_weight(t.row, x, wseed, wlo, whi);
         }
-    }
+    });
 }
 
-// Copies touched rows back from tmp into their (unchanged) capacity slots.
-__global__ void k_copy_back(const int32_t* rows, int64_t n_rows, const int32_t* newdeg, const int64_t* toff,
-                            const int64_t* noff, int64_t n_new, const int32_t* tmp, const uint32_t* tmpw,
-                            int64_t* beg, int32_t* deg, int32_t* adj, uint32_t* w) {
-    GRID_STRIDE(e, n_new) {
-        int64_t lo = 0, hi = n_rows - 1;
-        while (lo < hi) {
-            const int64_t m = (lo + hi + 1) >> 1;
-            if (noff[m] <= e) lo = m; else hi = m - 1;
-        }
-        const int64_t k = lo, j = e - noff[k], r = rows[k];
-        adj[beg[r] + j] = tmp[toff[k] + j];
-        if (w) w[beg[r] + j] = tmpw[toff[k] + j];
-    }
+// Copies the merged rests back into their rows (capacities unchanged), and the new lengths.
+__global__ void k_copy_back(const Touched* touched, int64_t n_rows, const int64_t* noff, const int32_t* tmp,
+                            const uint32_t* tmpw, int32_t* deg, int32_t* adj, uint32_t* w) {
+    walk_segments(noff, n_rows, [&](int64_t k, int64_t j) {
+        const int64_t to = touched[k].beg + touched[k].keep + j;
+        adj[to] = tmp[noff[k] + j];
+        if (w) w[to] = tmpw[noff[k] + j];
+    });
+    GRID_STRIDE(k, n_rows) deg[touched[k].row] = touched[k].newdeg;
 }
 
-__global__ void k_set_deg(const int32_t* rows, int64_t n_rows, const int32_t* newdeg, int32_t* deg) {
-    GRID_STRIDE(k, n_rows) deg[rows[k]] = newdeg[k];
+__global__ void k_set_deg(const Touched* touched, int64_t n_rows, int32_t* deg) {
+    GRID_STRIDE(k, n_rows) deg[touched[k].row] = touched[k].newdeg;
 }
 
 __global__ void k_mark_rows(const uint64_t* a, int64_t na, const uint64_t* b, int64_t nb, uint8_t* flag) {
     GRID_STRIDE(i, na + nb) flag[(i < na ? a[i] : b[i - na]) >> 32] = 1;
 }
 
-__global__ void k_row_len_plus_ins(const int32_t* rows, int64_t n_rows, const int64_t* i_lo, CSRView c,
-                                   int64_t* out) {
-    GRID_STRIDE(k, n_rows) out[k] = (int64_t)c.deg[rows[k]] + (i_lo[n_rows + k] - i_lo[k]);
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[n_rows] = 0;
-}
-
-__global__ void k_i32_to_i64(const int32_t* in, int64_t n, int64_t* out) {
-    GRID_STRIDE(k, n) out[k] = in[k];
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = 0;
-}
-
-// Full re-layout: new capacities from new lengths, then every row copied (touched rows from tmp).
+// Full re-layout: new capacities from new lengths, then every row copied (the merged rests of touched rows from tmp).
 __global__ void k_new_caps(int64_t V, const int32_t* deg, int64_t* capv) {
     GRID_STRIDE(v, V) capv[v] = row_capacity(deg[v]);
     if (blockIdx.x == 0 && threadIdx.x == 0) capv[V] = 0;
@@ -230,28 +214,23 @@ __global__ void k_new_caps(int64_t V, const int32_t* deg, int64_t* capv) {
 
 __global__ void k_relayout_rows(int64_t V, const int64_t* old_beg, const int32_t* old_adj, const uint32_t* old_w,
                                 const int32_t* deg, const int64_t* new_beg, int32_t* new_adj, uint32_t* new_w,
-                                const int32_t* touched_slot, const int64_t* toff, const int32_t* tmp,
-                                const uint32_t* tmpw) {
-    // one warp per row
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t v = warp; v < V; v += nwarps) {
+                                const int32_t* touched_slot, const Touched* touched, const int64_t* noff,
+                                const int32_t* tmp, const uint32_t* tmpw) {
+    walk_segments(new_beg, V, [&](int64_t v, int64_t j) {
+        if (j >= deg[v]) return;  // (slack)
         const int32_t k = touched_slot[v];
-        const int32_t* src = k >= 0 ? tmp + toff[k] : old_adj + old_beg[v];
-        const uint32_t* srcw = k >= 0 ? tmpw + toff[k] : (old_w ? old_w + old_beg[v] : nullptr);
-        const int64_t d = deg[v], nb = new_beg[v];
-        for (int64_t j = lane; j < d; j += 32) {
-            new_adj[nb + j] = src[j];
-            if (new_w) new_w[nb + j] = srcw[j];
-        }
-    }
+        const int64_t to = new_beg[v] + j, from = old_beg[v] + j;
+        const bool merged = k >= 0 && j >= touched[k].keep;
+        const int64_t m = merged ? noff[k] + j - touched[k].keep : 0;
+        new_adj[to] = merged ? tmp[m] : old_adj[from];
+        if (new_w) new_w[to] = merged ? tmpw[m] : old_w[from];
+    });
 }
 
 __global__ void k_fill_i32(int32_t* p, int64_t n, int32_t v) { GRID_STRIDE(i, n) p[i] = v; }
 
-__global__ void k_mark_slots(const int32_t* rows, int64_t n_rows, int32_t* slot) {
-    GRID_STRIDE(k, n_rows) slot[rows[k]] = (int32_t)k;
+__global__ void k_mark_slots(const Touched* touched, int64_t n_rows, int32_t* slot) {
+    GRID_STRIDE(k, n_rows) slot[touched[k].row] = (int32_t)k;
 }
 
 __global__ void k_bin_flags(int64_t V, const int32_t* deg, int32_t small, int32_t large, uint8_t* f0, uint8_t* f1,
@@ -478,7 +457,7 @@ int store_build_sym(gir_dev* g) {
     GIR_TRY(ensure_n(g, g->scratch[3], 2 * E + 1, &keep));
     GIR_TRY(compact_offsets(g, g->fw, cb));
     if (E > 0) {
-        k_sym_keys<<<grid_for(g, E, kBlock), kBlock, 0, g->stream>>>(V, E, cb, view(g->fw), keys, keep);
+        k_sym_keys<<<grid_for(g, E, kBlock), kBlock, 0, g->stream>>>(V, cb, view(g->fw), keys, keep);
         GIR_LAUNCH(g, "k_sym_keys");
     }
     int64_t n = 0;
@@ -498,7 +477,7 @@ int store_compact_csr(gir_dev* g, const DevCSR& c, int64_t* beg_out, int32_t* ad
     // beg_out / adj_out: device pointers (V+1 / cap entries)
     GIR_TRY(compact_offsets(g, c, beg_out));
     if (c.E > 0 && adj_out && cap > 0) {
-        k_compact_copy<<<grid_for(g, c.E, kBlock), kBlock, 0, g->stream>>>(g->V, c.E, beg_out, view(c), adj_out, cap);
+        k_compact_copy<<<grid_for(g, c.E, kBlock), kBlock, 0, g->stream>>>(g->V, beg_out, view(c), adj_out, cap);
         GIR_LAUNCH(g, "k_compact_copy");
     }
     return GIR_OK;
@@ -516,9 +495,10 @@ int store_apply_ops(gir_dev* g, DevCSR& c, const uint64_t* ins, int64_t n_ins, c
     if (n_ins + n_del == 0) return GIR_OK;
     const int64_t V = g->V;
     const int64_t n_ops = n_ins + n_del;
-    int32_t *rows = nullptr, *newdeg = nullptr, *tmp = nullptr;
+    int32_t *rows = nullptr, *tmp = nullptr;
     uint8_t* flag = nullptr;
-    int64_t *i_lo = nullptr, *d_lo = nullptr, *eoff = nullptr, *noff = nullptr;
+    int64_t *eoff = nullptr, *noff = nullptr;
+    Touched* touched = nullptr;
     uint32_t* tmpw = nullptr;
     GIR_TRY(ensure_n(g, g->scratch[4], V + 1, &flag));
     GIR_TRY(ensure_n(g, g->scratch[5], V + 1, &rows));
@@ -530,22 +510,15 @@ int store_apply_ops(gir_dev* g, DevCSR& c, const uint64_t* ins, int64_t n_ins, c
     GIR_TRY(select_flagged_iota(g, flag, rows, V, &n_rows));
 
     int32_t* overflow = nullptr;
-    GIR_TRY(ensure_n(g, g->scratch[9], 2 * n_rows + 2, &i_lo));
-    GIR_TRY(ensure_n(g, g->scratch[13], 2 * n_rows + 2, &d_lo));
-    GIR_TRY(ensure_n(g, g->scratch[14], n_rows + 1, &newdeg));
+    GIR_TRY(ensure_n(g, g->scratch[9], n_rows + 1, &touched));
     GIR_TRY(ensure_n(g, g->scratch[10], n_rows + 1, &eoff));
     GIR_TRY(ensure_n(g, g->scratch[11], n_rows + 1, &noff));
     GIR_TRY(ensure_n(g, g->scratch[12], 4, &overflow));
     GIR_CUDA(g, cudaMemsetAsync(overflow, 0, 2 * sizeof(int32_t), g->stream));
     k_touched_rows<<<grid_for(g, n_rows, kBlock), kBlock, 0, g->stream>>>(ins, n_ins, del, n_del, rows, n_rows, view(c),
-                                                                           i_lo, d_lo, newdeg, overflow);
+                                                                           touched, eoff, noff, overflow);
     GIR_LAUNCH(g, "k_touched_rows");
-    // element space: old entries + inserts of every touched row
-    k_row_len_plus_ins<<<grid_for(g, n_rows, kBlock), kBlock, 0, g->stream>>>(rows, n_rows, i_lo, view(c), eoff);
-    GIR_LAUNCH(g, "k_row_len_plus_ins");
     GIR_TRY(exclusive_scan_i64(g, eoff, eoff, n_rows + 1));
-    k_i32_to_i64<<<grid_for(g, n_rows, kBlock), kBlock, 0, g->stream>>>(newdeg, n_rows, noff);
-    GIR_LAUNCH(g, "k_i32_to_i64");
     GIR_TRY(exclusive_scan_i64(g, noff, noff, n_rows + 1));
     int64_t h[2] = {0, 0};
     int32_t ovf = 0;
@@ -555,13 +528,13 @@ int store_apply_ops(gir_dev* g, DevCSR& c, const uint64_t* ins, int64_t n_ins, c
     GIR_CUDA(g, cudaStreamSynchronize(g->stream));
     const int64_t n_elems = h[0], n_new = h[1];
     const bool wts = weights && c.w;
-    // tmp holds each touched row's new content at noff[k] (the merged rows are written there)
+    // tmp holds the merged rest of touched row k at noff[k]
     GIR_TRY(ensure_n(g, g->stage_out, n_new + 4, &tmp));
     if (wts) GIR_TRY(ensure_n(g, g->scratch[3], n_new + 4, &tmpw));
     if (n_elems > 0) {
         k_merge_rows<<<grid_for(g, n_elems, kBlock), kBlock, 0, g->stream>>>(
-            ins, del, rows, n_rows, i_lo, d_lo, eoff, n_elems, noff, newdeg, view(c), tmp, tmpw, wts, g->wrule_seed,
-            g->wrule_lo, g->wrule_hi, overflow + 1);
+            ins, del, touched, n_rows, eoff, noff, view(c), tmp, tmpw, wts, g->wrule_seed, g->wrule_lo, g->wrule_hi,
+            overflow + 1);
         GIR_LAUNCH(g, "k_merge_rows");
     }
     int32_t inconsistent = 0;
@@ -570,14 +543,9 @@ int store_apply_ops(gir_dev* g, DevCSR& c, const uint64_t* ins, int64_t n_ins, c
     if (inconsistent)
         return fail(g, GIR_ERR_MALFORMED, "edge update: the backward CSR is not the transpose of the forward CSR");
     if (!ovf) {
-        if (n_new > 0) {
-            k_copy_back<<<grid_for(g, n_new, kBlock), kBlock, 0, g->stream>>>(rows, n_rows, newdeg, noff, noff, n_new,
-                                                                              tmp, tmpw, c.beg, c.deg, c.adj,
-                                                                              wts ? c.w : nullptr);
-            GIR_LAUNCH(g, "k_copy_back");
-        }
-        k_set_deg<<<grid_for(g, n_rows, kBlock), kBlock, 0, g->stream>>>(rows, n_rows, newdeg, c.deg);
-        GIR_LAUNCH(g, "k_set_deg");
+        k_copy_back<<<grid_for(g, n_new > n_rows ? n_new : n_rows, kBlock), kBlock, 0, g->stream>>>(
+            touched, n_rows, noff, tmp, tmpw, c.deg, c.adj, wts ? c.w : nullptr);
+        GIR_LAUNCH(g, "k_copy_back");
     } else {
         // Some row outgrew its slack: new layout for the whole CSR.
         trace_mark(g, "store: merge before relayout");
@@ -585,11 +553,11 @@ int store_apply_ops(gir_dev* g, DevCSR& c, const uint64_t* ins, int64_t n_ins, c
         int64_t* capv = nullptr;
         GIR_TRY(ensure_n(g, g->scratch[0], V + 1, &slot));
         GIR_TRY(ensure_n(g, g->scratch[1], V + 1, &capv));
-        k_set_deg<<<grid_for(g, n_rows, kBlock), kBlock, 0, g->stream>>>(rows, n_rows, newdeg, c.deg);
+        k_set_deg<<<grid_for(g, n_rows, kBlock), kBlock, 0, g->stream>>>(touched, n_rows, c.deg);
         GIR_LAUNCH(g, "k_set_deg");
         k_fill_i32<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(slot, V, -1);
         GIR_LAUNCH(g, "k_fill_i32");
-        k_mark_slots<<<grid_for(g, n_rows, kBlock), kBlock, 0, g->stream>>>(rows, n_rows, slot);
+        k_mark_slots<<<grid_for(g, n_rows, kBlock), kBlock, 0, g->stream>>>(touched, n_rows, slot);
         GIR_LAUNCH(g, "k_mark_slots");
         k_new_caps<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, c.deg, capv);
         GIR_LAUNCH(g, "k_new_caps");
@@ -603,8 +571,8 @@ int store_apply_ops(gir_dev* g, DevCSR& c, const uint64_t* ins, int64_t n_ins, c
         uint32_t* nw = nullptr;
         GIR_TRY(dev_alloc_n(g, &nadj, total > 0 ? total : 4));
         if (c.w) GIR_TRY(dev_alloc_n(g, &nw, total > 0 ? total : 4));
-        k_relayout_rows<<<grid_for(g, V * 32, kBlock), kBlock, 0, g->stream>>>(V, c.beg, c.adj, c.w, c.deg, nbeg, nadj,
-                                                                                 nw, slot, noff, tmp, tmpw);
+        k_relayout_rows<<<grid_for(g, total, kBlock), kBlock, 0, g->stream>>>(V, c.beg, c.adj, c.w, c.deg, nbeg, nadj,
+                                                                                 nw, slot, touched, noff, tmp, tmpw);
         GIR_LAUNCH(g, "k_relayout_rows");
         dev_free(g, c.beg);
         dev_free(g, c.adj);
