@@ -97,6 +97,45 @@ struct ForestLevel {
     }
 };
 
+// The same level bottom-up: every vertex without a parent takes the first entry of its row that is in
+// the frontier (bits) and in its SCC.
+__global__ void __launch_bounds__(kBlock) k_forest_up(int64_t V, CSRView sym, const int32_t* scc, const uint32_t* bits,
+                                                      int32_t* parent, Queue out, unsigned long long* cnt) {
+    __shared__ int32_t s_st[kBlock / 32][kStage];
+    int n_st = 0;
+    auto deg = [&](int32_t x) { return sym.deg[x]; };
+    for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < V; base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t v = base + threadIdx.x;
+        const bool want = v < V && parent[v] == -1;
+        const int32_t mine = want ? scc[v] : -1;
+        const int32_t p = first_hit(sym.adj, want ? sym.beg[v] : 0, want ? sym.deg[v] : 0, want, mine,
+                                    [&](int32_t w, int32_t c) { return ((bits[w >> 5] >> (w & 31)) & 1u) && scc[w] == c; });
+        if (p >= 0) parent[v] = p;
+        queue_push(p >= 0, (int32_t)v, s_st[threadIdx.x >> 5], n_st, out, deg, cnt);
+    }
+    queue_flush(s_st[threadIdx.x >> 5], n_st, out, deg, cnt);
+}
+
+// Bottom-up where the frontier's rows hold over four times as many entries as there are vertices left
+// (a vertex left reads a few entries to its first hit; 4.8M-vertex R-MAT: both levels of over 2^22
+// entries, 0.6 ms each top-down).
+struct ForestUp {
+    CSRView sym;
+    const int32_t* scc;
+    int32_t* parent;
+    uint32_t* bits;
+    int64_t V;
+    bool wants(int64_t total, int64_t queued) const { return total > 4 * (V - queued); }
+    int launch(gir_dev* g, const Queue& in, int64_t nq, const Queue& out, unsigned long long* cnt) const {
+        GIR_CUDA(g, cudaMemsetAsync(bits, 0, sizeof(uint32_t) * (V / 32 + 1), g->stream));
+        k_frontier_bits<<<grid_for(g, nq, kBlock), kBlock, 0, g->stream>>>(in.v, nq, bits, bits);
+        GIR_LAUNCH(g, "k_frontier_bits");
+        k_forest_up<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, sym, scc, bits, parent, out, cnt);
+        GIR_LAUNCH(g, "k_forest_up");
+        return GIR_OK;
+    }
+};
+
 // ---- Deep graphs: a spanning forest without levels ---------------------------------------------
 // Tarjan-Vishkin takes any rooted spanning forest. Where the BFS forest is still growing after
 // deep_levels(V) levels (a road network has thousands), the forest comes from union-find over H
@@ -292,35 +331,37 @@ __global__ void k_pre_level(const int32_t* q, int64_t n, const int32_t* parent, 
 
 __global__ void k_pre_roots(const int32_t* q, int64_t n, int32_t* pre) { GRID_STRIDE(i, n) pre[q[i]] = 0; }
 
-// Per-vertex tree data packed for the non-tree sweep: one 16-byte gather per neighbour instead of
-// four scattered 4-byte ones. x = pre, y = nd, z = parent, w = scc.
-__global__ void k_pack_vinfo(int64_t V, const int32_t* pre, const int32_t* nd, const int32_t* parent,
-                             const int32_t* scc, int4* vinfo) {
-    GRID_STRIDE(v, V) vinfo[v] = make_int4(pre[v], nd[v], parent[v], scc[v]);
+// Per-vertex tree data packed for the sweeps over H: one 8-byte gather per neighbour. x = pre, y = scc.
+__global__ void k_pack_keys(int64_t V, const int32_t* pre, const int32_t* scc, int2* key) {
+    GRID_STRIDE(v, V) key[v] = make_int2(pre[v], scc[v]);
 }
 
-// Rule-1 unions from a sample before the full sweep: every vertex of H takes the first kSample
-// entries of its row, and the non-tree edges among them whose ends are unrelated in the forest
-// (neither an ancestor of the other) union the two ends' tree edges. After a flatten (every uf
-// entry its root), the full sweep's cheap uf[u] != uf[w] test rejects nearly every pair the
-// sample already joined (on a power-law graph the giant block takes most vertices), instead of
-// each pair walking two find chains. Unions are idempotent, so the sample changes no class.
+// Before the full sweep, a sample: every vertex of H takes the first kSample entries of its row for rule 1
+// and for its low and high. After the unions, and rule 2 with low and high of the sample carried up the
+// levels (both are facts, if not all of them), nearly every tree edge of a power-law graph is in its final
+// class: a pair already joined costs the sweep one test, and most rows nothing at all (k_sweep_len).
+// Unions are idempotent, so the sample changes no class.
 constexpr int kSample = 4;
 
-__global__ void k_nontree_sample(int64_t V, HView h, const int4* vinfo, int32_t* uf, unsigned long long* err) {
+__global__ void k_nontree_sample(int64_t V, HView h, const int2* key, const int32_t* nd, int32_t* low, int32_t* high,
+                                 int32_t* uf, unsigned long long* err) {
     GRID_STRIDE(u, V) {
         const int32_t d = h.sym.deg[u];
         if (d == 0) continue;
-        const int4 iu = vinfo[u];
+        const int2 ku = key[u];
         const int64_t b = h.sym.beg[u];
+        int32_t lo = ku.x, hi = ku.x;
         for (int j = 0; j < kSample && j < d; ++j) {
             const int32_t w = h.sym.adj[b + j];
-            const int4 iw = vinfo[w];
-            if (iu.w != iw.w || iw.z == (int32_t)u || iu.z == w) continue;  // other SCC, or a tree edge
-            const bool w_under_u = iw.x >= iu.x && iw.x < iu.x + iu.y;
-            const bool u_under_w = iu.x >= iw.x && iu.x < iw.x + iw.y;
-            if (!w_under_u && !u_under_w && uf[u] != uf[w]) uf_union(uf, (int32_t)u, w, err);
+            const int2 kw = key[w];
+            if (ku.y != kw.y) continue;  // other SCC
+            lo = kw.x < lo ? kw.x : lo;
+            hi = kw.x > hi ? kw.x : hi;
+            const bool apart = kw.x > ku.x ? kw.x >= ku.x + nd[u] : ku.x >= kw.x + nd[w];
+            if (apart && uf[u] != uf[w]) uf_union(uf, (int32_t)u, w, err);
         }
+        low[u] = lo;
+        high[u] = hi;
     }
 }
 
@@ -333,43 +374,83 @@ __global__ void k_uf_flatten(int32_t* uf, int64_t V) {
     }
 }
 
-// One sweep over the non-tree edges of H: low / high of every vertex from its own non-tree
-// neighbours, and rule 1 (once per edge, from its endpoint with the smaller pre) for edges
-// between unrelated endpoints.
-__device__ __forceinline__ void nontree_entry(int32_t u, int32_t w, const int4* vinfo, int32_t* low, int32_t* high,
-                                              int32_t* uf, unsigned long long* err) {
-    const int4 iu = vinfo[u], iw = vinfo[w];
-    if (iu.w != iw.w || iw.z == u || iu.z == w) return;  // other SCC, or a tree edge
-    const int32_t pw = iw.x;
-    if (pw < low[u]) atomicMin(&low[u], pw);  // (plain pre-checks: a hub's row is swept by many
-    if (pw > high[u]) atomicMax(&high[u], pw);  //  threads, most of which change nothing)
-    if (iu.x < pw && iu.x + iu.y <= pw && uf[u] != uf[w]) uf_union(uf, u, w, err);
+// Which rows the sweep below can leave out. After the sample nearly all tree edges are in one class G. Rule 2
+// has nothing left to say about a vertex whose tree edge is in its parent's class already ("decided", and
+// a root's child always), and low / high of a vertex matter only to itself and its ancestors: they are
+// needed under undecided vertices only. A row of class G whose vertex and ancestors are all decided is
+// left out: an edge from it to another vertex of G joins nothing, one to a vertex outside G is in that
+// vertex's row, which is swept and takes rule 1 in both directions.
+__global__ void k_need_level(const int32_t* q, int64_t n, const int32_t* parent, const int32_t* uf, uint8_t* need) {
+    GRID_STRIDE(i, n) {
+        const int32_t v = q[i], p = parent[v];
+        need[v] = need[p] || (parent[p] != p && uf[v] != uf[p]);
+    }
+}
+__global__ void k_sweep_len(int64_t V, const int32_t* hdeg, const int32_t* uf, const uint8_t* need, const int32_t* giant,
+                            int32_t* len) {
+    const int32_t g = *giant;
+    GRID_STRIDE(v, V) len[v] = uf[v] == g && !need[v] ? 0 : hdeg[v];
 }
 
-// Rows of at most kHeavyRow entries, a warp per 32 rows; the longer rows go to k_nontree_heavy,
-// which spreads their entries over the whole grid.
-__global__ void __launch_bounds__(kBlock) k_nontree(int64_t V, HView h, const int4* vinfo, int32_t* low, int32_t* high,
-                                                    int32_t* uf, unsigned long long* err) {
-    __shared__ int64_t s_excl[kBlock / 32][33];
-    __shared__ int32_t s_u[kBlock / 32][32];
-    const int wib = threadIdx.x >> 5;
-    warp_sweep_rows(
-        h.sym.beg, h.sym.deg, h.sym.adj, 0, V, s_excl[wib], s_u[wib],
-        [&](int32_t u, int32_t w, int64_t) { nontree_entry(u, w, vinfo, low, high, uf, err); }, kHeavyRow);
+// One sweep over the entries of H: low / high of every vertex from its neighbours, and rule 1 for edges
+// between unrelated endpoints. Tree edges need no test: a parent's pre never lies below the parent's own
+// subtree nor a child's beyond it, so neither changes what rule 2 reads off low and high, and an edge
+// between related ends is no rule-1 edge. Per entry one 8-byte gather, (pre, scc) of the neighbour; the
+// row's own values are the same for neighbouring lanes. A warp's lanes of one row reduce their minimum
+// and maximum by shuffles, so a row costs an atomic per 32 entries at most. Rows are cut into even runs
+// whatever their length. Bound by the L2's random gathers: 138M entries of the 4.8M-vertex R-MAT took
+// 2.1 ms (a warp per 32 rows, 16-byte gathers), 1.46 ms so, 0.11 ms with the rows above left out.
+__global__ void __launch_bounds__(kBlock) k_nontree(int64_t V, const int64_t* off, HView h, const int2* key,
+                                                    const int32_t* nd, int32_t* low, int32_t* high, int32_t* uf,
+                                                    unsigned long long* err) {
+    const int ln = lane_id();
+    struct Got {
+        int2 kw, ku;
+        int32_t end;
+    };
+    walk_rows_of<4>(
+        off, V, h.sym.beg, h.sym.adj,
+        [&](int32_t u, int32_t w) {
+            Got g;
+            g.kw = key[w];
+            g.ku = key[u];
+            g.end = g.ku.x + nd[u];
+            return g;
+        },
+        [&](bool on, int32_t u, int32_t w, int x, const Got& g) {
+            int32_t lo = INT32_MAX, hi = -1;
+            if (on && g.kw.y == g.ku.y) {
+                lo = hi = g.kw.x;
+                const int32_t ru = uf[u], rw = uf[w];
+                if (ru != rw && (g.kw.x > g.ku.x ? g.kw.x >= g.end : g.ku.x >= g.kw.x + nd[w])) uf_union(uf, u, w, err);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {  // the row's first lane ends up with its minimum and maximum
+                const int ox = __shfl_down_sync(0xffffffffu, x, o);
+                const int32_t ol = __shfl_down_sync(0xffffffffu, lo, o), oh = __shfl_down_sync(0xffffffffu, hi, o);
+                if (ln + o < 32 && ox == x) {
+                    lo = ol < lo ? ol : lo;
+                    hi = oh > hi ? oh : hi;
+                }
+            }
+            const int before = __shfl_up_sync(0xffffffffu, x, 1);
+            if (on && (ln == 0 || before != x)) {
+                if (lo < low[u]) atomicMin(&low[u], lo);
+                if (hi > high[u]) atomicMax(&high[u], hi);
+            }
+        });
 }
 
-__global__ void k_nontree_heavy(const int32_t* rows, const int64_t* pref, int64_t n, HView h, const int4* vinfo,
-                                int32_t* low, int32_t* high, int32_t* uf, unsigned long long* err) {
-    grid_sweep_heavy_rows(rows, pref, n, h.sym.beg, h.sym.adj,
-                          [&](int32_t u, int32_t w, int64_t) { nontree_entry(u, w, vinfo, low, high, uf, err); });
-}
-
-__global__ void k_lowhigh_level(const int32_t* q, int64_t n, const int32_t* parent, int32_t* low, int32_t* high) {
+// low / high of one level's vertices into their parents (need: only of the vertices that need them).
+__global__ void k_lowhigh_level(const int32_t* q, int64_t n, const int32_t* parent, const uint8_t* need, int32_t* low,
+                                int32_t* high) {
     GRID_STRIDE(i, n) {
         const int32_t v = q[i];
-        const int32_t p = parent[v];
-        atomicMin(&low[p], low[v]);
-        atomicMax(&high[p], high[v]);
+        if (need && !need[v]) continue;
+        const int32_t p = parent[v], lo = low[v], hi = high[v];
+        if (lo < low[p]) atomicMin(&low[p], lo);  // (plain pre-checks: a hub has a million children)
+        if (hi > high[p]) atomicMax(&high[p], hi);
     }
 }
 
@@ -491,7 +572,7 @@ static int euler_forest(gir_dev* g, const CSRView& h, const int32_t* scc, int32_
     const int gn = grid_for(g, n + 1, kBlock);
     k_tree_arcs<<<gn, kBlock, 0, g->stream>>>(picked, m, arcs);
     GIR_LAUNCH(g, "k_tree_arcs");
-    GIR_TRY(sort_keys_u64(g, arcs, atmp, n, 64));
+    GIR_TRY(sort_keys_u64(g, arcs, atmp, n, edge_key_bits(g->V)));
     k_euler_next<<<gn, kBlock, 0, g->stream>>>(arcs, n, scc, twin, ja);
     GIR_LAUNCH(g, "k_euler_next");
     for (int64_t reach = 1; reach < n; reach *= 2) {
@@ -591,8 +672,10 @@ int bct_build(gir_dev* g) {
     GIR_CUDA(g, cudaMemsetAsync(ctl, 0, sizeof(unsigned long long) * kLoopWords, g->stream));
     k_roots<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, scc, nontrivial, hdeg, parent, fq, ctl + W_Q);
     GIR_LAUNCH(g, "k_roots");
+    uint32_t* bits = nullptr;
+    GIR_TRY(ensure_n(g, g->work[5], V / 32 + 2, &bits));
     FrontierRun run;
-    GIR_TRY(run_frontier(g, ForestLevel{h.sym, scc, parent}, fq, ctl, run, V < kEulerMaxV ? deep_levels(V) : INT64_MAX));
+    GIR_TRY(run_frontier(g, ForestLevel{h.sym, scc, parent}, ForestUp{h.sym, scc, parent, bits, V}, fq, ctl, run, V < kEulerMaxV ? deep_levels(V) : INT64_MAX));
     const bool deep = !run.done();
     trace_mark(g, deep ? "bct: forest levels (given up)" : "bct: forest");
     std::vector<int64_t> lvl_off{0};
@@ -617,7 +700,7 @@ int bct_build(gir_dev* g) {
         GIR_LAUNCH(g, "k_child_keys");
         int64_t nc = 0;
         GIR_TRY(select_flagged_u64(g, keys, flag, ktmp, V, &nc));
-        GIR_TRY(sort_keys_u64(g, ktmp, keys, nc, 64));
+        GIR_TRY(sort_keys_u64(g, ktmp, keys, nc, edge_key_bits(g->V)));
         if (nc > 0) {
             k_child_nd<<<grid_for(g, nc, kBlock), kBlock, 0, g->stream>>>(ktmp, nc, nd, scan);
             GIR_LAUNCH(g, "k_child_nd");
@@ -642,33 +725,51 @@ int bct_build(gir_dev* g) {
     GIR_CUDA(g, cudaMemcpyAsync(high, pre, sizeof(int32_t) * V, cudaMemcpyDeviceToDevice, g->stream));
     k_uf_init<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(uf, V);
     GIR_LAUNCH(g, "k_uf_init");
-    int4* vinfo = nullptr;
-    GIR_TRY(ensure_n(g, g->work[5], V + 1, &vinfo));
-    k_pack_vinfo<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, pre, nd, parent, scc, vinfo);
-    GIR_LAUNCH(g, "k_pack_vinfo");
-    k_nontree_sample<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, h, vinfo, uf, &cnt[C_ERR]);
+    int2* key = nullptr;
+    GIR_TRY(ensure_n(g, g->work[5], V + 1, &key));
+    k_pack_keys<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, pre, scc, key);
+    GIR_LAUNCH(g, "k_pack_keys");
+    k_nontree_sample<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, h, key, nd, low, high, uf, &cnt[C_ERR]);
     GIR_LAUNCH(g, "k_nontree_sample");
+    auto carry_up = [&](const uint8_t* only) -> int {
+        for (int L = D - 1; L >= 1; --L) {
+            const int64_t n = lvl_off[L + 1] - lvl_off[L];
+            if (n == 0) continue;
+            k_lowhigh_level<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(order + lvl_off[L], n, parent, only, low,
+                                                                             high);
+            GIR_LAUNCH(g, "k_lowhigh_level");
+        }
+        return GIR_OK;
+    };
+    int32_t* len = hdeg;
+    uint8_t* need = nullptr;
+    if (!deep) {
+        GIR_TRY(carry_up(nullptr));
+        k_rule2<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, parent, pre, nd, low, high, uf, &cnt[C_ERR]);
+        GIR_LAUNCH(g, "k_rule2");
+    }
     k_uf_flatten<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(uf, V);
     GIR_LAUNCH(g, "k_uf_flatten");
-    k_nontree<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, h, vinfo, low, high, uf, &cnt[C_ERR]);
-    GIR_LAUNCH(g, "k_nontree");
-    {
-        int64_t n_heavy = 0;  // (first / scan are free after the preorder)
-        int32_t* heavy = reinterpret_cast<int32_t*>(first);
-        GIR_TRY(heavy_rows(g, h.sym.deg, V, kHeavyRow, flag, heavy, scan, &n_heavy));
-        if (n_heavy > 0) {
-            k_nontree_heavy<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(heavy, scan, n_heavy, h, vinfo, low, high,
-                                                                             uf, &cnt[C_ERR]);
-            GIR_LAUNCH(g, "k_nontree_heavy");
+    if (!deep) {
+        int32_t* giant = reinterpret_cast<int32_t*>(cnt + C_N);
+        need = flag;
+        len = off;  // (sibling offsets are no longer needed)
+        GIR_CUDA(g, cudaMemsetAsync(need, 0, V, g->stream));
+        for (int L = 1; L < D; ++L) {
+            const int64_t n = lvl_off[L + 1] - lvl_off[L];
+            if (n == 0) continue;
+            k_need_level<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(order + lvl_off[L], n, parent, uf, need);
+            GIR_LAUNCH(g, "k_need_level");
         }
+        GIR_TRY(sample_mode(g, g->sym, uf, giant));
+        k_sweep_len<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, hdeg, uf, need, giant, len);
+        GIR_LAUNCH(g, "k_sweep_len");
     }
+    GIR_TRY(scan_degrees(g, len, V, scan));  // (scan is free after the preorder)
+    k_nontree<<<g->num_sms * 8, kBlock, 0, g->stream>>>(V, scan, h, key, nd, low, high, uf, &cnt[C_ERR]);
+    GIR_LAUNCH(g, "k_nontree");
     if (deep) GIR_TRY(subtree_windows(g, order, n_tree, nd, low, high));
-    for (int L = D - 1; L >= 1; --L) {
-        const int64_t n = lvl_off[L + 1] - lvl_off[L];
-        if (n == 0) continue;
-        k_lowhigh_level<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(order + lvl_off[L], n, parent, low, high);
-        GIR_LAUNCH(g, "k_lowhigh_level");
-    }
+    else GIR_TRY(carry_up(need));
     trace_mark(g, "bct: low/high + rule 1");
     // 4. rule 2
     k_rule2<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, parent, pre, nd, low, high, uf, &cnt[C_ERR]);

@@ -178,8 +178,8 @@ int build_direction(gir_dev* g, DevCSR& c, const int32_t* beg, const int32_t* ad
     GIR_CUDA(g, cudaStreamSynchronize(g->stream));
     int64_t n = E;
     if (h_unsorted) {
-        if (w) GIR_TRY(sort_pairs_u64(g, keys, ktmp, wv, wtmp, E, 64));
-        else GIR_TRY(sort_keys_u64(g, keys, ktmp, E, 64));
+        if (w) GIR_TRY(sort_pairs_u64(g, keys, ktmp, wv, wtmp, E, edge_key_bits(g->V)));
+        else GIR_TRY(sort_keys_u64(g, keys, ktmp, E, edge_key_bits(g->V)));
         k_distinct<<<grid_for(g, E, kBlock), kBlock, 0, g->stream>>>(keys, E, flag);
         GIR_LAUNCH(g, "k_distinct");
         GIR_TRY(select_flagged_u64(g, keys, flag, ktmp, E, &n));
@@ -553,7 +553,7 @@ int apply_batch_impl(gir_dev* g, const int32_t* u, const int32_t* v, const uint8
     k_batch_keys<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>((const int32_t*)du, (const int32_t*)dv, n, V, keys,
                                                                    pos, cnt);
     if ((rc = cuda_check(g, cudaGetLastError(), "k_batch_keys")) ||
-        (rc = sort_pairs_u64_i64(g, keys, ktmp, pos, ptmp, n, 64))) {
+        (rc = sort_pairs_u64_i64(g, keys, ktmp, pos, ptmp, n, edge_key_bits(g->V)))) {
         cleanup();
         return rc;
     }
@@ -600,7 +600,7 @@ int apply_batch_impl(gir_dev* g, const int32_t* u, const int32_t* v, const uint8
     fsd = fsi + 2 * np + 2;
     k_pair_keys<<<grid_for(g, np, kBlock), kBlock, 0, g->stream>>>(ins_k, n_ins, del_k, n_del, pairs);
     GIR_LAUNCH(g, "k_pair_keys");
-    GIR_TRY(sort_keys_u64(g, pairs, ptmp2, np, 64));
+    GIR_TRY(sort_keys_u64(g, pairs, ptmp2, np, edge_key_bits(g->V)));
     k_distinct<<<grid_for(g, np, kBlock), kBlock, 0, g->stream>>>(pairs, np, pflag);
     GIR_LAUNCH(g, "k_distinct");
     int64_t npu = 0;
@@ -618,12 +618,12 @@ int apply_batch_impl(gir_dev* g, const int32_t* u, const int32_t* v, const uint8
     if (n_ins) {
         k_transpose_keys<<<grid_for(g, n_ins, kBlock), kBlock, 0, g->stream>>>(ins_k, n_ins, tk);
         GIR_LAUNCH(g, "k_transpose_keys");
-        GIR_TRY(sort_keys_u64(g, tk, ins_k, n_ins, 64));
+        GIR_TRY(sort_keys_u64(g, tk, ins_k, n_ins, edge_key_bits(g->V)));
     }
     if (n_del) {
         k_transpose_keys<<<grid_for(g, n_del, kBlock), kBlock, 0, g->stream>>>(del_k, n_del, tk2);
         GIR_LAUNCH(g, "k_transpose_keys");
-        GIR_TRY(sort_keys_u64(g, tk2, del_k, n_del, 64));
+        GIR_TRY(sort_keys_u64(g, tk2, del_k, n_del, edge_key_bits(g->V)));
     }
     GIR_TRY(store_apply_ops(g, g->bw, tk, n_ins, tk2, n_del, false));
     trace_mark(g, "batch: backward ops");
@@ -636,8 +636,8 @@ int apply_batch_impl(gir_dev* g, const int32_t* u, const int32_t* v, const uint8
     int64_t nsi = 0, nsd = 0;
     GIR_TRY(select_flagged_u64(g, sym_keys, fsi, sym_ins, 2 * npu, &nsi));
     GIR_TRY(select_flagged_u64(g, sym_keys, fsd, sym_del, 2 * npu, &nsd));
-    GIR_TRY(sort_keys_u64(g, sym_ins, sym_keys, nsi, 64));
-    GIR_TRY(sort_keys_u64(g, sym_del, sym_keys, nsd, 64));
+    GIR_TRY(sort_keys_u64(g, sym_ins, sym_keys, nsi, edge_key_bits(g->V)));
+    GIR_TRY(sort_keys_u64(g, sym_del, sym_keys, nsd, edge_key_bits(g->V)));
     if (g->bct_built && nsi + nsd > 0) {
         k_classify_pairs<<<grid_for(g, nsi + nsd, kBlock), kBlock, 0, g->stream>>>(
             sym_ins, nsi, sym_del, nsd, static_cast<const int32_t*>(g->scc.p), static_cast<const int32_t*>(g->blk_label.p),

@@ -295,6 +295,18 @@ int store_build_bins(gir_dev* g);
 int store_single_edit(gir_dev* g, int32_t u, int32_t v, int insert, unsigned long long* out, uint64_t* keys);
 
 // ---- CUB wrappers (prims.cu) ----
+// Radix passes cover the key bits [0, end_bit). Bits of a key u << 32 | v of two vertex ids (or an
+// invalid op's ~0, which still sorts last).
+inline int edge_key_bits(int64_t V) {
+    int n = 1;
+    while (V >> n) ++n;
+    return 32 + n;
+}
+// The value that most of 512 row slots of `c` hold in val[row] (slots drawn evenly, so rows weigh by their
+// length), into *out, or -1 where no value holds half of them. Device words throughout, no host read.
+int sample_mode(gir_dev* g, const DevCSR& c, const int32_t* val, int32_t* out);
+// Exclusive scan of the V row lengths into off (V + 1 entries).
+int scan_degrees(gir_dev* g, const int32_t* deg, int64_t V, int64_t* off);
 int sort_keys_u64(gir_dev* g, uint64_t* keys, uint64_t* tmp, int64_t n, int end_bit);
 int sort_pairs_u64(gir_dev* g, uint64_t* keys, uint64_t* ktmp, uint32_t* vals, uint32_t* vtmp, int64_t n, int end_bit);
 int sort_pairs_u32(gir_dev* g, uint32_t* keys, uint32_t* ktmp, uint32_t* vals, uint32_t* vtmp, int64_t n, int end_bit);
@@ -308,7 +320,6 @@ int select_flagged_i32(gir_dev* g, const int32_t* in, const uint8_t* flags, int3
 int select_flagged_iota(gir_dev* g, const uint8_t* flags, int32_t* out, int64_t n, int64_t* host_n);
 // The rows of `deg` (V entries) longer than max_deg, ascending, into rows (V entries), and the
 // exclusive scan of their lengths into pref (V + 1 entries); *n = their number. flag: V bytes.
-constexpr int32_t kHeavyRow = 4096;
 int heavy_rows(gir_dev* g, const int32_t* deg, int64_t V, int32_t max_deg, uint8_t* flag, int32_t* rows, int64_t* pref,
                int64_t* n);
 
@@ -398,20 +409,15 @@ __device__ __forceinline__ int64_t lower_bound_dev(const T* a, int64_t lo, int64
 // so a row of any length costs its warp ceil(len/32) rounds. Must be called by all threads of
 // the grid (every lane of a warp takes part in every round). `scan` is per-warp shared scratch
 // of 33 int64 and 32 int32.
-// With max_deg >= 0, rows longer than max_deg are left out: a warp walks all of its 32 rows, so a
-// hub row would keep one warp busy long after the rest of the grid is idle; sweep those rows with
-// grid_sweep_heavy_rows instead (rows and offsets from heavy_rows).
 template <class F>
 __device__ __forceinline__ void warp_sweep_rows(const int64_t* beg, const int32_t* deg, const int32_t* adj,
-                                                int64_t v0, int64_t v1, int64_t* s_excl, int32_t* s_u, F&& f,
-                                                int32_t max_deg = -1) {
+                                                int64_t v0, int64_t v1, int64_t* s_excl, int32_t* s_u, F&& f) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t base = v0 + warp * 32; base < v1; base += nwarps * 32) {
         const int64_t v = base + lane;
-        int64_t cnt = v < v1 ? deg[v] : 0;
-        if (max_deg >= 0 && cnt > max_deg) cnt = 0;
+        const int64_t cnt = v < v1 ? deg[v] : 0;
         int64_t incl = cnt;
         for (int o = 1; o < 32; o <<= 1) {
             const int64_t t = __shfl_up_sync(0xffffffffu, incl, o);
@@ -439,53 +445,51 @@ __device__ __forceinline__ void warp_sweep_rows(const int64_t* beg, const int32_
     }
 }
 
-// Calls f(u, w, edge_index) for every entry of the rows rows[0 .. n) (pref: the exclusive scan of
-// their lengths, n + 1 entries), the entries spread evenly over the whole grid: the companion of
-// warp_sweep_rows(..., max_deg) for the rows it leaves out.
-template <class F>
-__device__ __forceinline__ void grid_sweep_heavy_rows(const int32_t* rows, const int64_t* pref, int64_t n,
-                                                      const int64_t* beg, const int32_t* adj, F&& f) {
-    if (n <= 0) return;
-    const int64_t total = pref[n];
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-        int64_t lo = 0, hi = n - 1;  // largest r with pref[r] <= e
-        while (lo < hi) {
-            const int64_t m = (lo + hi + 1) >> 1;
-            if (pref[m] <= e) lo = m; else hi = m - 1;
-        }
-        const int32_t u = rows[lo];
-        const int64_t k = beg[u] + (e - pref[lo]);
-        f(u, adj[k], k);
+// Largest i in [lo, n) with off[i] <= key (off[lo] <= key), by one warp, 32 probes a round.
+template <class T>
+__device__ __forceinline__ int64_t warp_find(const T* off, int64_t lo, int64_t n, int64_t key) {
+    int64_t hi = n - 1;
+    while (hi > lo) {
+        const int64_t step = (hi - lo + 31) / 32;
+        const int64_t i = lo + (int64_t)(lane_id() + 1) * step;
+        const int t = __popc(__ballot_sync(0xffffffffu, i <= hi && (int64_t)off[i] <= key));
+        if (t > 0) lo += (int64_t)t * step;
+        hi = lo + step - 1 < hi ? lo + step - 1 : hi;
     }
+    return lo;
+}
+
+// The window of 32 segments after the one at i0 (position p is its end): jumps past a run of empty
+// segments, which may be most of them, by one search.
+template <class T>
+__device__ __forceinline__ int64_t next_window(const T* off, int64_t i0, int64_t n, int64_t p) {
+    i0 += 32;
+    return i0 + 32 < n && (int64_t)off[i0 + 32] <= p ? warp_find(off, i0 + 32, n, p) : i0;
+}
+
+// Run length of a warp over `total` entries: even shares, at most 512 entries.
+__device__ __forceinline__ int64_t walk_run(int64_t total, int64_t nwarps) {
+    const int64_t run = ((total + nwarps - 1) / nwarps + 31) & ~(int64_t)31;
+    return run < 512 ? run : 512;
 }
 
 // Calls f(k, j) for every entry of n segments laid end to end, entry j of segment k, where off is the
-// exclusive scan of their lengths (n + 1 entries; any order of launch, whole warps only). Every warp
-// takes runs of 512 consecutive entries: one 32-ary search finds a run's first segment, then 32
-// segments at a time sit one per lane and an entry finds its own by shuffles. A binary search of the
-// offsets per entry had made the update merges' and the compact copies' kernels 5 - 10 times slower.
+// exclusive scan of their lengths (n + 1 entries); whole warps call it. Every warp takes runs of 512
+// consecutive entries: one 32-ary search finds a run's first segment, then 32 segments at a time sit
+// one per lane and an entry finds its own by shuffles. A binary search of the offsets per entry had
+// made the update merges' and the compact copies' kernels 3 - 6 times slower.
 template <class T, class F>
 __device__ __forceinline__ void walk_segments(const T* off, int64_t n, F&& f) {
-    constexpr int64_t kWalk = 512;
     if (n <= 0) return;
-    const int ln = threadIdx.x & 31;
+    const int ln = lane_id();
     const int64_t total = off[n];
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    int64_t run = ((total + nwarps - 1) / nwarps + 31) & ~(int64_t)31;
-    run = run < kWalk ? run : kWalk;
+    const int64_t run = walk_run(total, nwarps);
     for (int64_t c0 = warp * run; c0 < total; c0 += nwarps * run) {
         const int64_t c1 = c0 + run < total ? c0 + run : total;
-        int64_t lo = 0, hi = n - 1;  // largest i with off[i] <= c0
-        while (hi > lo) {
-            const int64_t step = (hi - lo + 31) / 32;
-            const int64_t i = lo + (int64_t)(ln + 1) * step;
-            const int t = __popc(__ballot_sync(0xffffffffu, i <= hi && off[i] <= c0));
-            if (t > 0) lo += (int64_t)t * step;
-            hi = lo + step - 1 < hi ? lo + step - 1 : hi;
-        }
         int64_t p = c0;
-        for (int64_t i0 = lo; p < c1; i0 += 32) {
+        for (int64_t i0 = warp_find(off, 0, n, c0); p < c1; i0 = next_window(off, i0, n, p)) {
             const int64_t ij = i0 + ln;
             const int64_t at = ij < n ? (int64_t)off[ij] - c0 : INT64_MAX;
             const uint32_t relj = at <= 0 ? 0u : (at < 0x7fffffff ? (uint32_t)at : 0x7fffffffu);
@@ -499,6 +503,55 @@ __device__ __forceinline__ void walk_segments(const T* off, int64_t n, F&& f) {
                     if (__shfl_sync(0xffffffffu, relj, x + b) <= rel) x += b;
                 const int64_t ax = __shfl_sync(0xffffffffu, at, x);
                 if (p + ln < wend) f(i0 + x, (int64_t)rel - ax);
+            }
+            p = wend;
+        }
+    }
+}
+
+// The same over the rows of a CSR with gathers per entry: use(on, u, w, x, load(u, w)) for every entry
+// w of row u, every lane of a warp calling `use` together (on: the lane has an entry; x: its row within
+// the warp's window, ascending with the lane). off: exclusive scan of the row lengths. U entries a lane
+// are loaded before the first is used, so that many dependent gathers are in flight.
+template <int U, class Load, class Use>
+__device__ __forceinline__ void walk_rows_of(const int64_t* off, int64_t V, const int64_t* beg, const int32_t* adj,
+                                             Load&& load, Use&& use) {
+    using T = decltype(load((int32_t)0, (int32_t)0));
+    const int ln = lane_id();
+    const int64_t total = off[V];
+    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t run = walk_run(total, nwarps);
+    for (int64_t c0 = warp * run; c0 < total; c0 += nwarps * run) {
+        const int64_t c1 = c0 + run < total ? c0 + run : total;
+        int64_t p = c0;
+        for (int64_t i0 = warp_find(off, 0, V, c0); p < c1; i0 = next_window(off, i0, V, p)) {
+            const int64_t ij = i0 + ln;
+            const int64_t at = ij < V ? off[ij] - c0 : INT64_MAX;
+            const int64_t baj = ij < V ? beg[ij] - at : 0;  // the row's first index, less its offset in the run
+            const uint32_t relj = at <= 0 ? 0u : (at < 0x7fffffff ? (uint32_t)at : 0x7fffffffu);
+            const int64_t wnext = i0 + 32 < V ? off[i0 + 32] : total;
+            const int64_t wend = wnext < c1 ? wnext : c1;
+            for (; p < wend; p += 32 * U) {
+                int x[U];
+                int32_t w[U];
+                T got[U];
+#pragma unroll
+                for (int i = 0; i < U; ++i) {
+                    const int64_t pos = p + 32 * i + ln;
+                    const uint32_t rel = (uint32_t)(pos - c0);
+                    x[i] = 0;
+#pragma unroll
+                    for (int b = 16; b; b >>= 1)
+                        if (__shfl_sync(0xffffffffu, relj, x[i] + b) <= rel) x[i] += b;
+                    const int64_t bx = __shfl_sync(0xffffffffu, baj, x[i]);
+                    w[i] = pos < wend ? adj[bx + rel] : -1;
+                }
+#pragma unroll
+                for (int i = 0; i < U; ++i)
+                    if (w[i] >= 0) got[i] = load((int32_t)(i0 + x[i]), w[i]);
+#pragma unroll
+                for (int i = 0; i < U; ++i) use(w[i] >= 0, (int32_t)(i0 + x[i]), w[i], x[i], got[i]);
             }
             p = wend;
         }

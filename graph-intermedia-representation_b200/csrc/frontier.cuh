@@ -205,6 +205,9 @@ __device__ __forceinline__ void walk_rows(const Queue& q, int64_t nq, int64_t to
         }
         p = wend;
         i0 += 32;
+        // (entries without a row keep their slots: jump past a run of them)
+        if (p < c1 && i0 + 32 < nq && (int64_t)__ldcg((const unsigned long long*)q.off + i0 + 32) <= p)
+            i0 = queue_find(q.off, i0 + 32, nq, (uint64_t)p);
     }
 }
 
@@ -302,12 +305,60 @@ struct FrontierRun {
     bool done() const { return started && (packed >> kQShift) == 0; }
 };
 
+// ---- Bottom-up levels of the builds ------------------------------------------------------------
+// Where a frontier's rows hold far more entries than there are vertices left, the vertices left look
+// for the frontier instead: a bitmap of the frontier (V / 8 bytes, so the gathers mostly stay in the
+// L1) and each row read only as far as its first hit.
+__global__ static void k_frontier_bits(const int32_t* q, int64_t n, uint32_t* fwd, uint32_t* bwd) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t e = q[i], v = e >= 0 ? e : ~e;
+        atomicOr((e >= 0 ? fwd : bwd) + (v >> 5), 1u << (v & 31));
+    }
+}
+
+// First entry w of row [b, b + d) for which hit(w, key), or -1; the row starts on a 16-byte boundary.
+// Every lane of the warp calls it (want: this lane has a row, key: a value that goes with it): a lane reads the first 32 entries of its own
+// row, four at a time; what is left of longer rows the warp reads together, row after row.
+template <class Hit>
+__device__ __forceinline__ int32_t first_hit(const int32_t* adj, int64_t b, int32_t d, bool want, int32_t key, const Hit& hit) {
+    int32_t found = -1, at = 0;
+    if (want) {
+        const int32_t own = d < 32 ? d : 32;
+        for (; at + 4 <= own && found < 0; at += 4) {
+            const int4 a = *reinterpret_cast<const int4*>(adj + b + at);
+            if (hit(a.x, key)) found = a.x;
+            else if (hit(a.y, key)) found = a.y;
+            else if (hit(a.z, key)) found = a.z;
+            else if (hit(a.w, key)) found = a.w;
+        }
+        for (; at < own && found < 0; ++at) {
+            const int32_t w = adj[b + at];
+            if (hit(w, key)) found = w;
+        }
+    }
+    for (unsigned todo = __ballot_sync(0xffffffffu, want && found < 0 && at < d); todo; todo &= todo - 1) {
+        const int src = __ffs(todo) - 1;
+        const int64_t rb = __shfl_sync(0xffffffffu, b, src);
+        const int32_t rd = __shfl_sync(0xffffffffu, d, src), rkey = __shfl_sync(0xffffffffu, key, src);
+        int32_t got = -1;
+        for (int32_t k = 32; k < rd && got < 0; k += 32) {
+            const int32_t w = k + lane_id() < rd ? adj[rb + k + lane_id()] : -1;
+            const unsigned m = __ballot_sync(0xffffffffu, w >= 0 && hit(w, rkey));
+            if (m) got = __shfl_sync(0xffffffffu, w, __ffs(m) - 1);
+        }
+        if (lane_id() == src) found = got;
+    }
+    return found;
+}
+
 // Runs up to max_levels more levels. Before the first call the caller zeroes ctl (kLoopWords words),
 // puts the first frontier at the front of the queue arrays and its packed size in ctl[W_Q].
 // kLoopMaxEdges: a larger level runs as its own launch at full occupancy (as the BFS levels do).
 constexpr int64_t kLoopMaxEdges = 1ll << 22;
-template <class Op>
-int run_frontier(gir_dev* g, Op op, Queue q, unsigned long long* ctl, FrontierRun& r, int64_t max_levels) {
+// A large level runs bottom-up where bu.wants(its row entries, entries queued so far).
+template <class Op, class BottomUp>
+int run_frontier(gir_dev* g, Op op, const BottomUp& bu, Queue q, unsigned long long* ctl, FrontierRun& r,
+                 int64_t max_levels) {
     void* hp = nullptr;
     GIR_TRY(pinned(g, kPinnedBytes, &hp));
     unsigned long long* hc = static_cast<unsigned long long*>(hp);
@@ -315,9 +366,13 @@ int run_frontier(gir_dev* g, Op op, Queue q, unsigned long long* ctl, FrontierRu
         const int64_t nq = (int64_t)(r.packed >> kQShift), total = (int64_t)(r.packed & kQEdges);
         if (r.started && total > kLoopMaxEdges) {
             GIR_CUDA(g, cudaMemsetAsync(ctl + W_SLOTS, 0, sizeof(unsigned long long), g->stream));
-            k_frontier_level<Op><<<g->num_sms * 8, kLevelThreads, 0, g->stream>>>(
-                op, Queue{q.v + r.lo, q.off + r.lo}, nq, total, Queue{q.v + r.lo + nq, q.off + r.lo + nq}, ctl + W_SLOTS);
-            GIR_LAUNCH(g, "k_frontier_level");
+            const Queue in{q.v + r.lo, q.off + r.lo}, out{q.v + r.lo + nq, q.off + r.lo + nq};
+            if (bu.wants(total, r.lo + nq)) {
+                GIR_TRY(bu.launch(g, in, nq, out, ctl + W_SLOTS));
+            } else {
+                k_frontier_level<Op><<<g->num_sms * 8, kLevelThreads, 0, g->stream>>>(op, in, nq, total, out, ctl + W_SLOTS);
+                GIR_LAUNCH(g, "k_frontier_level");
+            }
             GIR_CUDA(g, cudaMemcpyAsync(hc, ctl + W_SLOTS, sizeof(unsigned long long), cudaMemcpyDeviceToHost, g->stream));
             GIR_CUDA(g, cudaStreamSynchronize(g->stream));
             r.lo += nq;

@@ -224,6 +224,48 @@ __global__ void k_heavy_lengths(const int32_t* deg, const int32_t* rows, int64_t
 }
 }  // namespace
 
+constexpr int kModeSamples = 512;
+__global__ void __launch_bounds__(kModeSamples) k_sample_mode(int64_t V, const int64_t* beg, const int32_t* val,
+                                                              int32_t* out) {
+    __shared__ int32_t s_val[kModeSamples];
+    __shared__ unsigned long long s_best;
+    const int i = threadIdx.x;
+    const int64_t slots = beg[V];
+    uint64_t z = (uint64_t)(i + 1) * 0x9e3779b97f4a7c15ULL;
+    z = (z ^ (z >> 31)) * 0xbf58476d1ce4e5b9ULL;
+    const int64_t at = slots > 0 ? (int64_t)((z >> 17) % (uint64_t)slots) : 0;
+    int64_t lo = 0, hi = V - 1;  // largest row starting at or before the slot
+    while (lo < hi) {
+        const int64_t m = (lo + hi + 1) >> 1;
+        if (beg[m] <= at) lo = m; else hi = m - 1;
+    }
+    s_val[i] = val[lo];
+    if (i == 0) s_best = 0;
+    __syncthreads();
+    int same = 0;
+    for (int k = 0; k < kModeSamples; ++k) same += s_val[k] == s_val[i];
+    atomicMax(&s_best, ((unsigned long long)same << 32) | (uint32_t)s_val[i]);
+    __syncthreads();
+    if (i == 0) *out = (int)(s_best >> 32) * 2 >= kModeSamples ? (int32_t)(uint32_t)s_best : -1;
+}
+
+int sample_mode(gir_dev* g, const DevCSR& c, const int32_t* val, int32_t* out) {
+    k_sample_mode<<<1, kModeSamples, 0, g->stream>>>(g->V, c.beg, val, out);
+    GIR_LAUNCH(g, "k_sample_mode");
+    return GIR_OK;
+}
+
+__global__ void k_widen(const int32_t* in, int64_t n, int64_t* out) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= n; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = i < n ? in[i] : 0;
+}
+
+int scan_degrees(gir_dev* g, const int32_t* deg, int64_t V, int64_t* off) {
+    k_widen<<<grid_for(g, V + 1, 256), 256, 0, g->stream>>>(deg, V, off);
+    GIR_LAUNCH(g, "k_widen");
+    return exclusive_scan_i64(g, off, off, V + 1);
+}
+
 int heavy_rows(gir_dev* g, const int32_t* deg, int64_t V, int32_t max_deg, uint8_t* flag, int32_t* rows, int64_t* pref,
                int64_t* n) {
     *n = 0;

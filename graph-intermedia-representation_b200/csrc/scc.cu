@@ -180,6 +180,50 @@ struct ReachBoth {
     }
 };
 
+// The same level bottom-up, on rows that start on 16-byte boundaries (the handle's graph): a vertex
+// without the forward mark looks for an in-neighbour in the forward frontier, one without the backward
+// mark for an out-neighbour in the backward frontier.
+__global__ void __launch_bounds__(kBlock) k_reach_up(int64_t V, CSRView fw, CSRView bw, const uint32_t* fwd,
+                                                     const uint32_t* bwd, int32_t* mark, Queue out,
+                                                     unsigned long long* cnt) {
+    __shared__ int32_t s_st[kBlock / 32][kStage];
+    int n_st = 0;
+    auto deg = [&](int32_t e) { return e >= 0 ? fw.deg[e] : bw.deg[~e]; };
+    for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < V; base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t v = base + threadIdx.x;
+        const int32_t m = v < V ? mark[v] : 3;
+        const bool wf = !(m & 1), wb = !(m & 2);
+        const bool f = first_hit(bw.adj, wf ? bw.beg[v] : 0, wf ? bw.deg[v] : 0, wf, 0,
+                                 [&](int32_t w, int32_t) { return (fwd[w >> 5] >> (w & 31)) & 1u; }) >= 0;
+        const bool b = first_hit(fw.adj, wb ? fw.beg[v] : 0, wb ? fw.deg[v] : 0, wb, 0,
+                                 [&](int32_t w, int32_t) { return (bwd[w >> 5] >> (w & 31)) & 1u; }) >= 0;
+        if (f || b) mark[v] = m | (f ? 1 : 0) | (b ? 2 : 0);
+        queue_push(f, (int32_t)v, s_st[threadIdx.x >> 5], n_st, out, deg, cnt);
+        queue_push(b, ~(int32_t)v, s_st[threadIdx.x >> 5], n_st, out, deg, cnt);
+    }
+    queue_flush(s_st[threadIdx.x >> 5], n_st, out, deg, cnt);
+}
+
+// Bottom-up where the frontier's rows hold over four times as many entries as there are (vertex,
+// direction) pairs left (4.8M-vertex R-MAT: both levels of over 2^22 entries, 0.62 ms each top-down).
+struct ReachUp {
+    CSRView fw, bw;
+    int32_t* mark;
+    uint32_t* bits;  // two bitmaps
+    int64_t V;
+    bool aligned;
+    bool wants(int64_t total, int64_t queued) const { return aligned && total > 4 * (2 * V - queued); }
+    int launch(gir_dev* g, const Queue& in, int64_t nq, const Queue& out, unsigned long long* cnt) const {
+        uint32_t* bwd = bits + V / 32 + 1;
+        GIR_CUDA(g, cudaMemsetAsync(bits, 0, sizeof(uint32_t) * 2 * (V / 32 + 1), g->stream));
+        k_frontier_bits<<<grid_for(g, nq, kBlock), kBlock, 0, g->stream>>>(in.v, nq, bits, bwd);
+        GIR_LAUNCH(g, "k_frontier_bits");
+        k_reach_up<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, fw, bw, bits, bwd, mark, out, cnt);
+        GIR_LAUNCH(g, "k_reach_up");
+        return GIR_OK;
+    }
+};
+
 // Marks of the assigned vertices, and the pivot in both directions as the first frontier.
 __global__ void k_reach_init(int64_t V, const int32_t* label, int32_t pivot, CSRView fw, CSRView bw, int32_t* mark,
                              Queue q, unsigned long long* ctl) {
@@ -277,31 +321,53 @@ __global__ void k_apply_min(int64_t V, int32_t* label, const int32_t* mn, unsign
     if (lane_id() == 0 && c) atomicAdd(n_classes, c);
 }
 
-// Cross-SCC edge keys (label(u) << 32 | label(w)) at the edge's own slot, flagged; the flags of
-// slack slots stay 0 (cleared by the caller), so a compaction over the capacity collects them.
-__global__ void __launch_bounds__(kBlock) k_cross_keys(int64_t V, CSRView fw, const int32_t* label, uint64_t* keys,
-                                                       uint8_t* flag) {
-    __shared__ int64_t s_excl[kWarps][33];
-    __shared__ int32_t s_u[kWarps][32];
-    const int wib = threadIdx.x >> 5;
-    warp_sweep_rows(
-        fw.beg, fw.deg, fw.adj, 0, V, s_excl[wib], s_u[wib],
-        [&](int32_t u, int32_t w, int64_t e) {
-            const int32_t a = label[u], b = label[w];
-            keys[e] = ((uint64_t)(uint32_t)a << 32) | (uint32_t)b;
-            flag[e] = a != b;
-        },
-        kHeavyRow);
+// Rows whose entries hold every cross edge. Where one SCC G holds most edges, its rows are left out: an
+// edge with its tail outside G is in that vertex's forward row, and one from G to a vertex outside in
+// that vertex's backward row. Without such an SCC (*giant = -1) all forward rows and no backward ones.
+__global__ void k_cross_len(int64_t V, const int32_t* deg, const int32_t* label, const int32_t* giant, int back,
+                            int32_t* len) {
+    const int32_t g = *giant;
+    GRID_STRIDE(v, V) len[v] = g >= 0 ? (label[v] != g ? deg[v] : 0) : (back ? 0 : deg[v]);
 }
 
-// The rows k_cross_keys leaves out (longer than kHeavyRow), their entries spread over the grid.
-__global__ void k_cross_keys_heavy(const int32_t* rows, const int64_t* pref, int64_t n, CSRView fw, const int32_t* label,
-                                   uint64_t* keys, uint8_t* flag) {
-    grid_sweep_heavy_rows(rows, pref, n, fw.beg, fw.adj, [&](int32_t u, int32_t w, int64_t e) {
-        const int32_t a = label[u], b = label[w];
-        keys[e] = ((uint64_t)(uint32_t)a << 32) | (uint32_t)b;
-        flag[e] = a != b;
+// Cross-SCC edge keys (label(u) << 32 | label(w)), appended to `keys` in any order (they are sorted next)
+// through a per-warp buffer; a run of equal keys within a step (a singleton's edges into the giant SCC)
+// is appended once. Rows are cut into even runs whatever their length (off: scan of the row lengths); with
+// `back` the rows are backward ones and only edges from G count. 69M edges of the 4.8M-vertex R-MAT: keys
+// and flags at every edge's slot and a compaction took 1.1 ms, all rows this way 0.41 ms, without
+// the giant SCC's rows 0.25 ms.
+constexpr int kKeyStage = 128;
+__global__ void __launch_bounds__(kBlock) k_cross_keys(int64_t V, const int64_t* off, CSRView c, const int32_t* label,
+                                                       const int32_t* giant, int back, uint64_t* keys,
+                                                       unsigned long long* n) {
+    __shared__ uint64_t s_keys[kWarps][kKeyStage];
+    uint64_t* buf = s_keys[threadIdx.x >> 5];
+    int held = 0;
+    const int ln = lane_id();
+    auto flush = [&]() {
+        unsigned long long at = 0;
+        if (ln == 0) at = atomicAdd(n, (unsigned long long)held);
+        at = __shfl_sync(0xffffffffu, at, 0);
+        for (int i = ln; i < held; i += 32) keys[at + i] = buf[i];
+        __syncwarp();
+        held = 0;
+    };
+    const uint32_t from = (uint32_t)*giant;
+    auto load = [&](int32_t u, int32_t w) {
+        return ((uint64_t)(uint32_t)label[back ? w : u] << 32) | (uint32_t)label[back ? u : w];
+    };
+    walk_rows_of<4>(off, V, c.beg, c.adj, load, [&](bool on, int32_t, int32_t, int, uint64_t key) {
+        const bool cross = on && (key >> 32) != (key & 0xffffffffULL) && (!back || (uint32_t)(key >> 32) == from);
+        const uint64_t before = __shfl_up_sync(0xffffffffu, key, 1);
+        const bool put = cross && (ln == 0 || before != key);
+        const unsigned m = __ballot_sync(0xffffffffu, put);
+        if (!m) return;
+        if (held + __popc(m) > kKeyStage) flush();
+        if (put) buf[held + __popc(m & ((1u << ln) - 1))] = key;
+        __syncwarp();
+        held += __popc(m);
     });
+    if (held) flush();
 }
 
 __global__ void k_distinct_u64(const uint64_t* keys, int64_t n, uint8_t* flag) {
@@ -497,14 +563,14 @@ static int scc_by_quotient(gir_dev* g, int32_t* label, int64_t* n_scc, bool* use
         GIR_TRY(t.get(&flag, n));
         k_quotient_keys<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, fw, cls, keys, cnt + 3);
         GIR_LAUNCH(g, "k_quotient_keys");
-        GIR_TRY(sort_keys_u64(g, keys, tmp, n, 64));
+        GIR_TRY(sort_keys_u64(g, keys, tmp, n, edge_key_bits(g->V)));
         k_distinct_u64<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(keys, n, flag);
         GIR_LAUNCH(g, "k_distinct_u64");
         int64_t m = 0;
         GIR_TRY(select_flagged_u64(g, keys, flag, tmp, n, &m));
         k_flip_keys<<<grid_for(g, m, kBlock), kBlock, 0, g->stream>>>(tmp, m, flip);
         GIR_LAUNCH(g, "k_flip_keys");
-        GIR_TRY(sort_keys_u64(g, flip, keys, m, 64));
+        GIR_TRY(sort_keys_u64(g, flip, keys, m, edge_key_bits(g->V)));
         int64_t* beg[2];
         int32_t *deg[2], *adj[2];
         for (int i = 0; i < 2; ++i) {
@@ -642,14 +708,17 @@ static int scc_labels(gir_dev* g, const CSRView fw, const CSRView bw, bool whole
         k_reach_init<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, label, pivot, fw, bw, mark, q, ctl);
         GIR_LAUNCH(g, "k_reach_init");
         const ReachBoth op{fw, bw, mark};
+        uint32_t* bits = nullptr;
+        GIR_TRY(ensure_n(g, g->scratch[11], 2 * (V / 32 + 1), &bits));
+        const ReachUp up{fw, bw, mark, bits, V, whole};
         FrontierRun run;
-        GIR_TRY(run_frontier(g, op, q, ctl, run, whole ? deep_levels(V) : INT64_MAX));
+        GIR_TRY(run_frontier(g, op, up, q, ctl, run, whole ? deep_levels(V) : INT64_MAX));
         if (!run.done()) {
             bool used = false;
             GIR_TRY(scc_by_quotient(g, label, n_scc, &used));
             trace_mark(g, "scc: reciprocal classes");
             if (used) return GIR_OK;
-            GIR_TRY(run_frontier(g, op, q, ctl, run, INT64_MAX));
+            GIR_TRY(run_frontier(g, op, up, q, ctl, run, INT64_MAX));
         }
         k_reach_label<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, mark, pivot, label);
         GIR_LAUNCH(g, "k_reach_label");
@@ -808,38 +877,39 @@ int scc_build_dag(gir_dev* g) {
     const int64_t V = g->V;
     int32_t* label = static_cast<int32_t*>(g->scc.p);
     // condensation edges: cross keys, radix sort, unique
-    const int64_t cap = g->fw.cap;
+    const int64_t E = g->fw.E;
     uint64_t *keys = nullptr, *tmp = nullptr;
     uint8_t* flag = nullptr;
+    int64_t* off = nullptr;
     unsigned long long* cnt = nullptr;
-    GIR_TRY(ensure_n(g, g->scratch[7], cap + 1, &keys));
-    GIR_TRY(ensure_n(g, g->scratch[8], cap + 1, &tmp));
-    GIR_TRY(ensure_n(g, g->scratch[9], cap + 1, &flag));
+    // (the rank keys share keys / tmp: up to one per vertex)
+    const int64_t room = E > V ? E : V;
+    GIR_TRY(ensure_n(g, g->scratch[7], room + 1, &keys));
+    GIR_TRY(ensure_n(g, g->scratch[8], room + 1, &tmp));
+    GIR_TRY(ensure_n(g, g->scratch[9], room + 1, &flag));
+    GIR_TRY(ensure_n(g, g->scratch[10], V + 1, &off));
     GIR_TRY(ensure_n(g, g->scratch[6], 2 * C_N, &cnt));
     void* hp = nullptr;
     GIR_TRY(pinned(g, 256, &hp));
     unsigned long long* hc = static_cast<unsigned long long*>(hp);
-    GIR_CUDA(g, cudaMemsetAsync(flag, 0, cap + 1, g->stream));
-    if (V > 0) {
-        // the long rows' list in tmp (free until the compaction; cap >= 4V, every row has room
-        // for 4 entries): rows int32[V], their length scan int64[V + 1], flags uint8[V]
-        int32_t* heavy = reinterpret_cast<int32_t*>(tmp);
-        int64_t* hpref = reinterpret_cast<int64_t*>(tmp) + (V + 1) / 2 + 1;
-        uint8_t* hflag = reinterpret_cast<uint8_t*>(hpref + V + 2);
-        int64_t n_heavy = 0;
-        GIR_TRY(heavy_rows(g, g->fw.deg, V, kHeavyRow, hflag, heavy, hpref, &n_heavy));
-        k_cross_keys<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, view(g->fw), label, keys, flag);
-        GIR_LAUNCH(g, "k_cross_keys");
-        if (n_heavy > 0) {
-            k_cross_keys_heavy<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(heavy, hpref, n_heavy, view(g->fw), label,
-                                                                               keys, flag);
-            GIR_LAUNCH(g, "k_cross_keys_heavy");
+    GIR_CUDA(g, cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * C_N, g->stream));
+    if (E > 0) {
+        int32_t *len = nullptr, *giant = reinterpret_cast<int32_t*>(cnt + C_N);
+        GIR_TRY(ensure_n(g, g->scratch[11], V + 1, &len));
+        GIR_TRY(sample_mode(g, g->fw, label, giant));
+        for (int back = 0; back < 2; ++back) {
+            const DevCSR& c = back ? g->bw : g->fw;
+            k_cross_len<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, c.deg, label, giant, back, len);
+            GIR_LAUNCH(g, "k_cross_len");
+            GIR_TRY(scan_degrees(g, len, V, off));
+            k_cross_keys<<<g->num_sms * 8, kBlock, 0, g->stream>>>(V, off, view(c), label, giant, back, keys, &cnt[C_Q]);
+            GIR_LAUNCH(g, "k_cross_keys");
         }
     }
-    int64_t n_cross = 0;
-    GIR_TRY(select_flagged_u64(g, keys, flag, tmp, cap, &n_cross));
-    std::swap(keys, tmp);
-    GIR_TRY(sort_keys_u64(g, keys, tmp, n_cross, 64));
+    GIR_CUDA(g, cudaMemcpyAsync(hc, cnt, sizeof(unsigned long long), cudaMemcpyDeviceToHost, g->stream));
+    GIR_CUDA(g, cudaStreamSynchronize(g->stream));
+    const int64_t n_cross = (int64_t)hc[C_Q];
+    GIR_TRY(sort_keys_u64(g, keys, tmp, n_cross, edge_key_bits(g->V)));
     int64_t n_dag = 0;
     uint64_t* dag = nullptr;
     GIR_TRY(ensure_n(g, g->dag, n_cross + 1, &dag));
@@ -878,7 +948,7 @@ int scc_build_dag(gir_dev* g) {
     GIR_CUDA(g, cudaMemcpyAsync(hc, cnt, sizeof(unsigned long long) * C_N, cudaMemcpyDeviceToHost, g->stream));
     GIR_CUDA(g, cudaStreamSynchronize(g->stream));
     const int64_t ns = (int64_t)hc[C_Q];
-    GIR_TRY(sort_keys_u64(g, keys, tmp, ns, 64));
+    GIR_TRY(sort_keys_u64(g, keys, tmp, ns, edge_key_bits(g->V)));
     if (ns > 0) {
         k_rank_scatter<<<grid_for(g, ns, kBlock), kBlock, 0, g->stream>>>(keys, ns, rank_of);
         GIR_LAUNCH(g, "k_rank_scatter");

@@ -462,7 +462,7 @@ int store_build_sym(gir_dev* g) {
     }
     int64_t n = 0;
     GIR_TRY(select_flagged_u64(g, keys, keep, tmp, 2 * E, &n));
-    GIR_TRY(sort_keys_u64(g, tmp, keys, n, 64));
+    GIR_TRY(sort_keys_u64(g, tmp, keys, n, edge_key_bits(g->V)));
     if (n > 0) {
         k_distinct_flags<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(tmp, n, keep);
         GIR_LAUNCH(g, "k_distinct_flags");
