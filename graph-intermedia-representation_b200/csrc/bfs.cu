@@ -34,11 +34,60 @@ constexpr int kBlock = 256;
 // [4] the device-decided direction of the next level and [5..8] its features (learned schedule)
 enum { C_Q = 0, C_PAIRS = 1, C_MEDGES = 2, C_DIR = 4, C_FEAT = 5, C_N = 9 };
 
-__device__ __forceinline__ void write_levels(int32_t* level, int64_t V, int32_t v, uint64_t nb, int32_t L) {
+// Where levels go. Written straight into the output's rows, every (vertex, lane) pair is a 4-byte write
+// into another 32-byte sector; with many lanes the levels below kPlaneLevels are kept in four bit planes
+// per vertex instead (one sector: bit s of plane b is bit b of lane s's code, 15 - level, 0 for none), and
+// k_expand_levels writes every row of the output once, coalesced, after the search. (The minus-one fill
+// of the output goes with it.)
+constexpr int kPlaneLevels = 15;
+struct Levels {
+    int32_t* out;
+    int64_t V;
+    unsigned long long* plane;  // 4 per vertex, zeroed; null: every level goes straight to the output
+};
+// The planes cost a sector per vertex and pass, the straight writes a sector per pair. 64 lanes, 4.8M
+// vertices: 5.1 ms a call with straight writes, 2.7 ms so; small calls keep those and save the launch.
+constexpr int kPlaneMinLanes = 8;
+constexpr int64_t kPlaneMinPairs = 1ll << 23;
+
+// Level L of the lanes nb of vertex v. Several threads may write lanes of one vertex.
+__device__ __forceinline__ void write_levels(const Levels& l, int32_t v, uint64_t nb, int32_t L) {
+    if (l.plane && L < kPlaneLevels) {
+        const int code = kPlaneLevels - L;
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+            if ((code >> b) & 1) atomicOr(l.plane + 4 * (int64_t)v + b, (unsigned long long)nb);
+        return;
+    }
     while (nb) {
         const int s = __ffsll((long long)nb) - 1;
         nb &= nb - 1;
-        level[(int64_t)s * V + v] = L;
+        l.out[(int64_t)s * l.V + v] = L;
+    }
+}
+// The same by a warp whose lanes all hold v and nb.
+__device__ __forceinline__ void write_levels_warp(const Levels& l, int32_t v, uint64_t nb, int32_t L) {
+    const int ln = lane_id();
+    if (l.plane && L < kPlaneLevels) {
+        if (nb && ln < 4 && (((kPlaneLevels - L) >> ln) & 1)) atomicOr(l.plane + 4 * (int64_t)v + ln, (unsigned long long)nb);
+        return;
+    }
+    if ((nb >> ln) & 1ull) l.out[(int64_t)ln * l.V + v] = L;
+    if ((nb >> 32 >> ln) & 1ull) l.out[(int64_t)(ln + 32) * l.V + v] = L;
+}
+
+// The output rows from the planes: a thread per vertex, so a warp writes 128 bytes of each row. Lanes that
+// were seen without a code have their level in the output already. Bound by the output's writes.
+__global__ void __launch_bounds__(kBlock) k_expand_levels(Levels l, const uint64_t* seen, int nl) {
+    GRID_STRIDE(v, l.V) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(l.plane + 4 * v);
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(l.plane + 4 * v + 2);
+        const uint64_t done = seen[v] & ~(a.x | a.y | b.x | b.y);
+        for (int s = 0; s < nl; ++s) {
+            const int code = (int)((a.x >> s) & 1) | (int)((a.y >> s) & 1) << 1 | (int)((b.x >> s) & 1) << 2 |
+                             (int)((b.y >> s) & 1) << 3;
+            if (!((done >> s) & 1)) __stcs(l.out + (int64_t)s * l.V + v, code ? kPlaneLevels - code : -1);
+        }
     }
 }
 
@@ -56,7 +105,7 @@ struct RowLen {
 // Sources: lane s of the group starts at every vertex of set s (set_beg is device memory). Counts
 // the sources' (vertex, lane) pairs and out-edges with the queue.
 __global__ void k_init_sources(const int64_t* set_beg, int n_lanes, const int32_t* srcs, int64_t V, uint64_t* seen,
-                               uint64_t* front, Queue q, unsigned long long* cnt, int32_t* level, const int32_t* deg) {
+                               uint64_t* front, Queue q, unsigned long long* cnt, Levels level, const int32_t* deg) {
     __shared__ int32_t s_stage[kBlock / 32][kStage];
     int n_st = 0;
     const int64_t lo = set_beg[0], hi = set_beg[n_lanes];
@@ -74,7 +123,7 @@ __global__ void k_init_sources(const int64_t* set_beg, int n_lanes, const int32_
             const unsigned long long bit = 1ull << s;
             if (!(atomicOr((unsigned long long*)&seen[v], bit) & bit)) {
                 on = atomicOr((unsigned long long*)&front[v], bit) == 0ull;
-                level[(int64_t)s * V + v] = 0;
+                write_levels(level, v, bit, 0);
                 ++pairs;
                 medges += (unsigned long long)deg[v];
             }
@@ -99,8 +148,7 @@ struct LevelMasks {
     const uint64_t* front;
     uint64_t* seen;
     uint64_t* next;
-    int32_t* level;
-    int64_t V;
+    Levels level;
 };
 
 // A top-down level (walk_rows). One pass does the whole level: the atomicOr on seen[w] hands every
@@ -125,7 +173,7 @@ struct TopDown {
         const unsigned long long nb = bits & ~atomicOr((unsigned long long*)k.seen + w, bits);
         if (!nb) return false;
         const bool fresh = atomicOr((unsigned long long*)k.next + w, nb) == 0ull;
-        write_levels(k.level, k.V, w, nb, L);
+        write_levels(k.level, w, nb, L);
         const unsigned c = __popcll(nb);
         pairs += c;
         medges += (unsigned long long)c * (unsigned long long)fw.deg[w];
@@ -176,7 +224,7 @@ __device__ __forceinline__ void bu_threads(const int32_t* ids, int64_t n, int64_
                 if (nb) {
                     k.next[v] = nb;
                     k.seen[v] = s | nb;
-                    write_levels(k.level, k.V, v, nb, L);
+                    write_levels(k.level, v, nb, L);
                     const unsigned c = __popcll(nb);
                     acc.pairs += c;
                     acc.medges += (unsigned long long)c * (unsigned long long)outdeg[v];
@@ -217,9 +265,7 @@ __device__ __forceinline__ void bu_warps(const int32_t* ids, int64_t n, int64_t 
             acc.medges += (unsigned long long)c * (unsigned long long)outdeg[v];
         }
         queue_push(lane == 0 && nb != 0, v, acc.s_buf, acc.n, out, RowLen{outdeg}, cnt);
-        // lanes split the level writes of this vertex
-        if ((nb >> lane) & 1ull) k.level[(int64_t)lane * k.V + v] = L;
-        if ((nb >> 32 >> lane) & 1ull) k.level[(int64_t)(lane + 32) * k.V + v] = L;
+        write_levels_warp(k.level, v, nb, L);
     }
 }
 
@@ -254,8 +300,10 @@ __device__ __forceinline__ void bu_ctas(const int32_t* ids, int64_t n, const CSR
             acc.pairs += c;
             acc.medges += (unsigned long long)c * (unsigned long long)outdeg[v];
         }
-        if (threadIdx.x < 32) queue_push(threadIdx.x == 0 && nb != 0, v, acc.s_buf, acc.n, out, RowLen{outdeg}, cnt);
-        if (threadIdx.x < 64 && ((nb >> threadIdx.x) & 1ull)) k.level[(int64_t)threadIdx.x * k.V + v] = L;
+        if (threadIdx.x < 32) {
+            queue_push(threadIdx.x == 0 && nb != 0, v, acc.s_buf, acc.n, out, RowLen{outdeg}, cnt);
+            write_levels_warp(k.level, v, nb, L);
+        }
         __syncthreads();
     }
 }
@@ -300,7 +348,7 @@ struct PersistArgs {
     uint64_t* seen;
     uint64_t* front[3];       // the frontier's masks, the next frontier's (zero) and the last one's (zero)
     Queue q[3];               // frontier, next frontier, last frontier (empty)
-    int32_t* level;
+    Levels level;
     const int32_t* bins;
     int64_t bin_n[3];
     int64_t V;
@@ -364,7 +412,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_bfs_persistent(PersistAr
         if (!dir && vedges > kPersistMaxEdges) { reason = R_BIG; break; }
         unsigned long long* sl = a.ctl + P_SLOTS + S_W * (lev % 3);
         const Queue &qa = a.q[rot], &qb = a.q[(rot + 1) % 3], &qc = a.q[(rot + 2) % 3];
-        LevelMasks k{a.front[rot], a.seen, a.front[(rot + 1) % 3], a.level, a.V};
+        LevelMasks k{a.front[rot], a.seen, a.front[(rot + 1) % 3], a.level};
         uint64_t* old = a.front[(rot + 2) % 3];
         // (the slot after this level's was last read before the barrier of the level before)
         if (blockIdx.x == 0 && threadIdx.x < S_W) a.ctl[P_SLOTS + S_W * ((lev + 1) % 3) + threadIdx.x] = 0;
@@ -481,9 +529,7 @@ int bfs_run(gir_dev* g, const int64_t* set_beg_h, const int32_t* srcs_d, int64_t
     st = QueryStats{};
     g->trace_x.clear();
     g->trace_y.clear();
-    if (n_sets <= 0) return GIR_OK;
-    GIR_CUDA(g, cudaMemsetAsync(level_d, 0xff, sizeof(int32_t) * V * n_sets, g->stream));
-    if (V == 0) return GIR_OK;
+    if (n_sets <= 0 || V == 0) return GIR_OK;
     if (!g->bins_valid) GIR_TRY(store_build_bins(g));
 
     uint64_t *seen = nullptr, *front[3] = {nullptr, nullptr, nullptr};
@@ -529,12 +575,18 @@ int bfs_run(gir_dev* g, const int64_t* set_beg_h, const int32_t* srcs_d, int64_t
     for (int64_t g0 = 0; g0 < n_sets; g0 += 64) {
         const int nl = (int)((n_sets - g0) < 64 ? (n_sets - g0) : 64);
         const uint64_t all = nl == 64 ? ~0ull : ((1ull << nl) - 1);
-        int32_t* level = level_d + g0 * V;
+        Levels level{level_d + g0 * V, V, nullptr};
         GIR_CUDA(g, cudaMemsetAsync(seen, 0, sizeof(uint64_t) * V, g->stream));
         for (uint64_t* f : front) GIR_CUDA(g, cudaMemsetAsync(f, 0, sizeof(uint64_t) * V, g->stream));
         GIR_CUDA(g, cudaMemsetAsync(ctl, 0, sizeof(unsigned long long) * kCtlTrace, g->stream));
         GIR_CUDA(g, cudaMemcpyAsync(sbeg, set_beg_h + g0, sizeof(int64_t) * (nl + 1), cudaMemcpyHostToDevice, g->stream));
         const int64_t n_entries = set_beg_h[g0 + nl] - set_beg_h[g0];
+        if (n_entries > 0 && nl >= kPlaneMinLanes && (int64_t)nl * V >= kPlaneMinPairs) {
+            GIR_TRY(ensure_n(g, g->scratch[12], 4 * V, &level.plane));
+            GIR_CUDA(g, cudaMemsetAsync(level.plane, 0, sizeof(uint64_t) * 4 * V, g->stream));
+        } else {
+            GIR_CUDA(g, cudaMemsetAsync(level.out, 0xff, sizeof(int32_t) * V * nl, g->stream));
+        }
         if (n_entries == 0) continue;
         k_init_sources<<<grid_for(g, n_entries, kBlock), kBlock, 0, g->stream>>>(sbeg, nl, srcs_d, V, seen, front[0], q[0],
                                                                                 cnt, level, g->fw.deg);
@@ -665,7 +717,7 @@ int bfs_run(gir_dev* g, const int64_t* set_beg_h, const int32_t* srcs_d, int64_t
             }
             handed_back = false;
             GIR_CUDA(g, cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * C_N, g->stream));
-            const LevelMasks km{front[0], seen, front[1], level, V};
+            const LevelMasks km{front[0], seen, front[1], level};
             if (!bottom_up) {
                 const int64_t blocks = std::min<int64_t>((vedges / 32 + kBlock / 32) / (kBlock / 32), g->num_sms * 8);
                 GIR_TRY(timer.run([&]() -> int {
@@ -716,6 +768,11 @@ int bfs_run(gir_dev* g, const int64_t* set_beg_h, const int32_t* srcs_d, int64_t
             take_counters();
             ++L;
             st.iterations++;
+        }
+        if (level.plane) {
+            k_expand_levels<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(level, seen, nl);
+            GIR_LAUNCH(g, "k_expand_levels");
+            st.launches++;
         }
     }
     GIR_CUDA(g, cudaEventRecord(g->ev1, g->stream));
