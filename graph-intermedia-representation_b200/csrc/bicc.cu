@@ -8,8 +8,8 @@
 // SCC at once:
 //  1. BFS spanning forest of H from every SCC's smallest vertex (level-synchronous), or on a deep H a
 //     forest from union-find, rooted by Euler tours, with 2. and 3. to match (see "Deep graphs");
-//  2. subtree sizes nd (levels bottom-up) and preorder numbers pre (children grouped by parent
-//     by a radix sort, sibling offsets by a scan, levels top-down);
+//  2. subtree sizes nd (levels bottom-up, which also gives every vertex its offset among its siblings)
+//     and preorder numbers pre (levels top-down);
 //  3. low / high: min / max pre over each subtree and its non-tree neighbours;
 //  4. union-find over tree edges (edge (p(v), v) is named by v): rule 1 joins the edges of
 //     v and w for a non-tree edge {v, w} between unrelated vertices; rule 2 joins (p(v), v)
@@ -260,8 +260,7 @@ __global__ void k_win_step(const int32_t* at, int64_t n, int64_t len, const int3
     }
 }
 
-// The smallest H neighbour of every tree root (a BFS forest's first child): it decides which of its
-// blocks is the root's parent block.
+// The smallest H neighbour of every tree root: it decides which of its blocks is the root's parent block.
 __global__ void k_root_rows(int64_t V, const int32_t* scc, const int32_t* hdeg, int32_t* deg, int32_t* least) {
     GRID_STRIDE(v, V) {
         deg[v] = scc[v] == (int32_t)v ? hdeg[v] : 0;
@@ -283,42 +282,14 @@ __global__ void k_root_block_least(int64_t V, const int32_t* least, const int32_
 
 __global__ void k_fill_i32(int32_t* p, int64_t n, int32_t v) { GRID_STRIDE(i, n) p[i] = v; }
 
-// nd[parent] += nd[v] for the vertices of one level (deepest level first).
-__global__ void k_nd_level(const int32_t* q, int64_t n, const int32_t* parent, int32_t* nd) {
+// nd[parent] += nd[v] for the vertices of one level (deepest level first). What the sum held before, less
+// the parent itself, is the subtrees of the siblings that came earlier: the vertex's offset among them in
+// a preorder (any order of siblings makes one). Grouping the children by a sort and scanning their sizes
+// took another 0.3 ms of 4.5 ms on the 4.8M-vertex R-MAT, and fifteen launches on a small graph.
+__global__ void k_nd_level(const int32_t* q, int64_t n, const int32_t* parent, int32_t* nd, int32_t* off) {
     GRID_STRIDE(i, n) {
         const int32_t v = q[i];
-        atomicAdd(&nd[parent[v]], nd[v]);
-    }
-}
-
-// Children grouped by parent: key (parent << 32 | v) for non-root vertices.
-__global__ void k_child_keys(int64_t V, const int32_t* parent, uint64_t* keys, uint8_t* flag) {
-    GRID_STRIDE(v, V) {
-        const int32_t p = parent[v];
-        keys[v] = ((uint64_t)(uint32_t)p << 32) | (uint64_t)v;
-        flag[v] = p >= 0 && p != (int32_t)v;
-    }
-}
-
-// Sibling offsets: off[v] = sum of nd over the earlier children of parent(v).
-__global__ void k_child_nd(const uint64_t* keys, int64_t n, const int32_t* nd, int64_t* scan_in) {
-    GRID_STRIDE(i, n) scan_in[i] = nd[(int64_t)(keys[i] & 0xffffffffULL)];
-    if (blockIdx.x == 0 && threadIdx.x == 0) scan_in[n] = 0;
-}
-
-__global__ void k_group_first(const uint64_t* keys, int64_t n, int64_t* first_of_parent) {
-    GRID_STRIDE(i, n) {
-        const int64_t p = (int64_t)(keys[i] >> 32);
-        if (i == 0 || (int64_t)(keys[i - 1] >> 32) != p) first_of_parent[p] = i;
-    }
-}
-
-__global__ void k_sibling_off(const uint64_t* keys, int64_t n, const int64_t* scan, const int64_t* first_of_parent,
-                              int32_t* off) {
-    GRID_STRIDE(i, n) {
-        const int64_t p = (int64_t)(keys[i] >> 32);
-        const int64_t v = (int64_t)(keys[i] & 0xffffffffULL);
-        off[v] = (int32_t)(scan[i] - scan[first_of_parent[p]]);
+        off[v] = atomicAdd(&nd[parent[v]], nd[v]) - 1;
     }
 }
 
@@ -343,34 +314,43 @@ __global__ void k_pack_keys(int64_t V, const int32_t* pre, const int32_t* scc, i
 // Unions are idempotent, so the sample changes no class.
 constexpr int kSample = 4;
 
-__global__ void k_nontree_sample(int64_t V, HView h, const int2* key, const int32_t* nd, int32_t* low, int32_t* high,
-                                 int32_t* uf, unsigned long long* err) {
+// The first pass takes low and high and, without atomics, puts every tree edge under the first of the
+// smaller ones it is joined to; after a flatten the second joins loosely (uf_hook: the sweep below does not
+// depend on it).
+__global__ void k_nontree_first(int64_t V, HView h, const int2* key, const int32_t* nd, int32_t* low, int32_t* high,
+                                int32_t* uf) {
     GRID_STRIDE(u, V) {
         const int32_t d = h.sym.deg[u];
-        if (d == 0) continue;
         const int2 ku = key[u];
         const int64_t b = h.sym.beg[u];
-        int32_t lo = ku.x, hi = ku.x;
+        int32_t lo = ku.x, hi = ku.x, under = (int32_t)u;
         for (int j = 0; j < kSample && j < d; ++j) {
             const int32_t w = h.sym.adj[b + j];
             const int2 kw = key[w];
             if (ku.y != kw.y) continue;  // other SCC
             lo = kw.x < lo ? kw.x : lo;
             hi = kw.x > hi ? kw.x : hi;
-            const bool apart = kw.x > ku.x ? kw.x >= ku.x + nd[u] : ku.x >= kw.x + nd[w];
-            if (apart && uf[u] != uf[w]) uf_union(uf, (int32_t)u, w, err);
+            if (under == (int32_t)u && w < under && (kw.x > ku.x ? kw.x >= ku.x + nd[u] : ku.x >= kw.x + nd[w])) under = w;
         }
         low[u] = lo;
         high[u] = hi;
+        uf[u] = under;
     }
 }
 
-// Every uf entry to its root (read-only walks, then one write; no union runs meanwhile).
-__global__ void k_uf_flatten(int32_t* uf, int64_t V) {
-    GRID_STRIDE(v, V) {
-        int32_t x = uf[v];
-        while (uf[x] != x) x = uf[x];
-        uf[v] = x;
+__global__ void k_nontree_sample(int64_t V, HView h, const int2* key, const int32_t* nd, int32_t* uf) {
+    GRID_STRIDE(u, V) {
+        const int32_t d = h.sym.deg[u];
+        const int64_t b = h.sym.beg[u];
+        const int32_t ru = uf[u];
+        for (int j = 0; j < kSample && j < d; ++j) {
+            const int32_t w = h.sym.adj[b + j], rw = uf[w];
+            if (ru == rw) continue;
+            const int2 ku = key[u], kw = key[w];
+            if (ku.y != kw.y) continue;
+            const bool apart = kw.x > ku.x ? kw.x >= ku.x + nd[u] : ku.x >= kw.x + nd[w];
+            if (apart) uf_hook(uf, ru, rw);
+        }
     }
 }
 
@@ -485,17 +465,8 @@ __global__ void k_block_ids(const int32_t* reps, int64_t nb, int32_t* id_of_rep)
     GRID_STRIDE(b, nb) id_of_rep[reps[b]] = (int32_t)b;
 }
 
-// label_block and heads. A tree root's first block (that of its child with pre 1) is its parent
-// block (head -1); its other blocks hang from it.
-// Pass 1: the block of every tree root's first child (pre 1) becomes the root's parent block.
-__global__ void k_root_block(int64_t V, const int32_t* parent, const int32_t* pre, const int32_t* uf,
-                             const int32_t* id_of_rep, int32_t* label) {
-    GRID_STRIDE(v, V) {
-        const int32_t p = parent[v];
-        if (p != (int32_t)v && parent[p] == p && pre[v] == 1) label[p] = id_of_rep[uf[v]];
-    }
-}
-
+// label_block and heads. Pass 1 (k_root_block_least): the block of every tree root's smallest H neighbour
+// becomes the root's parent block (head -1); its other blocks hang from it.
 // Pass 2: parent blocks of the other vertices, and heads: a block's head is the parent p of its
 // topmost child ends (p is a tree root, or p's own parent edge is in another block); the root's
 // parent block has head -1.
@@ -618,9 +589,8 @@ int bct_build(gir_dev* g) {
     HView h{view(g->sym), scc};  // (row lengths replaced by the H lengths below)
     int32_t *parent = nullptr, *order = nullptr, *nd = nullptr, *pre = nullptr, *off = nullptr;
     int32_t *low = nullptr, *high = nullptr, *uf = nullptr, *reps = nullptr, *id_of_rep = nullptr;
-    uint64_t *keys = nullptr, *ktmp = nullptr;
     uint8_t* flag = nullptr;
-    int64_t *scan = nullptr, *first = nullptr;
+    int64_t* scan = nullptr;
     unsigned long long* cnt = nullptr;
     GIR_TRY(ensure_n(g, g->scratch[0], V + 1, &parent));
     GIR_TRY(ensure_n(g, g->scratch[2], V + 1, &order));
@@ -630,11 +600,8 @@ int bct_build(gir_dev* g) {
     GIR_TRY(ensure_n(g, g->scratch[6], V + 1, &low));
     GIR_TRY(ensure_n(g, g->scratch[7], V + 1, &high));
     GIR_TRY(ensure_n(g, g->scratch[8], V + 1, &uf));
-    GIR_TRY(ensure_n(g, g->scratch[9], V + 1, &keys));
-    GIR_TRY(ensure_n(g, g->scratch[10], V + 1, &ktmp));
     GIR_TRY(ensure_n(g, g->scratch[11], V + 1, &flag));
     GIR_TRY(ensure_n(g, g->scratch[12], V + 2, &scan));
-    GIR_TRY(ensure_n(g, g->scratch[13], V + 1, &first));
     GIR_TRY(ensure_n(g, g->scratch[14], 2 * C_N, &cnt));
     void* hp = nullptr;
     GIR_TRY(pinned(g, 256, &hp));
@@ -692,24 +659,10 @@ int bct_build(gir_dev* g) {
         for (int L = D - 1; L >= 1; --L) {
             const int64_t n = lvl_off[L + 1] - lvl_off[L];
             if (n == 0) continue;
-            k_nd_level<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(order + lvl_off[L], n, parent, nd);
+            k_nd_level<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(order + lvl_off[L], n, parent, nd, off);
             GIR_LAUNCH(g, "k_nd_level");
         }
-        //    preorder: children grouped by parent, sibling offsets, then levels top-down
-        k_child_keys<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, parent, keys, flag);
-        GIR_LAUNCH(g, "k_child_keys");
-        int64_t nc = 0;
-        GIR_TRY(select_flagged_u64(g, keys, flag, ktmp, V, &nc));
-        GIR_TRY(sort_keys_u64(g, ktmp, keys, nc, edge_key_bits(g->V)));
-        if (nc > 0) {
-            k_child_nd<<<grid_for(g, nc, kBlock), kBlock, 0, g->stream>>>(ktmp, nc, nd, scan);
-            GIR_LAUNCH(g, "k_child_nd");
-            GIR_TRY(exclusive_scan_i64(g, scan, scan, nc + 1));
-            k_group_first<<<grid_for(g, nc, kBlock), kBlock, 0, g->stream>>>(ktmp, nc, first);
-            GIR_LAUNCH(g, "k_group_first");
-            k_sibling_off<<<grid_for(g, nc, kBlock), kBlock, 0, g->stream>>>(ktmp, nc, scan, first, off);
-            GIR_LAUNCH(g, "k_sibling_off");
-        }
+        //    preorder: levels top-down
         k_pre_roots<<<grid_for(g, lvl_off[1], kBlock), kBlock, 0, g->stream>>>(order, lvl_off[1], pre);
         GIR_LAUNCH(g, "k_pre_roots");
         for (int L = 1; L < D; ++L) {
@@ -721,16 +674,20 @@ int bct_build(gir_dev* g) {
     }
     trace_mark(g, "bct: subtree sizes + preorder");
     // 3. low / high and rule 1
-    GIR_CUDA(g, cudaMemcpyAsync(low, pre, sizeof(int32_t) * V, cudaMemcpyDeviceToDevice, g->stream));
-    GIR_CUDA(g, cudaMemcpyAsync(high, pre, sizeof(int32_t) * V, cudaMemcpyDeviceToDevice, g->stream));
-    k_uf_init<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(uf, V);
-    GIR_LAUNCH(g, "k_uf_init");
     int2* key = nullptr;
     GIR_TRY(ensure_n(g, g->work[5], V + 1, &key));
     k_pack_keys<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, pre, scc, key);
     GIR_LAUNCH(g, "k_pack_keys");
-    k_nontree_sample<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, h, key, nd, low, high, uf, &cnt[C_ERR]);
-    GIR_LAUNCH(g, "k_nontree_sample");
+    k_nontree_first<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, h, key, nd, low, high, uf);
+    GIR_LAUNCH(g, "k_nontree_first");
+    k_uf_flatten<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(uf, V);
+    GIR_LAUNCH(g, "k_uf_flatten");
+    for (int r = 0; r < 2; ++r) {
+        k_nontree_sample<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, h, key, nd, uf);
+        GIR_LAUNCH(g, "k_nontree_sample");
+        k_uf_flatten<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(uf, V);
+        GIR_LAUNCH(g, "k_uf_flatten");
+    }
     auto carry_up = [&](const uint8_t* only) -> int {
         for (int L = D - 1; L >= 1; --L) {
             const int64_t n = lvl_off[L + 1] - lvl_off[L];
@@ -765,7 +722,7 @@ int bct_build(gir_dev* g) {
         k_sweep_len<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, hdeg, uf, need, giant, len);
         GIR_LAUNCH(g, "k_sweep_len");
     }
-    GIR_TRY(scan_degrees(g, len, V, scan));  // (scan is free after the preorder)
+    GIR_TRY(scan_degrees(g, len, V, scan));
     k_nontree<<<g->num_sms * 8, kBlock, 0, g->stream>>>(V, scan, h, key, nd, low, high, uf, &cnt[C_ERR]);
     GIR_LAUNCH(g, "k_nontree");
     if (deep) GIR_TRY(subtree_windows(g, order, n_tree, nd, low, high));
@@ -785,20 +742,15 @@ int bct_build(gir_dev* g) {
     k_block_ids<<<grid_for(g, nb, kBlock), kBlock, 0, g->stream>>>(reps, nb, id_of_rep);
     GIR_LAUNCH(g, "k_block_ids");
     GIR_TRY(ensure_n(g, g->blk_head, nb + 1, &head));
-    if (deep) {
-        int32_t *rdeg = pre, *least = high;  // (neither is read any more)
-        k_root_rows<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, scc, hdeg, rdeg, least);
-        GIR_LAUNCH(g, "k_root_rows");
-        CSRView rows = h.sym;
-        rows.deg = rdeg;
-        k_root_least<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, rows, scc, least);
-        GIR_LAUNCH(g, "k_root_least");
-        k_root_block_least<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, least, uf, id_of_rep, label);
-        GIR_LAUNCH(g, "k_root_block_least");
-    } else {
-        k_root_block<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, parent, pre, uf, id_of_rep, label);
-        GIR_LAUNCH(g, "k_root_block");
-    }
+    int32_t *rdeg = pre, *least = high;  // (neither is read any more)
+    k_root_rows<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, scc, hdeg, rdeg, least);
+    GIR_LAUNCH(g, "k_root_rows");
+    CSRView rows = h.sym;
+    rows.deg = rdeg;
+    k_root_least<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, rows, scc, least);
+    GIR_LAUNCH(g, "k_root_least");
+    k_root_block_least<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, least, uf, id_of_rep, label);
+    GIR_LAUNCH(g, "k_root_block_least");
     k_block_assign<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, parent, nd, uf, id_of_rep, label, head);
     GIR_LAUNCH(g, "k_block_assign");
     k_bcnt<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, head, nb, bcnt);

@@ -105,17 +105,23 @@ __global__ void k_pair_keys(const uint64_t* a, int64_t na, const uint64_t* b, in
     }
 }
 
-__global__ void k_pair_presence(const uint64_t* pairs, int64_t n, CSRView fw, int64_t V, uint8_t* pres) {
-    GRID_STRIDE(i, n) {
+__global__ void k_pair_presence(const uint64_t* pairs, const int64_t* n, CSRView fw, int64_t V, uint8_t* pres) {
+    GRID_STRIDE(i, *n) {
         const int32_t x = (int32_t)(pairs[i] >> 32), y = (int32_t)(pairs[i] & 0xffffffffULL);
         pres[i] = csr_has(fw, V, x, y) || csr_has(fw, V, y, x);
     }
 }
 
-// Symmetric ops: both directions of every pair whose undirected presence changed.
-__global__ void k_sym_ops(const uint64_t* pairs, int64_t n, const uint8_t* before, CSRView fw, int64_t V,
-                          uint64_t* keys2, uint8_t* f_ins, uint8_t* f_del) {
-    GRID_STRIDE(i, n) {
+// Symmetric ops: both directions of every pair whose undirected presence changed (n_pairs: a device word,
+// at most n_max; the slots beyond it are not flagged).
+__global__ void k_sym_ops(const uint64_t* pairs, const int64_t* n_pairs, int64_t n_max, const uint8_t* before, CSRView fw,
+                          int64_t V, uint64_t* keys2, uint8_t* f_ins, uint8_t* f_del) {
+    const int64_t n = *n_pairs;
+    GRID_STRIDE(i, n_max) {
+        if (i >= n) {
+            f_ins[2 * i] = f_ins[2 * i + 1] = f_del[2 * i] = f_del[2 * i + 1] = 0;
+            continue;
+        }
         const uint64_t p = pairs[i];
         const int32_t x = (int32_t)(p >> 32), y = (int32_t)(p & 0xffffffffULL);
         const bool after = csr_has(fw, V, x, y) || csr_has(fw, V, y, x);
@@ -307,6 +313,9 @@ int create_impl(const int32_t* fw_beg, const int32_t* fw_adj, const int32_t* bw_
 //    (not an edge of H) or is an inserted pair whose endpoints already share a block (a
 //    block's vertices are those with it as parent block plus its head).
 enum { F_SCC_SPLIT = 4, F_SCC_CYCLE = 5, F_DAG = 6, F_BCT = 7, F_N = 8 };
+// The batch's device words after those: two counts of compactions, the number of touched pairs, and the
+// flag of a merge that does not fit its CSR.
+enum { F_COUNT = 8, F_PAIRS = 10, F_BAD = 11, F_WORDS = 12 };
 
 __global__ void k_classify_directed(const uint64_t* ins, int64_t n_ins, const uint64_t* del, int64_t n_del,
                                     const int32_t* scc, const int32_t* rank, unsigned long long* cnt) {
@@ -544,12 +553,14 @@ int apply_batch_impl(gir_dev* g, const int32_t* u, const int32_t* v, const uint8
     if ((rc = ensure_n(g, g->work[0], n + 1, &keys)) || (rc = ensure_n(g, g->work[1], n + 1, &ktmp)) ||
         (rc = ensure_n(g, g->work[2], n + 1, &pos)) || (rc = ensure_n(g, g->work[3], n + 1, &ptmp)) ||
         (rc = ensure_n(g, g->work[4], 2 * n + 2, &f_ins)) || (rc = ensure_n(g, g->work[5], n + 1, &ins_k)) ||
-        (rc = ensure_n(g, g->work[6], n + 1, &del_k)) || (rc = ensure_n(g, g->work[7], F_N, &cnt))) {
+        (rc = ensure_n(g, g->work[6], n + 1, &del_k)) || (rc = ensure_n(g, g->work[7], F_WORDS, &cnt))) {
         cleanup();
         return rc;
     }
     f_del = f_ins + n + 1;
-    cudaMemsetAsync(cnt, 0, F_N * sizeof(unsigned long long), g->stream);
+    int64_t* const counts = reinterpret_cast<int64_t*>(cnt + F_COUNT);
+    int32_t* const bad = reinterpret_cast<int32_t*>(cnt + F_BAD);
+    cudaMemsetAsync(cnt, 0, F_WORDS * sizeof(unsigned long long), g->stream);
     k_batch_keys<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>((const int32_t*)du, (const int32_t*)dv, n, V, keys,
                                                                    pos, cnt);
     if ((rc = cuda_check(g, cudaGetLastError(), "k_batch_keys")) ||
@@ -559,25 +570,28 @@ int apply_batch_impl(gir_dev* g, const int32_t* u, const int32_t* v, const uint8
     }
     k_batch_classify<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(keys, pos, n, (const uint8_t*)dins, view(g->fw),
                                                                        V, f_ins, f_del, cnt + 1);
-    int64_t n_ins = 0, n_del = 0;
+    void* hp = nullptr;
     if ((rc = cuda_check(g, cudaGetLastError(), "k_batch_classify")) ||
-        (rc = select_flagged_u64(g, keys, f_ins, ins_k, n, &n_ins)) ||
-        (rc = select_flagged_u64(g, keys, f_del, del_k, n, &n_del))) {
+        (rc = select_flagged_u64_to(g, keys, f_ins, ins_k, n, counts)) ||
+        (rc = select_flagged_u64_to(g, keys, f_del, del_k, n, counts + 1)) || (rc = pinned(g, kPinnedBytes, &hp))) {
         cleanup();
         return rc;
     }
-    unsigned long long hc[2] = {0, 0};
-    cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, g->stream);
-    uint64_t one_key = 0;  // the change of a batch with exactly one (the single-edge latency path)
-    if (n_ins + n_del == 1)
-        cudaMemcpyAsync(&one_key, n_ins ? ins_k : del_k, sizeof(uint64_t), cudaMemcpyDeviceToHost, g->stream);
+    unsigned long long* const hc = static_cast<unsigned long long*>(hp);
+    cudaMemcpyAsync(hc, cnt, F_WORDS * sizeof(unsigned long long), cudaMemcpyDeviceToHost, g->stream);
     if ((rc = cuda_check(g, cudaStreamSynchronize(g->stream), "batch counters"))) { cleanup(); return rc; }
     cleanup();
+    const int64_t n_ins = (int64_t)hc[F_COUNT], n_del = (int64_t)hc[F_COUNT + 1];
     g->b_invalid = (int64_t)hc[0];
     g->b_noop = (int64_t)hc[1];
     g->b_ins = n_ins;
     g->b_del = n_del;
     if (n_ins + n_del == 0) return GIR_OK;
+    uint64_t one_key = 0;  // the change of a batch with exactly one (the single-edge latency path)
+    if (n_ins + n_del == 1) {
+        GIR_CUDA(g, cudaMemcpyAsync(&one_key, n_ins ? ins_k : del_k, sizeof(uint64_t), cudaMemcpyDeviceToHost, g->stream));
+        GIR_CUDA(g, cudaStreamSynchronize(g->stream));
+    }
     GIR_TRY(inc_log(g, ins_k, n_ins, del_k, n_del));
     trace_mark(g, "batch: normalize");
     if (g->scc_built) {
@@ -603,15 +617,15 @@ int apply_batch_impl(gir_dev* g, const int32_t* u, const int32_t* v, const uint8
     GIR_TRY(sort_keys_u64(g, pairs, ptmp2, np, edge_key_bits(g->V)));
     k_distinct<<<grid_for(g, np, kBlock), kBlock, 0, g->stream>>>(pairs, np, pflag);
     GIR_LAUNCH(g, "k_distinct");
-    int64_t npu = 0;
-    GIR_TRY(select_flagged_u64(g, pairs, pflag, ptmp2, np, &npu));
+    int64_t* const npu = reinterpret_cast<int64_t*>(cnt + F_PAIRS);  // (at most np)
+    GIR_TRY(select_flagged_u64_to(g, pairs, pflag, ptmp2, np, npu));
     std::swap(pairs, ptmp2);
-    k_pair_presence<<<grid_for(g, npu, kBlock), kBlock, 0, g->stream>>>(pairs, npu, view(g->fw), V, before);
+    k_pair_presence<<<grid_for(g, np, kBlock), kBlock, 0, g->stream>>>(pairs, npu, view(g->fw), V, before);
     GIR_LAUNCH(g, "k_pair_presence");
 
     trace_mark(g, "batch: pairs");
     // forward, then backward (transposed keys, re-sorted)
-    GIR_TRY(store_apply_ops(g, g->fw, ins_k, n_ins, del_k, n_del, true));
+    GIR_TRY(store_apply_ops(g, g->fw, ins_k, n_ins, del_k, n_del, true, bad));
     trace_mark(g, "batch: forward ops");
     GIR_TRY(ensure_n(g, g->work[4], np + 2, &tk));
     uint64_t* tk2 = tk + n_ins + 1;
@@ -625,17 +639,21 @@ int apply_batch_impl(gir_dev* g, const int32_t* u, const int32_t* v, const uint8
         GIR_LAUNCH(g, "k_transpose_keys");
         GIR_TRY(sort_keys_u64(g, tk2, del_k, n_del, edge_key_bits(g->V)));
     }
-    GIR_TRY(store_apply_ops(g, g->bw, tk, n_ins, tk2, n_del, false));
+    GIR_TRY(store_apply_ops(g, g->bw, tk, n_ins, tk2, n_del, false, bad));
     trace_mark(g, "batch: backward ops");
 
     // symmetrized view: pairs whose undirected presence changed
-    k_sym_ops<<<grid_for(g, npu, kBlock), kBlock, 0, g->stream>>>(pairs, npu, before, view(g->fw), V, sym_keys, fsi, fsd);
+    k_sym_ops<<<grid_for(g, np, kBlock), kBlock, 0, g->stream>>>(pairs, npu, np, before, view(g->fw), V, sym_keys, fsi,
+                                                                 fsd);
     GIR_LAUNCH(g, "k_sym_ops");
-    GIR_TRY(ensure_n(g, g->work[5], 2 * npu + 2, &sym_ins));
-    GIR_TRY(ensure_n(g, g->work[6], 2 * npu + 2, &sym_del));
-    int64_t nsi = 0, nsd = 0;
-    GIR_TRY(select_flagged_u64(g, sym_keys, fsi, sym_ins, 2 * npu, &nsi));
-    GIR_TRY(select_flagged_u64(g, sym_keys, fsd, sym_del, 2 * npu, &nsd));
+    GIR_TRY(ensure_n(g, g->work[5], 2 * np + 2, &sym_ins));
+    GIR_TRY(ensure_n(g, g->work[6], 2 * np + 2, &sym_del));
+    GIR_TRY(select_flagged_u64_to(g, sym_keys, fsi, sym_ins, 2 * np, counts));
+    GIR_TRY(select_flagged_u64_to(g, sym_keys, fsd, sym_del, 2 * np, counts + 1));
+    GIR_CUDA(g, cudaMemcpyAsync(hc, cnt, F_WORDS * sizeof(unsigned long long), cudaMemcpyDeviceToHost, g->stream));
+    GIR_CUDA(g, cudaStreamSynchronize(g->stream));
+    if (hc[F_BAD]) return store_ops_bad(g);
+    const int64_t nsi = (int64_t)hc[F_COUNT], nsd = (int64_t)hc[F_COUNT + 1];
     GIR_TRY(sort_keys_u64(g, sym_ins, sym_keys, nsi, edge_key_bits(g->V)));
     GIR_TRY(sort_keys_u64(g, sym_del, sym_keys, nsd, edge_key_bits(g->V)));
     if (g->bct_built && nsi + nsd > 0) {
@@ -644,13 +662,15 @@ int apply_batch_impl(gir_dev* g, const int32_t* u, const int32_t* v, const uint8
             static_cast<const int32_t*>(g->blk_head.p), cnt);
         GIR_LAUNCH(g, "k_classify_pairs");
     }
-    GIR_TRY(store_apply_ops(g, g->sym, sym_ins, nsi, sym_del, nsd, false));
+    GIR_TRY(store_apply_ops(g, g->sym, sym_ins, nsi, sym_del, nsd, false, bad));
     trace_mark(g, "batch: symmetric ops");
 
     GIR_TRY(invalidate_after_update(g));
-    unsigned long long fl[F_N] = {};
-    GIR_CUDA(g, cudaMemcpyAsync(fl, cnt, sizeof(fl), cudaMemcpyDeviceToHost, g->stream));
+    GIR_CUDA(g, cudaMemcpyAsync(hc, cnt, F_WORDS * sizeof(unsigned long long), cudaMemcpyDeviceToHost, g->stream));
     GIR_CUDA(g, cudaStreamSynchronize(g->stream));
+    if (hc[F_BAD]) return store_ops_bad(g);
+    unsigned long long fl[F_N];
+    std::memcpy(fl, hc, sizeof(fl));
     g->b_ms[0] = now_ms() - t_start;
     if (deferred) {
         g->pend = true;

@@ -285,8 +285,12 @@ int store_free(gir_dev* g, DevCSR& c);
 int store_build_sym(gir_dev* g);
 int store_compact_csr(gir_dev* g, const DevCSR& c, int64_t* beg_out, int32_t* adj_out, int64_t cap);
 int store_has_edges(gir_dev* g, const DevCSR& c, const int32_t* u, const int32_t* v, int64_t n, uint8_t* out);
+// `bad`: a device word, zero at the start of a batch; a merge whose ops do not fit its CSR sets it, changes
+// nothing and the caller finds out at its next read (or store_apply_ops itself at the next CSR's: then it
+// returns GIR_ERR_MALFORMED, as store_ops_bad does).
 int store_apply_ops(gir_dev* g, DevCSR& c, const uint64_t* ins, int64_t n_ins, const uint64_t* del, int64_t n_del,
-                    bool weights);
+                    bool weights, int32_t* bad);
+int store_ops_bad(gir_dev* g);
 int store_build_bins(gir_dev* g);
 // One change u -> v applied in place to the fw / bw / sym rows when they have room (store.cu):
 // out[0] 0 no-op, 1 applied, 2 no room (nothing changed); out[1] 1 / 2 when the undirected pair
@@ -315,9 +319,12 @@ int exclusive_scan_i64(gir_dev* g, const int64_t* in, int64_t* out, int64_t n);
 int sum_i64(gir_dev* g, const int64_t* in, int64_t n, int64_t* host_out);
 // Compacts the entries of `in` whose flag is non-zero into `out`; *host_n = count.
 int select_flagged_u64(gir_dev* g, const uint64_t* in, const uint8_t* flags, uint64_t* out, int64_t n, int64_t* host_n);
+// The same with the count left on the device.
+int select_flagged_u64_to(gir_dev* g, const uint64_t* in, const uint8_t* flags, uint64_t* out, int64_t n, int64_t* d_n);
 int select_flagged_i32(gir_dev* g, const int32_t* in, const uint8_t* flags, int32_t* out, int64_t n, int64_t* host_n);
 // Indices i in [0, n) with flags[i] != 0, ascending.
 int select_flagged_iota(gir_dev* g, const uint8_t* flags, int32_t* out, int64_t n, int64_t* host_n);
+int select_flagged_iota_to(gir_dev* g, const uint8_t* flags, int32_t* out, int64_t n, int64_t* d_n);
 // The rows of `deg` (V entries) longer than max_deg, ascending, into rows (V entries), and the
 // exclusive scan of their lengths into pref (V + 1 entries); *n = their number. flag: V bytes.
 int heavy_rows(gir_dev* g, const int32_t* deg, int64_t V, int32_t max_deg, uint8_t* flag, int32_t* rows, int64_t* pref,

@@ -153,7 +153,7 @@ __device__ __forceinline__ int64_t queue_find(const uint64_t* off, int64_t lo, i
 // entries in registers (one load each) and finds a position's entry by shuffles; two positions a
 // thread keep two rows of dependent loads in flight. The operation:
 //   op.row(entry, beg, pay)    first index of the entry's row, and 64 bits that go with it
-//   op.adj(index, pay)         the neighbour at an index of the row (>= 0)
+//   op.adj(index, pay)         the neighbour at an index of the row (>= 0); may change its copy of pay
 //   op.want(w, pay)            the bits the neighbour may take (0: none); a plain read
 //   op.apply(w, pay, bits, e)  takes them by an atomic; true when e joins the next queue
 //   op.deg(entry)              row length
@@ -350,6 +350,12 @@ __device__ __forceinline__ int32_t first_hit(const int32_t* adj, int64_t b, int3
     }
     return found;
 }
+
+// An operation without bottom-up levels.
+struct TopDownOnly {
+    bool wants(int64_t, int64_t) const { return false; }
+    int launch(gir_dev*, const Queue&, int64_t, const Queue&, unsigned long long*) const { return GIR_OK; }
+};
 
 // Runs up to max_levels more levels. Before the first call the caller zeroes ctl (kLoopWords words),
 // puts the first frontier at the front of the queue arrays and its packed size in ctl[W_Q].

@@ -185,15 +185,26 @@ int sum_i64(gir_dev* g, const int64_t* in, int64_t n, int64_t* host_out) {
     return GIR_OK;
 }
 
+// Compaction with the count left on the device (d_n).
+template <class It, class T>
+static int select_flagged_to(gir_dev* g, It in, const uint8_t* flags, T* out, int64_t n, int64_t* d_n) {
+    if (n <= 0) {
+        GIR_CUDA(g, cudaMemsetAsync(d_n, 0, sizeof(int64_t), g->stream));
+        return GIR_OK;
+    }
+    size_t bytes = 0;
+    GIR_CUDA(g, cub::DeviceSelect::Flagged(nullptr, bytes, in, flags, out, d_n, n, g->stream));
+    GIR_TRY(ensure(g, g->cub_tmp, bytes));
+    GIR_CUDA(g, cub::DeviceSelect::Flagged(g->cub_tmp.p, bytes, in, flags, out, d_n, n, g->stream));
+    return GIR_OK;
+}
+
 template <class It, class T>
 static int select_flagged(gir_dev* g, It in, const uint8_t* flags, T* out, int64_t n, int64_t* host_n) {
     int64_t* d_n = nullptr;
     GIR_TRY(ensure_n(g, g->scratch[15], 1, &d_n));
     if (n <= 0) { *host_n = 0; return GIR_OK; }
-    size_t bytes = 0;
-    GIR_CUDA(g, cub::DeviceSelect::Flagged(nullptr, bytes, in, flags, out, d_n, n, g->stream));
-    GIR_TRY(ensure(g, g->cub_tmp, bytes));
-    GIR_CUDA(g, cub::DeviceSelect::Flagged(g->cub_tmp.p, bytes, in, flags, out, d_n, n, g->stream));
+    GIR_TRY(select_flagged_to(g, in, flags, out, n, d_n));
     void* h = nullptr;
     GIR_TRY(pinned(g, 64, &h));
     GIR_CUDA(g, cudaMemcpyAsync(h, d_n, sizeof(int64_t), cudaMemcpyDeviceToHost, g->stream));
@@ -202,6 +213,12 @@ static int select_flagged(gir_dev* g, It in, const uint8_t* flags, T* out, int64
     return GIR_OK;
 }
 
+int select_flagged_u64_to(gir_dev* g, const uint64_t* in, const uint8_t* flags, uint64_t* out, int64_t n, int64_t* d_n) {
+    return select_flagged_to(g, in, flags, out, n, d_n);
+}
+int select_flagged_iota_to(gir_dev* g, const uint8_t* flags, int32_t* out, int64_t n, int64_t* d_n) {
+    return select_flagged_to(g, cub::CountingInputIterator<int32_t>(0), flags, out, n, d_n);
+}
 int select_flagged_u64(gir_dev* g, const uint64_t* in, const uint8_t* flags, uint64_t* out, int64_t n, int64_t* host_n) {
     return select_flagged(g, in, flags, out, n, host_n);
 }

@@ -40,9 +40,10 @@ enum { C_Q = 0, C_ACT = 1, C_ROOTS = 2, C_PIV = 3, C_ACT_E = 4, C_N = 8 };
 
 // Active in/out degree counts (self-loops excluded) and the first trim frontier.
 __global__ void k_trim_init(int64_t V, CSRView fw, CSRView bw, int32_t* label, int32_t* indeg, int32_t* outdeg,
-                            int32_t* q, unsigned long long* cnt) {
+                            Queue q, unsigned long long* cnt) {
     __shared__ int32_t s_st[kBlock / 32][kStage];
     int n_st = 0;
+    auto deg = [&](int32_t v) { return (int64_t)fw.deg[v] + bw.deg[v]; };
     for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < V; base += (int64_t)gridDim.x * blockDim.x) {
         const int64_t v = base + threadIdx.x;
         bool trim = false;
@@ -57,32 +58,39 @@ __global__ void k_trim_init(int64_t V, CSRView fw, CSRView bw, int32_t* label, i
             trim = (o == 0 || in == 0);
             label[v] = trim ? (int32_t)v : -1;
         }
-        stage_append(trim, (int32_t)v, s_st[threadIdx.x >> 5], n_st, q, &cnt[C_Q]);
+        queue_push(trim, (int32_t)v, s_st[threadIdx.x >> 5], n_st, q, deg, cnt);
     }
-    stage_flush(s_st[threadIdx.x >> 5], n_st, q, &cnt[C_Q]);
+    queue_flush(s_st[threadIdx.x >> 5], n_st, q, deg, cnt);
 }
 
-// One trim round over the removed vertices of the last round: lower the counts of their
-// neighbours; a neighbour whose count reaches 0 is removed (claimed once by CAS).
-__global__ void __launch_bounds__(kBlock) k_trim_out(const int32_t* q, const unsigned long long* qlen, CSRView fw,
-                                                     int32_t* label, int32_t* indeg, int32_t* nq,
-                                                     unsigned long long* cnt) {
-    warp_expand(q, (int64_t)*qlen, fw, nq, &cnt[C_Q], [&](int32_t u, int32_t w) {
-        if (w == u) return false;
-        if (atomicSub(&indeg[w], 1) == 1) return atomicCAS(&label[w], -1, w) == -1;
-        return false;
-    });
-}
-
-__global__ void __launch_bounds__(kBlock) k_trim_in(const int32_t* q, const unsigned long long* qlen, CSRView bw,
-                                                    int32_t* label, int32_t* outdeg, int32_t* nq,
-                                                    unsigned long long* cnt) {
-    warp_expand(q, (int64_t)*qlen, bw, nq, &cnt[C_Q], [&](int32_t u, int32_t w) {
-        if (w == u) return false;
-        if (atomicSub(&outdeg[w], 1) == 1) return atomicCAS(&label[w], -1, w) == -1;
-        return false;
-    });
-}
+// One trim round over the removed vertices of the last round (frontier.cuh): lower the counts of their
+// neighbours; a neighbour whose count reaches 0 is removed (claimed once by CAS). A removed vertex's row
+// here is its forward row with its backward row behind it; pay holds the vertex, its forward length from
+// bit 32 on, and bit 63 for an entry of the backward row.
+struct Trim {
+    CSRView fw, bw;
+    int32_t *label, *indeg, *outdeg;
+    __device__ __forceinline__ int64_t deg(int32_t v) const { return (int64_t)fw.deg[v] + bw.deg[v]; }
+    __device__ __forceinline__ void row(int32_t v, int64_t& beg, unsigned long long& pay) const {
+        beg = 0;
+        pay = ((unsigned long long)(uint32_t)fw.deg[v] << 32) | (uint32_t)v;
+    }
+    __device__ __forceinline__ int32_t adj(int64_t i, unsigned long long& pay) const {
+        const int32_t v = (int32_t)(uint32_t)pay;
+        const int64_t n = (int64_t)(pay >> 32);
+        if (i < n) return fw.adj[fw.beg[v] + i];
+        pay |= 1ull << 63;
+        return bw.adj[bw.beg[v] + i - n];
+    }
+    __device__ __forceinline__ unsigned long long want(int32_t w, unsigned long long pay) const {
+        return w != (int32_t)(uint32_t)pay;
+    }
+    __device__ __forceinline__ bool apply(int32_t w, unsigned long long pay, unsigned long long, int32_t& e) {
+        e = w;
+        if (atomicSub((pay >> 63 ? outdeg : indeg) + w, 1) != 1) return false;
+        return atomicCAS(&label[w], -1, w) == -1;
+    }
+};
 
 // Trim-2 (iSpan's trim_2_from_fq, gir_constructor/includes/scc_cpu/trim_2_3.h:161, as an
 // algorithm source): u and v form an SCC of two when each is the other's only unassigned in-
@@ -374,31 +382,59 @@ __global__ void k_distinct_u64(const uint64_t* keys, int64_t n, uint8_t* flag) {
     GRID_STRIDE(i, n) flag[i] = (i == 0 || keys[i] != keys[i - 1]);
 }
 
-// One round of longest-path levels over the condensation edges: level(b) >= level(a) + 1 for
-// every edge a -> b. Edge-parallel with a plain pre-check, so only raises take an atomic (no
-// hot counter: a node with many in-edges, like the giant SCC, is raised a few times, not
-// decremented once per edge as in Kahn's algorithm).
-__global__ void k_dag_level_round(const uint64_t* keys, int64_t n, int32_t* level, unsigned long long* changed) {
-    unsigned long long c = 0;
-    GRID_STRIDE(i, n) {
-        const uint64_t k = keys[i];
-        const int32_t a = (int32_t)(k >> 32), b = (int32_t)(k & 0xffffffffULL);
-        const int32_t cand = level[a] + 1;
-        if (cand > level[b] && atomicMax(&level[b], cand) < cand) ++c;
+// Longest-path levels over the condensation edges: level(b) >= level(a) + 1 for every edge a -> b, in
+// rounds until nothing changes, all of them in one cooperative launch with a grid barrier a round (a
+// launch, two copies and a host read a round had been 22 us). Edge-parallel with a plain pre-check, so
+// only raises take an atomic (no hot counter: a node with many in-edges, like the giant SCC, is raised a
+// few times, not decremented once per edge as in Kahn's algorithm).
+// ctl: [0..2] raises of a round (in turn), [3] error, [5] raises of the last round, [6] the largest level
+// raised to (a round may carry a level far); the barrier's counter from word 16 on.
+constexpr int kDagWords = 32;
+__global__ void __launch_bounds__(kLoopThreads, 2) k_dag_levels(const uint64_t* keys, int64_t n, int32_t* level,
+                                                                unsigned long long* ctl, int max_rounds) {
+    unsigned int* bar = reinterpret_cast<unsigned int*>(ctl + 16);
+    unsigned long long raised = 0;
+    int32_t top = 0;
+    int round = 0;
+    while (round < max_rounds) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) ctl[(round + 1) % 3] = 0;
+        unsigned long long c = 0;
+        GRID_STRIDE(i, n) {
+            const uint64_t k = keys[i];
+            const int32_t a = (int32_t)(k >> 32), b = (int32_t)(k & 0xffffffffULL);
+            const int32_t cand = __ldcg(level + a) + 1;
+            if (cand > __ldcg(level + b) && atomicMax(&level[b], cand) < cand) {
+                ++c;
+                top = cand > top ? cand : top;
+            }
+        }
+        c = warp_sum_u64(c);
+        if (lane_id() == 0 && c) atomicAdd(&ctl[round % 3], c);
+        if (!grid_barrier(bar, ctl + 3, kLoopSpins)) return;
+        raised = __ldcg(ctl + round % 3);
+        ++round;
+        if (raised == 0) break;
     }
-    for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if (lane_id() == 0 && c) atomicAdd(changed, c);
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (lane_id() == 0 && top) atomicMax(&ctl[6], (unsigned long long)top);
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctl[5] = raised;
 }
 
-__global__ void k_rank_keys(int64_t V, const int32_t* label, const int32_t* level, uint64_t* keys,
-                            unsigned long long* n) {
-    GRID_STRIDE(v, V) {
-        if (label[v] == (int32_t)v) keys[atomicAdd(n, 1ull)] = ((uint64_t)(uint32_t)level[v] << 32) | (uint32_t)v;
+// Keys (level << vb | label) of the SCCs, vb the bits of a vertex id.
+__global__ void __launch_bounds__(kBlock) k_rank_keys(int64_t V, const int32_t* label, const int32_t* level, int vb,
+                                                      uint64_t* keys, unsigned long long* n) {
+    __shared__ int s_w[kWarps];
+    __shared__ unsigned long long s_base;
+    for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < V; base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t v = base + threadIdx.x;
+        const bool on = v < V && label[v] == (int32_t)v;
+        const unsigned long long at = block_slot(on, n, s_w, &s_base);
+        if (on) keys[at] = ((uint64_t)(uint32_t)level[v] << vb) | (uint64_t)v;
     }
 }
 
-__global__ void k_rank_scatter(const uint64_t* keys, int64_t n, int32_t* rank_of) {
-    GRID_STRIDE(i, n) rank_of[(int64_t)(keys[i] & 0xffffffffULL)] = (int32_t)i;
+__global__ void k_rank_scatter(const uint64_t* keys, int64_t n, int vb, int32_t* rank_of) {
+    GRID_STRIDE(i, n) rank_of[(int64_t)(keys[i] & ((1ull << vb) - 1))] = (int32_t)i;
 }
 
 __global__ void k_rank_gather(int64_t V, const int32_t* label, const int32_t* rank_of, int32_t* rank) {
@@ -412,7 +448,7 @@ __global__ void k_rank_gather(int64_t V, const int32_t* label, const int32_t* ra
 // neighbours by union-find leaves, on a graph that is undirected or nearly so (a road network), a few
 // classes and only the edges between the other vertices; the SCCs of that small quotient graph are
 // the SCCs of the graph.
-__global__ void k_reciprocal(int64_t V, CSRView fw, CSRView bw, CSRView sym, uint8_t* full, int32_t* cls,
+__global__ void k_reciprocal(int64_t V, CSRView fw, CSRView bw, CSRView sym, uint8_t* full,
                              unsigned long long* n_full) {
     unsigned long long c = 0;
     GRID_STRIDE(v, V) {
@@ -422,7 +458,6 @@ __global__ void k_reciprocal(int64_t V, CSRView fw, CSRView bw, CSRView sym, uin
         const int32_t self = p < fb + o && fw.adj[p] == (int32_t)v;
         const bool f = o - self == sym.deg[v] && bw.deg[v] - self == sym.deg[v];
         full[v] = f;
-        cls[v] = (int32_t)v;
         c += f;
     }
     c = warp_sum_u64(c);
@@ -440,14 +475,6 @@ __global__ void __launch_bounds__(kBlock) k_class_link(int64_t V, CSRView sym, i
     const int wib = threadIdx.x >> 5;
     warp_sweep_rows(sym.beg, sym.deg, sym.adj, 0, V, s_excl[wib], s_u[wib],
                     [&](int32_t u, int32_t w, int64_t) { uf_union(cls, u, w, err); });
-}
-
-__global__ void k_class_flatten(int64_t V, int32_t* cls) {
-    GRID_STRIDE(v, V) {
-        int32_t x = cls[v];
-        while (cls[x] != x) x = cls[x];
-        cls[v] = x;
-    }
 }
 
 // Keys (class(u) << 32 | class(w)) of the edges between classes; counted only while keys is null.
@@ -532,7 +559,7 @@ static int scc_by_quotient(gir_dev* g, int32_t* label, int64_t* n_scc, bool* use
         return GIR_OK;
     };
     GIR_CUDA(g, cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * 8, g->stream));
-    k_reciprocal<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, view(g->fw), view(g->bw), view(g->sym), full, cls, cnt);
+    k_reciprocal<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, view(g->fw), view(g->bw), view(g->sym), full, cnt);
     GIR_LAUNCH(g, "k_reciprocal");
     GIR_TRY(read());
     if ((int64_t)hc[0] * 2 < V) return GIR_OK;
@@ -540,10 +567,14 @@ static int scc_by_quotient(gir_dev* g, int32_t* label, int64_t* n_scc, bool* use
     sym.deg = mdeg;
     k_mask_deg<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, g->sym.deg, full, 1, mdeg);
     GIR_LAUNCH(g, "k_mask_deg");
+    k_uf_first<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(sym, V, cls);
+    GIR_LAUNCH(g, "k_uf_first");
+    k_uf_flatten<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(cls, V);
+    GIR_LAUNCH(g, "k_uf_flatten");
     k_class_link<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, sym, cls, cnt + 1);
     GIR_LAUNCH(g, "k_class_link");
-    k_class_flatten<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, cls);
-    GIR_LAUNCH(g, "k_class_flatten");
+    k_uf_flatten<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(cls, V);
+    GIR_LAUNCH(g, "k_uf_flatten");
     // (an edge between classes has two ends that are not full)
     fw.deg = mdeg;
     k_mask_deg<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, g->fw.deg, full, 0, mdeg);
@@ -634,18 +665,18 @@ static int scc_labels(gir_dev* g, const CSRView fw, const CSRView bw, bool whole
     trace_mark(g, "scc: start");
     // 1. trim-1
     GIR_CUDA(g, cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * 2 * C_N, g->stream));
-    k_trim_init<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, fw, bw, label, indeg, outdeg, qa, cnt);
+    Queue q{qa, nullptr};
+    unsigned long long* ctl = nullptr;
+    GIR_TRY(ensure_n(g, g->scratch[7], 2 * V + 2, &q.off));
+    GIR_TRY(ensure_n(g, g->scratch[10], kLoopWords, &ctl));
+    GIR_CUDA(g, cudaMemsetAsync(ctl, 0, sizeof(unsigned long long) * kLoopWords, g->stream));
+    k_trim_init<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, fw, bw, label, indeg, outdeg, q, ctl + W_Q);
     GIR_LAUNCH(g, "k_trim_init");
     int64_t n = 0;
-    GIR_TRY(lp.read(&n));
-    GIR_TRY(run_queue(qa, qb, n, [&](int32_t* in, int32_t* out, int64_t m) -> int {
-        // removed vertices lower both neighbour counts; both kernels append to `out`
-        k_trim_out<<<blocks_for_queue(m), kBlock, 0, g->stream>>>(in, qlen, fw, label, indeg, out, cnt);
-        GIR_LAUNCH(g, "k_trim_out");
-        k_trim_in<<<blocks_for_queue(m), kBlock, 0, g->stream>>>(in, qlen, bw, label, outdeg, out, cnt);
-        GIR_LAUNCH(g, "k_trim_in");
-        return GIR_OK;
-    }));
+    {
+        FrontierRun run;
+        GIR_TRY(run_frontier(g, Trim{fw, bw, label, indeg, outdeg}, TopDownOnly{}, q, ctl, run, INT64_MAX));
+    }
 
     // trim-2: SCCs of two vertices, through in-neighbours, then through out-neighbours
     {
@@ -700,10 +731,6 @@ static int scc_labels(gir_dev* g, const CSRView fw, const CSRView bw, bool whole
     if (rule != 3 && lp.hc[C_PIV] != 0) {
         const int32_t pivot = (int32_t)((lp.hc[C_PIV] - 1) & 0xffffffffULL);
         // both searches start from the pivot (marked both ways)
-        Queue q{qa, nullptr};
-        unsigned long long* ctl = nullptr;
-        GIR_TRY(ensure_n(g, g->scratch[7], 2 * V + 2, &q.off));
-        GIR_TRY(ensure_n(g, g->scratch[10], kLoopWords, &ctl));
         GIR_CUDA(g, cudaMemsetAsync(ctl, 0, sizeof(unsigned long long) * kLoopWords, g->stream));
         k_reach_init<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, label, pivot, fw, bw, mark, q, ctl);
         GIR_LAUNCH(g, "k_reach_init");
@@ -930,27 +957,39 @@ int scc_build_dag(gir_dev* g) {
     GIR_TRY(ensure_n(g, g->scratch[5], V + 1, &rank_of));
     GIR_TRY(ensure_n(g, g->scc_rank, V + 1, &rank));
     GIR_CUDA(g, cudaMemsetAsync(level, 0, sizeof(int32_t) * V, g->stream));
-    for (int64_t round = 0; n_dag > 0 && round <= V; ++round) {
-        GIR_CUDA(g, cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * C_N, g->stream));
-        k_dag_level_round<<<grid_for(g, n_dag, kBlock), kBlock, 0, g->stream>>>(dag, n_dag, level, &cnt[C_Q]);
-        GIR_LAUNCH(g, "k_dag_level_round");
-        GIR_CUDA(g, cudaMemcpyAsync(hc, cnt, sizeof(unsigned long long) * C_N, cudaMemcpyDeviceToHost, g->stream));
-        GIR_CUDA(g, cudaStreamSynchronize(g->stream));
-        if (hc[C_Q] == 0) break;
+    int64_t top = 0;  // the largest level
+    if (n_dag > 0) {
+        unsigned long long* ctl = nullptr;
+        GIR_TRY(ensure_n(g, g->scratch[10], kDagWords, &ctl));
+        int per_sm = 1;
+        GIR_CUDA(g, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dag_levels, kLoopThreads, 0));
+        while (true) {
+            GIR_CUDA(g, cudaMemsetAsync(ctl, 0, sizeof(unsigned long long) * kDagWords, g->stream));
+            int max_rounds = 1 << 22;  // (the barrier's counter is 32 bits wide)
+            const uint64_t* dag_c = dag;
+            int64_t n_c = n_dag;
+            void* args[] = {&dag_c, &n_c, &level, &ctl, &max_rounds};
+            GIR_CUDA(g, cudaLaunchCooperativeKernel((const void*)k_dag_levels, g->num_sms * (per_sm > 1 ? 2 : 1),
+                                                    kLoopThreads, args, 0, g->stream));
+            GIR_CUDA(g, cudaMemcpyAsync(hc, ctl, sizeof(unsigned long long) * 7, cudaMemcpyDeviceToHost, g->stream));
+            GIR_CUDA(g, cudaStreamSynchronize(g->stream));
+            if (hc[3]) return fail(g, GIR_ERR_TIMEOUT, "scc: a grid barrier of the DAG levels ran out its bound");
+            top = (int64_t)hc[6] > top ? (int64_t)hc[6] : top;
+            if (hc[5] == 0) break;
+        }
     }
     trace_mark(g, "scc: levels");
-    // rank = position in (level, label) order
+    // rank = position in (level, label) order (no more key bits than the largest of either)
+    const int vb = edge_key_bits(V) - 32;
     GIR_CUDA(g, cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * C_N, g->stream));
     if (V > 0) {
-        k_rank_keys<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, label, level, keys, &cnt[C_Q]);
+        k_rank_keys<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, label, level, vb, keys, &cnt[C_Q]);
         GIR_LAUNCH(g, "k_rank_keys");
     }
-    GIR_CUDA(g, cudaMemcpyAsync(hc, cnt, sizeof(unsigned long long) * C_N, cudaMemcpyDeviceToHost, g->stream));
-    GIR_CUDA(g, cudaStreamSynchronize(g->stream));
-    const int64_t ns = (int64_t)hc[C_Q];
-    GIR_TRY(sort_keys_u64(g, keys, tmp, ns, edge_key_bits(g->V)));
+    const int64_t ns = g->n_scc;
+    GIR_TRY(sort_keys_u64(g, keys, tmp, ns, vb + edge_key_bits(top) - 32));
     if (ns > 0) {
-        k_rank_scatter<<<grid_for(g, ns, kBlock), kBlock, 0, g->stream>>>(keys, ns, rank_of);
+        k_rank_scatter<<<grid_for(g, ns, kBlock), kBlock, 0, g->stream>>>(keys, ns, vb, rank_of);
         GIR_LAUNCH(g, "k_rank_scatter");
         k_rank_gather<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, label, rank_of, rank);
         GIR_LAUNCH(g, "k_rank_gather");

@@ -120,11 +120,19 @@ struct Touched {
 
 // Per touched row (from the merged op list `rows`, sorted distinct); elen / nlen = entries of its rest
 // before (old ones and inserts) and after the merge.
+// n_rows is a device word; the slots beyond it, up to n_ops, become empty rows.
 __global__ void k_touched_rows(const uint64_t* ins, int64_t n_ins, const uint64_t* del, int64_t n_del,
-                               const int32_t* rows, int64_t n_rows, CSRView c, Touched* touched, int64_t* elen,
-                               int64_t* nlen, int32_t* overflow) {
-    GRID_STRIDE(k, n_rows) {
+                               const int32_t* rows, const int64_t* n_rows, CSRView c, Touched* touched, int64_t* elen,
+                               int64_t* nlen, int32_t* overflow, int32_t* bad) {
+    const int64_t n_ops = n_ins + n_del, n = *n_rows;
+    GRID_STRIDE(k, n_ops) {
         Touched t;
+        if (k >= n) {
+            t.row = -1;
+            touched[k] = t;
+            elen[k] = nlen[k] = 0;
+            continue;
+        }
         t.row = rows[k];
         const uint64_t r = (uint64_t)(uint32_t)t.row;
         t.ib = lower_bound_dev(ins, (int64_t)0, n_ins, r << 32);
@@ -140,7 +148,7 @@ __global__ void k_touched_rows(const uint64_t* ins, int64_t n_ins, const uint64_
         t.keep = (int32_t)(lower_bound_dev(c.adj, t.beg, t.beg + t.deg, (int32_t)first) - t.beg);
         t.newdeg = (int32_t)nd;
         if (nd < t.keep) {  // more deletions than entries: the ops do not match this CSR
-            atomicExch(overflow + 1, 1);
+            atomicExch(bad, 1);
             t.newdeg = t.keep;
         }
         if (t.beg + nd > c.beg[r + 1]) atomicExch(overflow, 1);
@@ -148,7 +156,7 @@ __global__ void k_touched_rows(const uint64_t* ins, int64_t n_ins, const uint64_
         elen[k] = t.deg - t.keep + (t.ie - t.ib);
         nlen[k] = t.newdeg - t.keep;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) elen[n_rows] = nlen[n_rows] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) elen[n_ops] = nlen[n_ops] = 0;
 }
 
 // Merges the rest of every touched row into `tmp` (at noff[k]): surviving old entries and inserted
@@ -187,19 +195,30 @@ __global__ void k_merge_rows(const uint64_t* ins, const uint64_t* del, const Tou
     });
 }
 
+// The sizes the host needs, in one place to read: entries to merge, entries merged, a row outgrew its
+// slack, the batch's bad flag.
+__global__ void k_merge_sizes(const int64_t* eoff, const int64_t* noff, int64_t n, const int32_t* overflow,
+                              const int32_t* bad, int64_t* out) {
+    out[0] = eoff[n];
+    out[1] = noff[n];
+    out[2] = *overflow;
+    out[3] = *bad;
+}
+
 // Copies the merged rests back into their rows (capacities unchanged), and the new lengths.
 __global__ void k_copy_back(const Touched* touched, int64_t n_rows, const int64_t* noff, const int32_t* tmp,
-                            const uint32_t* tmpw, int32_t* deg, int32_t* adj, uint32_t* w) {
+                            const uint32_t* tmpw, int32_t* deg, int32_t* adj, uint32_t* w, const int32_t* bad) {
+    if (*bad) return;
     walk_segments(noff, n_rows, [&](int64_t k, int64_t j) {
         const int64_t to = touched[k].beg + touched[k].keep + j;
         adj[to] = tmp[noff[k] + j];
         if (w) w[to] = tmpw[noff[k] + j];
     });
-    GRID_STRIDE(k, n_rows) deg[touched[k].row] = touched[k].newdeg;
+    GRID_STRIDE(k, n_rows) if (touched[k].row >= 0) deg[touched[k].row] = touched[k].newdeg;
 }
 
 __global__ void k_set_deg(const Touched* touched, int64_t n_rows, int32_t* deg) {
-    GRID_STRIDE(k, n_rows) deg[touched[k].row] = touched[k].newdeg;
+    GRID_STRIDE(k, n_rows) if (touched[k].row >= 0) deg[touched[k].row] = touched[k].newdeg;
 }
 
 __global__ void k_mark_rows(const uint64_t* a, int64_t na, const uint64_t* b, int64_t nb, uint8_t* flag) {
@@ -230,7 +249,7 @@ __global__ void k_relayout_rows(int64_t V, const int64_t* old_beg, const int32_t
 __global__ void k_fill_i32(int32_t* p, int64_t n, int32_t v) { GRID_STRIDE(i, n) p[i] = v; }
 
 __global__ void k_mark_slots(const Touched* touched, int64_t n_rows, int32_t* slot) {
-    GRID_STRIDE(k, n_rows) slot[touched[k].row] = (int32_t)k;
+    GRID_STRIDE(k, n_rows) if (touched[k].row >= 0) slot[touched[k].row] = (int32_t)k;
 }
 
 __global__ void k_bin_flags(int64_t V, const int32_t* deg, int32_t small, int32_t large, uint8_t* f0, uint8_t* f1,
@@ -490,8 +509,12 @@ int store_has_edges(gir_dev* g, const DevCSR& c, const int32_t* u, const int32_t
     return GIR_OK;
 }
 
+int store_ops_bad(gir_dev* g) {
+    return fail(g, GIR_ERR_MALFORMED, "edge update: the backward CSR is not the transpose of the forward CSR");
+}
+
 int store_apply_ops(gir_dev* g, DevCSR& c, const uint64_t* ins, int64_t n_ins, const uint64_t* del, int64_t n_del,
-                    bool weights) {
+                    bool weights, int32_t* bad) {
     if (n_ins + n_del == 0) return GIR_OK;
     const int64_t V = g->V;
     const int64_t n_ops = n_ins + n_del;
@@ -506,49 +529,52 @@ int store_apply_ops(gir_dev* g, DevCSR& c, const uint64_t* ins, int64_t n_ins, c
     GIR_CUDA(g, cudaMemsetAsync(flag, 0, V, g->stream));
     k_mark_rows<<<grid_for(g, n_ops, kBlock), kBlock, 0, g->stream>>>(ins, n_ins, del, n_del, flag);
     GIR_LAUNCH(g, "k_mark_rows");
-    int64_t n_rows = 0;
-    GIR_TRY(select_flagged_iota(g, flag, rows, V, &n_rows));
-
+    // (their number stays on the device: at most one per op)
+    const int64_t n_rows = n_ops;
     int32_t* overflow = nullptr;
+    int64_t* words = nullptr;  // number of rows, then the sizes the host reads
     GIR_TRY(ensure_n(g, g->scratch[9], n_rows + 1, &touched));
     GIR_TRY(ensure_n(g, g->scratch[10], n_rows + 1, &eoff));
     GIR_TRY(ensure_n(g, g->scratch[11], n_rows + 1, &noff));
-    GIR_TRY(ensure_n(g, g->scratch[12], 4, &overflow));
-    GIR_CUDA(g, cudaMemsetAsync(overflow, 0, 2 * sizeof(int32_t), g->stream));
-    k_touched_rows<<<grid_for(g, n_rows, kBlock), kBlock, 0, g->stream>>>(ins, n_ins, del, n_del, rows, n_rows, view(c),
-                                                                           touched, eoff, noff, overflow);
+    GIR_TRY(ensure_n(g, g->scratch[12], 8, &words));
+    overflow = reinterpret_cast<int32_t*>(words + 6);
+    GIR_TRY(select_flagged_iota_to(g, flag, rows, V, words));
+    GIR_CUDA(g, cudaMemsetAsync(overflow, 0, sizeof(int32_t), g->stream));
+    k_touched_rows<<<grid_for(g, n_rows, kBlock), kBlock, 0, g->stream>>>(ins, n_ins, del, n_del, rows, words, view(c),
+                                                                           touched, eoff, noff, overflow, bad);
     GIR_LAUNCH(g, "k_touched_rows");
     GIR_TRY(exclusive_scan_i64(g, eoff, eoff, n_rows + 1));
     GIR_TRY(exclusive_scan_i64(g, noff, noff, n_rows + 1));
-    int64_t h[2] = {0, 0};
-    int32_t ovf = 0;
-    GIR_CUDA(g, cudaMemcpyAsync(&h[0], eoff + n_rows, sizeof(int64_t), cudaMemcpyDeviceToHost, g->stream));
-    GIR_CUDA(g, cudaMemcpyAsync(&h[1], noff + n_rows, sizeof(int64_t), cudaMemcpyDeviceToHost, g->stream));
-    GIR_CUDA(g, cudaMemcpyAsync(&ovf, overflow, sizeof(int32_t), cudaMemcpyDeviceToHost, g->stream));
+    k_merge_sizes<<<1, 1, 0, g->stream>>>(eoff, noff, n_rows, overflow, bad, words + 1);
+    GIR_LAUNCH(g, "k_merge_sizes");
+    void* hp = nullptr;
+    GIR_TRY(pinned(g, kPinnedBytes, &hp));
+    int64_t* h = static_cast<int64_t*>(hp);
+    GIR_CUDA(g, cudaMemcpyAsync(h, words + 1, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, g->stream));
     GIR_CUDA(g, cudaStreamSynchronize(g->stream));
     const int64_t n_elems = h[0], n_new = h[1];
+    const bool ovf = h[2] != 0;
+    if (h[3]) return store_ops_bad(g);
     const bool wts = weights && c.w;
     // tmp holds the merged rest of touched row k at noff[k]
     GIR_TRY(ensure_n(g, g->stage_out, n_new + 4, &tmp));
     if (wts) GIR_TRY(ensure_n(g, g->scratch[3], n_new + 4, &tmpw));
     if (n_elems > 0) {
         k_merge_rows<<<grid_for(g, n_elems, kBlock), kBlock, 0, g->stream>>>(
-            ins, del, touched, n_rows, eoff, noff, view(c), tmp, tmpw, wts, g->wrule_seed, g->wrule_lo, g->wrule_hi,
-            overflow + 1);
+            ins, del, touched, n_rows, eoff, noff, view(c), tmp, tmpw, wts, g->wrule_seed, g->wrule_lo, g->wrule_hi, bad);
         GIR_LAUNCH(g, "k_merge_rows");
     }
-    int32_t inconsistent = 0;
-    GIR_CUDA(g, cudaMemcpyAsync(&inconsistent, overflow + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, g->stream));
-    GIR_CUDA(g, cudaStreamSynchronize(g->stream));
-    if (inconsistent)
-        return fail(g, GIR_ERR_MALFORMED, "edge update: the backward CSR is not the transpose of the forward CSR");
     if (!ovf) {
         k_copy_back<<<grid_for(g, n_new > n_rows ? n_new : n_rows, kBlock), kBlock, 0, g->stream>>>(
-            touched, n_rows, noff, tmp, tmpw, c.deg, c.adj, wts ? c.w : nullptr);
+            touched, n_rows, noff, tmp, tmpw, c.deg, c.adj, wts ? c.w : nullptr, bad);
         GIR_LAUNCH(g, "k_copy_back");
     } else {
         // Some row outgrew its slack: new layout for the whole CSR.
         trace_mark(g, "store: merge before relayout");
+        int32_t inconsistent = 0;
+        GIR_CUDA(g, cudaMemcpyAsync(&inconsistent, bad, sizeof(int32_t), cudaMemcpyDeviceToHost, g->stream));
+        GIR_CUDA(g, cudaStreamSynchronize(g->stream));
+        if (inconsistent) return store_ops_bad(g);
         int32_t* slot = nullptr;
         int64_t* capv = nullptr;
         GIR_TRY(ensure_n(g, g->scratch[0], V + 1, &slot));
