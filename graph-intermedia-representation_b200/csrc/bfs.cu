@@ -170,13 +170,14 @@ struct TopDown {
         return lanes & ~__ldcg((const unsigned long long*)k.seen + w);
     }
     __device__ __forceinline__ bool apply(int32_t w, unsigned long long, unsigned long long bits, int32_t& e) {
+        const unsigned d = (unsigned)fw.deg[w];
         const unsigned long long nb = bits & ~atomicOr((unsigned long long*)k.seen + w, bits);
         if (!nb) return false;
         const bool fresh = atomicOr((unsigned long long*)k.next + w, nb) == 0ull;
         write_levels(k.level, w, nb, L);
         const unsigned c = __popcll(nb);
         pairs += c;
-        medges += (unsigned long long)c * (unsigned long long)fw.deg[w];
+        medges += (unsigned long long)c * d;
         e = w;
         return fresh;
     }
@@ -323,7 +324,8 @@ __device__ __forceinline__ void bu_ctas(const int32_t* ids, int64_t n, const CSR
 // 10 us on a lattice. Before, a level was two phases (expand, commit) with a barrier of eight CTAs
 // per SM after each and a warp took 32 frontier vertices whatever the frontier's size: 64 sources on
 // a 4.8M-vertex R-MAT 11.4 ms a call, now 5.1 ms; 37 sets on 0.78M vertices 3.0 -> 0.89 ms; 8 sources
-// on a 701 x 701 lattice 29.1 -> 11.3 ms; one source on 4,096 vertices 317 -> 145 us.
+// on a 701 x 701 lattice 29.3 -> 10.4 ms (11.4 before the barrier's one-way arrival, the first look
+// by interpolation and the degree loaded beside the claim); one source on 4,096 vertices 317 -> 145 us.
 constexpr int kPersistThreads = 1024;
 constexpr int kPersistWarps = kPersistThreads / 32;
 constexpr int64_t kPersistMaxEdges = 1ll << 22;   // a frontier's out-edges
@@ -384,6 +386,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_bfs_persistent(PersistAr
     double nf = (double)pairs0 / a.lanes, mf = (double)medges0 / a.lanes, mu = a.mu0 - mf;
     unsigned long long edges = a.count_first ? medges0 : 0, reached = a.count_first ? pairs0 : 0;
     unsigned long long pr = pairs0, me = medges0;
+    unsigned met = 0;
     for (lev = 0; lev < a.max_levels; ++lev) {
         const int64_t nq = (int64_t)(packed >> kQShift), vedges = (int64_t)(packed & kQEdges);
         if (nq == 0) { reason = R_DONE; break; }
@@ -433,7 +436,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_bfs_persistent(PersistAr
         }
         block_publish<kPersistWarps>(sh, acc.s_buf, acc.n, qb, RowLen{a.fw.deg}, &sl[S_Q], acc.pairs, acc.medges,
                                      &sl[S_PAIRS]);
-        if (!grid_barrier(bar, err, kBarrierSpins)) break;
+        if (!grid_barrier(bar, err, kBarrierSpins, met)) break;
         n_last = nq;
         packed = ldcg_u64(&sl[S_Q]);
         pr = ldcg_u64(&sl[S_PAIRS]);

@@ -92,6 +92,7 @@ struct ForestLevel {
         return __ldcg(parent + w) == -1 && scc[w] == (int32_t)(who >> 32);
     }
     __device__ __forceinline__ bool apply(int32_t w, unsigned long long who, unsigned long long, int32_t& e) {
+        touch_l1(sym.deg + w);  // (read at the level's end)
         e = w;
         return atomicCAS(&parent[w], -1, (int32_t)(uint32_t)who) == -1;
     }

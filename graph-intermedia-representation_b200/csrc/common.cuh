@@ -577,29 +577,36 @@ __device__ __forceinline__ void warp_append(bool pred, int32_t value, int32_t* q
 }
 
 // Grid-wide barrier of a cooperative launch: every CTA meets here. `bar` is one counter on its own
-// 128-byte line, zeroed by the host before the launch; arrivals only count up, so a CTA waits until
-// the counter reaches the end of its own round (one atomic and the polls, no reset and no second
-// word). The wait is bounded: after `spins_max` polls a CTA sets *err and leaves; every CTA also
-// leaves once it sees *err set. Returns false once any CTA has flagged an error.
-__device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned long long* err, unsigned spins_max) {
+// 128-byte line, zeroed by the host before the launch; arrivals only count up, so a CTA waits until the
+// counter reaches the end of its round (`round`: the barriers passed so far, the same in every CTA). One
+// release reduction without a result and acquire polls: no reset, no second word, no wait for the
+// atomic's return. The wait is bounded: after `spins_max` polls a CTA sets *err and leaves; every CTA
+// also leaves once it sees *err set. Returns false once any CTA has flagged an error.
+__device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned long long* err, unsigned spins_max,
+                                             unsigned& round) {
+    ++round;
     __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence();
-        const unsigned int mine = atomicAdd(bar, 1u);
-        const unsigned int end = mine - mine % gridDim.x + gridDim.x;
-        volatile unsigned int* now = bar;
-        unsigned int spins = 0;
-        while ((int)(*now - end) < 0) {
+        const unsigned int end = round * gridDim.x;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        unsigned int spins = 0, now;
+        while (true) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(bar) : "memory");
+            if ((int)(now - end) >= 0) break;
             if (++spins > spins_max) {
                 atomicExch(err, 1ull);
                 break;
             }
             if ((spins & 63) == 0 && __ldcg(err) != 0ull) break;
         }
-        __threadfence();
     }
     __syncthreads();
     return __ldcg(err) == 0ull;
+}
+
+// Starts a load into the L1 without waiting for it.
+__device__ __forceinline__ void touch_l1(const int32_t* p) {
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
 // Staged queue appends: a warp collects its entries in a shared-memory buffer of kStage slots

@@ -147,6 +147,20 @@ __device__ __forceinline__ int64_t queue_find(const uint64_t* off, int64_t lo, i
     }
     return lo;
 }
+// The same over the whole queue of n entries and `total` row positions, from a first look at the 32
+// entries about where the key would be if all rows were alike: one round instead of three where they
+// nearly are (a road network).
+__device__ __forceinline__ int64_t queue_guess(const uint64_t* off, int64_t n, int64_t total, int64_t key) {
+    int64_t at = (int64_t)((float)key / (float)total * (float)n) - 16;
+    at = at + 32 > n ? n - 32 : at;
+    at = at < 0 ? 0 : at;
+    const int64_t i = at + lane_id();
+    const unsigned m =
+        __ballot_sync(0xffffffffu, i < n && (int64_t)__ldcg((const unsigned long long*)off + i) <= key);
+    if (m == 0) return queue_find(off, 0, at, (uint64_t)key);
+    if (m == 0xffffffffu && at + 32 < n) return queue_find(off, at + 31, n, (uint64_t)key);
+    return at + __popc(m) - 1;
+}
 
 // Visits the row positions [c0, c1) of the frontier (as the queue's offsets count them), by one warp;
 // i0 is the largest entry whose offset is at most c0, and c1 - c0 is below 2^31. A warp holds 32 queue
@@ -221,7 +235,7 @@ __device__ __forceinline__ void walk_level(const Queue& q, int64_t nq, int64_t t
     run = run < kRun ? run : kRun;
     for (int64_t c0 = warp * run; c0 < total; c0 += nwarps * run) {
         const int64_t c1 = c0 + run < total ? c0 + run : total;
-        walk_rows(q, nq, total, c0, c1, queue_find(q.off, 0, nq, (uint64_t)c0), op, out, cnt, s_buf, s_n);
+        walk_rows(q, nq, total, c0, c1, queue_guess(q.off, nq, total, c0), op, out, cnt, s_buf, s_n);
     }
 }
 
@@ -252,6 +266,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_frontier_loop(Op op, Queue 
     unsigned long long packed = __ldcg(ctl + W_Q);
     int64_t lo = (int64_t)__ldcg(ctl + W_LO);
     int lev = 0;
+    unsigned met = 0;
     if (blockIdx.x == 0 && threadIdx.x == 0) ctl[W_LVL] = packed;
     for (; lev < max_levels; ++lev) {
         const int64_t nq = (int64_t)(packed >> kQShift), total = (int64_t)(packed & kQEdges);
@@ -262,7 +277,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_frontier_loop(Op op, Queue 
         int n_st = 0;
         walk_level(in, nq, total, warp, nwarps, op, out, sl, s_stage[wib], n_st);
         block_publish<32>(sh, s_stage[wib], n_st, out, [&](int32_t x) { return op.deg(x); }, sl);
-        if (!grid_barrier(bar, ctl + W_ERR, kLoopSpins)) break;
+        if (!grid_barrier(bar, ctl + W_ERR, kLoopSpins, met)) break;
         lo += nq;
         packed = __ldcg(sl);
         if (blockIdx.x == 0 && threadIdx.x == 0) ctl[W_LVL + 1 + lev] = packed;

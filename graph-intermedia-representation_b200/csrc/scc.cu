@@ -183,6 +183,7 @@ struct ReachBoth {
         return __ldcg(mark + w) & bit ? 0ull : bit;
     }
     __device__ __forceinline__ bool apply(int32_t w, unsigned long long back, unsigned long long bit, int32_t& e) {
+        touch_l1((back ? bw.deg : fw.deg) + w);  // (read at the level's end)
         e = back ? ~w : w;
         return (atomicOr(&mark[w], (int)bit) & (int)bit) == 0;
     }
@@ -396,6 +397,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_dag_levels(const uint64_t* 
     unsigned long long raised = 0;
     int32_t top = 0;
     int round = 0;
+    unsigned met = 0;
     while (round < max_rounds) {
         if (blockIdx.x == 0 && threadIdx.x == 0) ctl[(round + 1) % 3] = 0;
         unsigned long long c = 0;
@@ -410,7 +412,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_dag_levels(const uint64_t* 
         }
         c = warp_sum_u64(c);
         if (lane_id() == 0 && c) atomicAdd(&ctl[round % 3], c);
-        if (!grid_barrier(bar, ctl + 3, kLoopSpins)) return;
+        if (!grid_barrier(bar, ctl + 3, kLoopSpins, met)) return;
         raised = __ldcg(ctl + round % 3);
         ++round;
         if (raised == 0) break;

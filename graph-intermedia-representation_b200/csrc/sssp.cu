@@ -410,6 +410,7 @@ __device__ __forceinline__ void relax_edges(const Group& a, uint64_t kend, int32
     }
     if (!__any_sync(0xffffffffu, (near | far) != 0ull)) return;
     if (!kHeavy) {
+        if (kCg && near) touch_l1(reinterpret_cast<const int32_t*>(a.rows + w) + 3);  // (read at the queue write)
         const bool to_near = near != 0ull && atomicOr(&next[w], near) == 0ull;
         queue_push<kSlots>(to_near, w, st.near, st.n_near, outq, LightLen{a.rows}, near_cnt);
     }
@@ -436,7 +437,7 @@ __device__ __forceinline__ void relax_rows(const Group& a, const Bucket& b, cons
     run = run < kRun ? run : kRun;
     for (int64_t c0 = warp * run; c0 < total; c0 += nwarps * run) {
         const int64_t c1 = c0 + run < total ? c0 + run : total;
-        int64_t i0 = queue_find(q.off, 0, nq, (uint64_t)c0);
+        int64_t i0 = kCg ? queue_guess(q.off, nq, total, c0) : queue_find(q.off, 0, nq, (uint64_t)c0);
         int64_t p = c0;
         while (p < c1) {
             // 32 queue entries, one per thread: where its edges start in the run, its row, its lanes
@@ -470,7 +471,8 @@ __device__ __forceinline__ void relax_rows(const Group& a, const Bucket& b, cons
                 if (pos < wend) {
                     w = __ldcs(a.wadj + bx + rel);
                     wt = __ldcs(a.ww + bx + rel);
-                    if (a.nl > 1) need &= ~__ldcg(a.done + w);
+                    // (in the loop a single lane is not worth a load that stands before its distance's own)
+                    if (a.nl > 1 && (!kCg || (need & (need - 1)))) need &= ~__ldcg(a.done + w);
                 } else {
                     need = 0;
                 }
@@ -498,7 +500,16 @@ __device__ __forceinline__ void phase_light(const Group& a, const Bucket& b, uns
     const int old = (b.rot + 2) % 3;
     if (tid == 0) a.ctl[X_NEAR + old] = 0ull;
     for (int64_t i = tid; i < b.n_clear; i += nthreads) a.mask[old][__ldcg(a.q[old].v + i)] = 0ull;
-    for (int64_t base = tid & ~(int64_t)31; base < nq; base += nthreads) {
+    // A short pass is a chain of dependent accesses: the second half of every CTA's warps settles while the
+    // first half relaxes; in a long one every warp does both.
+    const bool halves = kCg && (int64_t)(packed & kQEdges) <= nwarps * 16 && nq <= nthreads / 2;
+    const int64_t half = nwarps / 2;
+    if (halves && warp < half) {
+        relax_rows<D, kCg, false, kSlots>(a, b, q, mask, packed, warp, half, st);
+        return;
+    }
+    const int64_t first = halves ? (tid & ~(int64_t)31) - half * 32 : tid & ~(int64_t)31;
+    for (int64_t base = first; base < nq; base += halves ? nthreads - half * 32 : nthreads) {
         const int64_t i = base + lane_id();
         int32_t u = 0;
         bool settles = false;
@@ -510,7 +521,7 @@ __device__ __forceinline__ void phase_light(const Group& a, const Bucket& b, uns
         }
         queue_push<kSlots>(settles, u, st.set, st.n_set, a.setq, HeavyLen{a.rows}, a.ctl + X_SET);
     }
-    relax_rows<D, kCg, false, kSlots>(a, b, q, mask, packed, warp, nwarps, st);
+    if (!halves) relax_rows<D, kCg, false, kSlots>(a, b, q, mask, packed, warp, nwarps, st);
 }
 
 // The heavy pass of a bucket: its settled lanes are final and relax their heavy edges once, into later
@@ -635,8 +646,12 @@ __global__ void __launch_bounds__(kPassThreads, 6) k_relax(Group a, Bucket b) {
 // while the phases are small: on a road network, or for a single source, a pass has a few thousand
 // edges and was four launches and a host read. It hands back when a pass has more than max_edges edges
 // or the far queue more than max_far entries; the host launches such a phase at full occupancy and
-// comes back. Bound by latency, about 17 us a pass: 16 sources on a 901 x 901 lattice (1,600 passes)
-// 71 -> 25 ms, one source on 65,536 vertices 4.4 -> 1.5 ms.
+// comes back. Bound by latency, about 12 us a pass (a chain of dependent L2 accesses and the barrier): 16
+// sources on a 901 x 901 lattice (1,600 passes) 71 -> 18.7 ms, one source on 65,536 vertices 4.4 -> 1.3 ms.
+// Of that the first look by interpolation, prefetched row lengths, settling and relaxing on different
+// warps, no `done` load for a single lane and the barrier's one-way arrival gave 23.5 -> 18.7 ms; in the
+// host-launched phases, which have warps enough to hide the chain, the same cost 21.4 -> 23.2 ms a call of
+// 64 sources on the 4.8M-vertex R-MAT (more loads, more targets read), so they are for the loop alone.
 constexpr int kLoopSlots = 64;
 constexpr int kMaxPhases = 1 << 23;  // of one launch (its barrier's counter is 32 bits wide)
 
@@ -655,6 +670,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_bucket_loop(Group a, int64_
     auto rd = [&](int i) { return __ldcg(a.ctl + i); };
     Bucket b{(int)rd(X_PHASE), (int)rd(X_ROT), (int)rd(X_SPL), (int)rd(X_FQ), rd(X_LO), (int64_t)rd(X_NCLEAR),
              (int64_t)rd(X_NSETCLEAR), (int64_t)rd(X_PASSES)};
+    unsigned met = 0;
     for (int ph = 0; ph < kMaxPhases && b.phase != PH_DONE; ++ph) {
         Stage st{s_near[wib], s_set[wib], s_far[wib], s_map[wib], 0, 0, 0};
         const int nx = (b.rot + 1) % 3;
@@ -707,7 +723,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_bucket_loop(Group a, int64_
             queue_write(st.set, st.n_set, a.setq, HeavyLen{a.rows}, (s_base[1] >> kQShift) + s_n[1][wib],
                         (s_base[1] & kQEdges) + s_e[1][wib]);
         for (int i = ln; i < st.n_far; i += 32) a.farq[fq][s_base[2] + s_n[2][wib] + i] = st.far[i];
-        if (!grid_barrier(bar, a.ctl + X_ERR, kLoopSpins)) return;
+        if (!grid_barrier(bar, a.ctl + X_ERR, kLoopSpins, met)) return;
         next_phase(b, a.delta, entries, rd);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
