@@ -3,6 +3,8 @@
 // templates from the CUDA toolkit, instantiated here for sm_100a); the traversal kernels of
 // the hot path are this library's own.
 #include <cub/cub.cuh>
+#include <thrust/iterator/zip_iterator.h>
+#include <thrust/tuple.h>
 
 #include "common.cuh"
 
@@ -115,15 +117,22 @@ int stage_input(gir_dev* g, DevBuf& stage, const void* p, size_t bytes, const vo
     return GIR_OK;
 }
 
-int sort_keys_u64(gir_dev* g, uint64_t* keys, uint64_t* tmp, int64_t n, int end_bit) {
+int sort_keys_u64_swap(gir_dev* g, uint64_t*& keys, uint64_t*& tmp, int64_t n, int end_bit) {
     if (n <= 1) return GIR_OK;
     cub::DoubleBuffer<uint64_t> kb(keys, tmp);
     size_t bytes = 0;
     GIR_CUDA(g, cub::DeviceRadixSort::SortKeys(nullptr, bytes, kb, n, 0, end_bit, g->stream));
     GIR_TRY(ensure(g, g->cub_tmp, bytes));
     GIR_CUDA(g, cub::DeviceRadixSort::SortKeys(g->cub_tmp.p, bytes, kb, n, 0, end_bit, g->stream));
-    if (kb.Current() != keys)
-        GIR_CUDA(g, cudaMemcpyAsync(keys, kb.Current(), sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, g->stream));
+    keys = kb.Current();
+    tmp = kb.Alternate();
+    return GIR_OK;
+}
+
+int sort_keys_u64(gir_dev* g, uint64_t* keys, uint64_t* tmp, int64_t n, int end_bit) {
+    uint64_t *a = keys, *b = tmp;
+    GIR_TRY(sort_keys_u64_swap(g, a, b, n, end_bit));
+    if (a != keys) GIR_CUDA(g, cudaMemcpyAsync(keys, a, sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, g->stream));
     return GIR_OK;
 }
 
@@ -166,6 +175,26 @@ int exclusive_scan_i64(gir_dev* g, const int64_t* in, int64_t* out, int64_t n) {
     GIR_CUDA(g, cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, n, g->stream));
     GIR_TRY(ensure(g, g->cub_tmp, bytes));
     GIR_CUDA(g, cub::DeviceScan::ExclusiveSum(g->cub_tmp.p, bytes, in, out, n, g->stream));
+    return GIR_OK;
+}
+
+namespace {
+struct AddBoth {
+    __host__ __device__ thrust::tuple<int64_t, int64_t> operator()(const thrust::tuple<int64_t, int64_t>& x,
+                                                                   const thrust::tuple<int64_t, int64_t>& y) const {
+        return thrust::make_tuple(thrust::get<0>(x) + thrust::get<0>(y), thrust::get<1>(x) + thrust::get<1>(y));
+    }
+};
+}  // namespace
+
+int exclusive_scan_two_i64(gir_dev* g, int64_t* a, int64_t* b, int64_t n) {
+    if (n <= 0) return GIR_OK;
+    size_t bytes = 0;
+    const auto it = thrust::make_zip_iterator(thrust::make_tuple(a, b));
+    const thrust::tuple<int64_t, int64_t> zero(0, 0);
+    GIR_CUDA(g, cub::DeviceScan::ExclusiveScan(nullptr, bytes, it, it, AddBoth{}, zero, n, g->stream));
+    GIR_TRY(ensure(g, g->cub_tmp, bytes));
+    GIR_CUDA(g, cub::DeviceScan::ExclusiveScan(g->cub_tmp.p, bytes, it, it, AddBoth{}, zero, n, g->stream));
     return GIR_OK;
 }
 

@@ -118,26 +118,32 @@ struct Touched {
     int32_t row, deg, keep, newdeg;
 };
 
-// Per touched row (from the merged op list `rows`, sorted distinct); elen / nlen = entries of its rest
-// before (old ones and inserts) and after the merge.
-// n_rows is a device word; the slots beyond it, up to n_ops, become empty rows.
-__global__ void k_touched_rows(const uint64_t* ins, int64_t n_ins, const uint64_t* del, int64_t n_del,
-                               const int32_t* rows, const int64_t* n_rows, CSRView c, Touched* touched, int64_t* elen,
-                               int64_t* nlen, int32_t* overflow, int32_t* bad) {
-    const int64_t n_ops = n_ins + n_del, n = *n_rows;
+// A slot per op, inserts first: the first insert of a row, or where it has none its first deletion, holds
+// the row, the row's other ops hold an empty one (in the place of flags over all rows, a compaction of them
+// and its scratch: four launches of ten a merge). elen / nlen = entries of a row's rest before (old ones and
+// inserts) and after the merge.
+__global__ void k_touched_rows(const uint64_t* ins, int64_t n_ins, const uint64_t* del, int64_t n_del, CSRView c,
+                               Touched* touched, int64_t* elen, int64_t* nlen, int32_t* overflow, int32_t* bad) {
+    const int64_t n_ops = n_ins + n_del;
     GRID_STRIDE(k, n_ops) {
+        const bool is_ins = k < n_ins;
+        const int64_t kd = k - n_ins;
+        const uint64_t r = (is_ins ? ins[k] : del[kd]) >> 32;
+        bool head = is_ins ? k == 0 || ins[k - 1] >> 32 != r : kd == 0 || del[kd - 1] >> 32 != r;
         Touched t;
-        if (k >= n) {
-            t.row = -1;
+        t.row = -1;
+        if (head) {
+            t.ib = is_ins ? k : lower_bound_dev(ins, (int64_t)0, n_ins, r << 32);
+            head = is_ins || t.ib == n_ins || ins[t.ib] >> 32 != r;
+        }
+        if (!head) {
             touched[k] = t;
             elen[k] = nlen[k] = 0;
             continue;
         }
-        t.row = rows[k];
-        const uint64_t r = (uint64_t)(uint32_t)t.row;
-        t.ib = lower_bound_dev(ins, (int64_t)0, n_ins, r << 32);
-        t.ie = lower_bound_dev(ins, t.ib, n_ins, (r + 1) << 32);
-        t.db = lower_bound_dev(del, (int64_t)0, n_del, r << 32);
+        t.row = (int32_t)r;
+        t.ie = is_ins ? lower_bound_dev(ins, k + 1, n_ins, (r + 1) << 32) : t.ib;
+        t.db = is_ins ? lower_bound_dev(del, (int64_t)0, n_del, r << 32) : kd;
         t.de = lower_bound_dev(del, t.db, n_del, (r + 1) << 32);
         t.beg = c.beg[r];
         t.deg = c.deg[r];
@@ -196,12 +202,13 @@ __global__ void k_merge_rows(const uint64_t* ins, const uint64_t* del, const Tou
 }
 
 // The sizes the host needs, in one place to read: entries to merge, entries merged, a row outgrew its
-// slack, the batch's bad flag.
-__global__ void k_merge_sizes(const int64_t* eoff, const int64_t* noff, int64_t n, const int32_t* overflow,
+// slack (the flag is cleared for the next merge), the batch's bad flag.
+__global__ void k_merge_sizes(const int64_t* eoff, const int64_t* noff, int64_t n, int32_t* overflow,
                               const int32_t* bad, int64_t* out) {
     out[0] = eoff[n];
     out[1] = noff[n];
     out[2] = *overflow;
+    *overflow = 0;
     out[3] = *bad;
 }
 
@@ -219,10 +226,6 @@ __global__ void k_copy_back(const Touched* touched, int64_t n_rows, const int64_
 
 __global__ void k_set_deg(const Touched* touched, int64_t n_rows, int32_t* deg) {
     GRID_STRIDE(k, n_rows) if (touched[k].row >= 0) deg[touched[k].row] = touched[k].newdeg;
-}
-
-__global__ void k_mark_rows(const uint64_t* a, int64_t na, const uint64_t* b, int64_t nb, uint8_t* flag) {
-    GRID_STRIDE(i, na + nb) flag[(i < na ? a[i] : b[i - na]) >> 32] = 1;
 }
 
 // Full re-layout: new capacities from new lengths, then every row copied (the merged rests of touched rows from tmp).
@@ -514,43 +517,28 @@ int store_ops_bad(gir_dev* g) {
 }
 
 int store_apply_ops(gir_dev* g, DevCSR& c, const uint64_t* ins, int64_t n_ins, const uint64_t* del, int64_t n_del,
-                    bool weights, int32_t* bad) {
+                    bool weights, int32_t* bad, int32_t* overflow) {
     if (n_ins + n_del == 0) return GIR_OK;
     const int64_t V = g->V;
-    const int64_t n_ops = n_ins + n_del;
-    int32_t *rows = nullptr, *tmp = nullptr;
-    uint8_t* flag = nullptr;
-    int64_t *eoff = nullptr, *noff = nullptr;
+    const int64_t n_rows = n_ins + n_del;  // slots, one per op
+    int32_t* tmp = nullptr;
+    int64_t *eoff = nullptr, *noff = nullptr, *words = nullptr;  // (words: the sizes the host reads)
     Touched* touched = nullptr;
     uint32_t* tmpw = nullptr;
-    GIR_TRY(ensure_n(g, g->scratch[4], V + 1, &flag));
-    GIR_TRY(ensure_n(g, g->scratch[5], V + 1, &rows));
-    // rows touched by any op, ascending and distinct
-    GIR_CUDA(g, cudaMemsetAsync(flag, 0, V, g->stream));
-    k_mark_rows<<<grid_for(g, n_ops, kBlock), kBlock, 0, g->stream>>>(ins, n_ins, del, n_del, flag);
-    GIR_LAUNCH(g, "k_mark_rows");
-    // (their number stays on the device: at most one per op)
-    const int64_t n_rows = n_ops;
-    int32_t* overflow = nullptr;
-    int64_t* words = nullptr;  // number of rows, then the sizes the host reads
     GIR_TRY(ensure_n(g, g->scratch[9], n_rows + 1, &touched));
     GIR_TRY(ensure_n(g, g->scratch[10], n_rows + 1, &eoff));
     GIR_TRY(ensure_n(g, g->scratch[11], n_rows + 1, &noff));
-    GIR_TRY(ensure_n(g, g->scratch[12], 8, &words));
-    overflow = reinterpret_cast<int32_t*>(words + 6);
-    GIR_TRY(select_flagged_iota_to(g, flag, rows, V, words));
-    GIR_CUDA(g, cudaMemsetAsync(overflow, 0, sizeof(int32_t), g->stream));
-    k_touched_rows<<<grid_for(g, n_rows, kBlock), kBlock, 0, g->stream>>>(ins, n_ins, del, n_del, rows, words, view(c),
-                                                                           touched, eoff, noff, overflow, bad);
+    GIR_TRY(ensure_n(g, g->scratch[12], 4, &words));
+    k_touched_rows<<<grid_for(g, n_rows, kBlock), kBlock, 0, g->stream>>>(ins, n_ins, del, n_del, view(c), touched, eoff,
+                                                                           noff, overflow, bad);
     GIR_LAUNCH(g, "k_touched_rows");
-    GIR_TRY(exclusive_scan_i64(g, eoff, eoff, n_rows + 1));
-    GIR_TRY(exclusive_scan_i64(g, noff, noff, n_rows + 1));
-    k_merge_sizes<<<1, 1, 0, g->stream>>>(eoff, noff, n_rows, overflow, bad, words + 1);
+    GIR_TRY(exclusive_scan_two_i64(g, eoff, noff, n_rows + 1));
+    k_merge_sizes<<<1, 1, 0, g->stream>>>(eoff, noff, n_rows, overflow, bad, words);
     GIR_LAUNCH(g, "k_merge_sizes");
     void* hp = nullptr;
     GIR_TRY(pinned(g, kPinnedBytes, &hp));
     int64_t* h = static_cast<int64_t*>(hp);
-    GIR_CUDA(g, cudaMemcpyAsync(h, words + 1, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, g->stream));
+    GIR_CUDA(g, cudaMemcpyAsync(h, words, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, g->stream));
     GIR_CUDA(g, cudaStreamSynchronize(g->stream));
     const int64_t n_elems = h[0], n_new = h[1];
     const bool ovf = h[2] != 0;

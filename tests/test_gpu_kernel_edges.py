@@ -196,3 +196,78 @@ def test_sssp_phases_inside_and_outside_the_bucket_loop(pkg, orc):
         one = d.sssp(src[:1], delta=7 * scale, weights=pkg.native.WEIGHT_STORED)
         np.testing.assert_array_equal(one[0], got[0])
         d.close()
+
+
+@pytest.mark.parametrize("lanes", [7, 8, 9, 64])
+def test_bfs_levels_kept_in_bit_planes(pkg, orc, lanes):
+    """Eight lanes or more over at least 2^23 (lane, vertex) pairs: levels below 15 go through bit planes,
+    the deeper ones of a tail straight to the output, unreached vertices and lanes without a source are -1."""
+    V = (1 << 20) + 77
+    rng = np.random.default_rng(lanes)
+    u, v = rng.integers(0, V - 200, 3 * V), rng.integers(0, V - 200, 3 * V)
+    tail = np.arange(V - 150, V)  # 50 vertices before it have no edge
+    u, v = np.r_[u, 5, tail[:-1]], np.r_[v, tail[0], tail[1:]]
+    g = _graph(pkg, V, u[u != v], v[u != v])
+    fb, fa = orc.normalize(V, g.fw_beg, g.fw_adj)
+    d = pkg.DeviceGraph.from_graph(g, weights=False)
+    src = rng.integers(0, V - 200, lanes).astype(np.int32)
+    src[1], src[2], src[3], src[-1] = V - 1, -1, V - 180, tail[0]
+    got = d.bfs(src)
+    for row, s in zip(got, src):
+        np.testing.assert_array_equal(row, orc.bfs(V, fb, fa, [int(s)]) if s >= 0 else np.full(V, -1))
+    d.close()
+
+
+def test_builds_with_levels_taken_bottom_up(pkg, orc):
+    """Levels of more than 2^22 row entries and a class that holds nearly every row: the rows of the giant
+    component, SCC and block are left out of the passes that look for the others."""
+    from test_gpu_layers import _oracle_match
+    core, V = 300_000, 360_000
+    rng = np.random.default_rng(3)
+    u, v = rng.integers(0, core, 20 * core), rng.integers(0, core, 20 * core)
+    w = np.arange(core, core + 30_000)  # hanging in or out by one edge, or by a small ring
+    x = np.arange(core + 30_000, V, 3)
+    u = np.r_[u, w[::2], rng.integers(0, core, 15_000), x, x + 1, x + 2, x[::2], rng.integers(0, core, 2_500)]
+    v = np.r_[v, rng.integers(0, core, 15_000), w[1::2], x + 1, x + 2, x, rng.integers(0, core, 5_000), x[1::4]]
+    g = _graph(pkg, V, u[u != v], v[u != v])
+    fb, fa = orc.normalize(V, g.fw_beg, g.fw_adj)
+    d = pkg.DeviceGraph.from_graph(g, weights=False)
+    d.build()
+    _oracle_match(pkg, orc, d, V, fb, fa, "bottom-up levels")
+    d.close()
+
+
+@pytest.mark.parametrize("V,n", [(2, 2), (40, 2), (40, 33), (40, 600), (700, 1), (700, 4096), (3000, 20_000)])
+def test_batches_that_change_both_directions_of_pairs(pkg, orc, V, n):
+    """Every way a batch can change a pair (one edge, both alike, one each way, one of two), several ops of
+    a key, rows with both inserts and deletions, rows with more ops than a warp, rows that outgrow their
+    slack: the three CSRs and the layers, with and without anything to insert or to delete."""
+    from test_gpu_layers import _oracle_match
+    rng = np.random.default_rng(V + n)
+    u, v = rng.integers(0, V, 4 * V), rng.integers(0, V, 4 * V)
+    u, v = np.r_[u, v[::3], 0], np.r_[v, u[::3], 1]
+    g = _graph(pkg, V, u[u != v], v[u != v])
+    fb, fa = orc.normalize(V, g.fw_beg, g.fw_adj)
+    d = pkg.DeviceGraph.from_graph(g)
+    d.build()
+    for step in range(4):
+        a, b = rng.integers(0, V, n), rng.integers(0, V, n)
+        a[: n // 4] = rng.integers(0, 1 + V // 20)  # one hub
+        rows, at = np.repeat(np.arange(V), np.diff(fb)), rng.integers(0, max(len(fa), 1), n)
+        if len(fa):
+            a[::3], b[::3] = rows[at[::3]], fa[at[::3]]
+        k = np.arange(n) % 5 == 1
+        a[k], b[k] = np.roll(b, 1)[k], np.roll(a, 1)[k]
+        a, b = a.astype(np.int32), b.astype(np.int32)
+        ins = (rng.random(n) < (0.5, 0.0, 1.0, 0.3)[step]).astype(np.uint8)
+        d.apply_batch(a, b, ins)
+        fb, fa, n_ins, n_del = orc.apply_batch(V, fb, fa, a, b, ins)
+        st = d.batch_stats()
+        assert (st["inserted"], st["deleted"]) == (n_ins, n_del)
+        tb, ta = orc.transpose(V, fb, fa)
+        for which, (eb, ea) in enumerate(((fb, fa), (tb, ta), orc.sym(V, fb, fa, tb, ta))):
+            gb, ga = d.csr(which)
+            np.testing.assert_array_equal(gb, eb)
+            np.testing.assert_array_equal(ga, ea)
+        _oracle_match(pkg, orc, d, V, fb, fa, f"step {step}")
+    d.close()
