@@ -759,40 +759,43 @@ __global__ void k_sssp_reached(const D* dist, int64_t V, int nl, const int32_t* 
     }
 }
 
-// dist[v * ld + s] -> out[row[s] * V + v], through 32 x 32 shared-memory tiles, a fixed grid
-// striding over the tiles. On the way it counts what k_sssp_reached counts (reached (vertex, lane)
-// pairs and their out-edges) from the same coalesced loads, with one atomicAdd per CTA.
+// dist[v * ld + s] -> out[row[s] * V + v], through 32 x 32 shared-memory tiles, a warp and a tile of its
+// own at a time (no CTA barrier), all 32 row loads in flight. On the way it counts what k_sssp_reached
+// counts (reached (vertex, lane) pairs and their out-edges), with one atomicAdd per CTA. Bound by DRAM: 64
+// lanes of 32 bits on 4.8M vertices move 3.7 GB; a CTA a tile with eight loads in two barriers, and the
+// out-degree loaded for every pair instead of once a tile and vertex, took 1.14 ms, this 0.76 (4.9 TB/s).
+constexpr int kTransposeWarps = 4;  // (the tiles of 64-bit distances fit the 48 KB of static shared memory)
 template <class D>
-__global__ void k_transpose(const D* dist, int64_t V, int nl, int ld, const int64_t* row, const int32_t* outdeg,
-                            uint64_t* out, unsigned long long* cnt) {
-    __shared__ uint64_t tile[32][33];
-    __shared__ unsigned long long s_r[8], s_e[8];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8 threads
+__global__ void __launch_bounds__(kTransposeWarps * 32) k_transpose(const D* dist, int64_t V, int nl, int ld,
+                                                                    const int64_t* row, const int32_t* outdeg,
+                                                                    uint64_t* out, unsigned long long* cnt) {
+    __shared__ D tiles[kTransposeWarps][32][33];
+    __shared__ unsigned long long s_r[kTransposeWarps], s_e[kTransposeWarps];
+    const int tx = lane_id(), ty = threadIdx.x >> 5;
+    D(*tile)[33] = tiles[ty];
     const int64_t tiles_v = (V + 31) / 32, tiles_s = (nl + 31) / 32;
     unsigned long long r_cnt = 0, e_cnt = 0;
-    for (int64_t t = blockIdx.x; t < tiles_v * tiles_s; t += gridDim.x) {
-        const int64_t v0 = (t % tiles_v) * 32;
-        const int s0 = (int)(t / tiles_v) * 32;
-        for (int r = ty; r < 32; r += 8) {
-            const int64_t v = v0 + r;
-            const int s = s0 + tx;
-            if (v < V && s < nl) {
-                const D d = dist[v * ld + s];
+    for (int64_t t = blockIdx.x * (int64_t)kTransposeWarps + ty; t < tiles_v * tiles_s;
+         t += (int64_t)gridDim.x * kTransposeWarps) {
+        const int64_t v0 = (t % tiles_v) * 32, v = v0 + tx;
+        const int s0 = (int)(t / tiles_v) * 32, s = s0 + tx;
+        const int nv = V - v0 < 32 ? (int)(V - v0) : 32, ns = nl - s0 < 32 ? nl - s0 : 32;
+        const unsigned deg = tx < nv ? (unsigned)outdeg[v] : 0u;
+#pragma unroll
+        for (int r = 0; r < 32; ++r)
+            if (r < nv && tx < ns) tile[r][tx] = __ldcs(dist + (v0 + r) * ld + s);
+        __syncwarp();
+        unsigned reached = 0;
+        if (tx < nv)
+            for (int r = 0; r < ns; ++r) {
+                const D d = tile[tx][r];
                 const bool fin = d != DistT<D>::inf;
-                tile[r][tx] = fin ? (uint64_t)d : kInf;
-                if (fin) {
-                    ++r_cnt;
-                    e_cnt += (unsigned long long)outdeg[v];
-                }
+                reached += fin;
+                __stcs(out + row[s0 + r] * V + v, fin ? (uint64_t)d : kInf);
             }
-        }
-        __syncthreads();
-        for (int r = ty; r < 32; r += 8) {
-            const int s = s0 + r;
-            const int64_t v = v0 + tx;
-            if (v < V && s < nl) out[row[s] * V + v] = tile[tx][r];
-        }
-        __syncthreads();
+        r_cnt += reached;
+        e_cnt += (unsigned long long)reached * deg;
+        __syncwarp();
     }
     for (int o = 16; o; o >>= 1) {
         r_cnt += __shfl_xor_sync(0xffffffffu, r_cnt, o);
@@ -805,7 +808,7 @@ __global__ void k_transpose(const D* dist, int64_t V, int nl, int ld, const int6
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned long long rr = 0, ee = 0;
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < kTransposeWarps; ++k) {
             rr += s_r[k];
             ee += s_e[k];
         }
@@ -1072,7 +1075,7 @@ int sssp_group(gir_dev* g, Work& wk, const DevCSR& ws, int nl, const int64_t* la
         return GIR_OK;
     }
     if (!direct) {  // (the transpose also counts the reached pairs and their edges)
-        k_transpose<D><<<g->num_sms * 8, 256, 0, g->stream>>>(dist, V, nl, ld, lane_row_d, g->fw.deg, out, ctl);
+        k_transpose<D><<<g->num_sms * 12, kTransposeWarps * 32, 0, g->stream>>>(dist, V, nl, ld, lane_row_d, g->fw.deg, out, ctl);
         GIR_LAUNCH(g, "k_transpose");
     } else {
         k_sssp_reached<D><<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(dist, V, nl, g->fw.deg, ctl);
