@@ -585,7 +585,11 @@ int bfs_run(gir_dev* g, const int64_t* set_beg_h, const int32_t* srcs_d, int64_t
         GIR_CUDA(g, cudaMemcpyAsync(sbeg, set_beg_h + g0, sizeof(int64_t) * (nl + 1), cudaMemcpyHostToDevice, g->stream));
         const int64_t n_entries = set_beg_h[g0 + nl] - set_beg_h[g0];
         if (n_entries > 0 && nl >= kPlaneMinLanes && (int64_t)nl * V >= kPlaneMinPairs) {
-            GIR_TRY(ensure_n(g, g->scratch[12], 4 * V, &level.plane));
+            const int rc = ensure_n(g, g->scratch[12], 4 * V, &level.plane);
+            if (rc == GIR_ERR_OOM) level.plane = nullptr;  // (the straight writes need no memory)
+            else GIR_TRY(rc);
+        }
+        if (level.plane) {
             GIR_CUDA(g, cudaMemsetAsync(level.plane, 0, sizeof(uint64_t) * 4 * V, g->stream));
         } else {
             GIR_CUDA(g, cudaMemsetAsync(level.out, 0xff, sizeof(int32_t) * V * nl, g->stream));

@@ -320,7 +320,6 @@ int sort_pairs_u64(gir_dev* g, uint64_t* keys, uint64_t* ktmp, uint32_t* vals, u
 int sort_pairs_u32(gir_dev* g, uint32_t* keys, uint32_t* ktmp, uint32_t* vals, uint32_t* vtmp, int64_t n, int end_bit);
 int sort_pairs_u64_i64(gir_dev* g, uint64_t* keys, uint64_t* ktmp, int64_t* vals, int64_t* vtmp, int64_t n, int end_bit);
 int exclusive_scan_i64(gir_dev* g, const int64_t* in, int64_t* out, int64_t n);
-int sum_i64(gir_dev* g, const int64_t* in, int64_t n, int64_t* host_out);
 // Compacts the entries of `in` whose flag is non-zero into `out`; *host_n = count.
 int select_flagged_u64(gir_dev* g, const uint64_t* in, const uint8_t* flags, uint64_t* out, int64_t n, int64_t* host_n);
 // The same with the count left on the device.
@@ -328,7 +327,6 @@ int select_flagged_u64_to(gir_dev* g, const uint64_t* in, const uint8_t* flags, 
 int select_flagged_i32(gir_dev* g, const int32_t* in, const uint8_t* flags, int32_t* out, int64_t n, int64_t* host_n);
 // Indices i in [0, n) with flags[i] != 0, ascending.
 int select_flagged_iota(gir_dev* g, const uint8_t* flags, int32_t* out, int64_t n, int64_t* host_n);
-int select_flagged_iota_to(gir_dev* g, const uint8_t* flags, int32_t* out, int64_t n, int64_t* d_n);
 // The rows of `deg` (V entries) longer than max_deg, ascending, into rows (V entries), and the
 // exclusive scan of their lengths into pref (V + 1 entries); *n = their number. flag: V bytes.
 int heavy_rows(gir_dev* g, const int32_t* deg, int64_t V, int32_t max_deg, uint8_t* flag, int32_t* rows, int64_t* pref,
@@ -567,17 +565,6 @@ __device__ __forceinline__ void walk_rows_of(const int64_t* off, int64_t V, cons
             p = wend;
         }
     }
-}
-
-// Warp-aggregated append: every lane with `pred` gets a distinct slot in `q` (counter `cnt`).
-__device__ __forceinline__ void warp_append(bool pred, int32_t value, int32_t* q, unsigned long long* cnt) {
-    const unsigned m = __ballot_sync(0xffffffffu, pred);
-    if (!m) return;
-    const int leader = __ffs(m) - 1;
-    unsigned long long base = 0;
-    if (lane_id() == leader) base = atomicAdd(cnt, (unsigned long long)__popc(m));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (pred) q[base + __popc(m & ((1u << lane_id()) - 1))] = value;
 }
 
 // Grid-wide barrier of a cooperative launch: every CTA meets here. `bar` is one counter on its own

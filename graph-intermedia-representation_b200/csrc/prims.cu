@@ -198,22 +198,6 @@ int exclusive_scan_two_i64(gir_dev* g, int64_t* a, int64_t* b, int64_t n) {
     return GIR_OK;
 }
 
-int sum_i64(gir_dev* g, const int64_t* in, int64_t n, int64_t* host_out) {
-    int64_t* d_out = nullptr;
-    GIR_TRY(ensure_n(g, g->scratch[15], 1, &d_out));
-    if (n <= 0) { *host_out = 0; return GIR_OK; }
-    size_t bytes = 0;
-    GIR_CUDA(g, cub::DeviceReduce::Sum(nullptr, bytes, in, d_out, n, g->stream));
-    GIR_TRY(ensure(g, g->cub_tmp, bytes));
-    GIR_CUDA(g, cub::DeviceReduce::Sum(g->cub_tmp.p, bytes, in, d_out, n, g->stream));
-    void* h = nullptr;
-    GIR_TRY(pinned(g, 64, &h));
-    GIR_CUDA(g, cudaMemcpyAsync(h, d_out, sizeof(int64_t), cudaMemcpyDeviceToHost, g->stream));
-    GIR_CUDA(g, cudaStreamSynchronize(g->stream));
-    *host_out = *static_cast<int64_t*>(h);
-    return GIR_OK;
-}
-
 // Compaction with the count left on the device (d_n).
 template <class It, class T>
 static int select_flagged_to(gir_dev* g, It in, const uint8_t* flags, T* out, int64_t n, int64_t* d_n) {
@@ -244,9 +228,6 @@ static int select_flagged(gir_dev* g, It in, const uint8_t* flags, T* out, int64
 
 int select_flagged_u64_to(gir_dev* g, const uint64_t* in, const uint8_t* flags, uint64_t* out, int64_t n, int64_t* d_n) {
     return select_flagged_to(g, in, flags, out, n, d_n);
-}
-int select_flagged_iota_to(gir_dev* g, const uint8_t* flags, int32_t* out, int64_t n, int64_t* d_n) {
-    return select_flagged_to(g, cub::CountingInputIterator<int32_t>(0), flags, out, n, d_n);
 }
 int select_flagged_u64(gir_dev* g, const uint64_t* in, const uint8_t* flags, uint64_t* out, int64_t n, int64_t* host_n) {
     return select_flagged(g, in, flags, out, n, host_n);
