@@ -285,9 +285,8 @@ int store_free(gir_dev* g, DevCSR& c);
 int store_build_sym(gir_dev* g);
 int store_compact_csr(gir_dev* g, const DevCSR& c, int64_t* beg_out, int32_t* adj_out, int64_t cap);
 int store_has_edges(gir_dev* g, const DevCSR& c, const int32_t* u, const int32_t* v, int64_t n, uint8_t* out);
-// `bad`: a device word, zero at the start of a batch; a merge whose ops do not fit its CSR sets it, changes
-// nothing and the caller finds out at its next read (or store_apply_ops itself at the next CSR's: then it
-// returns GIR_ERR_MALFORMED, as store_ops_bad does). `overflow`: a device word, zero before and after.
+// `bad`: a device word, zero at the start of a batch; ops that do not fit the CSR set it, change nothing and
+// give GIR_ERR_MALFORMED, as store_ops_bad does. `overflow`: a device word, zero before and after.
 int store_apply_ops(gir_dev* g, DevCSR& c, const uint64_t* ins, int64_t n_ins, const uint64_t* del, int64_t n_del,
                     bool weights, int32_t* bad, int32_t* overflow);
 int store_ops_bad(gir_dev* g);
@@ -314,8 +313,6 @@ int scan_degrees(gir_dev* g, const int32_t* deg, int64_t V, int64_t* off);
 int sort_keys_u64(gir_dev* g, uint64_t* keys, uint64_t* tmp, int64_t n, int end_bit);
 // The same without a copy where the sort ends in the other buffer: keys is the one with the result.
 int sort_keys_u64_swap(gir_dev* g, uint64_t*& keys, uint64_t*& tmp, int64_t n, int end_bit);
-// Exclusive scans of two arrays in one pass, in place.
-int exclusive_scan_two_i64(gir_dev* g, int64_t* a, int64_t* b, int64_t n);
 int sort_pairs_u64(gir_dev* g, uint64_t* keys, uint64_t* ktmp, uint32_t* vals, uint32_t* vtmp, int64_t n, int end_bit);
 int sort_pairs_u32(gir_dev* g, uint32_t* keys, uint32_t* ktmp, uint32_t* vals, uint32_t* vtmp, int64_t n, int end_bit);
 int sort_pairs_u64_i64(gir_dev* g, uint64_t* keys, uint64_t* ktmp, int64_t* vals, int64_t* vtmp, int64_t n, int end_bit);

@@ -3,8 +3,6 @@
 // templates from the CUDA toolkit, instantiated here for sm_100a); the traversal kernels of
 // the hot path are this library's own.
 #include <cub/cub.cuh>
-#include <thrust/iterator/zip_iterator.h>
-#include <thrust/tuple.h>
 
 #include "common.cuh"
 
@@ -175,26 +173,6 @@ int exclusive_scan_i64(gir_dev* g, const int64_t* in, int64_t* out, int64_t n) {
     GIR_CUDA(g, cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, n, g->stream));
     GIR_TRY(ensure(g, g->cub_tmp, bytes));
     GIR_CUDA(g, cub::DeviceScan::ExclusiveSum(g->cub_tmp.p, bytes, in, out, n, g->stream));
-    return GIR_OK;
-}
-
-namespace {
-struct AddBoth {
-    __host__ __device__ thrust::tuple<int64_t, int64_t> operator()(const thrust::tuple<int64_t, int64_t>& x,
-                                                                   const thrust::tuple<int64_t, int64_t>& y) const {
-        return thrust::make_tuple(thrust::get<0>(x) + thrust::get<0>(y), thrust::get<1>(x) + thrust::get<1>(y));
-    }
-};
-}  // namespace
-
-int exclusive_scan_two_i64(gir_dev* g, int64_t* a, int64_t* b, int64_t n) {
-    if (n <= 0) return GIR_OK;
-    size_t bytes = 0;
-    const auto it = thrust::make_zip_iterator(thrust::make_tuple(a, b));
-    const thrust::tuple<int64_t, int64_t> zero(0, 0);
-    GIR_CUDA(g, cub::DeviceScan::ExclusiveScan(nullptr, bytes, it, it, AddBoth{}, zero, n, g->stream));
-    GIR_TRY(ensure(g, g->cub_tmp, bytes));
-    GIR_CUDA(g, cub::DeviceScan::ExclusiveScan(g->cub_tmp.p, bytes, it, it, AddBoth{}, zero, n, g->stream));
     return GIR_OK;
 }
 

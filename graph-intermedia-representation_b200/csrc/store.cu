@@ -107,153 +107,125 @@ __global__ void k_has_edges(CSRView c, int64_t V, const int32_t* u, const int32_
 
 // ---- batched row updates -------------------------------------------------------------------
 // Ops are sorted, distinct keys (row << 32 | col): `ins` are absent edges to add, `del` present
-// edges to remove. For each touched row r: new length = deg - |del_r| + |ins_r|. The entries before
-// its first changed position stay where they are; the rest is merged into `tmp`. When every
-// touched row still fits its capacity the merged rests are copied back in place; otherwise the whole
-// CSR is re-laid-out with fresh slack.
+// edges to remove. Between two ops of a row its old entries keep their order and all move by the same
+// distance, so every op stands for a run: the entry it inserts, if it does, and the old entries after it as
+// far as the row's next op. The runs go through `tmp` and back to their new places; a row's entries before
+// its first op are not touched. When a row outgrows its capacity the whole CSR is re-laid-out with fresh
+// slack.
 
-// A touched row: its op ranges, its first changed position and its new length.
-struct Touched {
-    int64_t beg, ib, ie, db, de;
-    int32_t row, deg, keep, newdeg;
+// An op's run: `src` the first old entry of the run, `slot` where the run starts in the new row, `col` the
+// inserted column or -1, newdeg the row's new length in its first op and -1 in the others.
+struct OpRun {
+    int64_t src;
+    int32_t row, slot, col, newdeg;
 };
 
-// A slot per op, inserts first: the first insert of a row, or where it has none its first deletion, holds
-// the row, the row's other ops hold an empty one (in the place of flags over all rows, a compaction of them
-// and its scratch: four launches of ten a merge). elen / nlen = entries of a row's rest before (old ones and
-// inserts) and after the merge.
-__global__ void k_touched_rows(const uint64_t* ins, int64_t n_ins, const uint64_t* del, int64_t n_del, CSRView c,
-                               Touched* touched, int64_t* elen, int64_t* nlen, int32_t* overflow, int32_t* bad) {
+// len = entries of the op's run. Bound by its chains of binary searches: about ten dependent accesses for
+// each of the op's own place in the other list, in the row, and the next op's.
+__global__ void k_op_runs(const uint64_t* ins, int64_t n_ins, const uint64_t* del, int64_t n_del, CSRView c, OpRun* runs,
+                          int64_t* len, int32_t* overflow, int32_t* bad) {
     const int64_t n_ops = n_ins + n_del;
     GRID_STRIDE(k, n_ops) {
         const bool is_ins = k < n_ins;
-        const int64_t kd = k - n_ins;
-        const uint64_t r = (is_ins ? ins[k] : del[kd]) >> 32;
-        bool head = is_ins ? k == 0 || ins[k - 1] >> 32 != r : kd == 0 || del[kd - 1] >> 32 != r;
-        Touched t;
-        t.row = -1;
-        if (head) {
-            t.ib = is_ins ? k : lower_bound_dev(ins, (int64_t)0, n_ins, r << 32);
-            head = is_ins || t.ib == n_ins || ins[t.ib] >> 32 != r;
-        }
-        if (!head) {
-            touched[k] = t;
-            elen[k] = nlen[k] = 0;
-            continue;
-        }
+        const int64_t own = is_ins ? k : k - n_ins;
+        const uint64_t key = is_ins ? ins[own] : del[own];
+        const uint64_t r = key >> 32, row_key = r << 32;
+        const int32_t col = (int32_t)(key & 0xffffffffULL);
+        // the row's first ops, and this op's place in both lists
+        const int64_t ib = lower_bound_dev(ins, (int64_t)0, is_ins ? own : n_ins, row_key);
+        const int64_t db = lower_bound_dev(del, (int64_t)0, is_ins ? n_del : own, row_key);
+        const int64_t i = is_ins ? own : lower_bound_dev(ins, ib, n_ins, key);
+        const int64_t d = is_ins ? lower_bound_dev(del, db, n_del, key) : own;
+        const int64_t in = i + is_ins, dn = d + !is_ins;
+        uint64_t next = ~0ull;  // the row's next op
+        if (in < n_ins && ins[in] >> 32 == r) next = ins[in];
+        if (dn < n_del && del[dn] >> 32 == r && del[dn] < next) next = del[dn];
+        const int64_t beg = c.beg[r], end = beg + c.deg[r];
+        const int64_t p = lower_bound_dev(c.adj, beg, end, col);
+        const int64_t pn = next == ~0ull ? end : lower_bound_dev(c.adj, p, end, (int32_t)(next & 0xffffffffULL));
+        if (!is_ins && (p >= end || c.adj[p] != col)) atomicExch(bad, 1);  // the ops do not match this CSR
+        OpRun t;
+        t.src = p + !is_ins;
         t.row = (int32_t)r;
-        t.ie = is_ins ? lower_bound_dev(ins, k + 1, n_ins, (r + 1) << 32) : t.ib;
-        t.db = is_ins ? lower_bound_dev(del, (int64_t)0, n_del, r << 32) : kd;
-        t.de = lower_bound_dev(del, t.db, n_del, (r + 1) << 32);
-        t.beg = c.beg[r];
-        t.deg = c.deg[r];
-        const int64_t nd = (int64_t)t.deg - (t.de - t.db) + (t.ie - t.ib);
-        uint32_t first = 0xffffffffu;  // smallest column of an op
-        if (t.ib < t.ie) first = (uint32_t)ins[t.ib];
-        if (t.db < t.de && (uint32_t)del[t.db] < first) first = (uint32_t)del[t.db];
-        t.keep = (int32_t)(lower_bound_dev(c.adj, t.beg, t.beg + t.deg, (int32_t)first) - t.beg);
-        t.newdeg = (int32_t)nd;
-        if (nd < t.keep) {  // more deletions than entries: the ops do not match this CSR
-            atomicExch(bad, 1);
-            t.newdeg = t.keep;
+        t.slot = (int32_t)(p - beg - (d - db) + (i - ib));
+        t.col = is_ins ? col : -1;
+        t.newdeg = -1;
+        if (i == ib && d == db) {
+            const int64_t ie = lower_bound_dev(ins, in, n_ins, (r + 1) << 32);
+            const int64_t de = lower_bound_dev(del, dn, n_del, (r + 1) << 32);
+            const int64_t nd = end - beg - (de - db) + (ie - ib);
+            if (beg + nd > c.beg[r + 1]) atomicExch(overflow, 1);
+            t.newdeg = nd > 0 ? (int32_t)nd : 0;
         }
-        if (t.beg + nd > c.beg[r + 1]) atomicExch(overflow, 1);
-        touched[k] = t;
-        elen[k] = t.deg - t.keep + (t.ie - t.ib);
-        nlen[k] = t.newdeg - t.keep;
+        runs[k] = t;
+        len[k] = (pn > t.src ? pn - t.src : 0) + is_ins;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) elen[n_ops] = nlen[n_ops] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) len[n_ops] = 0;
 }
 
-// Merges the rest of every touched row into `tmp` (at noff[k]): surviving old entries and inserted
-// entries in sorted order. Element-parallel: each element computes its output slot with two binary
-// searches of its row's few ops. eoff: exclusive scan of elen. (100K ops on the 4.8M-vertex R-MAT, the
-// three CSRs together: 2.8 ms with a binary search of the rows per entry and every touched row copied
-// whole, 0.7 ms with walk_segments and the rests only; the copy back 2.1 -> 0.35 ms.)
-__global__ void k_merge_rows(const uint64_t* ins, const uint64_t* del, const Touched* touched, int64_t n_rows,
-                             const int64_t* eoff, const int64_t* noff, CSRView c, int32_t* tmp, uint32_t* tmpw,
-                             bool weights, uint64_t wseed, uint32_t wlo, uint32_t whi, int32_t* bad) {
-    walk_segments(eoff, n_rows, [&](int64_t k, int64_t e) {
-        const Touched t = touched[k];
-        const int64_t j = e + t.keep;
-        const uint64_t row_key = (uint64_t)(uint32_t)t.row << 32;
-        if (j < t.deg) {
-            const int32_t x = c.adj[t.beg + j];
-            const uint64_t key = row_key | (uint32_t)x;
-            const int64_t pd = lower_bound_dev(del, t.db, t.de, key);
-            if (pd < t.de && del[pd] == key) return;  // deleted
-            const int64_t pi = lower_bound_dev(ins, t.ib, t.ie, key);
-            const int64_t slot = j - (pd - t.db) + (pi - t.ib);
-            if (slot < t.keep || slot >= t.newdeg) { atomicExch(bad, 1); return; }  // ops not consistent with the row
-            tmp[noff[k] + slot - t.keep] = x;
-            if (weights) tmpw[noff[k] + slot - t.keep] = c.w[t.beg + j];
-        } else {
-            const int64_t q = j - t.deg;  // insert index within the row
-            const uint64_t key = ins[t.ib + q];
-            const int32_t x = (int32_t)(key & 0xffffffffULL);
-            const int64_t po = lower_bound_dev(c.adj, t.beg + t.keep, t.beg + t.deg, x) - t.beg;
-            const int64_t pd = lower_bound_dev(del, t.db, t.de, key);
-            const int64_t slot = q + po - (pd - t.db);
-            if (slot < t.keep || slot >= t.newdeg) { atomicExch(bad, 1); return; }
-            tmp[noff[k] + slot - t.keep] = x;
-            if (weights) tmpw[noff[k] + slot - t.keep] = new_edge_weight(t.row, x, wseed, wlo, whi);
-        }
+// The runs, end to end, into tmp (off: exclusive scan of their lengths): one read and one write an entry, and
+// the search for its run by shuffles, which bounds it (four entries a lane in flight: 0.73 -> 1.0 ms). 100K
+// ops on the 4.8M-vertex R-MAT, two batches of three CSRs: 0.73 ms; 1.34 ms where every entry of a touched
+// row's rest looked itself up among the row's inserts and deletions, and 2.8 ms each batch before that.
+__global__ void k_take_runs(const OpRun* runs, const int64_t* off, int64_t n, CSRView c, int32_t* tmp, uint32_t* tmpw,
+                            bool weights, uint64_t wseed, uint32_t wlo, uint32_t whi) {
+    walk_segments(off, n, [&](int64_t k, int64_t j) {
+        const OpRun t = runs[k];
+        const int64_t to = off[k] + j, from = t.src + j - (t.col >= 0);
+        const bool added = t.col >= 0 && j == 0;
+        tmp[to] = added ? t.col : c.adj[from];
+        if (weights) tmpw[to] = added ? new_edge_weight(t.row, t.col, wseed, wlo, whi) : c.w[from];
     });
 }
 
-// The sizes the host needs, in one place to read: entries to merge, entries merged, a row outgrew its
-// slack (the flag is cleared for the next merge), the batch's bad flag.
-__global__ void k_merge_sizes(const int64_t* eoff, const int64_t* noff, int64_t n, int32_t* overflow,
-                              const int32_t* bad, int64_t* out) {
-    out[0] = eoff[n];
-    out[1] = noff[n];
-    out[2] = *overflow;
+// The sizes the host needs, in one place to read: entries to move, a row outgrew its slack (the flag is
+// cleared for the next merge), the batch's bad flag.
+__global__ void k_merge_sizes(const int64_t* off, int64_t n, int32_t* overflow, const int32_t* bad, int64_t* out) {
+    out[0] = off[n];
+    out[1] = *overflow;
     *overflow = 0;
-    out[3] = *bad;
+    out[2] = *bad;
 }
 
-// Copies the merged rests back into their rows (capacities unchanged), and the new lengths.
-__global__ void k_copy_back(const Touched* touched, int64_t n_rows, const int64_t* noff, const int32_t* tmp,
-                            const uint32_t* tmpw, int32_t* deg, int32_t* adj, uint32_t* w, const int32_t* bad) {
-    if (*bad) return;
-    walk_segments(noff, n_rows, [&](int64_t k, int64_t j) {
-        const int64_t to = touched[k].beg + touched[k].keep + j;
-        adj[to] = tmp[noff[k] + j];
-        if (w) w[to] = tmpw[noff[k] + j];
+// The runs from tmp into their rows (which start at beg), and, where asked for, the rows' new lengths.
+__global__ void k_put_runs(const OpRun* runs, const int64_t* off, int64_t n, const int64_t* beg, const int32_t* tmp,
+                           const uint32_t* tmpw, int32_t* adj, uint32_t* w, int32_t* deg) {
+    walk_segments(off, n, [&](int64_t k, int64_t j) {
+        const OpRun t = runs[k];
+        const int64_t to = beg[t.row] + t.slot + j;
+        adj[to] = tmp[off[k] + j];
+        if (w) w[to] = tmpw[off[k] + j];
     });
-    GRID_STRIDE(k, n_rows) if (touched[k].row >= 0) deg[touched[k].row] = touched[k].newdeg;
+    if (deg) GRID_STRIDE(k, n) if (runs[k].newdeg >= 0) deg[runs[k].row] = runs[k].newdeg;
 }
 
-__global__ void k_set_deg(const Touched* touched, int64_t n_rows, int32_t* deg) {
-    GRID_STRIDE(k, n_rows) if (touched[k].row >= 0) deg[touched[k].row] = touched[k].newdeg;
+// Full re-layout: the new lengths and how far a row keeps its old entries (keep: all of them where it
+// has no op), new capacities, every row's kept entries copied, then the runs.
+__global__ void k_set_deg(const OpRun* runs, int64_t n, int32_t* deg, int32_t* keep) {
+    GRID_STRIDE(k, n)
+        if (runs[k].newdeg >= 0) {
+            deg[runs[k].row] = runs[k].newdeg;
+            keep[runs[k].row] = runs[k].slot;
+        }
 }
 
-// Full re-layout: new capacities from new lengths, then every row copied (the merged rests of touched rows from tmp).
 __global__ void k_new_caps(int64_t V, const int32_t* deg, int64_t* capv) {
     GRID_STRIDE(v, V) capv[v] = row_capacity(deg[v]);
     if (blockIdx.x == 0 && threadIdx.x == 0) capv[V] = 0;
 }
 
 __global__ void k_relayout_rows(int64_t V, const int64_t* old_beg, const int32_t* old_adj, const uint32_t* old_w,
-                                const int32_t* deg, const int64_t* new_beg, int32_t* new_adj, uint32_t* new_w,
-                                const int32_t* touched_slot, const Touched* touched, const int64_t* noff,
-                                const int32_t* tmp, const uint32_t* tmpw) {
+                                const int32_t* deg, const int32_t* keep, const int64_t* new_beg, int32_t* new_adj,
+                                uint32_t* new_w) {
     walk_segments(new_beg, V, [&](int64_t v, int64_t j) {
-        if (j >= deg[v]) return;  // (slack)
-        const int32_t k = touched_slot[v];
+        if (j >= deg[v] || j >= keep[v]) return;  // (slack, or a run's)
         const int64_t to = new_beg[v] + j, from = old_beg[v] + j;
-        const bool merged = k >= 0 && j >= touched[k].keep;
-        const int64_t m = merged ? noff[k] + j - touched[k].keep : 0;
-        new_adj[to] = merged ? tmp[m] : old_adj[from];
-        if (new_w) new_w[to] = merged ? tmpw[m] : old_w[from];
+        new_adj[to] = old_adj[from];
+        if (new_w) new_w[to] = old_w[from];
     });
 }
 
 __global__ void k_fill_i32(int32_t* p, int64_t n, int32_t v) { GRID_STRIDE(i, n) p[i] = v; }
-
-__global__ void k_mark_slots(const Touched* touched, int64_t n_rows, int32_t* slot) {
-    GRID_STRIDE(k, n_rows) if (touched[k].row >= 0) slot[touched[k].row] = (int32_t)k;
-}
 
 __global__ void k_bin_flags(int64_t V, const int32_t* deg, int32_t small, int32_t large, uint8_t* f0, uint8_t* f1,
                             uint8_t* f2, int32_t* ids) {
@@ -520,59 +492,50 @@ int store_apply_ops(gir_dev* g, DevCSR& c, const uint64_t* ins, int64_t n_ins, c
                     bool weights, int32_t* bad, int32_t* overflow) {
     if (n_ins + n_del == 0) return GIR_OK;
     const int64_t V = g->V;
-    const int64_t n_rows = n_ins + n_del;  // slots, one per op
+    const int64_t n = n_ins + n_del;
     int32_t* tmp = nullptr;
-    int64_t *eoff = nullptr, *noff = nullptr, *words = nullptr;  // (words: the sizes the host reads)
-    Touched* touched = nullptr;
+    int64_t *off = nullptr, *words = nullptr;  // (words: the sizes the host reads)
+    OpRun* runs = nullptr;
     uint32_t* tmpw = nullptr;
-    GIR_TRY(ensure_n(g, g->scratch[9], n_rows + 1, &touched));
-    GIR_TRY(ensure_n(g, g->scratch[10], n_rows + 1, &eoff));
-    GIR_TRY(ensure_n(g, g->scratch[11], n_rows + 1, &noff));
+    GIR_TRY(ensure_n(g, g->scratch[9], n, &runs));
+    GIR_TRY(ensure_n(g, g->scratch[10], n + 1, &off));
     GIR_TRY(ensure_n(g, g->scratch[12], 4, &words));
-    k_touched_rows<<<grid_for(g, n_rows, kBlock), kBlock, 0, g->stream>>>(ins, n_ins, del, n_del, view(c), touched, eoff,
-                                                                           noff, overflow, bad);
-    GIR_LAUNCH(g, "k_touched_rows");
-    GIR_TRY(exclusive_scan_two_i64(g, eoff, noff, n_rows + 1));
-    k_merge_sizes<<<1, 1, 0, g->stream>>>(eoff, noff, n_rows, overflow, bad, words);
+    k_op_runs<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(ins, n_ins, del, n_del, view(c), runs, off, overflow, bad);
+    GIR_LAUNCH(g, "k_op_runs");
+    GIR_TRY(exclusive_scan_i64(g, off, off, n + 1));
+    k_merge_sizes<<<1, 1, 0, g->stream>>>(off, n, overflow, bad, words);
     GIR_LAUNCH(g, "k_merge_sizes");
     void* hp = nullptr;
     GIR_TRY(pinned(g, kPinnedBytes, &hp));
     int64_t* h = static_cast<int64_t*>(hp);
-    GIR_CUDA(g, cudaMemcpyAsync(h, words, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, g->stream));
+    GIR_CUDA(g, cudaMemcpyAsync(h, words, 3 * sizeof(int64_t), cudaMemcpyDeviceToHost, g->stream));
     GIR_CUDA(g, cudaStreamSynchronize(g->stream));
-    const int64_t n_elems = h[0], n_new = h[1];
-    const bool ovf = h[2] != 0;
-    if (h[3]) return store_ops_bad(g);
+    const int64_t n_moved = h[0];
+    const bool ovf = h[1] != 0;
+    if (h[2]) return store_ops_bad(g);
     const bool wts = weights && c.w;
-    // tmp holds the merged rest of touched row k at noff[k]
-    GIR_TRY(ensure_n(g, g->stage_out, n_new + 4, &tmp));
-    if (wts) GIR_TRY(ensure_n(g, g->scratch[3], n_new + 4, &tmpw));
-    if (n_elems > 0) {
-        k_merge_rows<<<grid_for(g, n_elems, kBlock), kBlock, 0, g->stream>>>(
-            ins, del, touched, n_rows, eoff, noff, view(c), tmp, tmpw, wts, g->wrule_seed, g->wrule_lo, g->wrule_hi, bad);
-        GIR_LAUNCH(g, "k_merge_rows");
+    GIR_TRY(ensure_n(g, g->stage_out, n_moved + 4, &tmp));
+    if (wts) GIR_TRY(ensure_n(g, g->scratch[3], n_moved + 4, &tmpw));
+    if (n_moved > 0) {
+        k_take_runs<<<grid_for(g, n_moved, kBlock), kBlock, 0, g->stream>>>(runs, off, n, view(c), tmp, tmpw, wts,
+                                                                            g->wrule_seed, g->wrule_lo, g->wrule_hi);
+        GIR_LAUNCH(g, "k_take_runs");
     }
+    const int put_grid = grid_for(g, n_moved > n ? n_moved : n, kBlock);
     if (!ovf) {
-        k_copy_back<<<grid_for(g, n_new > n_rows ? n_new : n_rows, kBlock), kBlock, 0, g->stream>>>(
-            touched, n_rows, noff, tmp, tmpw, c.deg, c.adj, wts ? c.w : nullptr, bad);
-        GIR_LAUNCH(g, "k_copy_back");
+        k_put_runs<<<put_grid, kBlock, 0, g->stream>>>(runs, off, n, c.beg, tmp, tmpw, c.adj, wts ? c.w : nullptr, c.deg);
+        GIR_LAUNCH(g, "k_put_runs");
     } else {
         // Some row outgrew its slack: new layout for the whole CSR.
         trace_mark(g, "store: merge before relayout");
-        int32_t inconsistent = 0;
-        GIR_CUDA(g, cudaMemcpyAsync(&inconsistent, bad, sizeof(int32_t), cudaMemcpyDeviceToHost, g->stream));
-        GIR_CUDA(g, cudaStreamSynchronize(g->stream));
-        if (inconsistent) return store_ops_bad(g);
-        int32_t* slot = nullptr;
+        int32_t* keep = nullptr;
         int64_t* capv = nullptr;
-        GIR_TRY(ensure_n(g, g->scratch[0], V + 1, &slot));
+        GIR_TRY(ensure_n(g, g->scratch[0], V + 1, &keep));
         GIR_TRY(ensure_n(g, g->scratch[1], V + 1, &capv));
-        k_set_deg<<<grid_for(g, n_rows, kBlock), kBlock, 0, g->stream>>>(touched, n_rows, c.deg);
-        GIR_LAUNCH(g, "k_set_deg");
-        k_fill_i32<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(slot, V, -1);
+        k_fill_i32<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(keep, V, INT32_MAX);
         GIR_LAUNCH(g, "k_fill_i32");
-        k_mark_slots<<<grid_for(g, n_rows, kBlock), kBlock, 0, g->stream>>>(touched, n_rows, slot);
-        GIR_LAUNCH(g, "k_mark_slots");
+        k_set_deg<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(runs, n, c.deg, keep);
+        GIR_LAUNCH(g, "k_set_deg");
         k_new_caps<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, c.deg, capv);
         GIR_LAUNCH(g, "k_new_caps");
         int64_t* nbeg = nullptr;
@@ -585,9 +548,11 @@ int store_apply_ops(gir_dev* g, DevCSR& c, const uint64_t* ins, int64_t n_ins, c
         uint32_t* nw = nullptr;
         GIR_TRY(dev_alloc_n(g, &nadj, total > 0 ? total : 4));
         if (c.w) GIR_TRY(dev_alloc_n(g, &nw, total > 0 ? total : 4));
-        k_relayout_rows<<<grid_for(g, total, kBlock), kBlock, 0, g->stream>>>(V, c.beg, c.adj, c.w, c.deg, nbeg, nadj,
-                                                                                 nw, slot, touched, noff, tmp, tmpw);
+        k_relayout_rows<<<grid_for(g, total, kBlock), kBlock, 0, g->stream>>>(V, c.beg, c.adj, c.w, c.deg, keep, nbeg, nadj,
+                                                                              nw);
         GIR_LAUNCH(g, "k_relayout_rows");
+        k_put_runs<<<put_grid, kBlock, 0, g->stream>>>(runs, off, n, nbeg, tmp, tmpw, nadj, wts ? nw : nullptr, nullptr);
+        GIR_LAUNCH(g, "k_put_runs");
         dev_free(g, c.beg);
         dev_free(g, c.adj);
         dev_free(g, c.w);
