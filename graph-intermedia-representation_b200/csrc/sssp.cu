@@ -313,7 +313,8 @@ __device__ __forceinline__ D load_dist(const D* p) {
 //  - every thread steps through the lanes of its own edge (few lanes an edge);
 //  - eight threads take an edge, so four edges at once, each thread 16 bytes of the two distance rows at
 //    a time (many lanes an edge: the passes of a power-law graph, whose vertices are reached in most
-//    lanes at once). kU such steps are in flight: the rows come from L2 and HBM.
+//    lanes at once). The rows come from L2 and HBM; two such steps in flight (64 registers) measured as one
+//    (40, and more warps).
 // The minimum is taken without waiting for its result: a lane counts as improved by the plain read
 // before it. Where another thread lowered the lane in between, that thread queued it as well, and a far
 // entry that is no longer far is dropped by the far split, so the queues stay supersets of the lanes
