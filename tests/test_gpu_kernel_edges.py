@@ -271,3 +271,28 @@ def test_batches_that_change_both_directions_of_pairs(pkg, orc, V, n):
             np.testing.assert_array_equal(ga, ea)
         _oracle_match(pkg, orc, d, V, fb, fa, f"step {step}")
     d.close()
+
+
+@pytest.mark.parametrize("where", ["first", "middle", "last", "none"])
+def test_bottom_up_rows_to_their_last_entry(pkg, orc, where):
+    """Bottom-up levels of rows of every remainder of the warp's and the CTA's rounds, found by one entry of
+    the row: the first, one in between, the last, or none (lanes of the other sources find them)."""
+    deg = np.r_[31:35, 125:130, 157:166, 285:292, 4093:4102, 5117:5124, 8190:8196]
+    L, n = 8200, len(deg)  # leaves, then the hubs, then a vertex that reaches one leaf of every hub
+    V = L + n + 2
+    u = np.concatenate([np.arange(L - d, L) for d in deg])
+    v = np.repeat(L + np.arange(n), deg)
+    at = {"first": L - deg, "middle": L - deg // 2 - 1, "last": np.full(n, L - 1), "none": np.zeros(0, np.int64)}[where]
+    tail = np.arange(0, L, 50)
+    g = _graph(pkg, V, np.r_[u, np.full(len(at), V - 2), np.full(len(tail), V - 1)], np.r_[v, at, tail])
+    fb, fa = orc.normalize(V, g.fw_beg, g.fw_adj)
+    d = pkg.DeviceGraph.from_graph(g, weights=False)
+    d.set_param(pkg.native.PARAM_ALPHA, 1e9)
+    d.set_param(pkg.native.PARAM_BETA, 1e9)
+    for src in ([V - 2], [V - 2, V - 1, 0, L - 1, L + 3]):
+        got = d.bfs(np.array(src, np.int32))
+        for row, s in zip(got, src):
+            np.testing.assert_array_equal(row, orc.bfs(V, fb, fa, [s]))
+        if len(src) > 1 or where != "none":  # (a lone source without edges has no level to take)
+            assert d.query_stats()["bottom_up"] > 0
+    d.close()
