@@ -116,7 +116,7 @@ struct DistT<uint32_t> {
 template <>
 struct DistT<uint16_t> {
     static constexpr uint16_t inf = 0xffffu;
-    using acc = uint32_t;
+    using acc = uint32_t;  // (holds the sum of a distance and a weight below inf; see take() in relax_edges)
     __device__ static void atomic_min(uint16_t* p, uint16_t v) {
         const uintptr_t a = reinterpret_cast<uintptr_t>(p);
         unsigned int* wp = reinterpret_cast<unsigned int*>(a & ~(uintptr_t)3);
@@ -335,8 +335,9 @@ __device__ __forceinline__ void relax_edges(const Group& a, uint64_t kend, int32
     // takes one lane of a target from its tentative distance: 0 no gain, 1 near, 2 far
     auto take = [&](D* at, A du, A dw, uint32_t weight) -> int {
         const A nd = du + weight;
-        if (sizeof(D) == 2 && nd >= (A)DistT<D>::inf) {
-            // a 16-bit lane cannot hold it: the group is run again with 32-bit lanes
+        // (the weight by itself first: the sum of 32 bits could wrap)
+        if (sizeof(D) == 2 && (weight >= (A)DistT<D>::inf || nd >= (A)DistT<D>::inf)) {
+            // a 16-bit lane cannot hold it: the group is run again with wider lanes
             if (dw == (A)DistT<D>::inf) a.ctl[X_OVF] = 1ull;
             return 0;
         }

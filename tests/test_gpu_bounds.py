@@ -1,0 +1,45 @@
+"""Values and batches at the edges of what a call takes: the largest stored weights, weights through
+batches of many ops, backward rows that do not match the forward ones, memory that runs out."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _weighted(pkg, V, u, v, w):
+    key, first = np.unique(np.asarray(u, np.int64) * V + np.asarray(v, np.int64), return_index=True)
+    return pkg.graphs.from_edges(V, key // V, key % V, np.asarray(w, np.uint32)[first])
+
+
+@pytest.mark.parametrize("lanes", [2, 8, 64])
+@pytest.mark.parametrize("alike", [False, True])
+@pytest.mark.parametrize("all_wrap", [False, True])
+def test_sssp_weights_up_to_the_largest_word(pkg, orc, lanes, alike, all_wrap):
+    """Stored weights within a 16-bit distance of 2^32: narrow lanes cannot hold the sum with a source's
+    distance, and 32 bits of it wrap to a small one. `all_wrap`: every sum that does not fit wraps, so nothing
+    else has the group run again; `alike`: all lanes alike, so an edge is relaxed by eight threads."""
+    n = 600
+    rng = np.random.default_rng(lanes)
+    step = rng.integers(60, 100, n - 1)
+    at = np.r_[0, np.cumsum(step)]  # below 65,534
+    chain = np.arange(n)
+    src = (np.zeros(lanes, np.int64) if alike else rng.integers(0, 8, lanes)).astype(np.int32)
+    # from every vertex of the chain's rest an edge of nearly 2^32 leads out, to a leaf of its own
+    far = chain[20:]
+    big = (1 << 32) - rng.integers(1, at[far] - at[8] + 1)
+    big[::50] = (1 << 32) - (at[far] - at[8])[::50]
+    if not all_wrap:
+        big[::7] = rng.choice([0xFFFF, 0x10000, 0xFFFF0000, 0xFFFE], len(big[::7]))
+    V = n + len(far)
+    g = _weighted(pkg, V, np.r_[chain[:-1], chain[1:], far], np.r_[chain[1:], chain[:-1], n + np.arange(len(far))],
+                  np.r_[step, step, big])
+    fb, fa = orc.normalize(V, g.fw_beg, g.fw_adj)
+    exp = np.stack([orc.sssp(V, fb, fa, [int(s)], w=g.w) for s in src])
+    assert exp[:, :n].max() < 0xFFFF and exp[:, n:].max() > 0xFFFFFFFF
+    for bits in (16, 32, 64, 0):
+        for delta in (1, 64, 1 << 20, 1 << 40):
+            d = pkg.DeviceGraph.from_graph(g)  # (a handle remembers that 16 bits did not do)
+            d.set_param(pkg.native.PARAM_LANE_BITS, bits)
+            got = d.sssp(src, delta=delta, weights=pkg.native.WEIGHT_STORED)
+            np.testing.assert_array_equal(got, exp, err_msg=f"{bits} bits, delta {delta}")
+            d.close()
