@@ -143,7 +143,8 @@ __global__ void k_op_runs(const uint64_t* ins, int64_t n_ins, const uint64_t* de
         const int64_t beg = c.beg[r], end = beg + c.deg[r];
         const int64_t p = lower_bound_dev(c.adj, beg, end, col);
         const int64_t pn = next == ~0ull ? end : lower_bound_dev(c.adj, p, end, (int32_t)(next & 0xffffffffULL));
-        if (!is_ins && (p >= end || c.adj[p] != col)) atomicExch(bad, 1);  // the ops do not match this CSR
+        // an insert that is there already or a deletion that is not: the ops do not match this CSR
+        if (is_ins == (p < end && c.adj[p] == col)) atomicExch(bad, 1);
         OpRun t;
         t.src = p + !is_ins;
         t.row = (int32_t)r;

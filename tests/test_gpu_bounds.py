@@ -43,3 +43,27 @@ def test_sssp_weights_up_to_the_largest_word(pkg, orc, lanes, alike, all_wrap):
             got = d.sssp(src, delta=delta, weights=pkg.native.WEIGHT_STORED)
             np.testing.assert_array_equal(got, exp, err_msg=f"{bits} bits, delta {delta}")
             d.close()
+
+
+@pytest.mark.parametrize("insert", [True, False])
+@pytest.mark.parametrize("n", [2, 40])
+def test_backward_rows_that_do_not_match(pkg, insert, n):
+    """A backward CSR with as many edges as the forward one, but one of them elsewhere: a batch that inserts the
+    edge it holds already, or deletes the one it lacks, is malformed, and no backward row changes."""
+    V = 50
+    a = np.arange(V - 1)
+    g = pkg.graphs.from_edges(V, a, a + 1)
+    src, dst = a.copy(), a + 1
+    src[7], dst[7] = 7, 30  # (the forward rows have 7 -> 8)
+    b = pkg.graphs.from_edges(V, src, dst)
+    d = pkg.DeviceGraph.create(g.fw_beg, g.fw_adj, b.bw_beg, b.bw_adj, V)
+    before = [x.copy() for x in d.csr(1)]
+    u = np.r_[7, np.arange(9, 8 + n)].astype(np.int32)
+    v = np.r_[30 if insert else 8, np.zeros(n - 1, int)].astype(np.int32)  # (edges to vertex 0: new)
+    ins = np.r_[1 if insert else 0, np.ones(n - 1, int)].astype(np.uint8)
+    with pytest.raises(pkg.GirError, match="not the transpose") as e:
+        d.apply_batch(u, v, ins)
+    assert e.value.code == 5
+    for x, y in zip(d.csr(1), before):
+        np.testing.assert_array_equal(x, y)
+    d.close()
