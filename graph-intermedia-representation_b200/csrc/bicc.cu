@@ -687,13 +687,11 @@ int bct_build(gir_dev* g) {
     GIR_LAUNCH(g, "k_pack_keys");
     k_nontree_first<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, h, key, nd, low, high, uf);
     GIR_LAUNCH(g, "k_nontree_first");
-    k_uf_flatten<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(uf, V);
-    GIR_LAUNCH(g, "k_uf_flatten");
+    GIR_TRY(uf_flatten(g, uf, V));
     for (int r = 0; r < 2; ++r) {
         k_nontree_sample<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, h, key, nd, uf);
         GIR_LAUNCH(g, "k_nontree_sample");
-        k_uf_flatten<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(uf, V);
-        GIR_LAUNCH(g, "k_uf_flatten");
+        GIR_TRY(uf_flatten(g, uf, V));
     }
     auto carry_up = [&](const uint8_t* only) -> int {
         for (int L = D - 1; L >= 1; --L) {
@@ -712,8 +710,7 @@ int bct_build(gir_dev* g) {
         k_rule2<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, parent, pre, nd, low, high, uf, &cnt[C_ERR]);
         GIR_LAUNCH(g, "k_rule2");
     }
-    k_uf_flatten<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(uf, V);
-    GIR_LAUNCH(g, "k_uf_flatten");
+    GIR_TRY(uf_flatten(g, uf, V));
     if (!deep) {
         int32_t* giant = reinterpret_cast<int32_t*>(cnt + C_N);
         need = flag;

@@ -571,12 +571,10 @@ static int scc_by_quotient(gir_dev* g, int32_t* label, int64_t* n_scc, bool* use
     GIR_LAUNCH(g, "k_mask_deg");
     k_uf_first<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(sym, V, cls);
     GIR_LAUNCH(g, "k_uf_first");
-    k_uf_flatten<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(cls, V);
-    GIR_LAUNCH(g, "k_uf_flatten");
+    GIR_TRY(uf_flatten(g, cls, V));
     k_class_link<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, sym, cls, cnt + 1);
     GIR_LAUNCH(g, "k_class_link");
-    k_uf_flatten<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(cls, V);
-    GIR_LAUNCH(g, "k_uf_flatten");
+    GIR_TRY(uf_flatten(g, cls, V));
     // (an edge between classes has two ends that are not full)
     fw.deg = mdeg;
     k_mask_deg<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, g->fw.deg, full, 0, mdeg);

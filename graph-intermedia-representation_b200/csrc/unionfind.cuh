@@ -43,12 +43,16 @@ __device__ __forceinline__ void uf_hook(int32_t* uf, int32_t ra, int32_t rb) {
     if (lo != hi && uf[hi] > lo) atomicMin(&uf[hi], lo);
 }
 
-// Every entry to its root, run as a kernel of its own with no union meanwhile. A thread writes its own
-// entry only, at every step, so that the walks of all threads shorten one another's: a chain of n takes
+// Every entry to its root, run as a kernel of its own with no union meanwhile (uf_flatten). A thread writes
+// its own entry only, at every step, so that the walks of all threads shorten one another's: a chain of n takes
 // about log2 n steps (a lattice's first links form chains as long as its side). Long walks read past the
 // L1, which would hide the others' steps; short ones do not, since most end at one root, whose line the
 // L2 would serve one warp at a time (4.8M vertices: 106 us, 24 us so).
-__global__ static void k_uf_flatten(int32_t* uf, int64_t V) {
+// Every CTA is resident: an entry points at a smaller one, so whatever a walk meets is done or about to be
+// taken up. With more CTAs than fit, those of the first wave went on to their second vertices through entries
+// that no thread had started with, one step after another: 56 ms for a path of a million vertices in the order
+// of their ids (0.1 ms for the whole component build so).
+__global__ static void __launch_bounds__(256, 8) k_uf_flatten(int32_t* uf, int64_t V) {
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x) {
         int32_t x = uf[v];
         int steps = 0;
@@ -57,6 +61,14 @@ __global__ static void k_uf_flatten(int32_t* uf, int64_t V) {
             x = p;
         }
     }
+}
+inline int uf_flatten(gir_dev* g, int32_t* uf, int64_t V) {
+    constexpr int kThreads = 256;
+    if (V <= 0) return GIR_OK;
+    const int64_t want = (V + kThreads - 1) / kThreads, fit = (int64_t)g->num_sms * 8;
+    k_uf_flatten<<<(int)(want < fit ? want : fit), kThreads, 0, g->stream>>>(uf, V);
+    GIR_LAUNCH(g, "k_uf_flatten");
+    return GIR_OK;
 }
 
 // First links without atomics: every vertex with a smaller entry at the head of its (sorted) row goes

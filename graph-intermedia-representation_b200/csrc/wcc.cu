@@ -116,13 +116,11 @@ static int wcc_labels_sym(gir_dev* g, int32_t* label, int64_t* n_comp) {
     const CSRView s = view(g->sym);
     k_uf_first<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(s, V, label);
     GIR_LAUNCH(g, "k_uf_first");
-    k_uf_flatten<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(label, V);
-    GIR_LAUNCH(g, "k_uf_flatten");
+    GIR_TRY(uf_flatten(g, label, V));
     for (int r = 0; r < kHookRounds; ++r) {
         k_uf_hook_first_two<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(s, V, label);
         GIR_LAUNCH(g, "k_uf_hook_first_two");
-        k_uf_flatten<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(label, V);
-        GIR_LAUNCH(g, "k_uf_flatten");
+        GIR_TRY(uf_flatten(g, label, V));
     }
     GIR_TRY(sample_mode(g, g->sym, label, giant));
     trace_mark(g, "wcc: neighbour rounds + sample");

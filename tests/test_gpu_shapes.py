@@ -63,3 +63,47 @@ def test_blocks_of_a_star_whose_hub_is_the_root(pkg):
     V = 400_000
     first, last = (_build_ms(pkg, _star(pkg, V, hub), pkg.native.LAYER_BCT) for hub in (0, V - 1))
     assert first < 3 * last, (first, last)
+
+
+@pytest.mark.parametrize("layer", ["WCC", "BCT"])
+def test_builds_of_a_chain_in_the_order_of_its_ids(pkg, layer):
+    """A path for the components; for the blocks a ring whose vertices all hang on one hub, so that every edge of
+    the ring puts a tree edge under the one before it. The ids run along the chain, or in any order."""
+    V = 600_000
+    a = np.arange(1, V)
+    if layer == "WCC":
+        u, v = a - 1, a
+    else:
+        hub, rest = V // 2, np.delete(np.arange(V), V // 2)
+        u, v = np.r_[rest, np.full(V - 1, hub)], np.r_[np.roll(rest, 1), rest]
+    perm = np.random.default_rng(1).permutation(V)
+    which = getattr(pkg.native, f"LAYER_{layer}")
+    if layer == "WCC":
+        ms = []
+        for p in (np.arange(V), perm):
+            d = pkg.DeviceGraph.from_graph(_both(pkg, V, p[u], p[v]), weights=False)
+            best = 1e9
+            for _ in range(5):
+                t = time.perf_counter()
+                d.build(which)
+                best = min(best, 1e3 * (time.perf_counter() - t))
+            ms.append(best)
+            assert (d.labels(pkg.native.LABEL_WCC) == 0).all()
+            d.close()
+    else:
+        ms = [_build_ms(pkg, _both(pkg, V, p[u], p[v]), which) for p in (np.arange(V), perm)]
+    assert ms[0] < 3 * ms[1] + 1, ms
+
+
+def test_components_of_chains_of_every_length(pkg, orc):
+    """Paths in the order of their ids, side by side, with lengths about those of warps, CTAs and waves."""
+    length = np.array([1, 2, 31, 32, 33, 255, 256, 257, 4095, 4097, 70_000, 303_103, 303_105, 606_209])
+    V = int(length.sum())
+    end = np.cumsum(length)
+    a = np.delete(np.arange(V), end - 1)
+    g = _both(pkg, V, a, a + 1)
+    d = pkg.DeviceGraph.from_graph(g, weights=False)
+    d.build(pkg.native.LAYER_WCC)
+    np.testing.assert_array_equal(d.labels(pkg.native.LABEL_WCC), np.repeat(end - length, length))
+    assert d.counts()["n_wcc"] == len(length)
+    d.close()
