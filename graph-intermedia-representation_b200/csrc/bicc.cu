@@ -261,12 +261,20 @@ __global__ void k_win_step(const int32_t* at, int64_t n, int64_t len, const int3
     }
 }
 
-// The smallest H neighbour of every tree root: it decides which of its blocks is the root's parent block.
-__global__ void k_root_rows(int64_t V, const int32_t* scc, const int32_t* hdeg, int32_t* deg, int32_t* least) {
+// The smallest H neighbour of every tree root: it decides which of its blocks is the root's parent block. In a
+// BFS forest a root's neighbours are its children (no rows to read); consecutive children send one atomicMin.
+__global__ void k_root_child_least(int64_t V, const int32_t* parent, int32_t* least) {
     GRID_STRIDE(v, V) {
-        deg[v] = scc[v] == (int32_t)v ? hdeg[v] : 0;
-        least[v] = INT32_MAX;
+        const int32_t p = parent[v];
+        const bool child = p != (int32_t)v && parent[p] == p;
+        const unsigned grp = __match_any_sync(__activemask(), child ? p : -1);
+        if (child && __ffs(grp) - 1 == lane_id() && *(volatile int32_t*)&least[p] > (int32_t)v)
+            atomicMin(&least[p], (int32_t)v);
     }
+}
+// In the forest of a deep graph they need not be: the roots' rows.
+__global__ void k_root_rows(int64_t V, const int32_t* scc, const int32_t* hdeg, int32_t* deg) {
+    GRID_STRIDE(v, V) deg[v] = scc[v] == (int32_t)v ? hdeg[v] : 0;
 }
 // Rows are cut into even runs whatever their length (off: scan of the row lengths): a root may be the hub that
 // holds every row entry, and one warp for its whole row took 6.1 of 6.7 ms of the blocks of a star of 300,000
@@ -747,11 +755,18 @@ int bct_build(gir_dev* g) {
     GIR_LAUNCH(g, "k_block_ids");
     GIR_TRY(ensure_n(g, g->blk_head, nb + 1, &head));
     int32_t *rdeg = pre, *least = high;  // (neither is read any more)
-    k_root_rows<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, scc, hdeg, rdeg, least);
-    GIR_LAUNCH(g, "k_root_rows");
-    GIR_TRY(scan_degrees(g, rdeg, V, scan));
-    k_root_least<<<g->num_sms * 8, kBlock, 0, g->stream>>>(V, scan, h.sym, scc, least);
-    GIR_LAUNCH(g, "k_root_least");
+    k_fill_i32<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(least, V, INT32_MAX);
+    GIR_LAUNCH(g, "k_fill_i32");
+    if (deep) {
+        k_root_rows<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, scc, hdeg, rdeg);
+        GIR_LAUNCH(g, "k_root_rows");
+        GIR_TRY(scan_degrees(g, rdeg, V, scan));
+        k_root_least<<<g->num_sms * 8, kBlock, 0, g->stream>>>(V, scan, h.sym, scc, least);
+        GIR_LAUNCH(g, "k_root_least");
+    } else {
+        k_root_child_least<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, parent, least);
+        GIR_LAUNCH(g, "k_root_child_least");
+    }
     k_root_block_least<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, least, uf, id_of_rep, label);
     GIR_LAUNCH(g, "k_root_block_least");
     k_block_assign<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, parent, nd, uf, id_of_rep, label, head);
