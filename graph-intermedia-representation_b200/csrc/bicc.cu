@@ -151,13 +151,11 @@ struct ForestUp {
 // sixty launches in all (about 1.5 ms). The arcs' indices are 32 bits wide: below 2^30 vertices.
 constexpr int64_t kEulerMaxV = 1ll << 30;
 
-// Tree edges: the slot of the hooked root holds (u << 32 | w); ~0 elsewhere.
-__global__ void __launch_bounds__(kBlock) k_tree_link(int64_t V, CSRView h, const int32_t* scc, int32_t* uf,
-                                                      uint64_t* edge, unsigned long long* err) {
-    __shared__ int64_t s_excl[kBlock / 32][33];
-    __shared__ int32_t s_u[kBlock / 32][32];
-    const int wib = threadIdx.x >> 5;
-    warp_sweep_rows(h.beg, h.deg, h.adj, 0, V, s_excl[wib], s_u[wib], [&](int32_t u, int32_t w, int64_t) {
+// Tree edges: the slot of the hooked root holds (u << 32 | w); ~0 elsewhere. (off: scan of H's row lengths.)
+__global__ void __launch_bounds__(kBlock) k_tree_link(int64_t V, const int64_t* off, CSRView h, const int32_t* scc,
+                                                      int32_t* uf, uint64_t* edge, unsigned long long* err) {
+    walk_segments(off, V, [&](int64_t v, int64_t j) {
+        const int32_t u = (int32_t)v, w = h.adj[h.beg[v] + j];
         if (u > w || scc[u] != scc[w]) return;  // (every pair is in both rows)
         const int32_t hooked = uf_union(uf, u, w, err);
         if (hooked >= 0) edge[hooked] = ((uint64_t)(uint32_t)u << 32) | (uint32_t)w;
@@ -527,6 +525,8 @@ static int euler_forest(gir_dev* g, const CSRView& h, const int32_t* scc, int32_
     uint64_t *edge = nullptr, *picked = nullptr;
     int32_t* uf = nullptr;
     uint8_t* flag = nullptr;
+    int64_t *tour = nullptr, *down = nullptr;
+    GIR_TRY(t.get(&tour, V + 1));
     GIR_TRY(t.get(&edge, V));
     GIR_TRY(t.get(&picked, V));
     GIR_TRY(t.get(&uf, V));
@@ -535,7 +535,9 @@ static int euler_forest(gir_dev* g, const CSRView& h, const int32_t* scc, int32_
     GIR_CUDA(g, cudaMemsetAsync(pre, 0, sizeof(int32_t) * V, g->stream));
     k_uf_init<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(uf, V);
     GIR_LAUNCH(g, "k_uf_init");
-    k_tree_link<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, h, scc, uf, edge, err);
+    int64_t* off = tour;  // (the tours' offsets come later)
+    GIR_TRY(scan_degrees(g, h.deg, V, off));
+    k_tree_link<<<g->num_sms * 8, kBlock, 0, g->stream>>>(V, off, h, scc, uf, edge, err);
     GIR_LAUNCH(g, "k_tree_link");
     k_tree_flags<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, edge, flag);
     GIR_LAUNCH(g, "k_tree_flags");
@@ -546,13 +548,11 @@ static int euler_forest(gir_dev* g, const CSRView& h, const int32_t* scc, int32_
     uint64_t *arcs = nullptr, *atmp = nullptr;
     int32_t* twin = nullptr;
     int2 *ja = nullptr, *jb = nullptr;
-    int64_t *tour = nullptr, *down = nullptr;
     GIR_TRY(t.get(&arcs, n + 1));
     GIR_TRY(t.get(&atmp, n + 1));
     GIR_TRY(t.get(&twin, n + 1));
     GIR_TRY(t.get(&ja, n + 1));
     GIR_TRY(t.get(&jb, n + 1));
-    GIR_TRY(t.get(&tour, V + 1));
     GIR_TRY(t.get(&down, n + 1));
     if (m == 0) return GIR_OK;
     const int gn = grid_for(g, n + 1, kBlock);

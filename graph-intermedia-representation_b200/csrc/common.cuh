@@ -409,48 +409,6 @@ __device__ __forceinline__ int64_t lower_bound_dev(const T* a, int64_t lo, int64
     return lo;
 }
 
-// Calls f(u, w, edge_index) for every entry of the rows of vertices [v0, v1) of `c`. Warp-
-// cooperative: a warp takes 32 consecutive vertices, scans their row lengths and walks the
-// concatenated rows 32 entries at a time (consecutive lanes read consecutive entries of a row),
-// so a row of any length costs its warp ceil(len/32) rounds. Must be called by all threads of
-// the grid (every lane of a warp takes part in every round). `scan` is per-warp shared scratch
-// of 33 int64 and 32 int32.
-template <class F>
-__device__ __forceinline__ void warp_sweep_rows(const int64_t* beg, const int32_t* deg, const int32_t* adj,
-                                                int64_t v0, int64_t v1, int64_t* s_excl, int32_t* s_u, F&& f) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t base = v0 + warp * 32; base < v1; base += nwarps * 32) {
-        const int64_t v = base + lane;
-        const int64_t cnt = v < v1 ? deg[v] : 0;
-        int64_t incl = cnt;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int64_t t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        s_excl[lane] = incl - cnt;
-        if (lane == 31) s_excl[32] = incl;
-        s_u[lane] = (int32_t)v;
-        __syncwarp();
-        const int64_t total = s_excl[32];
-        for (int64_t p0 = 0; p0 < total; p0 += 32) {
-            const int64_t p = p0 + lane;
-            if (p < total) {
-                int lo = 0, hi = 31;
-                while (lo < hi) {
-                    const int m = (lo + hi + 1) >> 1;
-                    if (s_excl[m] <= p) lo = m; else hi = m - 1;
-                }
-                const int32_t u = s_u[lo];
-                const int64_t e = beg[u] + (p - s_excl[lo]);
-                f(u, adj[e], e);
-            }
-        }
-        __syncwarp();
-    }
-}
-
 // Largest i in [lo, n) with off[i] <= key (off[lo] <= key), by one warp, 32 probes a round.
 template <class T>
 __device__ __forceinline__ int64_t warp_find(const T* off, int64_t lo, int64_t n, int64_t key) {

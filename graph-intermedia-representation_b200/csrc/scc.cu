@@ -471,22 +471,17 @@ __global__ void k_mask_deg(int64_t V, const int32_t* deg, const uint8_t* full, i
     GRID_STRIDE(v, V) out[v] = (full[v] != 0) == (want != 0) ? deg[v] : 0;
 }
 
-__global__ void __launch_bounds__(kBlock) k_class_link(int64_t V, CSRView sym, int32_t* cls, unsigned long long* err) {
-    __shared__ int64_t s_excl[kWarps][33];
-    __shared__ int32_t s_u[kWarps][32];
-    const int wib = threadIdx.x >> 5;
-    warp_sweep_rows(sym.beg, sym.deg, sym.adj, 0, V, s_excl[wib], s_u[wib],
-                    [&](int32_t u, int32_t w, int64_t) { uf_union(cls, u, w, err); });
+// (off: scan of the row lengths, so that a hub's row is shared by many warps.)
+__global__ void __launch_bounds__(kBlock) k_class_link(int64_t V, const int64_t* off, CSRView sym, int32_t* cls,
+                                                       unsigned long long* err) {
+    walk_segments(off, V, [&](int64_t u, int64_t j) { uf_union(cls, (int32_t)u, sym.adj[sym.beg[u] + j], err); });
 }
 
 // Keys (class(u) << 32 | class(w)) of the edges between classes; counted only while keys is null.
-__global__ void __launch_bounds__(kBlock) k_quotient_keys(int64_t V, CSRView fw, const int32_t* cls, uint64_t* keys,
-                                                          unsigned long long* n) {
-    __shared__ int64_t s_excl[kWarps][33];
-    __shared__ int32_t s_u[kWarps][32];
-    const int wib = threadIdx.x >> 5;
-    warp_sweep_rows(fw.beg, fw.deg, fw.adj, 0, V, s_excl[wib], s_u[wib], [&](int32_t u, int32_t w, int64_t) {
-        const int32_t a = cls[u], b = cls[w];
+__global__ void __launch_bounds__(kBlock) k_quotient_keys(int64_t V, const int64_t* off, CSRView fw, const int32_t* cls,
+                                                          uint64_t* keys, unsigned long long* n) {
+    walk_segments(off, V, [&](int64_t u, int64_t j) {
+        const int32_t a = cls[u], b = cls[fw.adj[fw.beg[u] + j]];
         if (a == b) return;
         const unsigned m = __activemask();  // (one atomic for the threads that are here together)
         const int leader = __ffs(m) - 1;
@@ -547,10 +542,12 @@ static int scc_by_quotient(gir_dev* g, int32_t* label, int64_t* n_scc, bool* use
     Temps t{g, {}};
     uint8_t* full = nullptr;
     int32_t *cls = nullptr, *mdeg = nullptr;
+    int64_t* off = nullptr;
     unsigned long long* cnt = nullptr;  // [0] full vertices, [1] union-find errors, [2] keys, [3] keys, [4] classes
     GIR_TRY(t.get(&full, V));
     GIR_TRY(t.get(&cls, V));
     GIR_TRY(t.get(&mdeg, V));
+    GIR_TRY(t.get(&off, V + 1));
     GIR_TRY(t.get(&cnt, 8));
     void* hp = nullptr;
     GIR_TRY(pinned(g, 256, &hp));
@@ -572,14 +569,16 @@ static int scc_by_quotient(gir_dev* g, int32_t* label, int64_t* n_scc, bool* use
     k_uf_first<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(sym, V, cls);
     GIR_LAUNCH(g, "k_uf_first");
     GIR_TRY(uf_flatten(g, cls, V));
-    k_class_link<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, sym, cls, cnt + 1);
+    GIR_TRY(scan_degrees(g, mdeg, V, off));
+    k_class_link<<<g->num_sms * 8, kBlock, 0, g->stream>>>(V, off, sym, cls, cnt + 1);
     GIR_LAUNCH(g, "k_class_link");
     GIR_TRY(uf_flatten(g, cls, V));
     // (an edge between classes has two ends that are not full)
     fw.deg = mdeg;
     k_mask_deg<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, g->fw.deg, full, 0, mdeg);
     GIR_LAUNCH(g, "k_mask_deg");
-    k_quotient_keys<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, fw, cls, nullptr, cnt + 2);
+    GIR_TRY(scan_degrees(g, mdeg, V, off));
+    k_quotient_keys<<<g->num_sms * 8, kBlock, 0, g->stream>>>(V, off, fw, cls, nullptr, cnt + 2);
     GIR_LAUNCH(g, "k_quotient_keys");
     GIR_TRY(read());
     if (hc[1]) return fail(g, GIR_ERR_TIMEOUT, "scc: union-find exceeded its retry bound");
@@ -592,7 +591,7 @@ static int scc_by_quotient(gir_dev* g, int32_t* label, int64_t* n_scc, bool* use
         GIR_TRY(t.get(&flip, n));
         GIR_TRY(t.get(&tmp, n));
         GIR_TRY(t.get(&flag, n));
-        k_quotient_keys<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, fw, cls, keys, cnt + 3);
+        k_quotient_keys<<<g->num_sms * 8, kBlock, 0, g->stream>>>(V, off, fw, cls, keys, cnt + 3);
         GIR_LAUNCH(g, "k_quotient_keys");
         GIR_TRY(sort_keys_u64(g, keys, tmp, n, edge_key_bits(g->V)));
         k_distinct_u64<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(keys, n, flag);

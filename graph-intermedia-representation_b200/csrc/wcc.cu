@@ -62,8 +62,8 @@ __global__ void k_uf_hook_first_two(CSRView c, int64_t V, int32_t* parent) {
     }
 }
 
-// Rows of the vertices outside the sampled giant root, one warp per 32
-// vertices as in warp_sweep_rows.
+// Rows of the vertices outside the sampled giant root: a warp takes 32 vertices, scans their row lengths and
+// walks the rows laid end to end, 32 entries at a time.
 __global__ void __launch_bounds__(kBlock) k_uf_link_rest(CSRView c, int64_t V, const int32_t* giant_p,
                                                          int32_t* parent, unsigned long long* err) {
     const int32_t giant = *giant_p;  // (-1: none)

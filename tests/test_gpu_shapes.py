@@ -107,3 +107,48 @@ def test_components_of_chains_of_every_length(pkg, orc):
     np.testing.assert_array_equal(d.labels(pkg.native.LABEL_WCC), np.repeat(end - length, length))
     assert d.counts()["n_wcc"] == len(length)
     d.close()
+
+
+def _kite(pkg, V, path, p):
+    """A hub with leaves, and a path hanging on it: deep, with one row that holds nearly every entry."""
+    leaf, tail = np.arange(1, V - path), np.arange(V - path, V)
+    return _both(pkg, V, p[np.r_[np.zeros(len(leaf), np.int64), 0, tail[:-1]]], p[np.r_[leaf, tail[0], tail[1:]]])
+
+
+@pytest.mark.parametrize("hub", ["root", "anywhere"])
+@pytest.mark.parametrize("layer", ["SCC", "BCT"])
+def test_builds_of_a_deep_graph_with_a_long_row(pkg, layer, hub):
+    """The ways for deep graphs (reciprocal classes, the forest by union-find) on a hub's row: no more than a few
+    times what the hub costs without the path."""
+    V = 600_000
+    p = np.arange(V) if hub == "root" else np.random.default_rng(3).permutation(V)
+    which = getattr(pkg.native, f"LAYER_{layer}")
+    deep, flat = (_build_ms(pkg, _kite(pkg, V, path, p), which) for path in (300, 2))
+    assert deep < 4 * flat + 2, (deep, flat)
+
+
+@pytest.mark.parametrize("one_way", [0.0, 0.02, 0.3])
+def test_layers_of_deep_graphs_with_hubs(pkg, orc, one_way):
+    """A long path with hubs on it (rows beyond a warp's run), whose leaves are tied to one another here and there;
+    some edges only one way, so that classes, quotient and forest all take part."""
+    from test_gpu_layers import _oracle_match
+    n, leaves = 400, 3000
+    rng = np.random.default_rng(int(100 * one_way))
+    a = np.arange(n - 1)
+    u, v = [a], [a + 1]
+    at = n
+    for hub in (0, 1, 150, n - 1):
+        mine = np.arange(at, at + leaves)
+        at += leaves
+        u += [np.full(leaves, hub), mine[:600:3]]
+        v += [mine, mine[1:600:3]]
+    u, v = np.concatenate(u), np.concatenate(v)
+    one = rng.random(len(u)) < one_way
+    perm = rng.permutation(at)
+    for p in (np.arange(at), perm):
+        g = _graph(pkg, at, p[np.r_[u, v[~one]]], p[np.r_[v, u[~one]]])
+        fb, fa = orc.normalize(at, g.fw_beg, g.fw_adj)
+        d = pkg.DeviceGraph.from_graph(g, weights=False)
+        d.build()
+        _oracle_match(pkg, orc, d, at, fb, fa, f"one way {one_way}")
+        d.close()
