@@ -730,7 +730,7 @@ int bct_build(gir_dev* g) {
             k_need_level<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(order + lvl_off[L], n, parent, uf, need);
             GIR_LAUNCH(g, "k_need_level");
         }
-        GIR_TRY(sample_mode(g, g->sym, uf, giant));
+        GIR_TRY(sample_mode(g, g->sym, uf, kModeSamples / 2, giant));
         k_sweep_len<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, hdeg, uf, need, giant, len);
         GIR_LAUNCH(g, "k_sweep_len");
     }

@@ -305,9 +305,10 @@ inline int edge_key_bits(int64_t V) {
     while (V >> n) ++n;
     return 32 + n;
 }
-// The value that most of 512 row slots of `c` hold in val[row] (slots drawn evenly, so rows weigh by their
-// length), into *out, or -1 where no value holds half of them. Device words throughout, no host read.
-int sample_mode(gir_dev* g, const DevCSR& c, const int32_t* val, int32_t* out);
+// The value that most of kModeSamples row slots of `c` hold in val[row] (slots drawn evenly, so rows weigh by
+// their length), into *out, or -1 where no value is in `least` of them. Device words throughout, no host read.
+constexpr int kModeSamples = 512;
+int sample_mode(gir_dev* g, const DevCSR& c, const int32_t* val, int least, int32_t* out);
 // Exclusive scan of the V row lengths into off (V + 1 entries).
 int scan_degrees(gir_dev* g, const int32_t* deg, int64_t V, int64_t* off);
 int sort_keys_u64(gir_dev* g, uint64_t* keys, uint64_t* tmp, int64_t n, int end_bit);

@@ -229,9 +229,8 @@ __global__ void k_heavy_lengths(const int32_t* deg, const int32_t* rows, int64_t
 }
 }  // namespace
 
-constexpr int kModeSamples = 512;
 __global__ void __launch_bounds__(kModeSamples) k_sample_mode(int64_t V, const int64_t* beg, const int32_t* val,
-                                                              int32_t* out) {
+                                                              int least, int32_t* out) {
     __shared__ int32_t s_val[kModeSamples];
     __shared__ unsigned long long s_best;
     const int i = threadIdx.x;
@@ -251,11 +250,11 @@ __global__ void __launch_bounds__(kModeSamples) k_sample_mode(int64_t V, const i
     for (int k = 0; k < kModeSamples; ++k) same += s_val[k] == s_val[i];
     atomicMax(&s_best, ((unsigned long long)same << 32) | (uint32_t)s_val[i]);
     __syncthreads();
-    if (i == 0) *out = (int)(s_best >> 32) * 2 >= kModeSamples ? (int32_t)(uint32_t)s_best : -1;
+    if (i == 0) *out = (int)(s_best >> 32) >= least ? (int32_t)(uint32_t)s_best : -1;
 }
 
-int sample_mode(gir_dev* g, const DevCSR& c, const int32_t* val, int32_t* out) {
-    k_sample_mode<<<1, kModeSamples, 0, g->stream>>>(g->V, c.beg, val, out);
+int sample_mode(gir_dev* g, const DevCSR& c, const int32_t* val, int least, int32_t* out) {
+    k_sample_mode<<<1, kModeSamples, 0, g->stream>>>(g->V, c.beg, val, least, out);
     GIR_LAUNCH(g, "k_sample_mode");
     return GIR_OK;
 }

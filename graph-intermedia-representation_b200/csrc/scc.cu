@@ -922,7 +922,7 @@ int scc_build_dag(gir_dev* g) {
     if (E > 0) {
         int32_t *len = nullptr, *giant = reinterpret_cast<int32_t*>(cnt + C_N);
         GIR_TRY(ensure_n(g, g->scratch[11], V + 1, &len));
-        GIR_TRY(sample_mode(g, g->fw, label, giant));
+        GIR_TRY(sample_mode(g, g->fw, label, kModeSamples / 2, giant));
         for (int back = 0; back < 2; ++back) {
             const DevCSR& c = back ? g->bw : g->fw;
             k_cross_len<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, c.deg, label, giant, back, len);

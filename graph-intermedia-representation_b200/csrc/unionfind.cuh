@@ -37,10 +37,12 @@ __device__ __forceinline__ int32_t uf_union(int32_t* uf, int32_t a, int32_t b, u
 
 // A loose join for sampling rounds over a flattened forest: the larger of the two entries (a root) goes
 // under the smaller unless it is under a still smaller one. No search and no retry, but where one root
-// meets several the least wins and the other joins are lost, so exactness must not depend on it.
-__device__ __forceinline__ void uf_hook(int32_t* uf, int32_t ra, int32_t rb) {
+// meets several the least wins and the other joins are lost, so exactness must not depend on it. Returns
+// whether the two differed.
+__device__ __forceinline__ bool uf_hook(int32_t* uf, int32_t ra, int32_t rb) {
     const int32_t lo = ra < rb ? ra : rb, hi = ra < rb ? rb : ra;
     if (lo != hi && uf[hi] > lo) atomicMin(&uf[hi], lo);
+    return lo != hi;
 }
 
 // Every entry to its root, run as a kernel of its own with no union meanwhile (uf_flatten). A thread writes
@@ -51,8 +53,9 @@ __device__ __forceinline__ void uf_hook(int32_t* uf, int32_t ra, int32_t rb) {
 // Every CTA is resident: an entry points at a smaller one, so whatever a walk meets is done or about to be
 // taken up. With more CTAs than fit, those of the first wave went on to their second vertices through entries
 // that no thread had started with, one step after another: 56 ms for a path of a million vertices in the order
-// of their ids (0.1 ms for the whole component build so).
-__global__ static void __launch_bounds__(256, 8) k_uf_flatten(int32_t* uf, int64_t V) {
+// of their ids (0.1 ms for the whole component build so). go (if given): nothing to do where it is zero.
+__global__ static void __launch_bounds__(256, 8) k_uf_flatten(int32_t* uf, int64_t V, const int32_t* go) {
+    if (go && *go == 0) return;
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x) {
         int32_t x = uf[v];
         int steps = 0;
@@ -62,11 +65,11 @@ __global__ static void __launch_bounds__(256, 8) k_uf_flatten(int32_t* uf, int64
         }
     }
 }
-inline int uf_flatten(gir_dev* g, int32_t* uf, int64_t V) {
+inline int uf_flatten(gir_dev* g, int32_t* uf, int64_t V, const int32_t* go = nullptr) {
     constexpr int kThreads = 256;
     if (V <= 0) return GIR_OK;
     const int64_t want = (V + kThreads - 1) / kThreads, fit = (int64_t)g->num_sms * 8;
-    k_uf_flatten<<<(int)(want < fit ? want : fit), kThreads, 0, g->stream>>>(uf, V);
+    k_uf_flatten<<<(int)(want < fit ? want : fit), kThreads, 0, g->stream>>>(uf, V, go);
     GIR_LAUNCH(g, "k_uf_flatten");
     return GIR_OK;
 }

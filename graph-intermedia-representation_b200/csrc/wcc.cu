@@ -41,32 +41,53 @@ __global__ void k_uf_compress(int32_t* parent, int64_t V, unsigned long long* ro
 }
 
 // Afforest-style sampling over the symmetric view (every pair in both rows): every vertex goes under its
-// first neighbour (k_uf_first), then twice the roots of every vertex and its first two neighbours are
+// first neighbour (k_uf_first), then in a few rounds the roots of every vertex and its first two neighbours are
 // joined loosely (uf_hook) and the forest flattened; the most frequent root among sampled row slots is
 // taken as the giant component's, and only the rows of vertices outside it are linked exactly. An edge
 // between a giant vertex and any other is in the other vertex's row too, so skipping the giant's rows
-// loses no link. A larger root always goes under a smaller one, so every root stays its component's
-// smallest vertex.
+// loses no link (whatever share of the graph that root has). A larger root always goes under a smaller one, so
+// every root stays its component's smallest vertex.
 // (Exact unions of the second neighbours, whose compare-and-swaps meet at few roots, took 120 us on
 // 65,536 vertices and 230 us on 4.8M; two loose rounds with their flattens 20 and 165 us.)
-constexpr int kHookRounds = 2;
+// The shorter the rows, the fewer trees a round joins, and the exact links that follow are the slower the fewer
+// roots they meet at. Below eight row entries a vertex on average four rounds (a 80^3 grid with its ids permuted
+// 0.50 -> 0.13 ms; random graphs of 4 to 7 entries are done after two and pay 0.03); below 3.5 a round leaves a
+// third of the trees, and exact unions of the first two neighbours come first (ladder, permuted ids 0.69 -> 0.15
+// ms, random graph of two entries a vertex 0.45 -> 0.21, where two rounds had made the build 1.5 to 6 times
+// slower than these).
+inline int hook_rounds(int64_t V, int64_t E) { return 2 * E < 7 * V ? 0 : (E < 8 * V ? 4 : 2); }
 
-__global__ void k_uf_hook_first_two(CSRView c, int64_t V, int32_t* parent) {
+__global__ void k_uf_link_first_two(CSRView c, int64_t V, int32_t* parent, unsigned long long* err) {
+    GRID_STRIDE(v, V) {
+        const int32_t d = c.deg[v];
+        if (d == 0) continue;
+        const int64_t b = c.beg[v];
+        uf_union(parent, (int32_t)v, c.adj[b], err);
+        if (d > 1) uf_union(parent, (int32_t)v, c.adj[b + 1], err);
+    }
+}
+
+// A round: sets *hooked where it found trees to join; `before`, the word of the round before, says whether there
+// is anything left to do (a lattice in the order of its ids is one tree after the first links).
+__global__ void k_uf_hook_first_two(CSRView c, int64_t V, int32_t* parent, const int32_t* before, int32_t* hooked) {
+    if (before && *before == 0) return;
+    bool any = false;
     GRID_STRIDE(v, V) {
         const int32_t d = c.deg[v];
         if (d == 0) continue;
         const int64_t b = c.beg[v];
         const int32_t r = parent[v];
-        uf_hook(parent, r, parent[c.adj[b]]);
-        if (d > 1) uf_hook(parent, r, parent[c.adj[b + 1]]);
+        any |= uf_hook(parent, r, parent[c.adj[b]]);
+        if (d > 1) any |= uf_hook(parent, r, parent[c.adj[b + 1]]);
     }
+    if (__syncthreads_or(any) && threadIdx.x == 0 && __ldcg(hooked) == 0) *hooked = 1;
 }
 
 // Rows of the vertices outside the sampled giant root: a warp takes 32 vertices, scans their row lengths and
 // walks the rows laid end to end, 32 entries at a time.
 __global__ void __launch_bounds__(kBlock) k_uf_link_rest(CSRView c, int64_t V, const int32_t* giant_p,
                                                          int32_t* parent, unsigned long long* err) {
-    const int32_t giant = *giant_p;  // (-1: none)
+    const int32_t giant = *giant_p;
     __shared__ int64_t s_excl[kBlock / 32][33];
     __shared__ int32_t s_u[kBlock / 32][32];
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -108,21 +129,29 @@ __global__ void __launch_bounds__(kBlock) k_uf_link_rest(CSRView c, int64_t V, c
 static int wcc_labels_sym(gir_dev* g, int32_t* label, int64_t* n_comp) {
     const int64_t V = g->V;
     unsigned long long *roots = nullptr, *err = nullptr;
-    GIR_TRY(ensure_n(g, g->scratch[14], 4, &roots));
+    GIR_TRY(ensure_n(g, g->scratch[14], 5, &roots));
     err = roots + 1;
     int32_t* giant = reinterpret_cast<int32_t*>(roots + 2);
-    GIR_CUDA(g, cudaMemsetAsync(roots, 0, 2 * sizeof(unsigned long long), g->stream));
+    int32_t* hooked = giant + 1;  // a word per round
+    GIR_CUDA(g, cudaMemsetAsync(roots, 0, 5 * sizeof(unsigned long long), g->stream));
     if (V == 0) { *n_comp = 0; return GIR_OK; }
     const CSRView s = view(g->sym);
     k_uf_first<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(s, V, label);
     GIR_LAUNCH(g, "k_uf_first");
     GIR_TRY(uf_flatten(g, label, V));
-    for (int r = 0; r < kHookRounds; ++r) {
-        k_uf_hook_first_two<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(s, V, label);
-        GIR_LAUNCH(g, "k_uf_hook_first_two");
+    const int rounds = hook_rounds(V, g->sym.E);
+    if (rounds == 0) {
+        k_uf_link_first_two<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(s, V, label, err);
+        GIR_LAUNCH(g, "k_uf_link_first_two");
         GIR_TRY(uf_flatten(g, label, V));
     }
-    GIR_TRY(sample_mode(g, g->sym, label, giant));
+    for (int r = 0; r < rounds; ++r) {
+        k_uf_hook_first_two<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(s, V, label, r > 0 ? hooked + r - 1 : nullptr,
+                                                                             hooked + r);
+        GIR_LAUNCH(g, "k_uf_hook_first_two");
+        GIR_TRY(uf_flatten(g, label, V, hooked + r));
+    }
+    GIR_TRY(sample_mode(g, g->sym, label, 1, giant));
     trace_mark(g, "wcc: neighbour rounds + sample");
     k_uf_link_rest<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(s, V, giant, label, err);
     GIR_LAUNCH(g, "k_uf_link_rest");

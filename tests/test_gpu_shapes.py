@@ -152,3 +152,46 @@ def test_layers_of_deep_graphs_with_hubs(pkg, orc, one_way):
         d.build()
         _oracle_match(pkg, orc, d, at, fb, fa, f"one way {one_way}")
         d.close()
+
+
+def _ladder(n):
+    a, b = np.arange(n - 1), np.arange(n)
+    return 2 * n, np.r_[a, a + n, b], np.r_[a + 1, a + n + 1, b + n]
+
+
+def _grid3(s):
+    at = np.arange(s**3).reshape(s, s, s)
+    return s**3, np.r_[at[1:].ravel(), at[:, 1:].ravel(), at[:, :, 1:].ravel()], np.r_[
+        at[:-1].ravel(), at[:, :-1].ravel(), at[:, :, :-1].ravel()]
+
+
+@pytest.mark.parametrize("shape", [lambda: _ladder(300_000), lambda: _grid3(80)], ids=["ladder", "grid"])
+def test_components_of_short_rows_in_any_order(pkg, shape):
+    """Rows of three and of six entries, ids in order (one tree after the first links) and permuted (many): the
+    exact links that are left must not meet at a few roots."""
+    V, u, v = shape()
+    perm = np.random.default_rng(2).permutation(V)
+    order, mixed = (_build_ms(pkg, _both(pkg, V, p[u], p[v]), pkg.native.LAYER_WCC, 9) for p in (np.arange(V), perm))
+    assert mixed < 4 * order + 0.1, (mixed, order)
+
+
+@pytest.mark.parametrize("V,entries", [(5, 1), (300, 1), (300, 3), (20_000, 1), (20_000, 2), (20_000, 3.4), (20_000, 3.6),
+                                       (20_000, 5), (20_000, 7.9), (20_000, 8.1), (20_000, 14), (200_000, 2.2), (200_000, 6)])
+def test_components_at_every_row_length(pkg, orc, V, entries):
+    """About the average row lengths at which the sampling changes, with equal halves, isolated vertices and small
+    components beside: the smallest vertex of every component, against the oracle."""
+    rng = np.random.default_rng(int(10 * entries) + V)
+    m = int(V * entries / 2)
+    u, v = rng.integers(0, V, m), rng.integers(0, V, m)
+    for part in (False, True):
+        if part:  # two halves and a rest of small pieces
+            piece = np.minimum(u * 5 // (2 * V), 2)
+            v = np.where(piece < 2, piece * (2 * V // 5) + v % (2 * V // 5), np.minimum(u + v % 3, V - 1))
+        g = _graph(pkg, V, u[u != v], v[u != v])
+        fb, fa = orc.normalize(V, g.fw_beg, g.fw_adj)
+        d = pkg.DeviceGraph.from_graph(g, weights=False)
+        d.build(pkg.native.LAYER_WCC)
+        exp = orc.canon_labels(orc.wcc(V, fb, fa))
+        np.testing.assert_array_equal(d.labels(pkg.native.LABEL_WCC), exp)
+        assert d.counts()["n_wcc"] == len(np.unique(exp))
+        d.close()
