@@ -583,6 +583,16 @@ int bfs_run(gir_dev* g, const int64_t* set_beg_h, const int32_t* srcs_d, int64_t
         if (coop && per_sm > 0) persist_grid = g->num_sms;
     }
     const bool learned = g->schedule == GIR_SCHEDULE_LEARNED && g->sched_loaded && V >= 4096;
+    // Bit planes, for the groups of lanes that want them (the first group is the widest). Decided once a call:
+    // an allocation that fails has synchronized the stream and trimmed the pool by then.
+    auto wants_planes = [&](int64_t lanes) { return lanes >= kPlaneMinLanes && lanes * V >= kPlaneMinPairs; };
+    unsigned long long* plane = nullptr;
+    if (wants_planes(std::min<int64_t>(n_sets, 64)) && set_beg_h[n_sets] > set_beg_h[0]) {
+        const std::string err = g->err;
+        const int rc = ensure_n(g, g->scratch[12], 4 * V, &plane);
+        if (rc == GIR_ERR_OOM) g->err = err;  // (the straight writes need no memory: not this call's error)
+        else GIR_TRY(rc);
+    }
     std::vector<double> trace_rows;
     MainTimer timer{g, g->params[GIR_PARAM_PROFILE] != 0.0};
     GIR_CUDA(g, cudaEventRecord(g->ev0, g->stream));
@@ -596,11 +606,7 @@ int bfs_run(gir_dev* g, const int64_t* set_beg_h, const int32_t* srcs_d, int64_t
         GIR_CUDA(g, cudaMemsetAsync(ctl, 0, sizeof(unsigned long long) * kCtlTrace, g->stream));
         GIR_CUDA(g, cudaMemcpyAsync(sbeg, set_beg_h + g0, sizeof(int64_t) * (nl + 1), cudaMemcpyHostToDevice, g->stream));
         const int64_t n_entries = set_beg_h[g0 + nl] - set_beg_h[g0];
-        if (n_entries > 0 && nl >= kPlaneMinLanes && (int64_t)nl * V >= kPlaneMinPairs) {
-            const int rc = ensure_n(g, g->scratch[12], 4 * V, &level.plane);
-            if (rc == GIR_ERR_OOM) level.plane = nullptr;  // (the straight writes need no memory)
-            else GIR_TRY(rc);
-        }
+        if (n_entries > 0 && wants_planes(nl)) level.plane = plane;
         if (level.plane) {
             GIR_CUDA(g, cudaMemsetAsync(level.plane, 0, sizeof(uint64_t) * 4 * V, g->stream));
         } else {

@@ -24,7 +24,12 @@ int dev_alloc(gir_dev* g, void** p, size_t bytes) {
     *p = nullptr;
     const size_t want = ((bytes < 256 ? 256 : bytes) + 255) & ~(size_t)255;
     const double t0 = g->trace_on ? now_ms() : 0.0;
-    cudaError_t e = cudaMallocFromPoolAsync(p, want, g->pool, g->stream);
+    const double limit = g->params[GIR_PARAM_ALLOC_LIMIT];
+    auto take = [&]() {
+        return limit > 0 && (double)want > limit ? cudaErrorMemoryAllocation
+                                                 : cudaMallocFromPoolAsync(p, want, g->pool, g->stream);
+    };
+    cudaError_t e = take();
     if (e == cudaErrorMemoryAllocation) {
         if (g->trace_on) std::fprintf(stderr, "[gir] pool exhausted at %zu bytes: trimming\n", want);
         // The pool keeps freed blocks for reuse; when none fits, give its unused memory back to
@@ -32,7 +37,7 @@ int dev_alloc(gir_dev* g, void** p, size_t bytes) {
         cudaGetLastError();
         cudaStreamSynchronize(g->stream);
         cudaMemPoolTrimTo(g->pool, 0);
-        e = cudaMallocFromPoolAsync(p, want, g->pool, g->stream);
+        e = take();
     }
     if (g->trace_on && now_ms() - t0 > 1.0)
         std::fprintf(stderr, "[gir] pool allocation of %zu bytes took %.3f ms\n", want, now_ms() - t0);

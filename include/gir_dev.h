@@ -255,7 +255,9 @@ enum {
                                    and a group that meets a longer distance is rerun wider */
     GIR_PARAM_LANE_ORDER = 10,  /* SSSP lanes: 1 ordered by the sources' distance to the largest-in-degree
                                    vertex (lanes active in the same buckets share sectors), 0 query order */
-    GIR_PARAM_COUNT = 11
+    GIR_PARAM_ALLOC_LIMIT = 11, /* bytes: a later device allocation of the handle that is larger fails as it does
+                                   when device memory has run out; 0 no limit */
+    GIR_PARAM_COUNT = 12
 };
 int gir_dev_set_param(gir_dev_t* g, int which, double value);
 int gir_dev_get_param(gir_dev_t* g, int which, double* value);

@@ -67,3 +67,50 @@ def test_backward_rows_that_do_not_match(pkg, insert, n):
     for x, y in zip(d.csr(1), before):
         np.testing.assert_array_equal(x, y)
     d.close()
+
+
+@pytest.mark.parametrize("lanes", [64, 65, 130])
+def test_bfs_without_memory_for_the_bit_planes(pkg, orc, monkeypatch, capfd, lanes):
+    """The planes' 32 bytes a vertex cannot be had: the levels are written straight to the output, the call leaves
+    no error text, and it asks for the memory once, not once a group of 64 lanes."""
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("GIR_TRACE", "2")  # (failed allocations on stderr; read when a handle is made)
+    V = 140_000
+    rng = np.random.default_rng(lanes)
+    tail = np.arange(V - 40, V)  # more levels than the planes hold
+    u, v = np.r_[rng.integers(0, V - 60, 3 * V), 5, tail[:-1]], np.r_[rng.integers(0, V - 60, 3 * V), tail[0], tail[1:]]
+    key = np.unique(u[u != v] * V + v[u != v])
+    g = pkg.graphs.from_edges(V, key // V, key % V)
+    fb, fa = orc.normalize(V, g.fw_beg, g.fw_adj)
+    src = rng.integers(0, V - 60, lanes).astype(np.int32)
+    src[3] = -1
+    out = [torch.full((lanes, V), 7, dtype=torch.int32, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    failed = []
+    for limit, res in zip((0, 31 * V), out):
+        d = pkg.DeviceGraph.from_graph(g, weights=False)
+        d.set_param(pkg.native.PARAM_ALLOC_LIMIT, limit)
+        capfd.readouterr()
+        d.bfs(src, out=res)
+        failed.append(capfd.readouterr().err.count("pool exhausted"))
+        assert pkg.native.dev_lib().gir_dev_last_error(d.handle) == b""
+        d.close()
+    assert failed == [0, 1]
+    got = out[0].cpu().numpy()
+    np.testing.assert_array_equal(out[1].cpu().numpy(), got)
+    for i in (0, 3, lanes - 1):
+        np.testing.assert_array_equal(got[i], orc.bfs(V, fb, fa, [int(src[i])]) if src[i] >= 0 else np.full(V, -1))
+
+
+def test_allocation_limit_is_an_error_where_memory_is_needed(pkg):
+    g = pkg.graphs.rmat(12, seed=4)
+    d = pkg.DeviceGraph.from_graph(g, weights=False)
+    with pytest.raises(pkg.GirError):
+        d.set_param(pkg.native.PARAM_ALLOC_LIMIT, -1)
+    d.set_param(pkg.native.PARAM_ALLOC_LIMIT, 4096)
+    with pytest.raises(pkg.GirError) as e:
+        d.bfs(np.zeros(1, np.int32))
+    assert e.value.code == 3
+    d.set_param(pkg.native.PARAM_ALLOC_LIMIT, 0)
+    assert d.bfs(np.zeros(1, np.int32))[0, 0] == 0
+    d.close()
