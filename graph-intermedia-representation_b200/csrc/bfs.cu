@@ -577,10 +577,9 @@ int bfs_run(gir_dev* g, const int64_t* set_beg_h, const int32_t* srcs_d, int64_t
     // persistent levels (the device must take cooperative launches)
     int persist_grid = 0;
     {
-        int coop = 0, per_sm = 0;
-        GIR_CUDA(g, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, g->device));
-        GIR_CUDA(g, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bfs_persistent, kPersistThreads, 0));
-        if (coop && per_sm > 0) persist_grid = g->num_sms;
+        int per_sm = 0;
+        GIR_TRY(cooperative_ctas(g, (const void*)k_bfs_persistent, kPersistThreads, &per_sm));
+        if (per_sm > 0) persist_grid = g->num_sms;
     }
     const bool learned = g->schedule == GIR_SCHEDULE_LEARNED && g->sched_loaded && V >= 4096;
     // Bit planes, for the groups of lanes that want them (the first group is the widest). Decided once a call:

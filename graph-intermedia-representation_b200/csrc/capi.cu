@@ -1156,8 +1156,8 @@ int gir_dev_set_param(gir_dev_t* g, int which, double value) {
     } else if (which == GIR_PARAM_LANE_BITS) {
         if (!(value == 0.0 || value == 16.0 || value == 32.0 || value == 64.0))
             return fail(g, GIR_ERR_INVALID, "lane bits: 0 (the library decides), 16, 32 or 64");
-    } else if (which == GIR_PARAM_LANE_ORDER) {
-        if (!(value == 0.0 || value == 1.0)) return fail(g, GIR_ERR_INVALID, "lane order: 0 or 1");
+    } else if (which == GIR_PARAM_LANE_ORDER || which == GIR_PARAM_COOPERATIVE) {
+        if (!(value == 0.0 || value == 1.0)) return fail(g, GIR_ERR_INVALID, "lane order, cooperative launches: 0 or 1");
     } else if (which == GIR_PARAM_ALLOC_LIMIT) {
         if (!(value >= 0.0)) return fail(g, GIR_ERR_INVALID, "allocation limit: bytes, 0 for none");
     } else if (!(value > 0) && which != GIR_PARAM_PROFILE) {

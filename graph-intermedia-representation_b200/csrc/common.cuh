@@ -172,7 +172,7 @@ struct gir_dev {
 
     // Schedule
     int schedule = GIR_SCHEDULE_FIXED;
-    double params[GIR_PARAM_COUNT] = {15.0, 18.0, 16.0, 256.0, 32.0, 4096.0, 4.0, 0.0, -1.0, 0.0, 1.0, 0.0};
+    double params[GIR_PARAM_COUNT] = {15.0, 18.0, 16.0, 256.0, 32.0, 4096.0, 4.0, 0.0, -1.0, 0.0, 1.0, 0.0, 1.0};
     cudaEvent_t pev0 = nullptr, pev1 = nullptr;  // main-kernel timing (GIR_PARAM_PROFILE)
     gir::DevBuf sched_w;              // MLP parameters (fp32)
     gir::DevBuf sched_io;             // one decision's features and logits
@@ -236,6 +236,11 @@ constexpr size_t kKeepScratchBelow = 64u << 20;
 // valid across calls that ask for no more).
 constexpr size_t kPinnedBytes = 4096;
 int pinned(gir_dev* g, size_t bytes, void** out);
+
+// CTAs of `threads` threads of `kernel` that an SM holds in a cooperative launch; 0 where the handle's device
+// does not take such launches, the kernel does not fit, or GIR_PARAM_COOPERATIVE is off: the caller then
+// launches its levels one by one.
+int cooperative_ctas(gir_dev* g, const void* kernel, int threads, int* per_sm);
 
 bool is_device_ptr(const void* p);
 

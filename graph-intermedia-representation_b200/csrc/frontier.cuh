@@ -383,12 +383,21 @@ int run_frontier(gir_dev* g, Op op, const BottomUp& bu, Queue q, unsigned long l
     void* hp = nullptr;
     GIR_TRY(pinned(g, kPinnedBytes, &hp));
     unsigned long long* hc = static_cast<unsigned long long*>(hp);
+    int loop_ctas = 0;
+    GIR_TRY(cooperative_ctas(g, (const void*)k_frontier_loop<Op>, kLoopThreads, &loop_ctas));
+    if (loop_ctas == 0 && !r.started) {  // (every level is launched from here: the first frontier's size is read)
+        GIR_CUDA(g, cudaMemcpyAsync(hc, ctl + W_Q, sizeof(unsigned long long), cudaMemcpyDeviceToHost, g->stream));
+        GIR_CUDA(g, cudaStreamSynchronize(g->stream));
+        r.packed = hc[0];
+        r.levels.push_back((int64_t)(r.packed >> kQShift));
+        r.started = true;
+    }
     while (max_levels > 0 && !r.done()) {
         const int64_t nq = (int64_t)(r.packed >> kQShift), total = (int64_t)(r.packed & kQEdges);
-        if (r.started && total > kLoopMaxEdges) {
+        if (r.started && (total > kLoopMaxEdges || loop_ctas == 0)) {
             GIR_CUDA(g, cudaMemsetAsync(ctl + W_SLOTS, 0, sizeof(unsigned long long), g->stream));
             const Queue in{q.v + r.lo, q.off + r.lo}, out{q.v + r.lo + nq, q.off + r.lo + nq};
-            if (bu.wants(total, r.lo + nq)) {
+            if (total > kLoopMaxEdges && bu.wants(total, r.lo + nq)) {
                 GIR_TRY(bu.launch(g, in, nq, out, ctl + W_SLOTS));
             } else {
                 k_frontier_level<Op><<<g->num_sms * 8, kLevelThreads, 0, g->stream>>>(op, in, nq, total, out, ctl + W_SLOTS);

@@ -101,6 +101,15 @@ int pinned(gir_dev* g, size_t bytes, void** out) {
     return GIR_OK;
 }
 
+int cooperative_ctas(gir_dev* g, const void* kernel, int threads, int* per_sm) {
+    int coop = 0;
+    *per_sm = 0;
+    if (g->params[GIR_PARAM_COOPERATIVE] == 0.0) return GIR_OK;
+    GIR_CUDA(g, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, g->device));
+    if (coop) GIR_CUDA(g, cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, threads, 0));
+    return GIR_OK;
+}
+
 bool is_device_ptr(const void* p) {
     if (!p) return false;
     cudaPointerAttributes a;

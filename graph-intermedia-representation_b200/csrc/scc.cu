@@ -389,8 +389,10 @@ __global__ void k_distinct_u64(const uint64_t* keys, int64_t n, uint8_t* flag) {
 // only raises take an atomic (no hot counter: a node with many in-edges, like the giant SCC, is raised a
 // few times, not decremented once per edge as in Kahn's algorithm).
 // ctl: [0..2] raises of a round (in turn), [3] error, [5] raises of the last round, [6] the largest level
-// raised to (a round may carry a level far); the barrier's counter from word 16 on.
+// raised to (a round may carry a level far); the barrier's counter from word 16 on. Without kLoop one round,
+// for an ordinary launch: its raises are in [0].
 constexpr int kDagWords = 32;
+template <bool kLoop>
 __global__ void __launch_bounds__(kLoopThreads, 2) k_dag_levels(const uint64_t* keys, int64_t n, int32_t* level,
                                                                 unsigned long long* ctl, int max_rounds) {
     unsigned int* bar = reinterpret_cast<unsigned int*>(ctl + 16);
@@ -412,6 +414,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_dag_levels(const uint64_t* 
         }
         c = warp_sum_u64(c);
         if (lane_id() == 0 && c) atomicAdd(&ctl[round % 3], c);
+        if (!kLoop) break;
         if (!grid_barrier(bar, ctl + 3, kLoopSpins, met)) return;
         raised = __ldcg(ctl + round % 3);
         ++round;
@@ -419,7 +422,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_dag_levels(const uint64_t* 
     }
     top = __reduce_max_sync(0xffffffffu, top);
     if (lane_id() == 0 && top) atomicMax(&ctl[6], (unsigned long long)top);
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctl[5] = raised;
+    if (kLoop && blockIdx.x == 0 && threadIdx.x == 0) ctl[5] = raised;
 }
 
 // Keys (level << vb | label) of the SCCs, vb the bits of a vertex id.
@@ -960,21 +963,26 @@ int scc_build_dag(gir_dev* g) {
     if (n_dag > 0) {
         unsigned long long* ctl = nullptr;
         GIR_TRY(ensure_n(g, g->scratch[10], kDagWords, &ctl));
-        int per_sm = 1;
-        GIR_CUDA(g, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dag_levels, kLoopThreads, 0));
+        int per_sm = 0;
+        GIR_TRY(cooperative_ctas(g, (const void*)k_dag_levels<true>, kLoopThreads, &per_sm));
         while (true) {
             GIR_CUDA(g, cudaMemsetAsync(ctl, 0, sizeof(unsigned long long) * kDagWords, g->stream));
             int max_rounds = 1 << 22;  // (the barrier's counter is 32 bits wide)
             const uint64_t* dag_c = dag;
             int64_t n_c = n_dag;
             void* args[] = {&dag_c, &n_c, &level, &ctl, &max_rounds};
-            GIR_CUDA(g, cudaLaunchCooperativeKernel((const void*)k_dag_levels, g->num_sms * (per_sm > 1 ? 2 : 1),
-                                                    kLoopThreads, args, 0, g->stream));
+            if (per_sm > 0) {
+                GIR_CUDA(g, cudaLaunchCooperativeKernel((const void*)k_dag_levels<true>, g->num_sms * (per_sm > 1 ? 2 : 1),
+                                                        kLoopThreads, args, 0, g->stream));
+            } else {
+                k_dag_levels<false><<<grid_for(g, n_dag, kLoopThreads), kLoopThreads, 0, g->stream>>>(dag_c, n_c, level, ctl, 1);
+                GIR_LAUNCH(g, "k_dag_levels");
+            }
             GIR_CUDA(g, cudaMemcpyAsync(hc, ctl, sizeof(unsigned long long) * 7, cudaMemcpyDeviceToHost, g->stream));
             GIR_CUDA(g, cudaStreamSynchronize(g->stream));
             if (hc[3]) return fail(g, GIR_ERR_TIMEOUT, "scc: a grid barrier of the DAG levels ran out its bound");
             top = (int64_t)hc[6] > top ? (int64_t)hc[6] : top;
-            if (hc[5] == 0) break;
+            if (hc[per_sm > 0 ? 5 : 0] == 0) break;
         }
     }
     trace_mark(g, "scc: levels");

@@ -1026,7 +1026,10 @@ int sssp_group(gir_dev* g, Work& wk, const DevCSR& ws, int nl, const int64_t* la
         GIR_CUDA(g, cudaStreamSynchronize(g->stream));
         return GIR_OK;
     };
-    bool fresh = true;  // the first phase's size was not read: the loop looks at it
+    int loop_ctas = 0;  // (0: every phase is launched from here)
+    GIR_TRY(cooperative_ctas(g, (const void*)k_bucket_loop<D>, kLoopThreads, &loop_ctas));
+    bool fresh = loop_ctas > 0;  // the first phase's size was not read: the loop looks at it
+    if (!fresh) GIR_TRY(read());
     while (b.phase != PH_DONE) {
         int64_t edges = 0, entries = 0;
         if (!fresh) {
@@ -1035,7 +1038,7 @@ int sssp_group(gir_dev* g, Work& wk, const DevCSR& ws, int nl, const int64_t* la
             edges = (int64_t)(packed & kQEdges);
             entries = b.phase == PH_SPLIT ? (int64_t)hc[X_FAR + b.spl] : (int64_t)(packed >> kQShift);
         }
-        if (fresh || (edges <= kLoopMaxRelax && (b.phase != PH_SPLIT || entries <= kLoopMaxFar))) {
+        if (fresh || (loop_ctas > 0 && edges <= kLoopMaxRelax && (b.phase != PH_SPLIT || entries <= kLoopMaxFar))) {
             if (!fresh) {
                 hc[X_PHASE] = (unsigned long long)b.phase;
                 hc[X_ROT] = (unsigned long long)b.rot;

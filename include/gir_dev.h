@@ -257,7 +257,10 @@ enum {
                                    vertex (lanes active in the same buckets share sectors), 0 query order */
     GIR_PARAM_ALLOC_LIMIT = 11, /* bytes: a later device allocation of the handle that is larger fails as it does
                                    when device memory has run out; 0 no limit */
-    GIR_PARAM_COUNT = 12
+    GIR_PARAM_COOPERATIVE = 12, /* 1: frontier and bucket loops (BFS, SSSP, the layer builds) run level after level
+                                   in cooperative launches, where the device takes them; 0: every level and
+                                   phase is launched from the host (the results are the same) */
+    GIR_PARAM_COUNT = 13
 };
 int gir_dev_set_param(gir_dev_t* g, int which, double value);
 int gir_dev_get_param(gir_dev_t* g, int which, double* value);

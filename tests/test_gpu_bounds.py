@@ -114,3 +114,80 @@ def test_allocation_limit_is_an_error_where_memory_is_needed(pkg):
     d.set_param(pkg.native.PARAM_ALLOC_LIMIT, 0)
     assert d.bfs(np.zeros(1, np.int32))[0, 0] == 0
     d.close()
+
+
+def _host_level_graphs(pkg):
+    """Power-law, deep (past the builds' level limits), a deep DAG, one-way streets, nothing at all."""
+    from test_gpu_kernel_edges import _deep_shapes
+    rng = np.random.default_rng(6)
+    yield "rmat", pkg.graphs.rmat(13, seed=5)
+    for name, V, u, v in _deep_shapes():
+        if name in ("path 66", "path 700", "one-way, long range, loops", "joined paths"):
+            keep = (u != v) | ("loops" in name)
+            yield name, _weighted(pkg, V, u[keep], v[keep], rng.integers(1, 90, int(keep.sum())))
+    u = np.arange(5999)
+    far = rng.integers(0, 6000, (2, 4000))
+    far = far[:, far[0] != far[1]]
+    yield "dag", _weighted(pkg, 6000, np.r_[u[::2], np.minimum(*far)], np.r_[u[::2] + 1, np.maximum(*far)],
+                           rng.integers(1, 90, len(u[::2]) + far.shape[1]))
+    yield "empty", _weighted(pkg, 300, np.zeros(0, np.int64), np.zeros(0, np.int64), np.zeros(0))
+
+
+@pytest.mark.parametrize("learned", [False, True])
+def test_levels_and_phases_launched_from_the_host(pkg, orc, learned):
+    """Where a device takes no cooperative launches every BFS level, SSSP phase, build level and round of the DAG's
+    levels is a launch of its own: the same results, before and after a batch."""
+    from test_gpu_layers import _oracle_match
+    for name, g in _host_level_graphs(pkg):
+        V = g.V
+        fb, fa = orc.normalize(V, g.fw_beg, g.fw_adj)
+        d = pkg.DeviceGraph.from_graph(g)
+        d.set_param(pkg.native.PARAM_COOPERATIVE, 0)
+        if learned:
+            d.use_learned_schedule()
+        rng = np.random.default_rng(V)
+        weights = g.w
+        for step in range(2):
+            d.build()
+            _oracle_match(pkg, orc, d, V, fb, fa, f"{name}, step {step}")
+            for lanes in (1, 9, 65):
+                src = rng.integers(0, V, lanes).astype(np.int32)
+                src[-1] = -1 if lanes > 1 else src[0]
+                exp = np.stack([orc.bfs(V, fb, fa, [int(s)]) if s >= 0 else np.full(V, -1) for s in src])
+                np.testing.assert_array_equal(d.bfs(src), exp, err_msg=name)
+                st = d.query_stats()
+                assert st["persistent_levels"] == 0 and st["reached"] == (exp >= 0).sum()
+                for mode, w in ((pkg.native.WEIGHT_HASH, None), (pkg.native.WEIGHT_STORED, weights)):
+                    if w is None and mode == pkg.native.WEIGHT_STORED:
+                        continue
+                    got = d.sssp(src, delta=20, weights=mode)
+                    for i in {0, lanes // 2, lanes - 1}:
+                        e = orc.sssp(V, fb, fa, [int(src[i])], w=w) if src[i] >= 0 else np.full(V, 2**64 - 1, np.uint64)
+                        np.testing.assert_array_equal(got[i], e, err_msg=name)
+            if step == 0 and V > 1000:
+                a, b = rng.integers(0, V, 60).astype(np.int32), rng.integers(0, V, 60).astype(np.int32)
+                rows = np.repeat(np.arange(V), np.diff(fb))
+                at = rng.integers(0, len(fa), 30)
+                a[:30], b[:30] = rows[at], fa[at]
+                ins = (np.arange(60) >= 30).astype(np.uint8)
+                d.apply_batch(a, b, ins)
+                fb, fa, _, _ = orc.apply_batch(V, fb, fa, a, b, ins)
+                weights = None
+        d.close()
+
+
+def test_large_levels_without_cooperative_launches(pkg):
+    """Levels of over 2^22 row entries and passes of over 2^18 edges, which leave the loops where there are any: the
+    results of the loops."""
+    g = pkg.graphs.rmat(18, n_draws=24 << 18, seed=9)
+    src = np.flatnonzero(np.diff(g.fw_beg))[:: 3000][:40].astype(np.int32)
+    got = []
+    for coop in (1, 0):
+        d = pkg.DeviceGraph.from_graph(g)
+        d.set_param(pkg.native.PARAM_COOPERATIVE, coop)
+        d.build()
+        got.append([d.labels(k) for k in range(5)] + list(d.blocks()) + list(d.dag()) + [d.bfs(src), d.sssp(src)])
+        assert (d.query_stats()["launches"] > 0) and d.get_param(pkg.native.PARAM_COOPERATIVE) == coop
+        d.close()
+    for x, y in zip(*got):
+        np.testing.assert_array_equal(x, y)
