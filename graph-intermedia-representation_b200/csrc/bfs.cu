@@ -345,7 +345,6 @@ constexpr int64_t kPersistBuMaxV = 1ll << 20;     // vertices of a graph whose b
 constexpr int kPersistMaxLevels = 1 << 23;        // of one launch (its barrier's counter is 32 bits wide)
 constexpr int kPersistTrace = 8192;               // schedule decisions recorded per launch
 constexpr int kPersistTraceEager = 64;            // ... of which this many are read with the counters
-constexpr unsigned kBarrierSpins = 1u << 23;      // bounded barrier wait (a few seconds)
 
 // Device words of one call: the host levels' counters (C_*), the launch's control words, its counter
 // slots (one per level, reused every third level), the barrier's counter on its own 128-byte line,
@@ -448,7 +447,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_bfs_persistent(PersistAr
         }
         block_publish<kPersistWarps>(sh, acc.s_buf, acc.n, qb, RowLen{a.fw.deg}, &sl[S_Q], acc.pairs, acc.medges,
                                      &sl[S_PAIRS]);
-        if (!grid_barrier(bar, err, kBarrierSpins, met)) break;
+        if (!grid_barrier(bar, err, met)) break;
         n_last = nq;
         packed = ldcg_u64(&sl[S_Q]);
         pr = ldcg_u64(&sl[S_PAIRS]);

@@ -532,10 +532,12 @@ __device__ __forceinline__ void walk_rows_of(const int64_t* off, int64_t V, cons
 // 128-byte line, zeroed by the host before the launch; arrivals only count up, so a CTA waits until the
 // counter reaches the end of its round (`round`: the barriers passed so far, the same in every CTA). One
 // release reduction without a result and acquire polls: no reset, no second word, no wait for the
-// atomic's return. The wait is bounded: after `spins_max` polls a CTA sets *err and leaves; every CTA
-// also leaves once it sees *err set. Returns false once any CTA has flagged an error.
-__device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned long long* err, unsigned spins_max,
-                                             unsigned& round) {
+// atomic's return. The wait is bounded: after kBarrierSpins polls a CTA sets *err and leaves; every CTA
+// also leaves once it sees *err set. Returns false once any CTA has flagged an error. A poll takes 195 ns (one
+// thread of each of 148 CTAs), so the bound is 13 s; with polls that slept 64 ns in between, 260 ns each, it had
+// been 8.7.
+constexpr unsigned kBarrierSpins = 1u << 26;
+__device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned long long* err, unsigned& round) {
     ++round;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -545,7 +547,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned long lo
         while (true) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(bar) : "memory");
             if ((int)(now - end) >= 0) break;
-            if (++spins > spins_max) {
+            if (++spins > kBarrierSpins) {
                 atomicExch(err, 1ull);
                 break;
             }

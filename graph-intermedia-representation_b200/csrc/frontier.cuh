@@ -246,7 +246,6 @@ __device__ __forceinline__ void walk_level(const Queue& q, int64_t nq, int64_t t
 // Every level's queue follows the one before it in one pair of arrays, so these have to hold every
 // entry ever queued.
 constexpr int kLoopThreads = 1024;
-constexpr unsigned kLoopSpins = 1u << 23;  // bounded barrier wait (a few seconds)
 enum { W_Q = 0, W_LO = 1, W_LEVELS = 2, W_ERR = 3, W_SLOTS = 4, W_BAR = 16, W_LVL = 32 };
 constexpr int kLoopLevels = 64;                        // the most levels of a launch (their sizes go to W_LVL)
 constexpr int kLoopWords = W_LVL + kLoopLevels + 1;    // device words
@@ -277,7 +276,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_frontier_loop(Op op, Queue 
         int n_st = 0;
         walk_level(in, nq, total, warp, nwarps, op, out, sl, s_stage[wib], n_st);
         block_publish<32>(sh, s_stage[wib], n_st, out, [&](int32_t x) { return op.deg(x); }, sl);
-        if (!grid_barrier(bar, ctl + W_ERR, kLoopSpins, met)) break;
+        if (!grid_barrier(bar, ctl + W_ERR, met)) break;
         lo += nq;
         packed = __ldcg(sl);
         if (blockIdx.x == 0 && threadIdx.x == 0) ctl[W_LVL + 1 + lev] = packed;

@@ -98,7 +98,6 @@ __global__ void k_inc_dist(const uint64_t* st, int64_t V, uint64_t* out) {
 // before the barrier that opened level k, so one barrier per level suffices. Data other CTAs
 // write during the launch is read through L2 (ld.cg).
 constexpr int kIncThreads = 256;
-constexpr unsigned kIncSpins = 1u << 25;  // bounded barrier wait (a few seconds)
 enum { I_ERR = 0, I_CUTC = 1, I_QC = 4, I_NCUT = 8, I_ROUNDS = 9, I_RELAXED = 10, I_BAR = 32, I_WORDS = 64 };
 
 struct IncArgs {
@@ -155,7 +154,7 @@ __global__ void __launch_bounds__(kIncThreads) k_inc_persistent(IncArgs a) {
         }
         warp_push(push, v, a.cut, 0, ctl + I_CUTC);
     }
-    if (!grid_barrier(bar, err, kIncSpins, round)) return;
+    if (!grid_barrier(bar, err, round)) return;
     // 2b. the cut spreads down the dependence tree, level by level, behind itself in one list
     int64_t lo = 0, hi = (int64_t)__ldcg(ctl + I_CUTC);
     for (int k = 0; hi > lo; ++k) {
@@ -178,14 +177,14 @@ __global__ void __launch_bounds__(kIncThreads) k_inc_persistent(IncArgs a) {
                 warp_push(push, y, a.cut, hi, nc);
             }
         }
-        if (!grid_barrier(bar, err, kIncSpins, round)) return;
+        if (!grid_barrier(bar, err, round)) return;
         lo = hi;
         hi += (int64_t)__ldcg(nc);
     }
     const int64_t n_cut = hi;
     // 3. the cut vertices restart from their best valid in-neighbour (cut words are skipped by flag)
     for (int64_t i = tid; i < n_cut; i += nthr) a.st[__ldcg(&a.cut[i])] = kNone;
-    if (!grid_barrier(bar, err, kIncSpins, round)) return;
+    if (!grid_barrier(bar, err, round)) return;
     for (int64_t i = warp; i < n_cut; i += nwarps) {
         const int32_t x = __ldcg(&a.cut[i]);
         const int64_t b = a.bw.beg[x], e = b + a.bw.deg[x];
@@ -201,7 +200,7 @@ __global__ void __launch_bounds__(kIncThreads) k_inc_persistent(IncArgs a) {
         best = warp_min_u64(best);
         if (ln == 0) a.st[x] = best;
     }
-    if (!grid_barrier(bar, err, kIncSpins, round)) return;
+    if (!grid_barrier(bar, err, round)) return;
     // 4a. the re-seeded cut vertices start the first frontier (round 0 counts in ring slot 0)
     for (int64_t base = warp * 32; base < n_cut; base += nwarps * 32) {
         const int64_t i = base + ln;
@@ -214,7 +213,7 @@ __global__ void __launch_bounds__(kIncThreads) k_inc_persistent(IncArgs a) {
         }
         warp_push(push, x, a.q[0], 0, ctl + I_QC);
     }
-    if (!grid_barrier(bar, err, kIncSpins, round)) return;
+    if (!grid_barrier(bar, err, round)) return;
     // 4b. logged edges present now relax once
     for (int64_t base = warp * 32; base < a.np; base += nwarps * 32) {
         const int64_t i = base + ln;
@@ -232,7 +231,7 @@ __global__ void __launch_bounds__(kIncThreads) k_inc_persistent(IncArgs a) {
         }
         warp_push(push, v, a.q[0], 0, ctl + I_QC);
     }
-    if (!grid_barrier(bar, err, kIncSpins, round)) return;
+    if (!grid_barrier(bar, err, round)) return;
     // 5. propagation rounds: the frontier's flags are cleared before any of its distances is read
     int64_t n = (int64_t)__ldcg(ctl + I_QC), r = 0, relaxed = 0;
     for (; n > 0; ++r) {
@@ -246,7 +245,7 @@ __global__ void __launch_bounds__(kIncThreads) k_inc_persistent(IncArgs a) {
         if (tid == 0) ctl[I_QC + (r + 2) % 3] = 0ull;
         relaxed += n;
         for (int64_t i = tid; i < n; i += nthr) a.flag[__ldcg(&in[i])] = FLAG_CLEAR;
-        if (!grid_barrier(bar, err, kIncSpins, round)) return;
+        if (!grid_barrier(bar, err, round)) return;
         for (int64_t i = warp; i < n; i += nwarps) {
             const int32_t x = __ldcg(&in[i]);
             const int64_t b = a.fw.beg[x], e = b + a.fw.deg[x];
@@ -263,7 +262,7 @@ __global__ void __launch_bounds__(kIncThreads) k_inc_persistent(IncArgs a) {
                 warp_push(push, y, out, 0, nc);
             }
         }
-        if (!grid_barrier(bar, err, kIncSpins, round)) return;
+        if (!grid_barrier(bar, err, round)) return;
         n = (int64_t)__ldcg(nc);
     }
     if (tid == 0) {

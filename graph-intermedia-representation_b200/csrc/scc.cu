@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_dag_levels(const uint64_t* 
         c = warp_sum_u64(c);
         if (lane_id() == 0 && c) atomicAdd(&ctl[round % 3], c);
         if (!kLoop) break;
-        if (!grid_barrier(bar, ctl + 3, kLoopSpins, met)) return;
+        if (!grid_barrier(bar, ctl + 3, met)) return;
         raised = __ldcg(ctl + round % 3);
         ++round;
         if (raised == 0) break;

@@ -725,7 +725,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_bucket_loop(Group a, int64_
             queue_write(st.set, st.n_set, a.setq, HeavyLen{a.rows}, (s_base[1] >> kQShift) + s_n[1][wib],
                         (s_base[1] & kQEdges) + s_e[1][wib]);
         for (int i = ln; i < st.n_far; i += 32) a.farq[fq][s_base[2] + s_n[2][wib] + i] = st.far[i];
-        if (!grid_barrier(bar, a.ctl + X_ERR, kLoopSpins, met)) return;
+        if (!grid_barrier(bar, a.ctl + X_ERR, met)) return;
         next_phase(b, a.delta, entries, rd);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
