@@ -131,6 +131,15 @@ struct DistT<uint16_t> {
             old = prev;
         }
     }
+    // Both halves of an aligned word at once (0xffff: leave it).
+    __device__ static void atomic_min_pair(unsigned int* wp, unsigned int v) {
+        unsigned int old = *(volatile unsigned int*)wp;
+        for (unsigned int nw; (nw = __vminu2(old, v)) != old;) {
+            const unsigned int prev = atomicCAS(wp, old, nw);
+            if (prev == old) return;
+            old = prev;
+        }
+    }
 };
 
 // Sixteen bytes of a distance row: kVec neighbouring lanes. Rows are padded to a multiple of it (`ld`;
@@ -332,9 +341,9 @@ __device__ __forceinline__ void relax_edges(const Group& a, uint64_t kend, int32
     const A kend_a = kend < (uint64_t)(A)~(A)0 ? (A)kend : (A)~(A)0;
     const int ln = lane_id();
     unsigned long long near = 0, far = 0;
-    // takes one lane of a target from its tentative distance: 0 no gain, 1 near, 2 far
-    auto take = [&](D* at, A du, A dw, uint32_t weight) -> int {
-        const A nd = du + weight;
+    // judges one lane of a target by its tentative distance: 0 no gain, 1 near, 2 far
+    auto judge = [&](A du, A dw, uint32_t weight, A& nd) -> int {
+        nd = du + weight;
         // (the weight by itself first: the sum of 32 bits could wrap)
         if (sizeof(D) == 2 && (weight >= (A)DistT<D>::inf || nd >= (A)DistT<D>::inf)) {
             // a 16-bit lane cannot hold it: the group is run again with wider lanes
@@ -342,8 +351,14 @@ __device__ __forceinline__ void relax_edges(const Group& a, uint64_t kend, int32
             return 0;
         }
         if (nd >= dw) return 0;  // (most relaxations lose)
-        DistT<D>::atomic_min(at, (D)nd);
         return !kHeavy && nd < kend_a ? 1 : 2;
+    };
+    // and takes it
+    auto take = [&](D* at, A du, A dw, uint32_t weight) -> int {
+        A nd;
+        const int t = judge(du, dw, weight, nd);
+        if (t) DistT<D>::atomic_min(at, (D)nd);
+        return t;
     };
     const int lanes_max = __reduce_max_sync(0xffffffffu, __popcll(need)), live = __popc(any);
     if (a.ld == 1 || kThreadShare * lanes_max <= live) {
@@ -387,6 +402,24 @@ __device__ __forceinline__ void relax_edges(const Group& a, uint64_t kend, int32
                 if (!m) continue;
                 const Vec<D> du = load_vec<kCg>(du_row + at), dw = load_vec<true>(dw_row + at);
                 unsigned mn = 0, mf = 0;
+                if constexpr (sizeof(D) == 2) {
+                    // (two lanes share a word, and a swap of one had the other's fail: a swap for both)
+#pragma unroll
+                    for (int e = 0; e < kV; e += 2) {
+                        unsigned pair = 0xffffffffu;
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            A nd = 0;
+                            const int t = (m >> (e + h)) & 1u ? judge(du.v[e + h], dw.v[e + h], weight, nd) : 0;
+                            if (t) pair = h ? (pair & 0xffffu) | (nd << 16) : (pair & 0xffff0000u) | nd;
+                            mn |= (unsigned)(t & 1) << (e + h);
+                            mf |= (unsigned)(t >> 1) << (e + h);
+                        }
+                        if (pair != 0xffffffffu)
+                            DistT<uint16_t>::atomic_min_pair(reinterpret_cast<unsigned int*>(dw_row + at + e), pair);
+                    }
+                }
+                else
 #pragma unroll
                 for (int e = 0; e < kV; ++e) {
                     if ((m >> e) & 1u) {
