@@ -142,18 +142,24 @@ struct DistT<uint16_t> {
     }
 };
 
-// Sixteen bytes of a distance row: kVec neighbouring lanes. Rows are padded to a multiple of it (`ld`;
-// a single lane is not), so they can be read this way.
+// Sixteen bytes of a distance row: n neighbouring lanes. Rows are padded to a multiple of it (`ld`;
+// a single lane is not), so they can be read this way. Eight bytes of 16-bit lanes: with sixteen, 17 lanes kept
+// three of the eight threads of a row group at work (4.6 ms a call on a 1M-vertex R-MAT, 3.4 so).
 template <class D>
-struct alignas(16) Vec {
-    static constexpr int n = 16 / sizeof(D);
+struct alignas(sizeof(D) == 2 ? 8 : 16) Vec {
+    static constexpr int n = sizeof(D) == 2 ? 4 : 16 / sizeof(D);
     D v[n];
 };
 // Past the L1 (kCg) or through it.
 template <bool kCg, class D>
 __device__ __forceinline__ Vec<D> load_vec(const D* p) {
-    const uint4 r = kCg ? __ldcg(reinterpret_cast<const uint4*>(p)) : *reinterpret_cast<const uint4*>(p);
-    return *reinterpret_cast<const Vec<D>*>(&r);
+    if constexpr (sizeof(D) == 2) {
+        const uint2 r = kCg ? __ldcg(reinterpret_cast<const uint2*>(p)) : *reinterpret_cast<const uint2*>(p);
+        return *reinterpret_cast<const Vec<D>*>(&r);
+    } else {
+        const uint4 r = kCg ? __ldcg(reinterpret_cast<const uint4*>(p)) : *reinterpret_cast<const uint4*>(p);
+        return *reinterpret_cast<const Vec<D>*>(&r);
+    }
 }
 
 // OR over the eight threads of a row group.
@@ -320,7 +326,7 @@ __device__ __forceinline__ D load_dist(const D* p) {
 // Relaxes one edge per thread, u -> w of weight wt, in the lanes `need` (0: no edge), and queues what
 // improved. A warp takes the cheaper of two ways, by the work in front of it:
 //  - every thread steps through the lanes of its own edge (few lanes an edge);
-//  - eight threads take an edge, so four edges at once, each thread 16 bytes of the two distance rows at
+//  - eight threads take an edge, so four edges at once, each thread a Vec of the two distance rows at
 //    a time (many lanes an edge: the passes of a power-law graph, whose vertices are reached in most
 //    lanes at once). The rows come from L2 and HBM; two such steps in flight (64 registers) measured as one
 //    (40, and more warps).
@@ -601,7 +607,7 @@ __device__ __forceinline__ void phase_split(const Group& a, const Bucket& b, int
             // (lanes already final were reached by a shorter path since: dropped unread)
             m = __ldcg(a.farmask + w) & ~__ldcg(a.done + w);
         }
-        // Eight threads take an entry, so four at once, 16 bytes of its distance row per thread.
+        // Eight threads take an entry, so four at once, a Vec of its distance row per thread.
         unsigned long long my_near = 0, my_keep = 0;
         constexpr int kV = Vec<D>::n;
         const int sub = ln >> 3, k = ln & 7;
