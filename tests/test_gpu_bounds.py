@@ -191,3 +191,63 @@ def test_large_levels_without_cooperative_launches(pkg):
         d.close()
     for x, y in zip(*got):
         np.testing.assert_array_equal(x, y)
+
+
+def _batch_weights(pkg, V, n, step, rng, fb, fa):
+    """Ops of a batch: a hub's row, present edges, both directions of pairs, repeated keys."""
+    a, b = rng.integers(0, V, n), rng.integers(0, V, n)
+    a[: n // 4] = rng.integers(0, 1 + V // 20)  # one hub
+    rows, at = np.repeat(np.arange(V), np.diff(fb)), rng.integers(0, max(len(fa), 1), n)
+    if len(fa):
+        a[::3], b[::3] = rows[at[::3]], fa[at[::3]]
+    k = np.arange(n) % 5 == 1
+    a[k], b[k] = np.roll(b, 1)[k], np.roll(a, 1)[k]
+    ins = (rng.random(n) < (0.5, 0.0, 1.0, 0.3)[step]).astype(np.uint8)
+    return a.astype(np.int32), b.astype(np.int32), ins
+
+
+@pytest.mark.parametrize("rule", ["hash", "uniform"])
+@pytest.mark.parametrize("V,n", [(40, 2), (40, 33), (40, 600), (300, 4096), (300, 20_000)])
+def test_stored_weights_through_batches(pkg, orc, V, n, rule):
+    """Every edge's stored weight after batches of many ops: survivors keep theirs (in rows with inserts and
+    deletions, in rows that outgrow their slack and the layout that follows), inserted edges, among them those
+    deleted a batch before, get the rule's. No path of two edges is shorter than one (uniform rule) or the
+    oracle's distances say what is (hash rule), so the distances from every vertex hold every weight."""
+    rng = np.random.default_rng(V + n)
+    lo = 1 << 20
+    hi = lo + (1 << 19)
+    u, v = rng.integers(0, V, 4 * V), rng.integers(0, V, 4 * V)
+    u, v = np.r_[u, v[::3], 0], np.r_[v, u[::3], 1]
+    keep = u != v
+    w = rng.permutation(len(u)).astype(np.uint32) + (lo if rule == "uniform" else 1)
+    g = _weighted(pkg, V, u[keep], v[keep], w[keep])
+    fb, fa = orc.normalize(V, g.fw_beg, g.fw_adj)
+    weight = {(int(x), int(y)): int(z) for x, y, z in zip(np.repeat(np.arange(V), np.diff(fb)), fa, g.w)}
+    d = pkg.DeviceGraph.from_graph(g)
+    if rule == "uniform":
+        d.set_weight_rule(7, lo, hi)
+    d.build()
+    grown = False
+    for step in (0, 2, 1, 2, 3):
+        a, b, ins = _batch_weights(pkg, V, n, step, rng, fb, fa)
+        d.apply_batch(a, b, ins)
+        fb, fa, _, _ = orc.apply_batch(V, fb, fa, a, b, ins)
+        rows = np.repeat(np.arange(V), np.diff(fb))
+        gb, ga = d.csr(0)
+        np.testing.assert_array_equal(gb, fb)
+        np.testing.assert_array_equal(ga, fa)
+        if rule == "uniform":
+            new = pkg.graphs.uniform_weights(pkg.graphs.Graph(V, fb.astype(np.int32), fa, None, None), lo, hi, 7)
+        else:
+            new = [orc.edge_weight(int(x), int(y)) for x, y in zip(rows, fa)]
+        weight = {(int(x), int(y)): weight.get((int(x), int(y)), int(z)) for x, y, z in zip(rows, fa, new)}
+        now = np.array([weight[int(x), int(y)] for x, y in zip(rows, fa)], np.uint32)
+        src = np.arange(V, dtype=np.int32)
+        got = d.sssp(src, delta=1 << 21 if rule == "uniform" else 64, weights=pkg.native.WEIGHT_STORED)
+        if rule == "uniform":
+            np.testing.assert_array_equal(got[rows, fa], now)
+        for s in range(0, V, 1 if rule == "hash" else 37):
+            np.testing.assert_array_equal(got[s], orc.sssp(V, fb, fa, [s], w=now))
+        grown |= int(np.diff(fb).max()) > 2 * int(np.diff(g.fw_beg).max())
+    assert grown or n < 600  # (a row outgrew its slack: a new layout)
+    d.close()
