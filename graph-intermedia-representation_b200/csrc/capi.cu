@@ -640,7 +640,6 @@ int apply_batch_impl(gir_dev* g, const int32_t* u, const int32_t* v, const uint8
     GIR_TRY(invalidate_after_update(g));
     GIR_CUDA(g, cudaMemcpyAsync(hc, cnt, F_WORDS * sizeof(unsigned long long), cudaMemcpyDeviceToHost, g->stream));
     GIR_CUDA(g, cudaStreamSynchronize(g->stream));
-    if (hc[F_BAD]) return store_ops_bad(g);
     unsigned long long fl[F_N];
     std::memcpy(fl, hc, sizeof(fl));
     g->b_ms[0] = now_ms() - t_start;

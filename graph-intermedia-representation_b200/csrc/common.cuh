@@ -290,11 +290,10 @@ int store_free(gir_dev* g, DevCSR& c);
 int store_build_sym(gir_dev* g);
 int store_compact_csr(gir_dev* g, const DevCSR& c, int64_t* beg_out, int32_t* adj_out, int64_t cap);
 int store_has_edges(gir_dev* g, const DevCSR& c, const int32_t* u, const int32_t* v, int64_t n, uint8_t* out);
-// `bad`: a device word, zero at the start of a batch; ops that do not fit the CSR set it, change nothing and
-// give GIR_ERR_MALFORMED, as store_ops_bad does. `overflow`: a device word, zero before and after.
+// `bad`: a device word, zero at the start of a batch; ops that do not fit the CSR (an insert that it holds, a
+// deletion that it lacks) set it, change nothing and give GIR_ERR_MALFORMED. `overflow`: a device word, zero before and after.
 int store_apply_ops(gir_dev* g, DevCSR& c, const uint64_t* ins, int64_t n_ins, const uint64_t* del, int64_t n_del,
                     bool weights, int32_t* bad, int32_t* overflow);
-int store_ops_bad(gir_dev* g);
 int store_build_bins(gir_dev* g);
 // One change u -> v applied in place to the fw / bw / sym rows when they have room (store.cu):
 // out[0] 0 no-op, 1 applied, 2 no room (nothing changed); out[1] 1 / 2 when the undirected pair
@@ -444,8 +443,8 @@ __device__ __forceinline__ int64_t walk_run(int64_t total, int64_t nwarps) {
 }
 
 // Calls f(k, j) for every entry of n segments laid end to end, entry j of segment k, where off is the
-// exclusive scan of their lengths (n + 1 entries); whole warps call it. Every warp takes runs of 512
-// consecutive entries: one 32-ary search finds a run's first segment, then 32 segments at a time sit
+// exclusive scan of their lengths (n + 1 entries); whole warps call it. Every warp takes runs of at most 512
+// consecutive entries (walk_run): one 32-ary search finds a run's first segment, then 32 segments at a time sit
 // one per lane and an entry finds its own by shuffles. A binary search of the offsets per entry had
 // made the update merges' and the compact copies' kernels 3 - 6 times slower.
 template <class T, class F>

@@ -89,11 +89,6 @@ __global__ void k_ws_split(int64_t E, const K* keys, const uint32_t* cols, int w
     }
 }
 
-__global__ void k_deg_i64(int64_t V, const int32_t* deg, int64_t* out) {
-    GRID_STRIDE(v, V) out[v] = deg[v];
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[V] = 0;
-}
-
 // Distances inside a lane group are uint32 when every finite distance fits ((V - 1) * max weight
 // < 2^32 - 1): half the bytes, eight lanes per 32-byte sector, 32-bit atomics. Output is uint64.
 template <class D>
@@ -910,9 +905,7 @@ static int build_weight_sorted(gir_dev* g, int hash, int reverse, DevCSR& ws) {
     GIR_TRY(dev_alloc_n(g, &ws.w, E > 0 ? E : 1));
     ws.cap = ws.E = E;
     int64_t* cb = ws.beg;
-    k_deg_i64<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, c.deg, cb);
-    GIR_LAUNCH(g, "k_deg_i64");
-    GIR_TRY(exclusive_scan_i64(g, cb, cb, V + 1));
+    GIR_TRY(scan_degrees(g, c.deg, V, cb));
     GIR_CUDA(g, cudaMemcpyAsync(ws.deg, c.deg, sizeof(int32_t) * V, cudaMemcpyDeviceToDevice, g->stream));
     if (E == 0) return GIR_OK;
     uint32_t *cols = nullptr, *ctmp = nullptr;

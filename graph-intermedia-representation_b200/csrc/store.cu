@@ -65,12 +65,6 @@ __global__ void k_scatter_keys(const uint64_t* keys, const uint32_t* kw, int64_t
     }
 }
 
-// Compact offsets: cb[v] = sum of deg[0..v).
-__global__ void k_deg_to_i64(int64_t V, const int32_t* deg, int64_t* out) {
-    GRID_STRIDE(v, V) out[v] = deg[v];
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[V] = 0;
-}
-
 __global__ void k_sym_keys(int64_t V, const int64_t* cb, CSRView c, uint64_t* keys, uint8_t* keep) {
     walk_segments(cb, V, [&](int64_t u, int64_t j) {
         const int64_t i = cb[u] + j;
@@ -433,12 +427,6 @@ int store_build_csr_from_keys(gir_dev* g, DevCSR& c, const uint64_t* keys, int64
     return GIR_OK;
 }
 
-static int compact_offsets(gir_dev* g, const DevCSR& c, int64_t* cb) {
-    k_deg_to_i64<<<grid_for(g, g->V, kBlock), kBlock, 0, g->stream>>>(g->V, c.deg, cb);
-    GIR_LAUNCH(g, "k_deg_to_i64");
-    return exclusive_scan_i64(g, cb, cb, g->V + 1);
-}
-
 int store_build_sym(gir_dev* g) {
     // Symmetrized view (buildWCC, gir.cpp:599-625): {u,v} for every u -> v with u != v, both
     // directions, sorted and distinct.
@@ -450,7 +438,7 @@ int store_build_sym(gir_dev* g) {
     GIR_TRY(ensure_n(g, g->scratch[1], 2 * E + 1, &keys));
     GIR_TRY(ensure_n(g, g->scratch[2], 2 * E + 1, &tmp));
     GIR_TRY(ensure_n(g, g->scratch[3], 2 * E + 1, &keep));
-    GIR_TRY(compact_offsets(g, g->fw, cb));
+    GIR_TRY(scan_degrees(g, g->fw.deg, V, cb));
     if (E > 0) {
         k_sym_keys<<<grid_for(g, E, kBlock), kBlock, 0, g->stream>>>(V, cb, view(g->fw), keys, keep);
         GIR_LAUNCH(g, "k_sym_keys");
@@ -470,7 +458,7 @@ int store_build_sym(gir_dev* g) {
 
 int store_compact_csr(gir_dev* g, const DevCSR& c, int64_t* beg_out, int32_t* adj_out, int64_t cap) {
     // beg_out / adj_out: device pointers (V+1 / cap entries)
-    GIR_TRY(compact_offsets(g, c, beg_out));
+    GIR_TRY(scan_degrees(g, c.deg, g->V, beg_out));
     if (c.E > 0 && adj_out && cap > 0) {
         k_compact_copy<<<grid_for(g, c.E, kBlock), kBlock, 0, g->stream>>>(g->V, beg_out, view(c), adj_out, cap);
         GIR_LAUNCH(g, "k_compact_copy");
@@ -483,10 +471,6 @@ int store_has_edges(gir_dev* g, const DevCSR& c, const int32_t* u, const int32_t
     k_has_edges<<<grid_for(g, n, kBlock), kBlock, 0, g->stream>>>(view(c), g->V, u, v, n, out);
     GIR_LAUNCH(g, "k_has_edges");
     return GIR_OK;
-}
-
-int store_ops_bad(gir_dev* g) {
-    return fail(g, GIR_ERR_MALFORMED, "edge update: the backward CSR is not the transpose of the forward CSR");
 }
 
 int store_apply_ops(gir_dev* g, DevCSR& c, const uint64_t* ins, int64_t n_ins, const uint64_t* del, int64_t n_del,
@@ -513,7 +497,7 @@ int store_apply_ops(gir_dev* g, DevCSR& c, const uint64_t* ins, int64_t n_ins, c
     GIR_CUDA(g, cudaStreamSynchronize(g->stream));
     const int64_t n_moved = h[0];
     const bool ovf = h[1] != 0;
-    if (h[2]) return store_ops_bad(g);
+    if (h[2]) return fail(g, GIR_ERR_MALFORMED, "edge update: the backward CSR is not the transpose of the forward CSR");
     const bool wts = weights && c.w;
     GIR_TRY(ensure_n(g, g->stage_out, n_moved + 4, &tmp));
     if (wts) GIR_TRY(ensure_n(g, g->scratch[3], n_moved + 4, &tmpw));
