@@ -527,6 +527,33 @@ __device__ __forceinline__ void walk_rows_of(const int64_t* off, int64_t V, cons
     }
 }
 
+// Rows of more than kLongRow entries that a pass over all rows, a warp each, sets aside for the whole grid.
+// Calls f(item, k, on) for the entries k >= from of the rows of n listed items (len(item): the row's length), every
+// lane of a warp together (on: the lane has an entry); block-uniform call by CTAs of at most 256 threads. Chunks
+// of 1,024 entries are dealt to the CTAs in turn, and a CTA looks at 256 items at a time.
+constexpr int32_t kLongRow = 4096;
+template <class Len, class F>
+__device__ __forceinline__ void walk_long_rows(const int32_t* items, int64_t n, int32_t from, Len&& len, F&& f) {
+    constexpr int kChunk = 1024;
+    __shared__ int32_t s_item[256], s_len[256];
+    const int64_t grid = gridDim.x;
+    for (int64_t i0 = 0; i0 < n; i0 += blockDim.x) {
+        __syncthreads();
+        if (i0 + threadIdx.x < n) {
+            s_item[threadIdx.x] = items[i0 + threadIdx.x];
+            s_len[threadIdx.x] = len(s_item[threadIdx.x]);
+        }
+        __syncthreads();
+        const int here = n - i0 < (int64_t)blockDim.x ? (int)(n - i0) : (int)blockDim.x;
+        for (int j = 0; j < here; ++j) {
+            const int64_t d = s_len[j];
+            for (int64_t c = (blockIdx.x + grid - (i0 + j) % grid) % grid; from + c * kChunk < d; c += grid)
+                for (int64_t k = from + c * kChunk + threadIdx.x; k - (k & 31) < from + (c + 1) * kChunk; k += blockDim.x)
+                    f(s_item[j], (int32_t)k, k < d);
+        }
+    }
+}
+
 // Grid-wide barrier of a cooperative launch: every CTA meets here. `bar` is one counter on its own
 // 128-byte line, zeroed by the host before the launch; arrivals only count up, so a CTA waits until the
 // counter reaches the end of its round (`round`: the barriers passed so far, the same in every CTA). One

@@ -84,9 +84,11 @@ __global__ void k_uf_hook_first_two(CSRView c, int64_t V, int32_t* parent, const
 }
 
 // Rows of the vertices outside the sampled giant root: a warp takes 32 vertices, scans their row lengths and
-// walks the rows laid end to end, 32 entries at a time.
+// walks the rows laid end to end, 32 entries at a time. Long rows go to `list` (k_uf_link_long): one warp for a
+// hub of 1.5M entries outside the giant took 39 ms.
 __global__ void __launch_bounds__(kBlock) k_uf_link_rest(CSRView c, int64_t V, const int32_t* giant_p,
-                                                         int32_t* parent, unsigned long long* err) {
+                                                         int32_t* parent, unsigned long long* err, int32_t* list,
+                                                         unsigned int* n_list) {
     const int32_t giant = *giant_p;
     __shared__ int64_t s_excl[kBlock / 32][33];
     __shared__ int32_t s_u[kBlock / 32][32];
@@ -97,6 +99,10 @@ __global__ void __launch_bounds__(kBlock) k_uf_link_rest(CSRView c, int64_t V, c
         const int64_t v = base + lane;
         int64_t cnt = 0;
         if (v < V && parent[v] != giant) cnt = c.deg[v];
+        if (cnt > kLongRow) {
+            list[atomicAdd(n_list, 1u)] = (int32_t)v;
+            cnt = 0;
+        }
         int64_t incl = cnt;
         for (int o = 1; o < 32; o <<= 1) {
             const int64_t t = __shfl_up_sync(0xffffffffu, incl, o);
@@ -123,17 +129,27 @@ __global__ void __launch_bounds__(kBlock) k_uf_link_rest(CSRView c, int64_t V, c
     }
 }
 
+__global__ void __launch_bounds__(kBlock) k_uf_link_long(CSRView c, const int32_t* list, const unsigned int* n_list,
+                                                         int32_t* parent, unsigned long long* err) {
+    walk_long_rows(list, (int64_t)*n_list, 0, [&](int32_t v) { return c.deg[v]; }, [&](int32_t v, int32_t k, bool on) {
+        if (on) uf_union(parent, v, c.adj[c.beg[v] + k], err);
+    });
+}
+
 }  // namespace
 
 // Components of the symmetric view by the sampled union-find above; labels = smallest vertex id.
 static int wcc_labels_sym(gir_dev* g, int32_t* label, int64_t* n_comp) {
     const int64_t V = g->V;
     unsigned long long *roots = nullptr, *err = nullptr;
-    GIR_TRY(ensure_n(g, g->scratch[14], 5, &roots));
+    GIR_TRY(ensure_n(g, g->scratch[14], 6, &roots));
+    int32_t* list = nullptr;
+    GIR_TRY(ensure_n(g, g->scratch[13], g->sym.E / kLongRow + 1, &list));
+    unsigned int* n_list = reinterpret_cast<unsigned int*>(roots + 5);
     err = roots + 1;
     int32_t* giant = reinterpret_cast<int32_t*>(roots + 2);
     int32_t* hooked = giant + 1;  // a word per round
-    GIR_CUDA(g, cudaMemsetAsync(roots, 0, 5 * sizeof(unsigned long long), g->stream));
+    GIR_CUDA(g, cudaMemsetAsync(roots, 0, 6 * sizeof(unsigned long long), g->stream));
     if (V == 0) { *n_comp = 0; return GIR_OK; }
     const CSRView s = view(g->sym);
     k_uf_first<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(s, V, label);
@@ -153,8 +169,10 @@ static int wcc_labels_sym(gir_dev* g, int32_t* label, int64_t* n_comp) {
     }
     GIR_TRY(sample_mode(g, g->sym, label, 1, giant));
     trace_mark(g, "wcc: neighbour rounds + sample");
-    k_uf_link_rest<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(s, V, giant, label, err);
+    k_uf_link_rest<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(s, V, giant, label, err, list, n_list);
     GIR_LAUNCH(g, "k_uf_link_rest");
+    k_uf_link_long<<<g->num_sms * 8, kBlock, 0, g->stream>>>(s, list, n_list, label, err);
+    GIR_LAUNCH(g, "k_uf_link_long");
     k_uf_compress<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(label, V, roots);
     GIR_LAUNCH(g, "k_uf_compress");
     unsigned long long h[2] = {0, 0};

@@ -195,3 +195,37 @@ def test_components_at_every_row_length(pkg, orc, V, entries):
         np.testing.assert_array_equal(d.labels(pkg.native.LABEL_WCC), exp)
         assert d.counts()["n_wcc"] == len(np.unique(exp))
         d.close()
+
+
+def _beside_a_core(pkg, core, deg, pages, flip, hubs=1):
+    """A dense core, and beside it pages in rings of three that all link to a hub (one after another where there are
+    several), which links back to one: with `flip`, all edges the other way."""
+    rng = np.random.default_rng(core + deg)
+    u, v = rng.integers(0, core, (2, core * deg))
+    first = core + hubs
+    p = np.arange(first, first + pages // 3 * 3)
+    ring = p + np.where((p - first) % 3 == 2, -2, 1)
+    hub = core + (p - first) // 3 % hubs
+    e = [np.r_[u, p, p, core + np.arange(hubs)], np.r_[v, ring, hub, first + 3 * np.arange(hubs)]]
+    keep = e[0] != e[1]
+    e = [x[keep] for x in e]
+    return first + len(p), e[flip], e[1 - flip]
+
+
+def test_components_of_a_hub_beside_the_largest(pkg):
+    """The hub's rows are outside the component that holds most row entries."""
+    V, u, v = _beside_a_core(pkg, 8000, 1200, 600_000, 0)
+    hub, spread = (_build_ms(pkg, _graph(pkg, *a), pkg.native.LAYER_WCC)
+                   for a in ((V, u, v), _beside_a_core(pkg, 8000, 1200, 600_000, 0, hubs=3000)))
+    assert hub < 4 * spread + 1, (hub, spread)
+
+
+@pytest.mark.parametrize("hubs,pages", [(1, 4000), (1, 4090), (1, 4100), (1, 5121), (2, 12_000), (3, 60_000), (300, 1_500_000)])
+def test_components_with_rows_about_the_long_one(pkg, orc, hubs, pages):
+    V, u, v = _beside_a_core(pkg, 3000, 600 if pages < 100_000 else 2500, pages, 0, hubs)
+    g = _graph(pkg, V, u, v)
+    fb, fa = orc.normalize(V, g.fw_beg, g.fw_adj)
+    d = pkg.DeviceGraph.from_graph(g, weights=False)
+    d.build(pkg.native.LAYER_WCC)
+    np.testing.assert_array_equal(d.labels(pkg.native.LABEL_WCC), orc.canon_labels(orc.wcc(V, fb, fa)))
+    d.close()
