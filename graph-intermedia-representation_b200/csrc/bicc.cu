@@ -101,7 +101,7 @@ struct ForestLevel {
 // The same level bottom-up: every vertex without a parent takes the first entry of its row that is in
 // the frontier (bits) and in its SCC.
 __global__ void __launch_bounds__(kBlock) k_forest_up(int64_t V, CSRView sym, const int32_t* scc, const uint32_t* bits,
-                                                      int32_t* parent, Queue out, unsigned long long* cnt) {
+                                                      int32_t* parent, Queue out, unsigned long long* cnt, LongRows rest) {
     __shared__ int32_t s_st[kBlock / 32][kStage];
     int n_st = 0;
     auto deg = [&](int32_t x) { return sym.deg[x]; };
@@ -112,8 +112,26 @@ __global__ void __launch_bounds__(kBlock) k_forest_up(int64_t V, CSRView sym, co
         const int32_t p = first_hit(sym.adj, want ? sym.beg[v] : 0, want ? sym.deg[v] : 0, want, mine,
                                     [&](int32_t w, int32_t c) { return ((bits[w >> 5] >> (w & 31)) & 1u) && scc[w] == c; });
         if (p >= 0) parent[v] = p;
+        if (want && p < 0 && sym.deg[v] > kLongRow) rest.add((int32_t)v);
         queue_push(p >= 0, (int32_t)v, s_st[threadIdx.x >> 5], n_st, out, deg, cnt);
     }
+    queue_flush(s_st[threadIdx.x >> 5], n_st, out, deg, cnt);
+}
+
+__global__ void __launch_bounds__(kBlock) k_forest_up_long(CSRView sym, const int32_t* scc, const uint32_t* bits,
+                                                           int32_t* parent, Queue out, unsigned long long* cnt,
+                                                           LongRows rest) {
+    __shared__ int32_t s_st[kBlock / 32][kStage];
+    int n_st = 0;
+    auto deg = [&](int32_t x) { return sym.deg[x]; };
+    walk_long_rows(rest.item, (int64_t)*rest.n, kLongRow, deg, [&](int32_t v, int32_t k, bool on) {
+        bool join = false;
+        if (on && __ldcg(parent + v) == -1) {
+            const int32_t w = sym.adj[sym.beg[v] + k];
+            if (((bits[w >> 5] >> (w & 31)) & 1u) && scc[w] == scc[v]) join = atomicCAS(&parent[v], -1, w) == -1;
+        }
+        queue_push(join, v, s_st[threadIdx.x >> 5], n_st, out, deg, cnt);
+    });
     queue_flush(s_st[threadIdx.x >> 5], n_st, out, deg, cnt);
 }
 
@@ -124,15 +142,18 @@ struct ForestUp {
     CSRView sym;
     const int32_t* scc;
     int32_t* parent;
-    uint32_t* bits;
+    uint32_t* bits;  // the bitmap, the number of long rows, room for them
     int64_t V;
     bool wants(int64_t total, int64_t queued) const { return total > 4 * (V - queued); }
     int launch(gir_dev* g, const Queue& in, int64_t nq, const Queue& out, unsigned long long* cnt) const {
-        GIR_CUDA(g, cudaMemsetAsync(bits, 0, sizeof(uint32_t) * (V / 32 + 1), g->stream));
+        const LongRows rest{reinterpret_cast<int32_t*>(bits + V / 32 + 2), bits + V / 32 + 1};
+        GIR_CUDA(g, cudaMemsetAsync(bits, 0, sizeof(uint32_t) * (V / 32 + 2), g->stream));
         k_frontier_bits<<<grid_for(g, nq, kBlock), kBlock, 0, g->stream>>>(in.v, nq, bits, bits);
         GIR_LAUNCH(g, "k_frontier_bits");
-        k_forest_up<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, sym, scc, bits, parent, out, cnt);
+        k_forest_up<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, sym, scc, bits, parent, out, cnt, rest);
         GIR_LAUNCH(g, "k_forest_up");
+        k_forest_up_long<<<g->num_sms * 4, kBlock, 0, g->stream>>>(sym, scc, bits, parent, out, cnt, rest);
+        GIR_LAUNCH(g, "k_forest_up_long");
         return GIR_OK;
     }
 };
@@ -655,7 +676,7 @@ int bct_build(gir_dev* g) {
     k_roots<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, scc, nontrivial, hdeg, parent, fq, ctl + W_Q);
     GIR_LAUNCH(g, "k_roots");
     uint32_t* bits = nullptr;
-    GIR_TRY(ensure_n(g, g->work[5], V / 32 + 2, &bits));
+    GIR_TRY(ensure_n(g, g->work[5], V / 32 + 3 + g->sym.E / kLongRow, &bits));
     FrontierRun run;
     GIR_TRY(run_frontier(g, ForestLevel{h.sym, scc, parent}, ForestUp{h.sym, scc, parent, bits, V}, fq, ctl, run, V < kEulerMaxV ? deep_levels(V) : INT64_MAX));
     const bool deep = !run.done();

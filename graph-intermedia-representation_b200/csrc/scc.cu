@@ -194,7 +194,7 @@ struct ReachBoth {
 // mark for an out-neighbour in the backward frontier.
 __global__ void __launch_bounds__(kBlock) k_reach_up(int64_t V, CSRView fw, CSRView bw, const uint32_t* fwd,
                                                      const uint32_t* bwd, int32_t* mark, Queue out,
-                                                     unsigned long long* cnt) {
+                                                     unsigned long long* cnt, LongRows rest) {
     __shared__ int32_t s_st[kBlock / 32][kStage];
     int n_st = 0;
     auto deg = [&](int32_t e) { return e >= 0 ? fw.deg[e] : bw.deg[~e]; };
@@ -207,9 +207,30 @@ __global__ void __launch_bounds__(kBlock) k_reach_up(int64_t V, CSRView fw, CSRV
         const bool b = first_hit(fw.adj, wb ? fw.beg[v] : 0, wb ? fw.deg[v] : 0, wb, 0,
                                  [&](int32_t w, int32_t) { return (bwd[w >> 5] >> (w & 31)) & 1u; }) >= 0;
         if (f || b) mark[v] = m | (f ? 1 : 0) | (b ? 2 : 0);
+        if (wf && !f && bw.deg[v] > kLongRow) rest.add((int32_t)v);
+        if (wb && !b && fw.deg[v] > kLongRow) rest.add(~(int32_t)v);
         queue_push(f, (int32_t)v, s_st[threadIdx.x >> 5], n_st, out, deg, cnt);
         queue_push(b, ~(int32_t)v, s_st[threadIdx.x >> 5], n_st, out, deg, cnt);
     }
+    queue_flush(s_st[threadIdx.x >> 5], n_st, out, deg, cnt);
+}
+
+__global__ void __launch_bounds__(kBlock) k_reach_up_long(CSRView fw, CSRView bw, const uint32_t* fwd, const uint32_t* bwd,
+                                                          int32_t* mark, Queue out, unsigned long long* cnt, LongRows rest) {
+    __shared__ int32_t s_st[kBlock / 32][kStage];
+    int n_st = 0;
+    auto deg = [&](int32_t e) { return e >= 0 ? fw.deg[e] : bw.deg[~e]; };
+    walk_long_rows(rest.item, (int64_t)*rest.n, kLongRow, [&](int32_t e) { return e >= 0 ? bw.deg[e] : fw.deg[~e]; },
+                   [&](int32_t e, int32_t k, bool on) {
+                       const int32_t v = e >= 0 ? e : ~e, bit = e >= 0 ? 1 : 2;
+                       bool hit = false;
+                       if (on && !(__ldcg(mark + v) & bit)) {
+                           const int32_t w = e >= 0 ? bw.adj[bw.beg[v] + k] : fw.adj[fw.beg[v] + k];
+                           hit = ((e >= 0 ? fwd : bwd)[w >> 5] >> (w & 31)) & 1u;
+                       }
+                       const bool join = hit && !(atomicOr(&mark[v], bit) & bit);
+                       queue_push(join, e, s_st[threadIdx.x >> 5], n_st, out, deg, cnt);
+                   });
     queue_flush(s_st[threadIdx.x >> 5], n_st, out, deg, cnt);
 }
 
@@ -218,17 +239,21 @@ __global__ void __launch_bounds__(kBlock) k_reach_up(int64_t V, CSRView fw, CSRV
 struct ReachUp {
     CSRView fw, bw;
     int32_t* mark;
-    uint32_t* bits;  // two bitmaps
+    uint32_t* bits;  // two bitmaps, the number of long rows, room for those of both CSRs
     int64_t V;
     bool aligned;
     bool wants(int64_t total, int64_t queued) const { return aligned && total > 4 * (2 * V - queued); }
+    static int64_t words(int64_t V, int64_t E) { return 2 * (V / 32 + 1) + 1 + 2 * (E / kLongRow + 1); }
     int launch(gir_dev* g, const Queue& in, int64_t nq, const Queue& out, unsigned long long* cnt) const {
         uint32_t* bwd = bits + V / 32 + 1;
-        GIR_CUDA(g, cudaMemsetAsync(bits, 0, sizeof(uint32_t) * 2 * (V / 32 + 1), g->stream));
+        const LongRows rest{reinterpret_cast<int32_t*>(bwd + V / 32 + 2), bwd + V / 32 + 1};
+        GIR_CUDA(g, cudaMemsetAsync(bits, 0, sizeof(uint32_t) * (2 * (V / 32 + 1) + 1), g->stream));
         k_frontier_bits<<<grid_for(g, nq, kBlock), kBlock, 0, g->stream>>>(in.v, nq, bits, bwd);
         GIR_LAUNCH(g, "k_frontier_bits");
-        k_reach_up<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, fw, bw, bits, bwd, mark, out, cnt);
+        k_reach_up<<<grid_for(g, V, kBlock), kBlock, 0, g->stream>>>(V, fw, bw, bits, bwd, mark, out, cnt, rest);
         GIR_LAUNCH(g, "k_reach_up");
+        k_reach_up_long<<<g->num_sms * 4, kBlock, 0, g->stream>>>(fw, bw, bits, bwd, mark, out, cnt, rest);
+        GIR_LAUNCH(g, "k_reach_up_long");
         return GIR_OK;
     }
 };
@@ -738,7 +763,7 @@ static int scc_labels(gir_dev* g, const CSRView fw, const CSRView bw, bool whole
         GIR_LAUNCH(g, "k_reach_init");
         const ReachBoth op{fw, bw, mark};
         uint32_t* bits = nullptr;
-        GIR_TRY(ensure_n(g, g->scratch[11], 2 * (V / 32 + 1), &bits));
+        if (whole) GIR_TRY(ensure_n(g, g->scratch[11], ReachUp::words(V, g->fw.E), &bits));
         const ReachUp up{fw, bw, mark, bits, V, whole};
         FrontierRun run;
         GIR_TRY(run_frontier(g, op, up, q, ctl, run, whole ? deep_levels(V) : INT64_MAX));

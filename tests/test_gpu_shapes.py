@@ -214,9 +214,9 @@ def _beside_a_core(pkg, core, deg, pages, flip, hubs=1):
 
 def test_components_of_a_hub_beside_the_largest(pkg):
     """The hub's rows are outside the component that holds most row entries."""
-    V, u, v = _beside_a_core(pkg, 8000, 1200, 600_000, 0)
+    V, u, v = _beside_a_core(pkg, 8000, 600, 600_000, 0)
     hub, spread = (_build_ms(pkg, _graph(pkg, *a), pkg.native.LAYER_WCC)
-                   for a in ((V, u, v), _beside_a_core(pkg, 8000, 1200, 600_000, 0, hubs=3000)))
+                   for a in ((V, u, v), _beside_a_core(pkg, 8000, 600, 600_000, 0, hubs=3000)))
     assert hub < 4 * spread + 1, (hub, spread)
 
 
@@ -229,3 +229,57 @@ def test_components_with_rows_about_the_long_one(pkg, orc, hubs, pages):
     d.build(pkg.native.LAYER_WCC)
     np.testing.assert_array_equal(d.labels(pkg.native.LABEL_WCC), orc.canon_labels(orc.wcc(V, fb, fa)))
     d.close()
+
+
+def test_levels_that_look_through_a_long_row_in_vain(pkg):
+    """A core of over 2^22 row entries in a level, whose search reaches a hub only some levels later; pages that no
+    edge leads to are the rest of the hub's row. One hub, or as many entries on three thousand."""
+    core, deg, pages, tail = 8000, 500, 400_000, 6
+    rng = np.random.default_rng(1)
+    u, v = rng.integers(0, core, (2, core * deg))
+    ms = []
+    for hubs in (1, 3000):
+        chain = core + np.arange(tail)
+        hub = core + tail + np.arange(hubs)
+        page = core + tail + hubs + np.arange(pages)
+        V = core + tail + hubs + pages
+        a = np.r_[u, 0, chain[:-1], np.full(hubs, chain[-1]), hub, page]
+        b = np.r_[v, chain[0], chain[1:], hub, np.zeros(hubs, np.int64), hub[np.arange(pages) % hubs]]
+        ms.append(_build_ms(pkg, _graph(pkg, V, a[a != b], b[a != b]), pkg.native.LAYER_SCC))
+    assert ms[0] < 3 * ms[1] + 1, ms
+
+
+@pytest.mark.parametrize("where", ["before the line", "at the line", "last", "none"])
+def test_bottom_up_levels_and_long_rows(pkg, orc, where):
+    """A core of over 2^22 row entries in a level, and hubs whose only neighbours in the frontier come early in a
+    long row, about where the warp leaves off, last, or not at all: SCCs, DAG and blocks against the oracle."""
+    from test_gpu_layers import _oracle_match
+    core, pages, hubs = 3000, 9000, 6
+    rng = np.random.default_rng(len(where))
+    u, v = rng.integers(0, core, (2, core * 2200))
+    V = pages + core + 2 * hubs  # pages first, so that the core's entries come last in a hub's row (or the other way)
+    at = {"before the line": 4000, "at the line": 4096, "last": pages, "none": pages}[where]
+    page = np.r_[np.arange(at), np.arange(at + core, pages + core)]  # the core's ids lie from `at` on
+    u, v = u + at, v + at
+    into, out = V - 2 * hubs + np.arange(hubs), V - hubs + np.arange(hubs)
+    parts_u, parts_v = [u], [v]
+    for k in range(hubs):
+        mine = page[rng.random(len(page)) < (1.0, 0.9)[k % 2]]
+        parts_u += [mine, np.full(len(mine), out[k])]
+        parts_v += [np.full(len(mine), into[k]), mine]
+        if where != "none":  # a core vertex at one end of the row, both ways for half of the hubs
+            c = at + rng.integers(0, core, 3)
+            parts_u += [c, np.full(3, out[k])] + ([np.full(3, into[k]), c] if k % 2 else [])
+            parts_v += [np.full(3, into[k]), c] + ([c, np.full(3, out[k])] if k % 2 else [])
+    ring = page[: len(page) // 3 * 3].reshape(-1, 3)[::5]
+    parts_u.append(ring.ravel())
+    parts_v.append(np.roll(ring, 1, 1).ravel())
+    u, v = np.concatenate(parts_u), np.concatenate(parts_v)
+    g = _graph(pkg, V, u[u != v], v[u != v])
+    fb, fa = orc.normalize(V, g.fw_beg, g.fw_adj)
+    for pivot in (-1, 1, 2):
+        d = pkg.DeviceGraph.from_graph(g, weights=False)
+        d.set_param(pkg.native.PARAM_PIVOT, pivot)
+        d.build()
+        _oracle_match(pkg, orc, d, V, fb, fa, f"{where}, pivot {pivot}")
+        d.close()
