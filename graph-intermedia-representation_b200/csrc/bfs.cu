@@ -333,7 +333,8 @@ __device__ __forceinline__ void bu_ctas(const int32_t* ids, int64_t n, const CSR
 // read with ld.cg, past the SMs' incoherent L1; every barrier wait is bounded and sets an error flag
 // when it runs out.
 // Bound by latency: a level is a chain of about eight dependent L2 accesses and the barrier, about
-// 10 us on a lattice. Before, a level was two phases (expand, commit) with a barrier of eight CTAs
+// 10 us on a lattice. (64 registers a thread, the most that 1,024 threads have: 56 bytes of stores and 144 of loads
+// spill.) Before, a level was two phases (expand, commit) with a barrier of eight CTAs
 // per SM after each and a warp took 32 frontier vertices whatever the frontier's size: 64 sources on
 // a 4.8M-vertex R-MAT 11.4 ms a call, now 5.1 ms; 37 sets on 0.78M vertices 3.0 -> 0.89 ms; 8 sources
 // on a 701 x 701 lattice 29.3 -> 10.4 ms (11.4 before the barrier's one-way arrival, the first look

@@ -653,7 +653,9 @@ __device__ __forceinline__ void phase_split(const Group& a, const Bucket& b, int
 
 // ---- A phase launched from the host ------------------------------------------------------------
 // Bound by the latency of the distance rows' accesses, so occupancy counts: six CTAs an SM (40 registers)
-// 16.1 ms a call of 64 sources on the 4.8M-vertex R-MAT, four CTAs (64 registers) 16.6. Pairs of edge and
+// 16.1 ms a call of 64 sources on the 4.8M-vertex R-MAT, four CTAs (64 registers) 16.6. At 40 registers the light
+// phase of 32-bit lanes spills 248 bytes of stores and 372 of loads a thread, the heavy one 120 and 188 (the bucket
+// loop, at 64, 128 and 256); five CTAs, about 48 registers, are not measured. Pairs of edge and
 // lane dealt one to a thread, numbered by a scan, had taken 26.4 of 35 ms: about 140 instructions a pair
 // to find it, and every pair's distance read; now final lanes are dropped by one mask per edge (8 of 10
 // edges of the heavy passes have none left) and a row of 64 lanes costs about 20 instructions.
