@@ -269,6 +269,12 @@ def run_reference(args):
     world, rank, local = dist_setup()
     if rank != 0:
         return
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import oracle
+    if not oracle.ref_available():  # (the oracle is this repository's code, not the reference's)
+        print(json.dumps({"impl": "reference", "unavailable": "the reference compiled from its sources "
+                          "(oracle/_ref/libgirref.so) is not here, and its sources are not either"}), flush=True)
+        return
     os.environ.setdefault("OMP_NUM_THREADS", str(os.cpu_count()))
     os.environ.setdefault("OMP_PROC_BIND", "close")
     pkg = importlib.import_module("graph-intermedia-representation_b200")
