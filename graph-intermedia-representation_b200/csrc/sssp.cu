@@ -111,7 +111,7 @@ struct DistT<uint32_t> {
 template <>
 struct DistT<uint16_t> {
     static constexpr uint16_t inf = 0xffffu;
-    using acc = uint32_t;  // (holds the sum of a distance and a weight below inf; see take() in relax_edges)
+    using acc = uint32_t;  // (holds the sum of a distance and a weight below inf; see judge() in relax_edges)
     __device__ static void atomic_min(uint16_t* p, uint16_t v) {
         const uintptr_t a = reinterpret_cast<uintptr_t>(p);
         unsigned int* wp = reinterpret_cast<unsigned int*>(a & ~(uintptr_t)3);

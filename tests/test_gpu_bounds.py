@@ -251,3 +251,35 @@ def test_stored_weights_through_batches(pkg, orc, V, n, rule):
         grown |= int(np.diff(fb).max()) > 2 * int(np.diff(g.fw_beg).max())
     assert grown or n < 600  # (a row outgrew its slack: a new layout)
     d.close()
+
+
+def test_handles_on_several_threads(pkg):
+    """Builds and queries of three graphs at once, a thread and a handle each: their cooperative launches share the GPU."""
+    import threading
+    graphs = [pkg.graphs.rmat(14, seed=3), pkg.graphs.lattice(side=120, seed=4), pkg.graphs.rmat(16, seed=5)]
+    handles = [pkg.DeviceGraph.from_graph(g) for g in graphs]
+
+    def results(d, g):
+        src = np.flatnonzero(np.diff(g.fw_beg))[:70].astype(np.int32)
+        d.build()
+        return [d.labels(k) for k in range(5)] + [d.bfs(src[:9]), d.sssp(src[:9]), d.sssp(src[:1])]
+
+    alone = [results(d, g) for d, g in zip(handles, graphs)]
+    wrong = []
+
+    def loop(i):
+        try:
+            for _ in range(10):
+                if not all((x == y).all() for x, y in zip(results(handles[i], graphs[i]), alone[i])):
+                    wrong.append(i)
+        except Exception as e:  # (a failure in a thread would pass unseen)
+            wrong.append((i, repr(e)))
+
+    threads = [threading.Thread(target=loop, args=(i,)) for i in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    for d in handles:
+        d.close()
